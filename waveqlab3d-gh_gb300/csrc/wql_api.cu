@@ -140,7 +140,7 @@ struct wql_scn {
     void* Q[6] = {};
     void* DQ[6] = {};
     long long slab_np[6] = {};
-    void* G = nullptr;  // velocity gradient hand-off (FP32C with PML or attenuation)
+    void* G = nullptr;  // velocity gradient hand-off (FP32C with attenuation)
     void* eta = nullptr;   // anelastic memory variables (24 x np)
     void* Deta = nullptr;  // and their rates
     void* qs = nullptr;    // 1/Qs per point
@@ -578,7 +578,6 @@ int setup_block(wql_scn* S, int b) {
       if ((rc = S->alloc(&B.Q[s], 9 * slab * S->esz))) return rc;
       if ((rc = S->alloc(&B.DQ[s], 9 * slab * S->esz))) return rc;
     }
-    if (S->prec == WQL_FP32C && !S->anel && (rc = S->alloc(&B.G, 9 * B.np * S->esz))) return rc;
   }
   // anelastic: the TMA stencil hands the velocity gradient of every point
   // to the anelastic kernel
@@ -1128,6 +1127,9 @@ VolumeArgs<T> volume_args(wql_scn* S, int b, double A, double Bdt, bool last) {
   a.mms_Tp = (T)S->mms_Tp;
   B.maps.cur = S->cur;
   a.tma = &B.maps;
+  // the PML pre-kernel goes with the TMA stencil; it addresses a component
+  // with 32-bit byte offsets
+  a.pml_pre = B.npml > 0 && stencil_is_tma(a) && B.np < (1LL << 30) ? 1 : 0;
   return a;
 }
 
@@ -1231,8 +1233,8 @@ void stage_head(wql_scn* S, StepCtx& c, int stage) {
 
 void stage_block_pre(wql_scn* S, StepCtx& c, int stage, int b) {
   mark_begin(S, 2);
-  if (S->prec == WQL_FP64) c.launches += launch_pre<double>(volume_args<double>(S, b, stage_A(S, stage), stage_Bdt(S, stage), stage == 5), S->stream);
-  else c.launches += launch_pre<float>(volume_args<float>(S, b, stage_A(S, stage), stage_Bdt(S, stage), stage == 5), S->stream);
+  if (S->prec == WQL_FP64) c.launches += launch_pre<double>(volume_args<double>(S, b, stage_A(S, stage), stage_Bdt(S, stage), stage == 5), S->curv, S->stream);
+  else c.launches += launch_pre<float>(volume_args<float>(S, b, stage_A(S, stage), stage_Bdt(S, stage), stage == 5), S->curv, S->stream);
   mark_end(S);
 }
 
@@ -1478,7 +1480,7 @@ void run_stage(wql_scn* S, StepCtx& c, int stage) {
       const VolumeArgs<float> a0 = volume_args<float>(S, 0, A, Bdt, stage == 5);
       const VolumeArgs<float> a1 = volume_args<float>(S, 1, A, Bdt, stage == 5);
       mark_begin(S, 2);
-      c.launches += launch_pre2<float>(a0, a1, S->stream);
+      c.launches += launch_pre2<float>(a0, a1, S->curv, S->stream);
       mark_end(S);
     }
     mark_begin(S, 1);
@@ -2118,14 +2120,11 @@ int wql_estimate_device_bytes(const char* in_text, const char* base_dir, int pre
       const bool pml = (s2 % 2 == 0) ? bp.pml_lqrs[s2 / 2] : bp.pml_rqrs[s2 / 2];
       if (pml && bp.npml > 0) res += 2 * al(9 * (npd / dims[s2 / 2]) * bp.npml * esz);
     }
-    bool any_pml = false;
-    for (int s2 = 0; s2 < 3; ++s2) any_pml = any_pml || bp.pml_lqrs[s2] || bp.pml_rqrs[s2];
-    if (any_pml && bp.npml > 0 && precision == WQL_FP32C) res += al(9 * np * esz);
     if (P.response == "plastic") res += al(np * esz);
     if (P.response == "plastic" && P.plastic_model != "scec") res += 2 * al(np * esz);
     if (P.response == "anelastic") {
       res += 2 * al(24 * np * esz) + al(np * esz) + al(npd * 8);
-      if (precision == WQL_FP32C && !(any_pml && bp.npml > 0)) res += al(9 * np * esz);
+      if (precision == WQL_FP32C) res += al(9 * np * esz);
     }
     // set-up arrays of one block: x, metric, J, material (FP64)
     transient = std::max(transient, al(3 * npd * 8) + al(9 * npd * 8) + al(npd * 8) + al(3 * npd * 8));

@@ -14,7 +14,7 @@
 //   face  : per side 15 x nface (FP64): n(3), m(3), l(3), grad(3) of the
 //           face-normal coordinate, lambda, mu, rho
 //   Q/DQ  : PML auxiliary fields on slabs of npml layers per active side
-//   G     : 9 x np velocity gradient hand-off (FP32C with PML or attenuation)
+//   G     : 9 x np velocity gradient hand-off (FP32C with attenuation)
 //   eta/Deta, qs : 24 x np memory variables and their rates, 1/Qs per point
 //           (anelastic response only)
 #pragma once
@@ -86,10 +86,10 @@ struct VolumeArgs {
   T* Q[6];
   T* DQ[6];
   long long slab_np[6];
-  // velocity gradient g[c][j] (component c*3+j, stride np) of the PML points
-  // (of every point with the anelastic response), written by the TMA stencil
-  // kernel and read by the PML and anelastic kernels of the same stage;
-  // nullptr where those kernels form it themselves
+  int pml_pre;        // the slabs are advanced before the stencil (PML pre-kernel), not after it
+  // velocity gradient g[c][j] (component c*3+j, stride np) with the anelastic
+  // response, written by the TMA stencil kernel and read by the anelastic
+  // kernel of the same stage; nullptr where that kernel forms it itself
   T* G;
   int fd;             // difference operator: 0 SBP-6 central; upwind pair (D+ on v, D- on fluxes) of order 6 (1),
                       // of order 5 (2), or a table operator (3, ug)
@@ -252,14 +252,15 @@ void launch_stencil_tma_batch(const TmaBatchDesc* d_dev, int nd, long long total
 template <typename T>
 void launch_volume(const VolumeArgs<T>& a, bool curv, void* stream);
 // Before the stencil kernel of a variant without its own face pass: the
-// boundary and fault penalties folded into DF of the face points.  Returns
-// the number of launches.
+// boundary and fault penalties folded into DF of the face points, and the
+// PML slabs advanced with their damping folded into DF.  Returns the number
+// of launches.
 template <typename T>
-int launch_pre(const VolumeArgs<T>& a, void* stream);
+int launch_pre(const VolumeArgs<T>& a, bool curv, void* stream);
 // The same for both blocks of a scenario whose stencils both run as the TMA
-// kernel, in one launch.
+// kernel, in one launch each.
 template <typename T>
-int launch_pre2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, void* stream);
+int launch_pre2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, bool curv, void* stream);
 template <typename T>
 int launch_corrections(const VolumeArgs<T>& a, bool curv, void* stream);
 // One moment-tensor source: DF(4:9) -= am * delta on a box of points

@@ -256,11 +256,13 @@ __device__ __forceinline__ void add_correction(const VolumeArgs<T>& a, long long
 // the outer-boundary SAT of every side with a boundary code 1..3 that the
 // point lies on, times that axis's tau0/h (src/RHS_Interior.f90:1516-1703),
 // plus the fault SAT on the interface face (src/RHS_Interior.f90:1757-1772).
-// The caller subtracts tot from the rates.  Returns false if the point has
-// no penalised face.  Inlined: as a call its array arguments went through
+// The caller subtracts tot from the rates.  on_side(side, ubc) is called for
+// each boundary side with the forcing of a PML slab's auxiliary fields (not
+// yet scaled by tau0/h).  Returns false if the point has no penalised face.  Inlined: as a call its array arguments went through
 // the stack.
-template <typename T>
-__device__ __forceinline__ bool face_penalty(const VolumeArgs<T>& a, int i, int j, int k, const T* u, T* tot) {
+template <typename T, typename Fn>
+__device__ __forceinline__ bool face_penalty(const VolumeArgs<T>& a, int i, int j, int k, const T* u, T* tot,
+                                             Fn&& on_side) {
   const int nq = a.nq, nr = a.nr, ns = a.ns;
   bool any = false;
   for (int c = 0; c < 9; ++c) tot[c] = T(0);
@@ -278,6 +280,7 @@ __device__ __forceinline__ bool face_penalty(const VolumeArgs<T>& a, int i, int 
     T sat[9], ubc[9];
     boundary_sat(u, a.face[s2], nf, f, code, hi, a.bc_form, sat, ubc);
     for (int c = 0; c < 9; ++c) tot[c] += a.tau_h[ax2] * sat[c];
+    on_side(s2, ubc);
     any = true;
   }
   if (a.fault_sat && ((a.block == 0 && i == nq - 1) || (a.block == 1 && i == 0))) {

@@ -6,8 +6,9 @@
 // on every plane of the block.
 //
 // The boundary and fault penalties of the face points (src/RHS_Interior.f90:
-// 1516-1703, 1757-1772) are folded into DF beforehand by the face
-// pre-kernel, so this kernel has no face-dependent work.
+// 1516-1703, 1757-1772) and the PML damping of the slab points (:1782-2201)
+// are folded into DF beforehand by the pre-kernels, so this kernel has no
+// face- or slab-dependent work.
 //
 // A tile is 32 x 12 (q, r) points over a chunk of s planes; a CTA takes a
 // tile (or, launched persistently, tiles in turn) and marches along its
@@ -286,11 +287,12 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
   const int q = q0 + tx, r = r0 + ty;
   const bool own = q < nq && r >= spr.own_lo && r < spr.own_hi;
   const int kq = sbp_kind(q, nq), kr = sbp_kind(r, nr);
-  // PML points (every point with the anelastic response) hand their
-  // velocity gradient to the correction kernels (a.G)
-  const int npml = a.npml;
-  const bool pml_qr = a.G != nullptr && ((a.pml[0] && q < npml) || (a.pml[1] && q >= nq - npml) ||
-                                         (a.pml[2] && r < npml) || (a.pml[3] && r >= nr - npml));
+  // points whose DF the pre-kernels have set on a stage with A = 0: the
+  // block's faces and the PML slabs (here the q and r sides, true for the
+  // whole column)
+  const int npml = a.pml_pre ? a.npml : 0;
+  const bool fold_qr = q == 0 || q == nq - 1 || r == 0 || r == nr - 1 || (a.pml[0] && q < npml) ||
+                       (a.pml[1] && q >= nq - npml) || (a.pml[2] && r < npml) || (a.pml[3] && r >= nr - npml);
   const long long np = a.np;
   const long long sts = (long long)a.pq * nr;
   const long long col = q + (long long)a.pq * r;
@@ -533,7 +535,7 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
           }
         }
       }
-      if (a.G != nullptr && (a.anel || pml_qr || (a.pml[4] && s < npml) || (a.pml[5] && s >= ns - npml))) {
+      if (a.G != nullptr) {  // anelastic: every point hands its velocity gradient over
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -554,15 +556,15 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
       du[6] = mu * (g[0][1] + g[1][0]);
       du[7] = mu * (g[0][2] + g[2][0]);
       du[8] = mu * (g[1][2] + g[2][1]);
-      // the face pre-kernel has folded the boundary and fault penalties
-      // into DF of the face points: DF - tot/A, or -tot on the first stage
-      // (A = 0, where DF holds nothing else)
-      const bool face = q == 0 || q == nq - 1 || r == 0 || r == nr - 1 || s == 0 || s == ns - 1;
+      // the pre-kernels have folded the boundary and fault penalties and the
+      // PML damping into DF of their points: DF + term/A, or the term itself
+      // on the first stage (A = 0, where DF holds nothing else)
+      const bool fold = fold_qr || s == 0 || s == ns - 1 || (a.pml[4] && s < npml) || (a.pml[5] && s >= ns - npml);
 #pragma unroll
       for (int c = 0; c < 9; ++c) {
         const float f0 = fb(c, lr, lq);
         const float dfs = S[TL::OFF_DF + c * NC + ty * TQ + tx];
-        const float df = a.A != 0.0f ? a.A * dfs + du[c] : (face ? dfs : 0.0f) + du[c];
+        const float df = a.A != 0.0f ? a.A * dfs + du[c] : (fold ? dfs : 0.0f) + du[c];
         a.DF[c * np + p] = df;
         if (KAHAN) {
           const comp_t* CKs = reinterpret_cast<const comp_t*>(S + TL::OFF_CK);

@@ -24,6 +24,8 @@
 // constant metric.
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "wql_internal.h"
 #include "wql_stencil.cuh"
 
@@ -704,6 +706,16 @@ PmlBoxes pml_boxes(const VolumeArgs<T>& a) {
   return B;
 }
 
+// Offset of block point (i, j, k) within the slab of `side`.
+template <typename T>
+__device__ __forceinline__ long long slab_point(const VolumeArgs<T>& a, int side, int i, int j, int k) {
+  const int axis = side >> 1, npml = a.npml;
+  const bool hi = side & 1;
+  if (axis == 0) return (hi ? i - (a.nq - npml) : i) + (long long)npml * (j + (long long)a.nr * k);
+  if (axis == 1) return i + (long long)a.nq * ((hi ? j - (a.nr - npml) : j) + (long long)npml * k);
+  return i + (long long)a.nq * (j + (long long)a.nr * (hi ? k - (a.ns - npml) : k));
+}
+
 // FP32 fields: capped at 80 registers for three CTAs per SM (24 warps to
 // hide the latency of its dependent loads; measured 0.39 -> 0.31 ms per
 // correction launch on config 2 despite some spilling).
@@ -735,20 +747,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) pml_kernel(const 
   const T* __restrict__ F = a.Fin;
   const T* __restrict__ coef = a.coef;
   const bool shell = FD == 3 && ug_shell(a, idx, nn);
-  // velocity gradient at the point: from the TMA stencil of this stage
-  // (a.G), else formed here
+  // velocity gradient at the point
   T g[3][3];
   const T Jinv = CURV ? coef[9 * np + p] : T(1);
-  const bool have_g = a.G != nullptr;
-  if (have_g) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int jj = 0; jj < 3; ++jj) g[c][jj] = a.G[(c * 3 + jj) * np + p];
-  }
   // every loop over axes and sides is unrolled so that the per-axis index,
   // extent and stride are compile-time selections (no local-memory arrays)
-  if (!have_g) {
+  {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       T o[3];
@@ -791,10 +795,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) pml_kernel(const 
     // in the field precision
     const int off = hi ? ii + 1 - (n - npml) : (axis == 2 ? ii + 1 - npml : ii - npml);
     const T damp = (T)d0 * (fabs((T)off / (T)npml));
-    long long sp;
-    if (axis == 0) sp = (hi ? ii - (n - npml) : ii) + (long long)npml * (j + (long long)nr * k);
-    else if (axis == 1) sp = i + (long long)nq * ((hi ? ii - (n - npml) : ii) + (long long)npml * k);
-    else sp = i + (long long)nq * (j + (long long)nr * (hi ? ii - (n - npml) : ii));
+    const long long sp = slab_point(a, side, i, j, k);
     const long long snp = a.slab_np[side];
     T* __restrict__ Q = a.Q[side];
     T* __restrict__ DQ = a.DQ[side];
@@ -855,6 +856,285 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) pml_kernel(const 
     }
   }
   add_correction<T, KAHAN>(a, p, corr);
+}
+
+// ---------------------------------------------------------------------------
+// PML pre-kernel (FP32 fields whose stencil is the TMA kernel): the same slab
+// update as pml_kernel, run before the stencil of its stage.  Everything it
+// needs is stage input (F, Q, DQ), so the damping terms of the rates are
+// folded into DF (DF + corr/A, or corr on a stage with A = 0) and the
+// stencil's A*DF + du carries them: F_out and its compensation are not read
+// and written a second time, and no velocity gradient is handed over.  The
+// face pre-kernel, which runs first, has folded the boundary forcing of the
+// auxiliary fields into DQ at the slab's own face.
+//
+// The slab union is cut into regions along the slab edges, up to 26, so that
+// the sides a point lies in are the same for a whole CTA: the axis of a side
+// and the arrays of its fluxes are uniform, and every load of a neighbour is
+// a uniform base plus one 32-bit offset that all of the neighbour's
+// quantities share.  A CTA takes a tile of 256 points of one region, 32 x 4 x
+// 2 (q, r, s) points, or 8 x 8 x 4 in the regions of the q slabs, whose rows
+// are only npml points long: neighbouring rows share their stencil reads in
+// L1.  Each direction's neighbours are visited once for both the flux and the
+// velocity derivative; a closure row's columns are unrolled like the interior
+// row's, so their loads are in flight together (as a loop, their latencies
+// added up).
+struct PmlTiles {
+  int n;
+  int lo[26][3], dim[26][3];
+  int sides[26];       // bit per side
+  int lw[26], lr[26];  // log2 of the tile extents along q and r
+  int tq[26], tr[26];  // tiles along q and r
+  int start[27];       // CTAs before region b
+};
+
+template <typename T>
+PmlTiles pml_tiles(const VolumeArgs<T>& a) {
+  PmlTiles P;
+  P.n = 0;
+  P.start[0] = 0;
+  const int nn[3] = {a.nq, a.nr, a.ns}, w = a.npml;
+  // the intervals of each axis between its slab edges, with the sides they lie in
+  int cut[3][4], m[3], in[3][3];
+  for (int d = 0; d < 3; ++d) {
+    int e[4] = {0, a.pml[2 * d] ? w : 0, a.pml[2 * d + 1] ? nn[d] - w : nn[d], nn[d]};
+    if (e[1] > e[2]) std::swap(e[1], e[2]);
+    m[d] = 0;
+    cut[d][0] = 0;
+    for (int k = 0; k < 3; ++k) {
+      if (e[k + 1] <= e[k]) continue;
+      in[d][m[d]] = (a.pml[2 * d] && e[k] < w ? 1 << (2 * d) : 0) |
+                    (a.pml[2 * d + 1] && e[k] >= nn[d] - w ? 2 << (2 * d) : 0);
+      cut[d][++m[d]] = e[k + 1];
+    }
+  }
+  for (int z = 0; z < m[2]; ++z)
+    for (int y = 0; y < m[1]; ++y)
+      for (int x = 0; x < m[0]; ++x) {
+        const int sides = in[0][x] | in[1][y] | in[2][z], b = P.n;
+        if (!sides) continue;
+        const int c[3] = {x, y, z};
+        for (int d = 0; d < 3; ++d) {
+          P.lo[b][d] = cut[d][c[d]];
+          P.dim[b][d] = cut[d][c[d] + 1] - cut[d][c[d]];
+        }
+        P.sides[b] = sides;
+        const bool narrow = P.dim[b][0] <= 24;
+        P.lw[b] = narrow ? 3 : 5;
+        P.lr[b] = narrow ? 3 : 2;
+        const int ls = 8 - P.lw[b] - P.lr[b];
+        P.tq[b] = (P.dim[b][0] + (1 << P.lw[b]) - 1) >> P.lw[b];
+        P.tr[b] = (P.dim[b][1] + (1 << P.lr[b]) - 1) >> P.lr[b];
+        const int ts = (P.dim[b][2] + (1 << ls) - 1) >> ls;
+        P.start[b + 1] = P.start[b] + P.tq[b] * P.tr[b] * ts;
+        ++P.n;
+      }
+  return P;
+}
+
+// One or two blocks in a launch: CTAs [0, n0) take block 0's tiles.
+template <typename T>
+struct PmlPair {
+  VolumeArgs<T> a[2];
+  PmlTiles t[2];
+  int n0;
+};
+
+__device__ __forceinline__ float at(const float* base, unsigned byte) {
+  return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(base) + byte);
+}
+
+template <bool CURV, int FD>
+__device__ __forceinline__ void pml_pre_point(const VolumeArgs<float>& a, int i, int j, int k, unsigned sides,
+                                              const float* tab) {
+  const int nq = a.nq, nr = a.nr, ns = a.ns, npml = a.npml;
+  const long long np = a.np;
+  const unsigned o = 4u * (unsigned)(i + a.pq * (j + nr * k));  // byte offset of the point in a component
+  const float* __restrict__ F = a.Fin;
+  const float* __restrict__ coef = a.coef;
+  const float Jinv = CURV ? at(coef + 9 * np, o) : 1.0f;
+  const float lam = at(coef + (CURV ? 10 : 0) * np, o), mu = at(coef + (CURV ? 11 : 1) * np, o);
+  const float rinv = at(coef + (CURV ? 12 : 2) * np, o);
+  const float rhoinv = CURV ? rinv / Jinv : rinv;
+  const float l2m = lam + 2.0f * mu;
+  // on a stage with A = 0, DF and DQ hold only what the face pre-kernel put there
+  const bool keep = a.A != 0.0f;
+  float corr[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) corr[c] = 0.0f;
+#pragma unroll 1
+  while (sides) {
+    const int side = __ffs(sides) - 1;
+    sides &= sides - 1;
+    const int axis = side >> 1;
+    const bool hi = side & 1;
+    const int ii = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 0 ? nq : (axis == 1 ? nr : ns);
+    // flux components of physical axis `axis`: sigma_{c,axis}
+    const float* __restrict__ S0 = F + (axis == 0 ? 3 : (axis == 1 ? 6 : 7)) * np;
+    const float* __restrict__ S1 = F + (axis == 0 ? 6 : (axis == 1 ? 4 : 8)) * np;
+    const float* __restrict__ S2 = F + (axis == 0 ? 7 : (axis == 1 ? 8 : 5)) * np;
+    float sd[3] = {0.0f, 0.0f, 0.0f}, gv[3] = {0.0f, 0.0f, 0.0f};
+    // derivative along computational axis d of the velocities (o6[0..2]) and
+    // of the fluxes J*metric_axis(d)*sigma_{c,axis} (o6[3..5])
+    auto direction = [&](int d) {
+      const int id = d == 0 ? i : (d == 1 ? j : k), nd = d == 0 ? nq : (d == 1 ? nr : ns);
+      const unsigned st = 4u * (unsigned)(d == 0 ? 1 : (d == 1 ? a.pq : a.pq * nr));
+      const float* __restrict__ M = CURV ? coef + (d * 3 + axis) * np : coef;
+      float o6[6];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) o6[c] = 0.0f;
+      auto vel = [&](unsigned q, float w) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o6[c] += w * at(F + c * np, q);
+      };
+      auto flux = [&](unsigned q, float w) {
+        const float m = CURV ? w * at(M, q) : w;
+        o6[3] += m * at(S0, q);
+        o6[4] += m * at(S1, q);
+        o6[5] += m * at(S2, q);
+      };
+      const int kind = sbp_kind(id, nd);
+      if (kind == 0 && FD) {
+        const float cf[7] = WQL_UP_CF;
+#pragma unroll
+        for (int of = -4; of <= 4; ++of) {
+          if (of >= -2) vel(o + (unsigned)of * st, cf[of + 2]);
+          if (of <= 2) flux(o + (unsigned)of * st, -cf[2 - of]);
+        }
+      } else if (kind == 0) {
+        const float cs[3] = {float(kC1), float(kC2), float(kC3)};
+#pragma unroll
+        for (int s = 1; s <= 3; ++s) {
+          vel(o + (unsigned)s * st, cs[s - 1]);
+          flux(o + (unsigned)s * st, cs[s - 1]);
+          vel(o - (unsigned)s * st, -cs[s - 1]);
+          flux(o - (unsigned)s * st, -cs[s - 1]);
+        }
+      } else {
+        // left row kind = -1-row reads points 0.., right row kind = 1+row
+        // the mirrored points with negated weights (the upwind pair swaps
+        // its two tables there)
+        const int row = kind < 0 ? -kind - 1 : kind - 1;
+        constexpr int NC = FD ? 10 : 9;
+        const float sgn = kind < 0 ? 1.0f : -1.0f;
+        const unsigned dir = kind < 0 ? st : 0u - st;
+        const float* wv = tab + (FD && kind > 0 ? 60 : 0) + row * NC;
+        const float* wf = FD ? tab + (kind > 0 ? 0 : 60) + row * NC : wv;
+        const unsigned q = o - (unsigned)row * dir;
+#pragma unroll
+        for (int t = 0; t < NC; ++t) {
+          vel(q + (unsigned)t * dir, sgn * wv[t]);
+          flux(q + (unsigned)t * dir, sgn * wf[t]);
+        }
+      }
+      const float rh = a.rh[d];
+      const float mt = CURV ? at(M, o) * Jinv : a.cart_metric[d];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        gv[c] += mt * (rh * o6[c]);
+        sd[c] += rh * o6[3 + c];
+      }
+    };
+    if (CURV) {
+#pragma unroll 1
+      for (int d = 0; d < 3; ++d) direction(d);
+    } else {
+      direction(axis);
+    }
+    // Q and DQ are read after the derivatives (held across them, they spill)
+    float qv[9], dq[9];
+    const bool forced = (hi ? ii == n - 1 : ii == 0) && a.bc[side] >= 1 && a.bc[side] <= 3;
+    const long long sp = slab_point(a, side, i, j, k), snp = a.slab_np[side];
+    float* __restrict__ Q = a.Q[side] + sp;
+    float* __restrict__ DQ = a.DQ[side] + sp;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+      qv[c] = Q[c * snp];
+      dq[c] = keep || forced ? DQ[c * snp] : 0.0f;
+    }
+    const float sc = CURV ? Jinv : a.cart_metric[axis];
+    // damping profile in grid-index units (src/RHS_Interior.f90:1855,1973,2092)
+    const int off = hi ? ii + 1 - (n - npml) : (axis == 2 ? ii + 1 - npml : ii - npml);
+    const float damp = (float)a.pml_d0 * (fabsf((float)off / (float)npml));
+    const float cfs = 1.0f;
+    corr[0] -= damp * qv[0] * rhoinv;
+    corr[1] -= damp * qv[1] * rhoinv;
+    corr[2] -= damp * qv[2] * rhoinv;
+    corr[3] -= damp * (l2m * qv[3] + lam * qv[4] + lam * qv[5]);
+    corr[4] -= damp * (lam * qv[3] + l2m * qv[4] + lam * qv[5]);
+    corr[5] -= damp * (lam * qv[3] + lam * qv[4] + l2m * qv[5]);
+    corr[6] -= mu * damp * qv[6];
+    corr[7] -= mu * damp * qv[7];
+    corr[8] -= mu * damp * qv[8];
+    // velocity-gradient sources (src/RHS_Interior.f90:1890-1907, 2008-2025, 2125-2142)
+    float src[9];
+    src[0] = sd[0] * sc;
+    src[1] = sd[1] * sc;
+    src[2] = sd[2] * sc;
+    src[3] = axis == 0 ? gv[0] : 0.0f;
+    src[4] = axis == 1 ? gv[1] : 0.0f;
+    src[5] = axis == 2 ? gv[2] : 0.0f;
+    src[6] = axis == 0 ? gv[1] : (axis == 1 ? gv[0] : 0.0f);
+    src[7] = axis == 0 ? gv[2] : (axis == 2 ? gv[0] : 0.0f);
+    src[8] = axis == 1 ? gv[2] : (axis == 2 ? gv[1] : 0.0f);
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+      const float nw = (keep ? a.A * dq[c] : dq[c]) + src[c] - (damp + cfs) * qv[c];
+      DQ[c * snp] = nw;
+      Q[c * snp] = qv[c] + a.Bdt * nw;
+    }
+  }
+  const bool face = i == 0 || i == nq - 1 || j == 0 || j == nr - 1 || k == 0 || k == ns - 1;
+  const float inv = keep ? 1.0f / a.A : 1.0f;
+  float df[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) df[c] = keep || face ? at(a.DF + c * np, o) : 0.0f;
+#pragma unroll
+  for (int c = 0; c < 9; ++c)
+    *reinterpret_cast<float*>(reinterpret_cast<char*>(a.DF + c * np) + o) = df[c] + corr[c] * inv;
+}
+
+template <bool CURV, int FD>
+__global__ void __launch_bounds__(256, 3) pml_pre_kernel(const __grid_constant__ PmlPair<float> P) {
+  __shared__ float tab[120];
+  if (FD) {
+    if (threadIdx.x < 120) tab[threadIdx.x] = (&c_up_f[0][0][0])[threadIdx.x];
+  } else if (threadIdx.x < 54) {
+    tab[threadIdx.x] = (&c_sbp_f[0][0])[threadIdx.x];
+  }
+  __syncthreads();
+  const int blk = (int)blockIdx.x >= P.n0 ? 1 : 0;
+  const int t = (int)blockIdx.x - (blk ? P.n0 : 0);
+  const PmlTiles& B = P.t[blk];
+  int b = 0;
+  while (b < B.n - 1 && t >= B.start[b + 1]) ++b;
+  const int l = t - B.start[b], lw = B.lw[b], lr = B.lr[b];
+  const int bq = l % B.tq[b], br = (l / B.tq[b]) % B.tr[b], bs = l / (B.tq[b] * B.tr[b]);
+  const int e = threadIdx.x;
+  const int i = (bq << lw) + (e & ((1 << lw) - 1));
+  const int j = (br << lr) + ((e >> lw) & ((1 << lr) - 1));
+  const int k = (bs << (8 - lw - lr)) + (e >> (lw + lr));
+  if (i >= B.dim[b][0] || j >= B.dim[b][1] || k >= B.dim[b][2]) return;
+  pml_pre_point<CURV, FD>(P.a[blk], B.lo[b][0] + i, B.lo[b][1] + j, B.lo[b][2] + k, (unsigned)B.sides[b], tab);
+}
+
+// Launches the PML pre-kernel over one block (a1 null) or two.
+int launch_pml_pre(const VolumeArgs<float>& a0, const VolumeArgs<float>* a1, bool curv, cudaStream_t s) {
+  PmlPair<float> P;
+  const VolumeArgs<float>* a[2] = {&a0, a1 ? a1 : &a0};
+  int n[2];
+  for (int b = 0; b < 2; ++b) {
+    P.a[b] = *a[b];
+    P.t[b] = pml_tiles(*a[b]);
+    n[b] = a[b]->pml_pre ? P.t[b].start[P.t[b].n] : 0;
+  }
+  if (!a1) n[1] = 0;
+  P.n0 = n[0];
+  if (n[0] + n[1] == 0) return 0;
+  const unsigned g = (unsigned)(n[0] + n[1]);
+  if (a0.fd) curv ? pml_pre_kernel<true, 1><<<g, 256, 0, s>>>(P) : pml_pre_kernel<false, 1><<<g, 256, 0, s>>>(P);
+  else curv ? pml_pre_kernel<true, 0><<<g, 256, 0, s>>>(P) : pml_pre_kernel<false, 0><<<g, 256, 0, s>>>(P);
+  return 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -944,19 +1224,20 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
       if (!(hi ? (ii >= n - npml) : (ii < npml))) continue;
       const int off = hi ? ii + 1 - (n - npml) : (axis == 2 ? ii + 1 - npml : ii - npml);
       const T damp = (T)a.pml_d0 * (fabs((T)off / (T)npml));
-      long long sp;
-      if (axis == 0) sp = (hi ? ii - (n - npml) : ii) + (long long)npml * (j + (long long)nr * k);
-      else if (axis == 1) sp = i + (long long)nq * ((hi ? ii - (n - npml) : ii) + (long long)npml * k);
-      else sp = i + (long long)nq * (j + (long long)nr * (hi ? ii - (n - npml) : ii));
+      const long long sp = slab_point(a, side, i, j, k);
       const long long snp = a.slab_np[side];
       const T* Q = a.Q[side];
+      const T* DQ = a.DQ[side];
+      // the stage-input Q; after the PML pre-kernel has advanced it by
+      // B*dt*DQ that step is taken back (to the rounding of Q)
+      auto q_in = [&](int c) { return a.pml_pre ? Q[c * snp + sp] - a.Bdt * DQ[c * snp + sp] : Q[c * snp + sp]; };
       // Q components of the normal strain and the two shear strains of this axis
       const int cn = 3 + axis;
       const int c1 = axis == 0 ? 6 : (axis == 1 ? 6 : 7);
       const int c2 = axis == 0 ? 7 : 8;
-      dq[axis][0] = damp * Q[cn * snp + sp];
-      dq[axis][1] = damp * Q[c1 * snp + sp];
-      dq[axis][2] = damp * Q[c2 * snp + sp];
+      dq[axis][0] = damp * q_in(cn);
+      dq[axis][1] = damp * q_in(c1);
+      dq[axis][2] = damp * q_in(c2);
     }
     e[0] = e[0] - dq[0][0];
     e[1] = e[1] - dq[1][0];
@@ -1064,19 +1345,21 @@ __global__ void __launch_bounds__(256) face_kernel(const __grid_constant__ Volum
   T u[9], tot[9], corr[9];
   for (int c = 0; c < 9; ++c) u[c] = a.Fin[c * np + p];
   mms_deviation(a, p, u);
-  const bool any = face_penalty(a, i, j, k, u, tot);
+  const bool any = face_penalty(a, i, j, k, u, tot, [](int, const T (&)[9]) {});
   for (int c = 0; c < 9; ++c) corr[c] = -tot[c];
   if (any) add_correction<T, KAHAN>(a, p, corr);
 }
 
 // ---------------------------------------------------------------------------
 // Face pre-kernel (for the stencil variant without a face pass): the
-// boundary and fault penalty tot of each face point (face_penalty, as in the
-// face kernel) folded into the rates before the stencil kernel runs,
-// DF <- DF - tot/A, or DF <- -tot on a stage with A = 0, so that the
-// stencil's A*DF + du (or DF + du on face points when A = 0) carries it.
-// One thread per face point, a point on several faces taken by its lowest
-// side.
+// boundary and fault penalty tot of each face point (as in the face kernel)
+// folded into the rates before the stencil kernel runs, DF <- DF - tot/A, or
+// DF <- -tot on a stage with A = 0, so that the stencil's A*DF + du (or
+// DF + du on face points when A = 0) carries it.  On a PML side the same
+// boundary forcing enters the rates of the slab's auxiliary fields
+// (src/RHS_Interior.f90:1560-1700): it is folded into DQ in the same way,
+// for the PML pre-kernel to pick up.  One thread per face point, a point on
+// several faces taken by its lowest side.
 template <typename T>
 __device__ __forceinline__ void face_pre_point(const VolumeArgs<T>& a, long long t) {
   const int nq = a.nq, nr = a.nr, ns = a.ns;
@@ -1113,7 +1396,15 @@ __device__ __forceinline__ void face_pre_point(const VolumeArgs<T>& a, long long
     df[c] = keep ? a.DF[c * np + p] : T(0);
   }
   mms_deviation(a, p, u);
-  if (!face_penalty(a, i, j, k, u, tot)) return;
+  face_penalty(a, i, j, k, u, tot, [&](int s2, const T (&ubc)[9]) {
+    if (!a.pml_pre || !a.pml[s2]) return;
+    const long long sp = slab_point(a, s2, i, j, k), snp = a.slab_np[s2];
+    const T th = a.tau_h[s2 >> 1];
+    T* DQ = a.DQ[s2];
+#pragma unroll
+    for (int c = 0; c < 9; ++c) DQ[c * snp + sp] = keep ? DQ[c * snp + sp] - th * ubc[c] / a.A : -th * ubc[c];
+  });
+  // a face point without a penalised side still defines DF when A = 0
 #pragma unroll
   for (int c = 0; c < 9; ++c) a.DF[c * np + p] = keep ? df[c] - tot[c] / a.A : -tot[c];
 }
@@ -1337,7 +1628,7 @@ int launch_corr(const VolumeArgs<T>& a, cudaStream_t s) {
     else anelastic_kernel<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(a);
     ++n;
   }
-  if (a.npml > 0) {
+  if (a.npml > 0 && !a.pml_pre) {
     const PmlBoxes bx = pml_boxes(a);
     const unsigned nblk = (unsigned)((bx.start[bx.n] + 255) / 256);
     if (bx.start[bx.n] > 0) {
@@ -1387,15 +1678,16 @@ void launch_volume(const VolumeArgs<T>& a, bool curv, void* stream) {
 }
 
 template <typename T>
-int launch_pre(const VolumeArgs<T>& a, void* stream) {
+int launch_pre(const VolumeArgs<T>& a, bool curv, void* stream) {
   if (!stencil_is_tma(a)) return 0;
   const long long nface = 2LL * ((long long)a.nr * a.ns + (long long)a.nq * a.ns + (long long)a.nq * a.nr);
   face_pre_kernel<T><<<(unsigned)((nface + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a);
+  if constexpr (sizeof(T) == 4) return 1 + launch_pml_pre(a, nullptr, curv, (cudaStream_t)stream);
   return 1;
 }
 
 template <typename T>
-int launch_pre2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, void* stream) {
+int launch_pre2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, bool curv, void* stream) {
   FacePair<T> P;
   P.a[0] = a0;
   P.a[1] = a1;
@@ -1405,14 +1697,14 @@ int launch_pre2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, void* stream) 
   P.n0 = nface(a0);
   const long long n = P.n0 + nface(a1);
   face_pre_kernel2<T><<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(P);
-  return 1;
+  return 1 + launch_pml_pre(a0, &a1, curv, (cudaStream_t)stream);
 }
 
 template <typename T>
 int launch_corrections(const VolumeArgs<T>& a0, bool curv, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  // the PML velocity gradient comes from the stencil only when that was the
-  // TMA kernel (the only one that writes it)
+  // the velocity gradient of an anelastic block comes from the stencil only
+  // when that was the TMA kernel (the only one that writes it)
   VolumeArgs<T> a = a0;
   if (!stencil_is_tma(a)) a.G = nullptr;
   const bool kahan = a.C != nullptr;
@@ -1444,9 +1736,9 @@ template void launch_source<float>(const VolumeArgs<float>&, const int*, const i
 template void launch_volume<double>(const VolumeArgs<double>&, bool, void*);
 template void launch_volume<float>(const VolumeArgs<float>&, bool, void*);
 template int launch_corrections<double>(const VolumeArgs<double>&, bool, void*);
-template int launch_pre<double>(const VolumeArgs<double>&, void*);
-template int launch_pre<float>(const VolumeArgs<float>&, void*);
-template int launch_pre2<float>(const VolumeArgs<float>&, const VolumeArgs<float>&, void*);
+template int launch_pre<double>(const VolumeArgs<double>&, bool, void*);
+template int launch_pre<float>(const VolumeArgs<float>&, bool, void*);
+template int launch_pre2<float>(const VolumeArgs<float>&, const VolumeArgs<float>&, bool, void*);
 template int launch_corrections<float>(const VolumeArgs<float>&, bool, void*);
 template bool stencil_is_tma<float>(const VolumeArgs<float>&);
 template bool stencil_is_tma<double>(const VolumeArgs<double>&);
