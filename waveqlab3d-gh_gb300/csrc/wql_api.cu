@@ -1430,7 +1430,7 @@ int batch_step(wql_batch* B) {
         CK(cudaEventRecord(B->ev[i], B->members[i]->stream));
         CK(cudaStreamWaitEvent(B->stream, B->ev[i], 0));
       }
-      launch_stencil_tma_batch(B->d_dev + g.off, g.nd, g.total, curv == 1, true, B->stream);
+      launch_stencil_tma_batch(B->d_dev + g.off, g.nd, g.total, curv == 1, B->stream);
       CK(cudaEventRecord(B->joined, B->stream));
       for (size_t i : g.who) {
         CK(cudaStreamWaitEvent(B->members[i]->stream, B->joined, 0));
@@ -1485,7 +1485,7 @@ void run_stage(wql_scn* S, StepCtx& c, int stage) {
     }
     mark_begin(S, 1);
     launch_stencil_tma2(volume_args<float>(S, 0, A, Bdt, stage == 5), volume_args<float>(S, 1, A, Bdt, stage == 5),
-                        S->curv, true, S->stream);
+                        S->curv, S->stream);
     mark_end(S);
     c.launches += 1;
     for (int b = 0; b < 2; ++b) stage_block_post(S, c, stage, b);

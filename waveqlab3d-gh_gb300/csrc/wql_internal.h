@@ -217,10 +217,9 @@ int make_stencil_maps(StencilMaps& m, void* const F[2], void* coef, void* DF, vo
 // nq0 and nq1 points along q.
 int tma_tile_width(int nq0, int nq1, bool curv);
 // Launches the TMA stencil kernel (every plane of the block).
-void launch_stencil_tma(const VolumeArgs<float>& a, bool curv, bool kahan, void* stream);
+void launch_stencil_tma(const VolumeArgs<float>& a, bool curv, void* stream);
 // The same for both blocks of a scenario in one launch.
-void launch_stencil_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, bool curv, bool kahan,
-                         void* stream);
+void launch_stencil_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, bool curv, void* stream);
 // Whether the block's stencil runs as the TMA kernel (the tuning and the
 // block shape allow it).
 template <typename T>
@@ -243,8 +242,7 @@ long long fill_tma_desc(const VolumeArgs<float>& a, TmaBatchDesc& d);
 bool tma_eligible(const VolumeArgs<float>& a);
 // One launch over nd table entries (all curvilinear or all Cartesian, all
 // with or all without compensation).
-void launch_stencil_tma_batch(const TmaBatchDesc* d_dev, int nd, long long total_ctas, bool curv, bool kahan,
-                              void* stream);
+void launch_stencil_tma_batch(const TmaBatchDesc* d_dev, int nd, long long total_ctas, bool curv, void* stream);
 
 // One stage on one block: launch_volume runs the stencil kernel (DF and the
 // updated fields for every point); launch_corrections then adds the PML,

@@ -25,8 +25,11 @@
 //                      the remaining 7 coefficients, the rates DF and the
 //                      compensation C on the tile;
 //   lead (plane s+3) : the 9 field components and J*metric_s on the tile.
-// Each consumer thread keeps the velocities and the s-face momentum flux of
-// planes s-3..s+3 of its point in registers (the first six read directly at
+// Each consumer thread works on two neighbouring q points with packed FP32
+// instructions (a point per thread took about 900 issue slots a plane, a pair
+// takes about 1100 at twice the points: 0.774 -> 0.756 ms per launch on 2 x
+// 201^3, 0.140 -> 0.124 ms on the 2 x 76x101x151 upwind pair) and keeps the
+// velocities and the s-face momentum flux of planes s-3..s+3 in registers (the first six read directly at
 // the start of a chunk, then one pushed per step from the lead tile), so
 // the s derivative of a central row needs no shared memory (lead planes
 // outside 0..ns-1 load as zeros and are never used: the 12 s closure rows
@@ -54,9 +57,10 @@
 namespace wql {
 namespace {
 
-template <bool CURV, bool KAHAN, int FD, int TQ_ = kTmaTQ>
+template <bool CURV, int FD, int TQ_ = kTmaTQ>
 struct TmaTile {
   static constexpr int TQ = TQ_, TR = kTmaTR, NC = TQ * TR;
+  static constexpr int NT = (NC / 2 + 31) / 32 * 32;  // consumer threads: one per two q points, whole warps
   // r halo: 3 rows for the central operator, 4 for the upwind pair
   static constexpr int HR = FD ? 4 : 3;
   static constexpr int BQ = TQ + 16, BR = TR + 2 * HR;  // field box: q from q0-8, r from r0-HR
@@ -71,7 +75,7 @@ struct TmaTile {
   static constexpr int DF_W = 9 * NC;            // rates of the main plane
   // compensation of the main plane: 9 x NC bfloat16 in a slot of whole
   // 128-byte lines
-  static constexpr int CK_BOX = KAHAN ? 9 * NC * 2 : 0;  // bytes the copy delivers
+  static constexpr int CK_BOX = 9 * NC * 2;  // bytes the copy delivers
   static constexpr int CK_W = (CK_BOX / 4 + 31) / 32 * 32;
   static constexpr int OFF_F = 0;
   static constexpr int OFF_CA = OFF_F + F_W;
@@ -136,6 +140,48 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// Two FP32 values of neighbouring q points in one 64-bit register (the low
+// word is the even point): Blackwell's packed FP32 instructions do both in
+// one issue slot, each half rounded as the scalar instruction rounds it.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack(f2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 dot3(f2 a0, f2 x0, f2 a1, f2 x1, f2 a2, f2 x2) {
+  return fma2(a2, x2, fma2(a1, x1, mul2(a0, x0)));
+}
+// Two values rounded to the nearest bfloat16 (lo in the low half).
+__device__ __forceinline__ unsigned bf16_pair(float lo, float hi) {
+  unsigned r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+
 // s derivative of the six differenced quantities on a closure row (planes
 // 0..5 and ns-6..ns-1).  The s window already holds most of the planes a
 // closure row reads (planes s-3..s+3 for the central operator; velocities of
@@ -145,49 +191,50 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
 // compile-time constants, so the window stays in registers); the columns are
 // summed in the order of the operator table, zero weights skipped.
 template <bool CURV, int FD, int ROW, bool RIGHT, int T>
-__device__ __forceinline__ void s_close_col(const VolumeArgs<float>& a, long long p, const float (&qv)[7][6],
-                                            float acc[6]) {
+__device__ __forceinline__ void s_close_col(const VolumeArgs<float>& a, long long p, const f2 (&qv)[7][6],
+                                            f2 acc[6]) {
   constexpr float wv = (float)s_close_w(FD, RIGHT, false, ROW, T);
   constexpr float wf = (float)s_close_w(FD, RIGHT, true, ROW, T);
   constexpr int off = s_close_off(RIGHT, ROW, T);  // plane offset from s
   constexpr int iv = s_close_vpos(FD, RIGHT, ROW, T), iflux = s_close_fpos(FD, RIGHT, ROW, T);
   const long long np = a.np, pp = p + off * ((long long)a.pq * a.nr);
   const float* F = a.Fin;
+  auto g2 = [&](const float* base) { return *reinterpret_cast<const f2*>(base + pp); };
   if constexpr (wv != 0.0f) {
-    float x[3];
+    f2 x[3];
     if constexpr (iv >= 0 && iv <= 6) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) x[c] = qv[iv][c];
     } else {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = F[c * np + pp];
+      for (int c = 0; c < 3; ++c) x[c] = g2(F + c * np);
     }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[c] += wv * x[c];
+    for (int c = 0; c < 3; ++c) acc[c] = fma2(pack(wv, wv), x[c], acc[c]);
   }
   if constexpr (wf != 0.0f) {
-    float x[3];
+    f2 x[3];
     if constexpr (iflux >= 0 && iflux <= 6) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) x[c] = qv[iflux][3 + c];
     } else if constexpr (CURV) {
-      const float a0 = a.coef[6 * np + pp], a1 = a.coef[7 * np + pp], a2 = a.coef[8 * np + pp];
+      const f2 a0 = g2(a.coef + 6 * np), a1 = g2(a.coef + 7 * np), a2 = g2(a.coef + 8 * np);
 #pragma unroll
       for (int c = 0; c < 3; ++c)
-        x[c] = a0 * F[sig(c, 0) * np + pp] + a1 * F[sig(c, 1) * np + pp] + a2 * F[sig(c, 2) * np + pp];
+        x[c] = dot3(a0, g2(F + sig(c, 0) * np), a1, g2(F + sig(c, 1) * np), a2, g2(F + sig(c, 2) * np));
     } else {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = F[sig(c, 2) * np + pp];
+      for (int c = 0; c < 3; ++c) x[c] = g2(F + sig(c, 2) * np);
     }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[3 + c] += wf * x[c];
+    for (int c = 0; c < 3; ++c) acc[3 + c] = fma2(pack(wf, wf), x[c], acc[3 + c]);
   }
 }
 
 template <bool CURV, int FD, int ROW, bool RIGHT, int... T>
-__device__ __forceinline__ void s_close_row(const VolumeArgs<float>& a, long long p, const float (&qv)[7][6],
-                                            float o[6], std::integer_sequence<int, T...>) {
-  float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+__device__ __forceinline__ void s_close_row(const VolumeArgs<float>& a, long long p, const f2 (&qv)[7][6],
+                                            f2 o[6], std::integer_sequence<int, T...>) {
+  f2 acc[6] = {0, 0, 0, 0, 0, 0};
   (s_close_col<CURV, FD, ROW, RIGHT, T>(a, p, qv, acc), ...);
 #pragma unroll
   for (int c = 0; c < 6; ++c) o[c] = acc[c];
@@ -195,8 +242,8 @@ __device__ __forceinline__ void s_close_row(const VolumeArgs<float>& a, long lon
 
 // ks = sbp_kind(s, ns), nonzero: -1..-6 left rows 0..5, 1..6 right rows 0..5.
 template <bool CURV, int FD>
-__device__ __forceinline__ void s_closure(const VolumeArgs<float>& a, long long p, int ks, const float (&qv)[7][6],
-                                          float o[6]) {
+__device__ __forceinline__ void s_closure(const VolumeArgs<float>& a, long long p, int ks, const f2 (&qv)[7][6],
+                                          f2 o[6]) {
   using Cols = std::make_integer_sequence<int, FD ? 10 : 9>;
   switch (ks) {
     case -1: s_close_row<CURV, FD, 0, false>(a, p, qv, o, Cols{}); break;
@@ -223,11 +270,11 @@ struct MapArgs {
 // the CTA has used before this tile (the same count in every thread), so a
 // persistent CTA keeps its mbarriers and the producer runs ahead into the
 // next tile.  Returns false after a wait ran out (the error word is set).
-template <bool CURV, bool KAHAN, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
 __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapArgs& m, int schunk, int bx, int by,
-                                         int bz, int& tb) {
-  using TL = TmaTile<CURV, KAHAN, FD, TQW>;
-  constexpr int TQ = TL::TQ, TR = TL::TR, NC = TL::NC, BQ = TL::BQ, BR = TL::BR, HR = TL::HR;
+                                         int bz, const float* tab, int& tb) {
+  using TL = TmaTile<CURV, FD, TQW>;
+  constexpr int TQ = TL::TQ, TR = TL::TR, NC = TL::NC, NT = TL::NT, BQ = TL::BQ, BR = TL::BR, HR = TL::HR;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   // 128-byte aligned start, derived from the shared array itself so the
   // compiler keeps every access in the shared address space
@@ -245,8 +292,8 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
   const int s_end = min(ns, s_begin + schunk);
   const int nstep = s_end - s_begin;
 
-  if (tid >= NC) {  // producer warp: one thread issues every copy
-    if (tid == NC) {
+  if (tid >= NT) {  // producer warp: one thread issues every copy
+    if (tid == NT) {
       for (int t = 0; t < nstep; ++t) {
         const int T = tb + t;
         const int st = T % NS;
@@ -268,7 +315,7 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
         }
         tma_load_4d(S + TL::OFF_F, &m.fbox, &full[st], q0 - 8, r0 - HR, sp, 0);
         tma_load_4d(S + TL::OFF_DF, &m.df, &full[st], q0, r0, sp, 0);
-        if (KAHAN) tma_load_4d(S + TL::OFF_CK, &m.ck, &full[st], q0, r0, sp, 0);
+        tma_load_4d(S + TL::OFF_CK, &m.ck, &full[st], q0, r0, sp, 0);
         if (CURV) {
           tma_load_4d(S + TL::OFF_CA, &m.ca, &full[st], q0 - 8, r0, sp, 0);
           tma_load_4d(S + TL::OFF_CB, &m.cb, &full[st], q0, r0 - HR, sp, 3);
@@ -282,52 +329,62 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
     return true;
   }
 
-  // ---- consumers: one thread per (q, r) point of the tile
-  const int tx = tid % TQ, ty = tid / TQ;
+  // ---- consumers: one thread per pair of neighbouring q points (q, q+1) of the tile
+  const int tx = 2 * (tid % (TQ / 2));
+  const bool live = tid < NC / 2;  // the last warp of a 40-wide tile is half empty
+  const int ty = live ? tid / (TQ / 2) : TR - 1;
   const int q = q0 + tx, r = r0 + ty;
-  const bool own = q < nq && r >= spr.own_lo && r < spr.own_hi;
-  const int kq = sbp_kind(q, nq), kr = sbp_kind(r, nr);
+  // q = nq - 1 of an odd nq shares its pair with the pad column, which is
+  // inside the row pitch: its values are computed from zeros and stored
+  const bool own = live && q < nq && r >= spr.own_lo && r < spr.own_hi;
+  const int kq0 = sbp_kind(q, nq), kq1 = q + 1 < nq ? sbp_kind(q + 1, nq) : 0, kr = sbp_kind(r, nr);
   // points whose DF the pre-kernels have set on a stage with A = 0: the
   // block's faces and the PML slabs (here the q and r sides, true for the
   // whole column)
   const int npml = a.pml_pre ? a.npml : 0;
-  const bool fold_qr = q == 0 || q == nq - 1 || r == 0 || r == nr - 1 || (a.pml[0] && q < npml) ||
-                       (a.pml[1] && q >= nq - npml) || (a.pml[2] && r < npml) || (a.pml[3] && r >= nr - npml);
+  const bool fold_r = r == 0 || r == nr - 1 || (a.pml[2] && r < npml) || (a.pml[3] && r >= nr - npml);
+  auto fold_q = [&](int i) {
+    return i == 0 || i == nq - 1 || (a.pml[0] && i < npml) || (a.pml[1] && i >= nq - npml);
+  };
+  const bool fold0 = fold_r || fold_q(q), fold1 = fold_r || fold_q(q + 1);
   const long long np = a.np;
   const long long sts = (long long)a.pq * nr;
   const long long col = q + (long long)a.pq * r;
-  const int lq = tx + 8, lr = ty + HR;
+  const int lq = tx + 8, lr = ty + HR, li = ty * TQ + tx;
   const float c1 = float(kC1), c2 = float(kC2), c3 = float(kC3);
   const float cf[7] = WQL_UP_CF;
+  auto g2 = [](const float* p) { return *reinterpret_cast<const f2*>(p); };
 
   // s window: velocities of planes s-3..s+3 and the s-face flux of the same
   // planes (central operator), or velocities of s-2..s+4 and fluxes of
   // s-4..s+2 (upwind pair: the planes D+ and D- read)
-  float qv[7][6];
+  f2 qv[7][6];
   // the window's first six entries straight from global memory, all loads
   // in flight at once; planes outside the block stay zero (only central
   // rows read the window)
 #pragma unroll
   for (int i = 0; i < 7; ++i) {
 #pragma unroll
-    for (int c = 0; c < 6; ++c) qv[i][c] = 0.0f;
+    for (int c = 0; c < 6; ++c) qv[i][c] = 0;
     const int plv = s_begin + (FD ? -2 : -3) + i, pl = s_begin + (FD ? -4 : -3) + i;
     const float* F = a.Fin;
     if (i < 6 && plv >= 0 && plv < ns && q < nq && r < nr) {
       const long long pp = col + sts * plv;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) qv[i][c] = F[c * np + pp];
+      for (int c = 0; c < 3; ++c) qv[i][c] = g2(F + c * np + pp);
     }
     if (i < 6 && pl >= 0 && pl < ns && q < nq && r < nr) {
       const long long pp = col + sts * pl;
       if (CURV) {
-        const float a0 = a.coef[6 * np + pp], a1 = a.coef[7 * np + pp], a2 = a.coef[8 * np + pp];
+        const f2 a0 = g2(a.coef + 6 * np + pp), a1 = g2(a.coef + 7 * np + pp), a2 = g2(a.coef + 8 * np + pp);
+        f2 sg[6];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-          qv[i][3 + c] = a0 * F[sig(c, 0) * np + pp] + a1 * F[sig(c, 1) * np + pp] + a2 * F[sig(c, 2) * np + pp];
+        for (int c = 0; c < 6; ++c) sg[c] = g2(F + (3 + c) * np + pp);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) qv[i][3 + c] = dot3(a0, sg[sig(c, 0) - 3], a1, sg[sig(c, 1) - 3], a2, sg[sig(c, 2) - 3]);
       } else {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) qv[i][3 + c] = F[sig(c, 2) * np + pp];
+        for (int c = 0; c < 3; ++c) qv[i][3 + c] = g2(F + sig(c, 2) * np + pp);
       }
     }
   }
@@ -336,28 +393,26 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
     const int T = tb + t;
     const int st = T % NS;
     const int s = s_begin + t;  // output plane
-    const bool work = own;
     const int ks = sbp_kind(s, ns);
     const long long p = col + sts * s;
     if (!mbar_wait(&full[st], (T / NS) & 1)) {
       atomicExch(a.err, 2);
       return false;
     }
-    const float* S = sm + st * TL::STAGE_W;
+    float* S = sm + st * TL::STAGE_W;
     // push the lead plane(s) into the s window
     {
       const float* LF = S + TL::OFF_LF;
-      const int li = ty * TQ + tx;
-      float f[9];
+      f2 f[9];
 #pragma unroll
-      for (int c = 0; c < 9; ++c) f[c] = LF[c * NC + li];
+      for (int c = 0; c < 9; ++c) f[c] = g2(LF + c * NC + li);
 #pragma unroll
       for (int c = 0; c < 3; ++c) qv[6][c] = f[c];
       if (CURV) {
         const float* LC = S + TL::OFF_LC;
-        const float a0 = LC[li], a1 = LC[NC + li], a2 = LC[2 * NC + li];
+        const f2 a0 = g2(LC + li), a1 = g2(LC + NC + li), a2 = g2(LC + 2 * NC + li);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) qv[6][3 + c] = a0 * f[sig(c, 0)] + a1 * f[sig(c, 1)] + a2 * f[sig(c, 2)];
+        for (int c = 0; c < 3; ++c) qv[6][3 + c] = dot3(a0, f[sig(c, 0)], a1, f[sig(c, 1)], a2, f[sig(c, 2)]);
       } else {
 #pragma unroll
         for (int c = 0; c < 3; ++c) qv[6][3 + c] = f[sig(c, 2)];
@@ -369,39 +424,49 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
     // coefficients they come from (CA becomes the q flux on the q-extended
     // rows, CB the r flux on the r-extended columns); each position is
     // handled by one thread, which reads its coefficients first
-    float* FB = const_cast<float*>(S) + TL::OFF_F;
-    float* CA = const_cast<float*>(S) + TL::OFF_CA;
-    float* CB = const_cast<float*>(S) + TL::OFF_CB;
+    float* FB = S + TL::OFF_F;
+    float* CA = S + TL::OFF_CA;
+    float* CB = S + TL::OFF_CB;
     const float* CC = S + TL::OFF_CC;
-    auto fb = [&](int c, int rr, int qq) -> float { return FB[(c * BR + rr) * BQ + qq]; };
-    float mq[3] = {0.0f, 0.0f, 0.0f}, mr[3] = {0.0f, 0.0f, 0.0f};  // own J*metric_q, J*metric_r
+    auto fb2 = [&](int c, int rr, int qq) -> f2 { return g2(FB + (c * BR + rr) * BQ + qq); };
+    f2 mq[3], mr[3];  // own J*metric_q, J*metric_r
     if (CURV) {
-      auto qflux = [&](int row, int l, float m[3]) {
-        float sg[6];
+      // x: the first coefficient of the position, xs: words from one to the
+      // next; (rr, qq): the position in the field box
+      auto flux = [&](float* x, int xs, const f2 (&sg)[6], f2 (&m)[3]) {
 #pragma unroll
-        for (int c = 0; c < 6; ++c) sg[c] = fb(3 + c, row + HR, l);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) m[j] = CA[(j * TR + row) * BQ + l];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          CA[(c * TR + row) * BQ + l] = m[0] * sg[sig(c, 0) - 3] + m[1] * sg[sig(c, 1) - 3] + m[2] * sg[sig(c, 2) - 3];
-      };
-      auto rflux = [&](int l, int col_, float m[3]) {
-        float sg[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) sg[c] = fb(3 + c, l, col_ + 8);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) m[j] = CB[(j * BR + l) * TQ + col_];
+        for (int j = 0; j < 3; ++j) m[j] = g2(x + j * xs);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-          CB[(c * BR + l) * TQ + col_] = m[0] * sg[sig(c, 0) - 3] + m[1] * sg[sig(c, 1) - 3] + m[2] * sg[sig(c, 2) - 3];
+          *reinterpret_cast<f2*>(x + c * xs) =
+              dot3(m[0], sg[sig(c, 0) - 3], m[1], sg[sig(c, 1) - 3], m[2], sg[sig(c, 2) - 3]);
       };
-      qflux(ty, lq, mq);
-      rflux(lr, tx, mr);
-      float tmp[3];
-      if (tx < 16) qflux(ty, tx < 8 ? tx : tx + TQ, tmp);     // q halo: 8 columns each side
-      if (ty < 2 * HR) rflux(ty < HR ? ty : ty + TR, tx, tmp);  // r halo: HR rows each side
-      // a warp forms every q flux of its own row (the q derivative needs
+      f2 sg[6];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) sg[c] = fb2(3 + c, lr, lq);
+      flux(CA + ty * BQ + lq, TR * BQ, sg, mq);
+      flux(CB + lr * TQ + tx, BR * TQ, sg, mr);
+      // the halos: lanes 0..15 take the q halo of the warp's own two rows (4
+      // pairs each side), lanes 16..31 of all warps together the r halo (HR
+      // rows each side, TQ/2 pairs each)
+      const int lane = tid & 31, warp = tid >> 5;
+      constexpr int kRHalo = 2 * HR * (TQ / 2), kRPass = NT / 2;
+#pragma unroll
+      for (int e0 = 0; e0 < kRHalo; e0 += kRPass) {
+        const bool isq = lane < 16;
+        const int e = e0 + warp * 16 + (lane - 16);
+        if (isq ? e0 == 0 : e < kRHalo) {
+          const int h = lane & 7, rw = e / (TQ / 2);
+          const int row = isq ? 2 * warp + (lane >> 3) : (rw < HR ? rw : rw + TR);
+          const int qq = isq ? (h < 4 ? 2 * h : TQ + 2 * h) : 2 * (e % (TQ / 2)) + 8;
+          const int rr = isq ? row + HR : row;
+          f2 m[3];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) sg[c] = fb2(3 + c, rr, qq);
+          flux(isq ? CA + row * BQ + qq : CB + row * TQ + (qq - 8), isq ? TR * BQ : BR * TQ, sg, m);
+        }
+      }
+      // a warp forms every q flux of its own rows (the q derivative needs
       // only those: warp sync); the r fluxes of other rows come from other
       // warps: every consumer thread arrives here and waits (bounded) just
       // before the r derivative, so the q and s derivatives overlap the wait
@@ -409,22 +474,9 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
       mbar_arrive(fluxbar);
     }
 
-    if (work) {
-      // differenced quantities along q at box column l (row lr) and along r at box row l (column lq)
-      auto qvals = [&](int l, float o[6]) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) o[c] = fb(c, lr, l);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) o[3 + c] = CURV ? CA[(c * TR + ty) * BQ + l] : fb(sig(c, 0), lr, l);
-      };
-      auto rvals = [&](int l, float o[6]) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) o[c] = fb(c, l, lq);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) o[3 + c] = CURV ? CB[(c * BR + l) * TQ + tx] : fb(sig(c, 1), l, lq);
-      };
-      float g[3][3], dv[3];
-      const float Jinv = CURV ? CC[3 * NC + ty * TQ + tx] : 1.0f;
+    if (own) {
+      f2 g[3][3], dv[3];
+      const f2 Jinv = CURV ? g2(CC + 3 * NC + li) : 0;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const int d = k == 0 ? 0 : (k == 1 ? 2 : 1);  // q, s, then r
@@ -432,106 +484,170 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
           atomicExch(a.err, 3);
           return false;
         }
-        float o[6];
-        if (d == 2) {
+        f2 o[6];
+        if (d == 0) {
+          // the quantities along the row: box columns lq-4 .. lq+5 as five
+          // aligned pairs serve both points
+          auto row = [&](int c) -> const float* {
+            return c < 3 ? FB + (c * BR + lr) * BQ : (CURV ? CA + ((c - 3) * TR + ty) * BQ : FB + (sig(c - 3, 0) * BR + lr) * BQ);
+          };
+          if (kq0 == 0 || kq1 == 0) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+              const float* x = row(c) + lq;
+              const f2 m4 = g2(x - 4), m2 = g2(x - 2), z = g2(x), p2 = g2(x + 2), p4 = g2(x + 4);
+              float x0, x1, a1, a2, a3, a4, b2, b3, b4, b5;  // a_k at -k, b_k at +k
+              unpack(z, x0, x1);
+              unpack(m2, a2, a1);
+              unpack(m4, a4, a3);
+              unpack(p2, b2, b3);
+              unpack(p4, b4, b5);
+              if (FD) {
+                // offsets -2..4 of D+ (velocities), -4..2 of D- (fluxes)
+                f2 u;
+                if (c < 3) {
+                  u = mul2(pack(cf[0], cf[0]), m2);
+                  u = fma2(pack(cf[2], cf[2]), z, u);
+                  u = fma2(pack(cf[4], cf[4]), p2, u);
+                  u = fma2(pack(cf[6], cf[6]), p4, u);
+                  float u0, u1;
+                  unpack(u, u0, u1);
+                  u0 += cf[1] * a1 + cf[3] * x1 + cf[5] * b3;
+                  u1 += cf[1] * x0 + cf[3] * b2 + cf[5] * b4;
+                  o[c] = pack(u0, u1);
+                } else {
+                  u = mul2(pack(-cf[0], -cf[0]), p2);
+                  u = fma2(pack(-cf[2], -cf[2]), z, u);
+                  u = fma2(pack(-cf[4], -cf[4]), m2, u);
+                  u = fma2(pack(-cf[6], -cf[6]), m4, u);
+                  float u0, u1;
+                  unpack(u, u0, u1);
+                  u0 -= cf[1] * x1 + cf[3] * a1 + cf[5] * a3;
+                  u1 -= cf[1] * b2 + cf[3] * x0 + cf[5] * a2;
+                  o[c] = pack(u0, u1);
+                }
+              } else {
+                float u0, u1;
+                unpack(mul2(pack(c2, c2), sub2(p2, m2)), u0, u1);
+                u0 += c1 * (x1 - a1) + c3 * (b3 - a3);
+                u1 += c1 * (b2 - x0) + c3 * (b4 - a2);
+                o[c] = pack(u0, u1);
+              }
+            }
+          }
+          if (kq0 != 0 || kq1 != 0) {
+            // one or both points on a closure row: both rows of a pair read
+            // the same columns (points 0.. or n-1..) with their own weights
+            const bool left = kq0 < 0;
+            constexpr int NCOL = FD ? 10 : 9;
+            const int r0_ = kq0 ? (left ? -kq0 : kq0) - 1 : 0, r1_ = kq1 ? (left ? -kq1 : kq1) - 1 : 0;
+            const float sg0 = kq0 ? (left ? 1.0f : -1.0f) : 0.0f, sg1 = kq1 ? (left ? 1.0f : -1.0f) : 0.0f;
+            // the upwind pair's right rows swap its two tables
+            const float* wv = tab + (FD && !left ? 60 : 0);
+            const float* wf = FD ? tab + (left ? 60 : 0) : wv;
+            const int l0 = (left ? 0 : nq - 1) - q0 + 8, dl = left ? 1 : -1;
+            float u0[6], u1[6];
+#pragma unroll
+            for (int c = 0; c < 6; ++c) u0[c] = u1[c] = 0.0f;
+#pragma unroll 1
+            for (int e = 0; e < NCOL; ++e) {
+              const float v0 = sg0 * wv[r0_ * NCOL + e], v1 = sg1 * wv[r1_ * NCOL + e];
+              const float f0 = FD ? sg0 * wf[r0_ * NCOL + e] : v0, f1 = FD ? sg1 * wf[r1_ * NCOL + e] : v1;
+              const int l = l0 + e * dl;
+#pragma unroll
+              for (int c = 0; c < 6; ++c) {
+                const float x = row(c)[l];
+                u0[c] += (c < 3 ? v0 : f0) * x;
+                u1[c] += (c < 3 ? v1 : f1) * x;
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+              float i0 = 0.0f, i1 = 0.0f;
+              if (kq0 == 0 || kq1 == 0) unpack(o[c], i0, i1);
+              o[c] = pack(kq0 ? u0[c] : i0, kq1 ? u1[c] : i1);
+            }
+          }
+        } else if (d == 2) {
           if (ks == 0 && FD) {
 #pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = 0.0f;
+            for (int c = 0; c < 6; ++c) o[c] = 0;
 #pragma unroll
             for (int i = 0; i < 7; ++i) {
 #pragma unroll
-              for (int c = 0; c < 3; ++c) o[c] += cf[i] * qv[i][c];
+              for (int c = 0; c < 3; ++c) o[c] = fma2(pack(cf[i], cf[i]), qv[i][c], o[c]);
 #pragma unroll
-              for (int c = 3; c < 6; ++c) o[c] -= cf[6 - i] * qv[i][c];
+              for (int c = 3; c < 6; ++c) o[c] = fma2(pack(-cf[6 - i], -cf[6 - i]), qv[i][c], o[c]);
             }
           } else if (ks == 0) {
 #pragma unroll
             for (int c = 0; c < 6; ++c)
-              o[c] = c1 * (qv[4][c] - qv[2][c]) + c2 * (qv[5][c] - qv[1][c]) + c3 * (qv[6][c] - qv[0][c]);
+              o[c] = fma2(pack(c1, c1), sub2(qv[4][c], qv[2][c]),
+                          fma2(pack(c2, c2), sub2(qv[5][c], qv[1][c]), mul2(pack(c3, c3), sub2(qv[6][c], qv[0][c]))));
           } else {
-            float os[6];
+            f2 os[6];
             s_closure<CURV, FD>(a, p, ks, qv, os);
 #pragma unroll
             for (int c = 0; c < 6; ++c) o[c] = os[c];
           }
         } else {
-          const int kind = d == 0 ? kq : kr;
-          const int l0 = d == 0 ? lq : lr;
-          if (kind == 0 && FD) {
+          auto rvals = [&](int l, int c) -> f2 {
+            return c < 3 ? fb2(c, l, lq) : (CURV ? g2(CB + ((c - 3) * BR + l) * TQ + tx) : fb2(sig(c - 3, 1), l, lq));
+          };
+          if (kr == 0 && FD) {
 #pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = 0.0f;
+            for (int c = 0; c < 6; ++c) o[c] = 0;
 #pragma unroll
             for (int of = -4; of <= 4; ++of) {
-              float x[6];
-              if (d == 0) qvals(l0 + of, x);
-              else rvals(l0 + of, x);
               if (of >= -2)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) o[c] += cf[of + 2] * x[c];
+                for (int c = 0; c < 3; ++c) o[c] = fma2(pack(cf[of + 2], cf[of + 2]), rvals(lr + of, c), o[c]);
               if (of <= 2)
 #pragma unroll
-                for (int c = 3; c < 6; ++c) o[c] -= cf[2 - of] * x[c];
+                for (int c = 3; c < 6; ++c) o[c] = fma2(pack(-cf[2 - of], -cf[2 - of]), rvals(lr + of, c), o[c]);
             }
-          } else if (kind == 0) {
-            float xp[6], xm[6];
+          } else if (kr == 0) {
 #pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = 0.0f;
-#pragma unroll
-            for (int k = 1; k <= 3; ++k) {
-              if (d == 0) {
-                qvals(l0 + k, xp);
-                qvals(l0 - k, xm);
-              } else {
-                rvals(l0 + k, xp);
-                rvals(l0 - k, xm);
-              }
-              const float ck = k == 1 ? c1 : (k == 2 ? c2 : c3);
-#pragma unroll
-              for (int c = 0; c < 6; ++c) o[c] += ck * (xp[c] - xm[c]);
-            }
+            for (int c = 0; c < 6; ++c)
+              o[c] = fma2(pack(c1, c1), sub2(rvals(lr + 1, c), rvals(lr - 1, c)),
+                          fma2(pack(c2, c2), sub2(rvals(lr + 2, c), rvals(lr - 2, c)),
+                               mul2(pack(c3, c3), sub2(rvals(lr + 3, c), rvals(lr - 3, c)))));
           } else {
 #pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = 0.0f;
+            for (int c = 0; c < 6; ++c) o[c] = 0;
+            const bool left = kr < 0;
+            constexpr int NCOL = FD ? 10 : 9;
+            const int rw = (left ? -kr : kr) - 1;
+            const float sgn = left ? 1.0f : -1.0f;
+            const float* wv = tab + (FD && !left ? 60 : 0) + rw * NCOL;
+            const float* wf = FD ? tab + (left ? 60 : 0) + rw * NCOL : wv;
+            const int l0 = lr + (left ? -rw : rw), dl = left ? 1 : -1;
 #pragma unroll 1
-            for (int e = 0; e < (FD ? 10 : 9); ++e) {
-              float w, wf;
-              int off;
-              if (FD) {
-                up_entry<float>(kind, e, w, wf, off);
-              } else {
-                row_entry<float>(kind, e, w, off);
-                wf = w;
-              }
-              float x[6];
-              if (d == 0) qvals(l0 + off, x);
-              else rvals(l0 + off, x);
+            for (int e = 0; e < NCOL; ++e) {
+              const float v = sgn * wv[e], f = FD ? sgn * wf[e] : v;
 #pragma unroll
-              for (int c = 0; c < 3; ++c) o[c] += w * x[c];
-#pragma unroll
-              for (int c = 3; c < 6; ++c) o[c] += wf * x[c];
+              for (int c = 0; c < 6; ++c) o[c] = fma2(c < 3 ? pack(v, v) : pack(f, f), rvals(l0 + e * dl, c), o[c]);
             }
           }
         }
         const float rh = a.rh[d];
         if (CURV) {
-          float mt[3];
+          const f2 Jr = mul2(Jinv, pack(rh, rh));
+          f2 mt[3];
 #pragma unroll
-          for (int jj = 0; jj < 3; ++jj) {
-            const float cj = d == 0 ? mq[jj] : (d == 1 ? mr[jj] : CC[jj * NC + ty * TQ + tx]);
-            mt[jj] = cj * Jinv;
-          }
+          for (int jj = 0; jj < 3; ++jj) mt[jj] = mul2(d == 0 ? mq[jj] : (d == 1 ? mr[jj] : g2(CC + jj * NC + li)), Jr);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            dv[c] = k == 0 ? rh * o[3 + c] : dv[c] + rh * o[3 + c];
+            dv[c] = k == 0 ? mul2(pack(rh, rh), o[3 + c]) : fma2(pack(rh, rh), o[3 + c], dv[c]);
 #pragma unroll
-            for (int jj = 0; jj < 3; ++jj) g[c][jj] = k == 0 ? mt[jj] * (rh * o[c]) : g[c][jj] + mt[jj] * (rh * o[c]);
+            for (int jj = 0; jj < 3; ++jj) g[c][jj] = k == 0 ? mul2(mt[jj], o[c]) : fma2(mt[jj], o[c], g[c][jj]);
           }
         } else {
           const float sc = a.cart_metric[d] * rh;
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            dv[c] = k == 0 ? sc * o[3 + c] : dv[c] + sc * o[3 + c];
-            g[c][d] = sc * o[c];
+            dv[c] = k == 0 ? mul2(pack(sc, sc), o[3 + c]) : fma2(pack(sc, sc), o[3 + c], dv[c]);
+            g[c][d] = mul2(pack(sc, sc), o[c]);
           }
         }
       }
@@ -539,42 +655,49 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
-          for (int jj = 0; jj < 3; ++jj) a.G[(c * 3 + jj) * np + p] = g[c][jj];
+          for (int jj = 0; jj < 3; ++jj) *reinterpret_cast<f2*>(a.G + (c * 3 + jj) * np + p) = g[c][jj];
       }
-      const int ci = ty * TQ + tx;
-      const float lam = CURV ? CC[4 * NC + ci] : CC[0 * NC + ci];
-      const float mu = CURV ? CC[5 * NC + ci] : CC[1 * NC + ci];
-      const float rinv = CURV ? CC[6 * NC + ci] : CC[2 * NC + ci];
-      const float l2m = lam + 2.0f * mu;
-      float du[9];
-      du[0] = rinv * dv[0];
-      du[1] = rinv * dv[1];
-      du[2] = rinv * dv[2];
-      du[3] = l2m * g[0][0] + lam * (g[1][1] + g[2][2]);
-      du[4] = l2m * g[1][1] + lam * (g[0][0] + g[2][2]);
-      du[5] = l2m * g[2][2] + lam * (g[0][0] + g[1][1]);
-      du[6] = mu * (g[0][1] + g[1][0]);
-      du[7] = mu * (g[0][2] + g[2][0]);
-      du[8] = mu * (g[1][2] + g[2][1]);
+      const f2 lam = g2(CC + (CURV ? 4 : 0) * NC + li);
+      const f2 mu = g2(CC + (CURV ? 5 : 1) * NC + li);
+      const f2 rinv = g2(CC + (CURV ? 6 : 2) * NC + li);
+      const f2 l2m = fma2(pack(2.0f, 2.0f), mu, lam);
+      f2 du[9];
+      du[0] = mul2(rinv, dv[0]);
+      du[1] = mul2(rinv, dv[1]);
+      du[2] = mul2(rinv, dv[2]);
+      du[3] = fma2(l2m, g[0][0], mul2(lam, add2(g[1][1], g[2][2])));
+      du[4] = fma2(l2m, g[1][1], mul2(lam, add2(g[0][0], g[2][2])));
+      du[5] = fma2(l2m, g[2][2], mul2(lam, add2(g[0][0], g[1][1])));
+      du[6] = mul2(mu, add2(g[0][1], g[1][0]));
+      du[7] = mul2(mu, add2(g[0][2], g[2][0]));
+      du[8] = mul2(mu, add2(g[1][2], g[2][1]));
       // the pre-kernels have folded the boundary and fault penalties and the
       // PML damping into DF of their points: DF + term/A, or the term itself
       // on the first stage (A = 0, where DF holds nothing else)
-      const bool fold = fold_qr || s == 0 || s == ns - 1 || (a.pml[4] && s < npml) || (a.pml[5] && s >= ns - npml);
+      const bool fold_s = s == 0 || s == ns - 1 || (a.pml[4] && s < npml) || (a.pml[5] && s >= ns - npml);
+      const comp_t* CKs = reinterpret_cast<const comp_t*>(S + TL::OFF_CK);
+      const f2 A2 = pack(a.A, a.A), B2 = pack(a.Bdt, a.Bdt);
 #pragma unroll
       for (int c = 0; c < 9; ++c) {
-        const float f0 = fb(c, lr, lq);
-        const float dfs = S[TL::OFF_DF + c * NC + ty * TQ + tx];
-        const float df = a.A != 0.0f ? a.A * dfs + du[c] : (fold ? dfs : 0.0f) + du[c];
-        a.DF[c * np + p] = df;
-        if (KAHAN) {
-          const comp_t* CKs = reinterpret_cast<const comp_t*>(S + TL::OFF_CK);
-          const float y = a.Bdt * df - comp_get(CKs, c * NC + ty * TQ + tx);
-          const float tt = f0 + y;
-          comp_put(a.C, c * np + p, (tt - f0) - y);
-          a.Fout[c * np + p] = tt;
+        const f2 f0 = fb2(c, lr, lq);
+        const f2 dfs = g2(S + TL::OFF_DF + c * NC + li);
+        f2 df;
+        if (a.A != 0.0f) {
+          df = fma2(A2, dfs, du[c]);
         } else {
-          a.Fout[c * np + p] = f0 + a.Bdt * df;
+          float d0, d1;
+          unpack(dfs, d0, d1);
+          df = add2(pack(fold_s || fold0 ? d0 : 0.0f, fold_s || fold1 ? d1 : 0.0f), du[c]);
         }
+        *reinterpret_cast<f2*>(a.DF + c * np + p) = df;
+        // -C of the pair: two bfloat16 (low half the even point), widened
+        const unsigned ck = *reinterpret_cast<const unsigned*>(CKs + c * NC + li) ^ 0x80008000u;
+        const f2 y = fma2(B2, df, pack(__uint_as_float(ck << 16), __uint_as_float(ck & 0xffff0000u)));
+        const f2 tt = add2(f0, y);
+        float e0, e1;
+        unpack(sub2(sub2(tt, f0), y), e0, e1);
+        *reinterpret_cast<unsigned*>(a.C + c * np + p) = bf16_pair(e0, e1);
+        *reinterpret_cast<f2*>(a.Fout + c * np + p) = tt;
       }
     } else if (CURV && !mbar_wait(fluxbar, T & 1)) {  // the same phase for threads without a point
       atomicExch(a.err, 3);
@@ -595,27 +718,36 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
 }
 
 // Shared-memory ring of a persistent CTA: NS stages then the mbarriers.
-template <bool CURV, bool KAHAN, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
 struct Ring {
   float* sm;
   uint64_t *full, *empty, *fluxbar;
+  float* tab;  // closure weights
   __device__ Ring() {
-    using TL = TmaTile<CURV, KAHAN, FD, TQW>;
+    using TL = TmaTile<CURV, FD, TQW>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     sm = reinterpret_cast<float*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
     full = reinterpret_cast<uint64_t*>(sm + NS * TL::STAGE_W);
     empty = full + NS;
     fluxbar = empty + NS;
+    tab = reinterpret_cast<float*>(fluxbar + 1);
   }
   // one thread initialises the barriers once per CTA
   __device__ void init() {
-    using TL = TmaTile<CURV, KAHAN, FD, TQW>;
+    using TL = TmaTile<CURV, FD, TQW>;
+    // the closure weights: the q rows differ from lane to lane, which
+    // constant memory would serve one row at a time
+    if (FD) {
+      if (threadIdx.x < 120) tab[threadIdx.x] = (&c_up_f[0][0][0])[threadIdx.x];
+    } else if (threadIdx.x < 54) {
+      tab[threadIdx.x] = (&c_sbp_f[0][0])[threadIdx.x];
+    }
     if (threadIdx.x == 0) {
       for (int i = 0; i < NS; ++i) {
         mbar_init(&full[i], 1);
-        mbar_init(&empty[i], TL::NC / 32);
+        mbar_init(&empty[i], TL::NT / 32);
       }
-      mbar_init(fluxbar, TL::NC);
+      mbar_init(fluxbar, TL::NT);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -623,7 +755,7 @@ struct Ring {
   // the producer's copies of the last stages land before the CTA leaves
   // (tb = stages issued)
   __device__ void drain(int tb) {
-    if (threadIdx.x == TmaTile<CURV, KAHAN, FD, TQW>::NC)
+    if (threadIdx.x == TmaTile<CURV, FD, TQW>::NT)
       for (int T = max(0, tb - NS); T < tb; ++T) mbar_wait(&full[T % NS], (T / NS) & 1);
   }
 };
@@ -631,28 +763,28 @@ struct Ring {
 // Each CTA takes tiles w = blockIdx.x, blockIdx.x + gridDim.x, ... of the
 // tq x tr x nchunk tiles of the block (q fastest, so neighbouring CTAs share
 // halos in L2); with one CTA per tile that is one tile each.
-template <bool CURV, bool KAHAN, int NS, int FD, int TQW>
-__global__ void __launch_bounds__(TQW * kTmaTR + 32, 1)
+template <bool CURV, int NS, int FD, int TQW>
+__global__ void __launch_bounds__(TmaTile<CURV, FD, TQW>::NT + 32, 1)
     stencil_kernel_tma(const __grid_constant__ VolumeArgs<float> a, const __grid_constant__ MapArgs m, int schunk,
                        int tq, int tr, int ntile) {
-  Ring<CURV, KAHAN, NS, FD, TQW> ring;
+  Ring<CURV, NS, FD, TQW> ring;
   ring.init();
   int tb = 0;
   for (int w = blockIdx.x; w < ntile; w += gridDim.x)
-    if (!tma_body<CURV, KAHAN, NS, FD, TQW>(a, m, schunk, w % tq, (w / tq) % tr, w / (tq * tr), tb)) break;
+    if (!tma_body<CURV, NS, FD, TQW>(a, m, schunk, w % tq, (w / tq) % tr, w / (tq * tr), ring.tab, tb)) break;
   ring.drain(tb);
 }
 
 // One launch over many blocks (of one or many scenarios): CTA i works on the
 // descriptor whose CTA range holds i, found by binary search in the packed
 // table (descriptors sorted by cta0).
-template <bool CURV, bool KAHAN, int NS>
-__global__ void __launch_bounds__(kTmaTQ * kTmaTR + 32, 1)
+template <bool CURV, int NS>
+__global__ void __launch_bounds__(TmaTile<CURV, 0>::NT + 32, 1)
     stencil_kernel_tma_batch(const TmaBatchDesc* __restrict__ d, int nd, long long total) {
   // the entry's arguments are copied to shared memory: read from there they
   // cost no registers across the plane loop (held in registers they spill)
   __shared__ VolumeArgs<float> sa;
-  Ring<CURV, KAHAN, NS, 0> ring;
+  Ring<CURV, NS, 0> ring;
   const long long cta = blockIdx.x;
   int lo = 0, hi = nd - 1;
   while (lo < hi) {
@@ -668,14 +800,14 @@ __global__ void __launch_bounds__(kTmaTQ * kTmaTR + 32, 1)
   }
   // the table was written by a host copy: order that write before the
   // tensor-map proxy reads the entry's maps (in the thread that issues copies)
-  if (threadIdx.x == kTmaTQ * kTmaTR)
+  if (threadIdx.x == TmaTile<CURV, 0>::NT)
     for (int i = 0; i < 9; ++i)
       asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(&D.m[i]) : "memory");
   ring.init();  // its barrier also publishes sa
   int tb = 0;
   const long long l = cta - D.cta0;
-  tma_body<CURV, KAHAN, NS, 0>(sa, *reinterpret_cast<const MapArgs*>(&D.m), D.schunk, (int)(l % D.tq),
-                            (int)((l / D.tq) % D.tr), (int)(l / ((long long)D.tq * D.tr)), tb);
+  tma_body<CURV, NS, 0>(sa, *reinterpret_cast<const MapArgs*>(&D.m), D.schunk, (int)(l % D.tq),
+                            (int)((l / D.tq) % D.tr), (int)(l / ((long long)D.tq * D.tr)), ring.tab, tb);
   ring.drain(tb);
 }
 
@@ -690,20 +822,20 @@ struct TwoBlocks {
   int ntile0;
 };
 
-template <bool CURV, bool KAHAN, int NS, int FD, int TQW>
-__global__ void __launch_bounds__(TQW * kTmaTR + 32, 1)
+template <bool CURV, int NS, int FD, int TQW>
+__global__ void __launch_bounds__(TmaTile<CURV, FD, TQW>::NT + 32, 1)
     stencil_kernel_tma2(const __grid_constant__ TwoBlocks P) {
-  Ring<CURV, KAHAN, NS, FD, TQW> ring;
+  Ring<CURV, NS, FD, TQW> ring;
   ring.init();
   int tb = 0;
   const int w = blockIdx.x;
   if (w < P.ntile0) {
-    tma_body<CURV, KAHAN, NS, FD, TQW>(P.a[0], P.m[0], P.schunk[0], w % P.tq[0], (w / P.tq[0]) % P.tr[0],
-                              w / (P.tq[0] * P.tr[0]), tb);
+    tma_body<CURV, NS, FD, TQW>(P.a[0], P.m[0], P.schunk[0], w % P.tq[0], (w / P.tq[0]) % P.tr[0],
+                              w / (P.tq[0] * P.tr[0]), ring.tab, tb);
   } else {
     const int l = w - P.ntile0;
-    tma_body<CURV, KAHAN, NS, FD, TQW>(P.a[1], P.m[1], P.schunk[1], l % P.tq[1], (l / P.tq[1]) % P.tr[1],
-                              l / (P.tq[1] * P.tr[1]), tb);
+    tma_body<CURV, NS, FD, TQW>(P.a[1], P.m[1], P.schunk[1], l % P.tq[1], (l / P.tq[1]) % P.tr[1],
+                              l / (P.tq[1] * P.tr[1]), ring.tab, tb);
   }
   ring.drain(tb);
 }
@@ -757,22 +889,22 @@ MapArgs stage_maps(const StencilMaps& sm) {
   return m;
 }
 
-template <bool CURV, bool KAHAN, int FD, int TQW = kTmaTQ>
+template <bool CURV, int FD, int TQW = kTmaTQ>
 constexpr size_t tma_smem_bytes(int NS) {
-  return sizeof(float) * (size_t)NS * TmaTile<CURV, KAHAN, FD, TQW>::STAGE_W + (2 * NS + 1) * sizeof(uint64_t) + 128;
+  return sizeof(float) * (size_t)NS * TmaTile<CURV, FD, TQW>::STAGE_W + (2 * NS + 1) * sizeof(uint64_t) + 120 * sizeof(float) + 128;
 }
-static_assert(tma_smem_bytes<true, true, 0>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<false, true, 0>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<true, true, 1>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<false, true, 1>(kTmaStages) <= 227 * 1024,
+static_assert(tma_smem_bytes<true, 0>(kTmaStages) <= 227 * 1024 &&
+                  tma_smem_bytes<false, 0>(kTmaStages) <= 227 * 1024 &&
+                  tma_smem_bytes<true, 1>(kTmaStages) <= 227 * 1024 &&
+                  tma_smem_bytes<false, 1>(kTmaStages) <= 227 * 1024,
               "the stage ring must fit in the shared memory of one CTA");
-static_assert(tma_smem_bytes<false, true, 0, kTmaTQWide>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<false, true, 1, kTmaTQWide>(kTmaStages) <= 227 * 1024,
+static_assert(tma_smem_bytes<false, 0, kTmaTQWide>(kTmaStages) <= 227 * 1024 &&
+                  tma_smem_bytes<false, 1, kTmaTQWide>(kTmaStages) <= 227 * 1024,
               "the wide Cartesian stage ring must fit in the shared memory of one CTA");
 
 template <typename K>
 size_t prepare(K kern, int NS, int stage_words) {
-  const size_t smem = sizeof(float) * (size_t)NS * stage_words + (2 * NS + 1) * sizeof(uint64_t) + 128;
+  const size_t smem = sizeof(float) * (size_t)NS * stage_words + (2 * NS + 1) * sizeof(uint64_t) + 120 * sizeof(float) + 128;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   return smem;
 }
@@ -782,21 +914,21 @@ size_t prepare(K kern, int NS, int stage_words) {
 // tiles statically interleaved that measured slower on 2 x 201^3 blocks
 // (0.54 ms against 0.50 ms per launch): the chunks holding the s closure
 // rows take longer, and the hardware's dynamic CTA scheduling balances them.
-template <bool CURV, bool KAHAN, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
 void launch_tma(const VolumeArgs<float>& a, const StencilMaps& sm, cudaStream_t s) {
-  using TL = TmaTile<CURV, KAHAN, FD, TQW>;
-  auto kern = stencil_kernel_tma<CURV, KAHAN, NS, FD, TQW>;
+  using TL = TmaTile<CURV, FD, TQW>;
+  auto kern = stencil_kernel_tma<CURV, NS, FD, TQW>;
   static const size_t smem = prepare(kern, NS, TL::STAGE_W);
   const int tq = (a.nq + TL::TQ - 1) / TL::TQ, tr = (a.nr + TL::TR - 1) / TL::TR;
   const int schunk = chunk_planes(a);
   const int ntile = tq * tr * ((a.ns + schunk - 1) / schunk);
-  kern<<<ntile, TL::NC + 32, smem, s>>>(a, stage_maps(sm), schunk, tq, tr, ntile);
+  kern<<<ntile, TL::NT + 32, smem, s>>>(a, stage_maps(sm), schunk, tq, tr, ntile);
 }
 
-template <bool CURV, bool KAHAN, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
 void launch_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, cudaStream_t s) {
-  using TL = TmaTile<CURV, KAHAN, FD, TQW>;
-  auto kern = stencil_kernel_tma2<CURV, KAHAN, NS, FD, TQW>;
+  using TL = TmaTile<CURV, FD, TQW>;
+  auto kern = stencil_kernel_tma2<CURV, NS, FD, TQW>;
   static const size_t smem = prepare(kern, NS, TL::STAGE_W);
   TwoBlocks P;
   const VolumeArgs<float>* a[2] = {&a0, &a1};
@@ -815,16 +947,16 @@ void launch_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, cudaS
     ntile[b] = tiles[b] * ((a[b]->ns + P.schunk[b] - 1) / P.schunk[b]);
   }
   P.ntile0 = ntile[0];
-  kern<<<ntile[0] + ntile[1], TL::NC + 32, smem, s>>>(P);
+  kern<<<ntile[0] + ntile[1], TL::NT + 32, smem, s>>>(P);
 }
 
-template <bool CURV, bool KAHAN, int NS>
+template <bool CURV, int NS>
 void launch_tma_batch(const TmaBatchDesc* d, int nd, long long total, cudaStream_t s) {
-  using TL = TmaTile<CURV, KAHAN, 0>;
-  auto kern = stencil_kernel_tma_batch<CURV, KAHAN, NS>;
+  using TL = TmaTile<CURV, 0>;
+  auto kern = stencil_kernel_tma_batch<CURV, NS>;
   static const size_t smem = prepare(kern, NS, TL::STAGE_W);
   if (total <= 0) return;
-  kern<<<(unsigned)total, TL::NC + 32, smem, s>>>(d, nd, total);
+  kern<<<(unsigned)total, TL::NT + 32, smem, s>>>(d, nd, total);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -926,49 +1058,39 @@ int tma_tile_width(int nq0, int nq1, bool curv) {
   return used(kTmaTQWide) > used(kTmaTQ) + 0.02 ? kTmaTQWide : kTmaTQ;
 }
 
-void launch_stencil_tma_batch(const TmaBatchDesc* d, int nd, long long total, bool curv, bool kahan, void* stream) {
+void launch_stencil_tma_batch(const TmaBatchDesc* d, int nd, long long total, bool curv, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  if (curv) kahan ? launch_tma_batch<true, true, kTmaStages>(d, nd, total, s)
-                  : launch_tma_batch<true, false, kTmaStages>(d, nd, total, s);
-  else kahan ? launch_tma_batch<false, true, kTmaStages>(d, nd, total, s)
-             : launch_tma_batch<false, false, kTmaStages>(d, nd, total, s);
+  if (curv) launch_tma_batch<true, kTmaStages>(d, nd, total, s);
+  else launch_tma_batch<false, kTmaStages>(d, nd, total, s);
 }
 
-// The upwind pair runs with the compensated update only (the FP32 mode
-// always carries C); stencil_is_tma sends an uncompensated upwind block to
-// the per-point kernel.
-void launch_stencil_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, bool curv, bool kahan,
-                         void* stream) {
+void launch_stencil_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, bool curv, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  if (!curv && kahan && static_cast<const StencilMaps*>(a0.tma)->tq == kTmaTQWide) {
-    if (a0.fd) launch_tma2<false, true, kTmaStages, 1, kTmaTQWide>(a0, a1, s);
-    else launch_tma2<false, true, kTmaStages, 0, kTmaTQWide>(a0, a1, s);
-    return;
+  if (!curv && static_cast<const StencilMaps*>(a0.tma)->tq == kTmaTQWide) {
+    if (a0.fd) launch_tma2<false, kTmaStages, 1, kTmaTQWide>(a0, a1, s);
+    else launch_tma2<false, kTmaStages, 0, kTmaTQWide>(a0, a1, s);
+  } else if (a0.fd) {
+    if (curv) launch_tma2<true, kTmaStages, 1>(a0, a1, s);
+    else launch_tma2<false, kTmaStages, 1>(a0, a1, s);
+  } else {
+    if (curv) launch_tma2<true, kTmaStages, 0>(a0, a1, s);
+    else launch_tma2<false, kTmaStages, 0>(a0, a1, s);
   }
-  if (a0.fd) {
-    if (curv) launch_tma2<true, true, kTmaStages, 1>(a0, a1, s);
-    else launch_tma2<false, true, kTmaStages, 1>(a0, a1, s);
-    return;
-  }
-  if (curv) kahan ? launch_tma2<true, true, kTmaStages, 0>(a0, a1, s) : launch_tma2<true, false, kTmaStages, 0>(a0, a1, s);
-  else kahan ? launch_tma2<false, true, kTmaStages, 0>(a0, a1, s) : launch_tma2<false, false, kTmaStages, 0>(a0, a1, s);
 }
 
-void launch_stencil_tma(const VolumeArgs<float>& a, bool curv, bool kahan, void* stream) {
+void launch_stencil_tma(const VolumeArgs<float>& a, bool curv, void* stream) {
   const StencilMaps& sm = *static_cast<const StencilMaps*>(a.tma);
   cudaStream_t s = (cudaStream_t)stream;
-  if (!curv && kahan && sm.tq == kTmaTQWide) {
-    if (a.fd) launch_tma<false, true, kTmaStages, 1, kTmaTQWide>(a, sm, s);
-    else launch_tma<false, true, kTmaStages, 0, kTmaTQWide>(a, sm, s);
-    return;
+  if (!curv && sm.tq == kTmaTQWide) {
+    if (a.fd) launch_tma<false, kTmaStages, 1, kTmaTQWide>(a, sm, s);
+    else launch_tma<false, kTmaStages, 0, kTmaTQWide>(a, sm, s);
+  } else if (a.fd) {
+    if (curv) launch_tma<true, kTmaStages, 1>(a, sm, s);
+    else launch_tma<false, kTmaStages, 1>(a, sm, s);
+  } else {
+    if (curv) launch_tma<true, kTmaStages, 0>(a, sm, s);
+    else launch_tma<false, kTmaStages, 0>(a, sm, s);
   }
-  if (a.fd) {
-    if (curv) launch_tma<true, true, kTmaStages, 1>(a, sm, s);
-    else launch_tma<false, true, kTmaStages, 1>(a, sm, s);
-    return;
-  }
-  if (curv) kahan ? launch_tma<true, true, kTmaStages, 0>(a, sm, s) : launch_tma<true, false, kTmaStages, 0>(a, sm, s);
-  else kahan ? launch_tma<false, true, kTmaStages, 0>(a, sm, s) : launch_tma<false, false, kTmaStages, 0>(a, sm, s);
 }
 
 }  // namespace wql

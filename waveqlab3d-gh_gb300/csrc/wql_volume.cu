@@ -1569,7 +1569,7 @@ template <typename T>
 int effective_variant(const VolumeArgs<T>& a) {
   constexpr bool f32 = sizeof(T) == 4;
   int v = a.kernel != 0 ? a.kernel : (f32 ? 5 : 2);
-  if ((v == 5 || v == 6) && !f32) v = 2;
+  if ((v == 5 || v == 6) && !(f32 && a.C != nullptr)) v = 2;
   if (a.fd) {
     // the order-6 upwind pair: the TMA kernel (compensated FP32) or per
     // point; order 5 per point
@@ -1608,8 +1608,8 @@ void launch_stencil(const VolumeArgs<T>& a, cudaStream_t s) {
     case 4: launch_tiled<T, CURV, KAHAN, 64, 8, 1>(a, s); return;
     case 5:
     case 6:
-      if constexpr (f32) {
-        launch_stencil_tma(a, CURV, KAHAN, s);
+      if constexpr (f32 && KAHAN) {
+        launch_stencil_tma(a, CURV, s);
         return;
       }
       [[fallthrough]];
