@@ -97,6 +97,7 @@ int preset_of(const std::string& pb) {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool ordered = false;  // stream-ordered allocation (set-up scratch)
 };
 
 }  // namespace
@@ -152,6 +153,7 @@ struct wql_scn {
     double cart_metric[3] = {1, 1, 1};
     double tau_h[3] = {};
     StencilMaps maps{};  // TMA tensor maps (FP32 fields)
+    StencilPlan64 plan64{};  // split of the FP64 stencil kernel
   } B[2];
   int cur = 0;
   // interface (two block copies)
@@ -247,19 +249,22 @@ struct wql_scn {
     if (pin_done) cudaEventDestroy(pin_done);
     for (auto e : ev_pool) cudaEventDestroy(e);
     for (auto& a : allocs)
-      if (a.p) cudaFree(a.p);
+      if (a.p) a.ordered ? cudaFreeAsync(a.p, stream) : cudaFree(a.p);
     if (stream) cudaStreamDestroy(stream);
   }
 
-  int alloc(void** p, size_t bytes, bool zero = true) {
+  // ordered: from the device's stream-ordered pool, for set-up scratch that is
+  // released again: cudaFree waits for all work on the device, so a scenario
+  // being created beside running ones would wait for them.
+  int alloc(void** p, size_t bytes, bool zero = true, bool ordered = false) {
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = ordered ? cudaMallocAsync(p, bytes, stream) : cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
       *p = nullptr;
       return fail(WQL_E_OOM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed: " +
                                  cudaGetErrorString(e));
     }
-    allocs.push_back({*p, bytes});
+    allocs.push_back({*p, bytes, ordered});
     device_bytes += (long long)bytes;
     if (zero) {
       e = cudaMemsetAsync(*p, 0, bytes, stream);
@@ -270,7 +275,7 @@ struct wql_scn {
   void release(void* p) {
     for (auto& a : allocs)
       if (a.p == p) {
-        cudaFree(a.p);
+        a.ordered ? cudaFreeAsync(a.p, stream) : cudaFree(a.p);
         device_bytes -= (long long)a.bytes;
         a.p = nullptr;
       }
@@ -464,16 +469,16 @@ int setup_block(wql_scn* S, int b) {
   // geometry on the device (FP64) for the one-time precompute
   double *x = nullptr, *metric = nullptr, *J = nullptr, *mat = nullptr;
   int rc;
-  if ((rc = S->alloc((void**)&x, 3 * np * sizeof(double), false))) return rc;
+  if ((rc = S->alloc((void**)&x, 3 * np * sizeof(double), false, true))) return rc;
   for (int c = 0; c < 3; ++c)
     CK(cudaMemcpyAsync(x + c * np, G.x[c].data(), np * sizeof(double), cudaMemcpyHostToDevice, S->stream));
-  if ((rc = S->alloc((void**)&metric, 9 * np * sizeof(double), false))) return rc;
-  if ((rc = S->alloc((void**)&J, np * sizeof(double), false))) return rc;
+  if ((rc = S->alloc((void**)&metric, 9 * np * sizeof(double), false, true))) return rc;
+  if ((rc = S->alloc((void**)&J, np * sizeof(double), false, true))) return rc;
   launch_metrics(B.nq, B.nr, B.ns, x, metric, J, S->stream);
   CK(cudaGetLastError());
   // material: caller arrays (the reference's file media, src/material.f90:706-747)
   // or homogeneous from rho_s_p (src/material.f90:180-187)
-  if ((rc = S->alloc((void**)&mat, 3 * np * sizeof(double), false))) return rc;
+  if ((rc = S->alloc((void**)&mat, 3 * np * sizeof(double), false, true))) return rc;
   const double* user[3] = {S->media.lam[b], S->media.mu[b], S->media.rho[b]};
   if (user[0] || user[1] || user[2]) {
     if (!(user[0] && user[1] && user[2])) return fail(WQL_E_INPUT, "lam, mu and rho must be given together");
@@ -558,6 +563,11 @@ int setup_block(wql_scn* S, int b) {
     const int erc = make_stencil_maps(B.maps, B.F, B.coef, B.DF, B.C, B.nq, B.nr, B.ns, B.pq, S->curv, S->fd,
                                       tma_tile_width(S->P.btp[0].nqrs[0], S->P.btp[1].nqrs[0], S->curv));
     if (erc) return fail(WQL_E_CUDA, "cuTensorMapEncodeTiled failed for the stencil maps (error " + std::to_string(erc) + ")");
+  }
+  if (S->prec == WQL_FP64 && !S->fd) {
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S->ctx->device));
+    B.plan64 = make_plan64(B.nq, B.nr, B.ns, sms);
   }
   // boundary codes (src/BoundaryConditions.f90:15-48) and PML slabs (src/block.f90:163-178)
   B.bc[0] = bp.lqrs[0]; B.bc[1] = bp.rqrs[0];
@@ -1127,9 +1137,7 @@ VolumeArgs<T> volume_args(wql_scn* S, int b, double A, double Bdt, bool last) {
   a.mms_Tp = (T)S->mms_Tp;
   B.maps.cur = S->cur;
   a.tma = &B.maps;
-  // the PML pre-kernel goes with the TMA stencil; it addresses a component
-  // with 32-bit byte offsets
-  a.pml_pre = B.npml > 0 && stencil_is_tma(a) && B.np < (1LL << 30) ? 1 : 0;
+  a.plan64 = &B.plan64;
   return a;
 }
 
@@ -1231,11 +1239,29 @@ void stage_head(wql_scn* S, StepCtx& c, int stage) {
   }
 }
 
-void stage_block_pre(wql_scn* S, StepCtx& c, int stage, int b) {
+template <typename T>
+void stage_pre(wql_scn* S, StepCtx& c, int stage) {
+  const VolumeArgs<T> a0 = volume_args<T>(S, 0, stage_A(S, stage), stage_Bdt(S, stage), stage == 5);
+  const VolumeArgs<T> a1 = volume_args<T>(S, 1, stage_A(S, stage), stage_Bdt(S, stage), stage == 5);
   mark_begin(S, 2);
-  if (S->prec == WQL_FP64) c.launches += launch_pre<double>(volume_args<double>(S, b, stage_A(S, stage), stage_Bdt(S, stage), stage == 5), S->curv, S->stream);
-  else c.launches += launch_pre<float>(volume_args<float>(S, b, stage_A(S, stage), stage_Bdt(S, stage), stage == 5), S->curv, S->stream);
+  c.launches += launch_pre<T>(a0, &a1, S->curv, S->stream);
   mark_end(S);
+}
+void stage_pre(wql_scn* S, StepCtx& c, int stage) {
+  if (S->prec == WQL_FP64) stage_pre<double>(S, c, stage);
+  else stage_pre<float>(S, c, stage);
+}
+
+// Both blocks' stencils in one launch; false where their variant has none.
+template <typename T>
+bool stage_pair_stencil(wql_scn* S, StepCtx& c, int stage) {
+  const VolumeArgs<T> a0 = volume_args<T>(S, 0, stage_A(S, stage), stage_Bdt(S, stage), stage == 5);
+  const VolumeArgs<T> a1 = volume_args<T>(S, 1, stage_A(S, stage), stage_Bdt(S, stage), stage == 5);
+  mark_begin(S, 1);
+  const int n = launch_volume2<T>(a0, a1, S->curv, S->stream);
+  mark_end(S);
+  c.launches += n;
+  return n > 0;
 }
 
 void stage_block_stencil(wql_scn* S, StepCtx& c, int stage, int b) {
@@ -1420,7 +1446,7 @@ int batch_step(wql_batch* B) {
     for (size_t i = 0; i < n; ++i) {
       wql_scn* S = B->members[i];
       stage_head(S, c[i], stage);
-      for (int b = 0; b < 2; ++b) stage_block_pre(S, c[i], stage, b);
+      stage_pre(S, c[i], stage);
     }
     // the packed stencil launches: one group per mesh kind
     for (int curv = 0; curv < 2; ++curv) {
@@ -1466,36 +1492,13 @@ int batch_step(wql_batch* B) {
 
 // One RK stage of the current step (stages 1..5 in order).
 void run_stage(wql_scn* S, StepCtx& c, int stage) {
-  bool pair = false;  // both blocks through the TMA kernel: one stencil launch per stage
-  if (S->prec == WQL_FP32C) {
-    pair = true;
-    for (int b = 0; b < 2; ++b) pair = pair && stencil_is_tma(volume_args<float>(S, b, 0.0, 0.0, false));
-  }
   stage_head(S, c, stage);
-  if (pair) {
-    // both blocks' pre-kernels, the stencil launch, both blocks'
-    // corrections (the blocks touch disjoint arrays)
-    const double A = stage_A(S, stage), Bdt = stage_Bdt(S, stage);
-    {
-      const VolumeArgs<float> a0 = volume_args<float>(S, 0, A, Bdt, stage == 5);
-      const VolumeArgs<float> a1 = volume_args<float>(S, 1, A, Bdt, stage == 5);
-      mark_begin(S, 2);
-      c.launches += launch_pre2<float>(a0, a1, S->curv, S->stream);
-      mark_end(S);
-    }
-    mark_begin(S, 1);
-    launch_stencil_tma2(volume_args<float>(S, 0, A, Bdt, stage == 5), volume_args<float>(S, 1, A, Bdt, stage == 5),
-                        S->curv, S->stream);
-    mark_end(S);
-    c.launches += 1;
-    for (int b = 0; b < 2; ++b) stage_block_post(S, c, stage, b);
-  } else {
-    for (int b = 0; b < 2; ++b) {
-      stage_block_pre(S, c, stage, b);
-      stage_block_stencil(S, c, stage, b);
-      stage_block_post(S, c, stage, b);
-    }
-  }
+  // the blocks touch disjoint arrays: both blocks' pre-kernels, both
+  // stencils, both blocks' corrections
+  stage_pre(S, c, stage);
+  if (!(S->prec == WQL_FP64 ? stage_pair_stencil<double>(S, c, stage) : stage_pair_stencil<float>(S, c, stage)))
+    for (int b = 0; b < 2; ++b) stage_block_stencil(S, c, stage, b);
+  for (int b = 0; b < 2; ++b) stage_block_post(S, c, stage, b);
   S->cur ^= 1;
 }
 
@@ -2001,6 +2004,7 @@ int wql_autotune(wql_scn* scn, int reps, int* variant, int* schunk) {
         if (wide) cand.push_back({6, c});
       }
   } else {
+    cand.push_back({0, 0});
     for (int c : {8, 16, 32}) cand.push_back({2, c});
     cand.push_back({1, 0});
   }

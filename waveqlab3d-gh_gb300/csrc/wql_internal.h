@@ -60,6 +60,13 @@ struct UpG {
 };
 constexpr int kUgCol = 13, kUgRows = 8, kUgRowBlock = 3 * kUgRows * kUgCol, kUgWords = 4 * kUgCol + 4 * kUgRowBlock;
 
+// The split of a block for the FP64 stencil kernel: kq x kr tiles over (q, r)
+// of at most tw x th points, chunks of `chunk` planes.
+struct StencilPlan64 {
+  int kq, kr, tw, th, chunk;
+  int ok;
+};
+
 template <typename T>
 struct VolumeArgs {
   int nq, nr, ns;
@@ -86,7 +93,6 @@ struct VolumeArgs {
   T* Q[6];
   T* DQ[6];
   long long slab_np[6];
-  int pml_pre;        // the slabs are advanced before the stencil (PML pre-kernel), not after it
   // velocity gradient g[c][j] (component c*3+j, stride np) with the anelastic
   // response, written by the TMA stencil kernel and read by the anelastic
   // kernel of the same stage; nullptr where that kernel forms it itself
@@ -124,6 +130,7 @@ struct VolumeArgs {
   int* err;                      // device error word (pipeline wait timeouts)
   double pml_d0;                 // PML damping scale 3 ln(1000)
   const void* tma;               // host pointer to the block's StencilMaps (FP32 only)
+  const StencilPlan64* plan64;   // host pointer to the block's split (FP64, central operator; else nullptr)
   // manufactured solution (&mms_list use_mms): u_exact = T(t) S(x), where S
   // is sin*sin*sin for the velocities (ms[0..np)) and cos*cos*cos for the
   // stresses (ms[np..2np)); the forcing is T(t) mp - T'(t) S with mp the
@@ -220,6 +227,12 @@ int tma_tile_width(int nq0, int nq1, bool curv);
 void launch_stencil_tma(const VolumeArgs<float>& a, bool curv, void* stream);
 // The same for both blocks of a scenario in one launch.
 void launch_stencil_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, bool curv, void* stream);
+// The FP64 stencil kernel of the central operator over one block (a1 null) or
+// both; make_plan64 splits a block for `sms` SMs (ok = 0: the kernel does not
+// take it).
+StencilPlan64 make_plan64(int nq, int nr, int ns, int sms);
+void launch_stencil_fp64(const VolumeArgs<double>& a0, const VolumeArgs<double>* a1, bool curv, void* stream);
+
 // Whether the block's stencil runs as the TMA kernel (the tuning and the
 // block shape allow it).
 template <typename T>
@@ -244,21 +257,19 @@ bool tma_eligible(const VolumeArgs<float>& a);
 // with or all without compensation).
 void launch_stencil_tma_batch(const TmaBatchDesc* d_dev, int nd, long long total_ctas, bool curv, void* stream);
 
-// One stage on one block: launch_volume runs the stencil kernel (DF and the
-// updated fields for every point); launch_corrections then adds the PML,
-// boundary/fault penalty and plastic kernels and returns how many it issued.
+// One stage: launch_pre folds the boundary and fault penalties into DF of the
+// face points, advances the PML slabs and folds their damping into DF, over
+// one block (a1 null) or a scenario's two; launch_volume runs the stencil
+// kernel of one block (DF and the updated fields for every point), and
+// launch_volume2 that of both blocks in one launch where the blocks' variant
+// has one; launch_corrections then adds the attenuation, the manufactured
+// forcing and the plastic map.  They return the number of launches.
+template <typename T>
+int launch_pre(const VolumeArgs<T>& a0, const VolumeArgs<T>* a1, bool curv, void* stream);
 template <typename T>
 void launch_volume(const VolumeArgs<T>& a, bool curv, void* stream);
-// Before the stencil kernel of a variant without its own face pass: the
-// boundary and fault penalties folded into DF of the face points, and the
-// PML slabs advanced with their damping folded into DF.  Returns the number
-// of launches.
 template <typename T>
-int launch_pre(const VolumeArgs<T>& a, bool curv, void* stream);
-// The same for both blocks of a scenario whose stencils both run as the TMA
-// kernel, in one launch each.
-template <typename T>
-int launch_pre2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, bool curv, void* stream);
+int launch_volume2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, bool curv, void* stream);
 template <typename T>
 int launch_corrections(const VolumeArgs<T>& a, bool curv, void* stream);
 // One moment-tensor source: DF(4:9) -= am * delta on a box of points

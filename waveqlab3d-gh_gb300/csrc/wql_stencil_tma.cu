@@ -341,7 +341,7 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
   // points whose DF the pre-kernels have set on a stage with A = 0: the
   // block's faces and the PML slabs (here the q and r sides, true for the
   // whole column)
-  const int npml = a.pml_pre ? a.npml : 0;
+  const int npml = a.npml;
   const bool fold_r = r == 0 || r == nr - 1 || (a.pml[2] && r < npml) || (a.pml[3] && r >= nr - npml);
   auto fold_q = [&](int i) {
     return i == 0 || i == nq - 1 || (a.pml[0] && i < npml) || (a.pml[1] && i >= nq - npml);

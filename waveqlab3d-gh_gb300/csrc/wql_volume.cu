@@ -1,6 +1,7 @@
 // Volume kernels: one RK stage of the elastic velocity-stress system on one
-// block.  The stencil kernel does the bulk per grid point; small correction
-// kernels add the PML, boundary/fault penalties and the plastic map:
+// block.  Pre-kernels fold the boundary/fault penalties and the PML damping
+// into DF, the stencil kernel does the bulk per grid point, and correction
+// kernels add the sources, the attenuation and the plastic map:
 //
 //   DF <- A*DF + L(F)                 (scale_rates + set_rates,
 //                                      src/fields.f90:49-108,
@@ -24,6 +25,7 @@
 // constant metric.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <utility>
 
 #include "wql_internal.h"
@@ -55,327 +57,149 @@ __device__ __forceinline__ void load6(const T* __restrict__ F, const T* __restri
   }
 }
 
-// Apply the SBP-6 derivative along axis d (0-based index i of n, stride st)
-// to the six quantities of load6.  Result is not yet divided by h.
-template <typename T, bool CURV>
-__device__ __forceinline__ void diff6(const T* __restrict__ F, const T* __restrict__ coef,
-                                      long long np, long long p, int i, int n, long long st, int d,
-                                      T r[6]) {
-  T t[6], u[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) r[c] = T(0);
-  const int kind = sbp_kind(i, n);
-  if (kind == 0) {
-    const T cs[3] = {T(kC1), T(kC2), T(kC3)};
-#pragma unroll
-    for (int s = 1; s <= 3; ++s) {
-      load6<T, CURV>(F, coef, np, p + s * st, d, t);
-      load6<T, CURV>(F, coef, np, p - s * st, d, u);
-#pragma unroll
-      for (int c = 0; c < 6; ++c) r[c] += cs[s - 1] * (t[c] - u[c]);
-    }
-  } else if (kind < 0) {
-    const int row = -kind - 1;
-    const long long p0 = p - (long long)i * st;
-    for (int col = 0; col < 9; ++col) {
-      const T w = sbp_w<T>(row, col);
-      if (w != T(0)) {
-        load6<T, CURV>(F, coef, np, p0 + col * st, d, t);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) r[c] += w * t[c];
-      }
-    }
-  } else {
-    const int row = kind - 1;
-    const long long pn = p + (long long)(n - 1 - i) * st;
-    for (int col = 0; col < 9; ++col) {
-      const T w = -sbp_w<T>(row, col);
-      if (w != T(0)) {
-        load6<T, CURV>(F, coef, np, pn - col * st, d, t);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) r[c] += w * t[c];
-      }
-    }
-  }
-}
-
-// SBP-6 derivative along one axis of the three velocities only (no flux).
-template <typename T>
-__device__ __forceinline__ void diff_v(const T* __restrict__ F, long long np, long long p, int i, int n, long long st,
-                                       T r[3]) {
-  r[0] = r[1] = r[2] = T(0);
-  const int kind = sbp_kind(i, n);
-  if (kind == 0) {
-    const T cs[3] = {T(kC1), T(kC2), T(kC3)};
-#pragma unroll
-    for (int s = 1; s <= 3; ++s)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) r[c] += cs[s - 1] * (F[c * np + p + s * st] - F[c * np + p - s * st]);
-  } else if (kind < 0) {
-    const int row = -kind - 1;
-    const long long p0 = p - (long long)i * st;
-    for (int col = 0; col < 9; ++col) {
-      const T w = sbp_w<T>(row, col);
-      if (w != T(0))
-#pragma unroll
-        for (int c = 0; c < 3; ++c) r[c] += w * F[c * np + p0 + col * st];
-    }
-  } else {
-    const int row = kind - 1;
-    const long long pn = p + (long long)(n - 1 - i) * st;
-    for (int col = 0; col < 9; ++col) {
-      const T w = -sbp_w<T>(row, col);
-      if (w != T(0))
-#pragma unroll
-        for (int c = 0; c < 3; ++c) r[c] += w * F[c * np + pn - col * st];
-    }
-  }
-}
-
-// D_d of the three fluxes J*metric_j(d)*sigma_{c,j} (fixed physical axis j),
-// needed only inside PML slabs (the per-axis split of the divergence).
-template <typename T>
-__device__ void diff_pml_flux(const T* __restrict__ F, const T* __restrict__ coef, long long np,
-                              long long p, int i, int n, long long st, int d, int j, T r[3]) {
-  r[0] = r[1] = r[2] = T(0);
-  const int kind = sbp_kind(i, n);
-  auto acc = [&](long long q, T w) {
-    const T a = coef[(d * 3 + j) * np + q];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) r[c] += w * (a * F[sig(c, j) * np + q]);
-  };
-  if (kind == 0) {
-    const T cs[3] = {T(kC1), T(kC2), T(kC3)};
-    for (int s = 1; s <= 3; ++s) {
-      acc(p + s * st, cs[s - 1]);
-      acc(p - s * st, -cs[s - 1]);
-    }
-  } else if (kind < 0) {
-    const int row = -kind - 1;
-    const long long p0 = p - (long long)i * st;
-    for (int col = 0; col < 9; ++col) {
-      const T w = sbp_w<T>(row, col);
-      if (w != T(0)) acc(p0 + col * st, w);
-    }
-  } else {
-    const int row = kind - 1;
-    const long long pn = p + (long long)(n - 1 - i) * st;
-    for (int col = 0; col < 9; ++col) {
-      const T w = -sbp_w<T>(row, col);
-      if (w != T(0)) acc(pn - col * st, w);
-    }
-  }
-}
-
-
 // ---------------------------------------------------------------------------
-// Upwind SBP-6 (fd 1, src/JU_xJU_yJU_z6.f90:2680-3706, 17675-17983): D+ on
-// the velocities, D- on the fluxes.  Interior D+ weights on offsets -2..4
-// and D- weights on offsets -4..2; the closure rows of both operators cover
-// the same columns, so one load per column serves both.
-template <typename T, bool CURV, int FD>
-__device__ __forceinline__ void diff6_up(const T* __restrict__ F, const T* __restrict__ coef, long long np,
-                                         long long p, int i, int n, long long st, int d, T r[6]) {
-  constexpr int PHI = UpOp<FD>::PHI, NCOL = UpOp<FD>::NCOL;
-  T t[6];
+// Rows of the difference operators for the per-point kernels.  The weights of
+// the block's operator sit in shared memory (the closure rows of neighbouring
+// lanes differ, which constant memory would serve one row at a time):
+//   FD 0  SBP-6: [row 6][point 9]
+//   FD 1  upwind order 6: [D+, D-][row 6][point 10]
+//   FD 2  upwind order 5: [D+, D-][row 4][point 7]
+//   FD 3  a table operator: the whole table (UpG)
+template <int FD>
+constexpr int kRowWords = FD == 0 ? 54 : (FD == 1 ? 120 : (FD == 2 ? 56 : kUgWords));
+
+template <typename T, int FD>
+__device__ __forceinline__ void load_rows(T* tab, const UpG& g) {
+  const int nt = blockDim.x * blockDim.y;
+  for (int e = threadIdx.x + blockDim.x * threadIdx.y; e < kRowWords<FD>; e += nt) {
+    if constexpr (FD == 0) tab[e] = sbp_w<T>(e / 9, e % 9);
+    else if constexpr (FD == 1) tab[e] = up_w<T>(e / 60, e / 10 % 6, e % 10);
+    else if constexpr (FD == 2) tab[e] = upw<T, 2>(e / 28, e / 7 % 4, e % 7);
+    else tab[e] = ((const T*)g.w)[e];
+  }
+  __syncthreads();
+}
+
+// Calls vel(offset, weight) and flux(offset, weight) for the points of the
+// rows of the velocity and the flux operator at 0-based index i of n along
+// axis d (one operator for both in FD 0, D+ and D- else).  Interior rows and
+// closure columns are unrolled so that their loads are in flight together.
+// shell (FD 3): the point lies in the boundary shell, whose interior rows are
+// the near-boundary routine's.
+template <typename T, int FD, typename V, typename X>
+__device__ __forceinline__ void visit_row(const T* tab, const UpG& g, bool shell, int i, int n, int d, V&& vel,
+                                          X&& flux) {
+  if constexpr (FD == 3) {
+    if (i >= g.R && i < n - g.R) {
+      // orders 2..9 and the DRP operators: D+ within -4..5, D- within -5..4
+      const T* wp = tab + (shell ? 2 * kUgCol : 0);
 #pragma unroll
-  for (int c = 0; c < 6; ++c) r[c] = T(0);
-  const int kind = up_kind<FD>(i, n);
-  if (kind == 0) {
-#pragma unroll
-    for (int o = -PHI; o <= PHI; ++o) {
-      load6<T, CURV>(F, coef, np, p + o * st, d, t);
-      if (o >= -2)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) r[c] += up_cf<T, FD>(o) * t[c];
-      if (o <= 2)
-#pragma unroll
-        for (int c = 3; c < 6; ++c) r[c] -= up_cf<T, FD>(-o) * t[c];
+      for (int o = -5; o <= 5; ++o) {
+        if (o >= -4 && o >= g.plo && o < g.plo + g.pn) vel(o, wp[o - g.plo]);
+        if (o <= 4 && o >= g.mlo && o < g.mlo + g.mn) flux(o, wp[kUgCol + o - g.mlo]);
+      }
+    } else {
+      // left row i reads points 0.., right row k = n-1-i points n-1-t
+      const bool left = i < g.R;
+      const int row = left ? i : n - 1 - i;
+      const T* wp = tab + 4 * kUgCol + (left ? 0 : 2 * kUgRowBlock) + (d * kUgRows + row) * kUgCol;
+#pragma unroll 4
+      for (int t = 0; t < kUgCol; ++t) {
+        const int off = left ? t - row : row - t;
+        const T wv = wp[t], wf = wp[kUgRowBlock + t];
+        if (wv != T(0)) vel(off, wv);
+        if (wf != T(0)) flux(off, wf);
+      }
     }
   } else {
-    const long long base = kind < 0 ? p - (long long)i * st : p + (long long)(n - 1 - i) * st;
-    for (int col = 0; col < NCOL; ++col) {
-      T wv, wf;
-      int off;
-      upx_entry<T, FD>(kind, col, d, wv, wf, off);
-      if (wv != T(0) || wf != T(0)) {
-        load6<T, CURV>(F, coef, np, base + (kind < 0 ? col : -col) * st, d, t);
+    const int kind = FD ? up_kind<FD ? FD : 1>(i, n) : sbp_kind(i, n);
+    if (kind == 0 && FD) {
+      constexpr int PHI = UpOp<FD ? FD : 1>::PHI;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) r[c] += wv * t[c];
+      for (int o = -PHI; o <= PHI; ++o) {
+        if (o >= -2) vel(o, up_cf<T, FD ? FD : 1>(o));
+        if (o <= 2) flux(o, -up_cf<T, FD ? FD : 1>(-o));
+      }
+    } else if (kind == 0) {
+      const T cs[3] = {T(kC1), T(kC2), T(kC3)};
 #pragma unroll
-        for (int c = 3; c < 6; ++c) r[c] += wf * t[c];
+      for (int s = 1; s <= 3; ++s) {
+        vel(s, cs[s - 1]);
+        flux(s, cs[s - 1]);
+        vel(-s, -cs[s - 1]);
+        flux(-s, -cs[s - 1]);
+      }
+    } else {
+      // left row kind = -1-row reads points 0.., right row kind = 1+row the
+      // mirrored points with negated weights (the upwind pair swaps its two
+      // tables there)
+      constexpr int NC = FD ? UpOp<FD ? FD : 1>::NCOL : 9, NR = FD ? UpOp<FD ? FD : 1>::R : 6;
+      const bool left = kind < 0;
+      const int row = left ? -kind - 1 : kind - 1;
+      const T sgn = left ? T(1) : T(-1);
+      const T* wv = tab + (FD && !left ? NR * NC : 0) + row * NC;
+      const T* wf = FD ? tab + (left ? NR * NC : 0) + row * NC : wv;
+#pragma unroll
+      for (int t = 0; t < NC; ++t) {
+        const int off = left ? t - row : row - t;
+        if (FD == 0) {
+          const T w = wv[t];
+          if (w != T(0)) {
+            vel(off, sgn * w);
+            flux(off, sgn * w);
+          }
+        } else {
+          const T w = wv[t], x = wf[t];
+          if (w != T(0)) vel(off, sgn * w);
+          if (x != T(0)) flux(off, sgn * x);
+        }
       }
     }
   }
 }
 
-// D+ of the three velocities only, along axis d.
-template <typename T, int FD>
-__device__ __forceinline__ void diff_v_up(const T* __restrict__ F, long long np, long long p, int i, int n,
-                                          long long st, int d, T r[3]) {
-  constexpr int PHI = UpOp<FD>::PHI, NCOL = UpOp<FD>::NCOL;
-  r[0] = r[1] = r[2] = T(0);
-  const int kind = up_kind<FD>(i, n);
-  if (kind == 0) {
-#pragma unroll
-    for (int o = -2; o <= PHI; ++o)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) r[c] += up_cf<T, FD>(o) * F[c * np + p + o * st];
-  } else {
-    const long long base = kind < 0 ? p - (long long)i * st : p + (long long)(n - 1 - i) * st;
-    for (int col = 0; col < NCOL; ++col) {
-      T wv, wf;
-      int off;
-      upx_entry<T, FD>(kind, col, d, wv, wf, off);
-      if (wv != T(0))
-#pragma unroll
-        for (int c = 0; c < 3; ++c) r[c] += wv * F[c * np + base + (kind < 0 ? col : -col) * st];
-    }
-  }
-}
-
-// D- of the three fluxes J*metric_j(d)*sigma_{c,j} (PML split, as
-// diff_pml_flux).
-template <typename T, int FD>
-__device__ void diff_pml_flux_up(const T* __restrict__ F, const T* __restrict__ coef, long long np, long long p,
-                                 int i, int n, long long st, int d, int j, T r[3]) {
-  constexpr int PHI = UpOp<FD>::PHI, NCOL = UpOp<FD>::NCOL;
-  r[0] = r[1] = r[2] = T(0);
-  const int kind = up_kind<FD>(i, n);
-  auto acc = [&](long long q, T w) {
-    const T a = coef[(d * 3 + j) * np + q];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) r[c] += w * (a * F[sig(c, j) * np + q]);
-  };
-  if (kind == 0) {
-#pragma unroll
-    for (int o = -PHI; o <= 2; ++o) acc(p + o * st, -up_cf<T, FD>(-o));
-  } else {
-    const long long base = kind < 0 ? p - (long long)i * st : p + (long long)(n - 1 - i) * st;
-    for (int col = 0; col < NCOL; ++col) {
-      T wv, wf;
-      int off;
-      upx_entry<T, FD>(kind, col, d, wv, wf, off);
-      if (wf != T(0)) acc(base + (kind < 0 ? col : -col) * st, wf);
-    }
-  }
-}
-
-// ---- table upwind operators (fd 3), as the reference applies them: the
-// near-boundary routine JJU_x<order>_upwind(_drp) at points of the boundary
-// shell (its closure rows, and its interior case bp/bm on the axes where the
-// point is interior), the interior routine JJU_x<order>_interior_upwind(_drp)
-// (ip/im) at the other points (src/RHS_Interior.f90:40-125, 276-1512).
+// Whether point idx lies in the boundary shell of a table operator: outside
+// [lo, n-1-hi] on some axis, with lo and hi the closure rows R, or npml on a
+// PML side if larger (the interior limits of the interior routines,
+// src/RHS_Interior.f90:40-125, 276-1512).
 template <typename T>
-__device__ __forceinline__ T ugw(const UpG& g, int idx) {
-  return ((const T*)g.w)[idx];
-}
-
-// Whether point idx lies in the boundary shell: outside [lo, n-1-hi] on some
-// axis, with lo and hi the closure rows R, or npml on a PML side if larger
-// (the interior limits of the interior routines).
-template <typename T>
-__device__ __forceinline__ bool ug_shell(const VolumeArgs<T>& a, const int idx[3], const int nn[3]) {
+__device__ __forceinline__ bool ug_shell(const VolumeArgs<T>& a, int i, int j, int k) {
   bool shell = false;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
+    const int idx = d == 0 ? i : (d == 1 ? j : k), n = d == 0 ? a.nq : (d == 1 ? a.nr : a.ns);
     const int lo = a.pml[2 * d] ? max(a.ug.R, a.npml) : a.ug.R;
     const int hi = a.pml[2 * d + 1] ? max(a.ug.R, a.npml) : a.ug.R;
-    shell = shell || idx[d] < lo || idx[d] > nn[d] - 1 - hi;
+    shell = shell || idx < lo || idx > n - 1 - hi;
   }
   return shell;
 }
 
-// Weights of the D+ (plus) or D- row at 0-based index i of n along axis d:
-// calls f(offset from the point, weight) for each nonzero weight.
-template <typename T, typename Fn>
-__device__ __forceinline__ void ug_row(const UpG& g, bool shell, bool plus, int i, int n, int d, Fn&& f) {
-  if (i >= g.R && i < n - g.R) {
-    const int base = (shell ? 2 * kUgCol : 0) + (plus ? 0 : kUgCol);
-    const int lo = plus ? g.plo : g.mlo, cnt = plus ? g.pn : g.mn;
-    for (int k = 0; k < cnt; ++k) {
-      const T w = ugw<T>(g, base + k);
-      if (w != T(0)) f(lo + k, w);
-    }
-  } else if (i < g.R) {  // left row i, points 0..12
-    const int base = 4 * kUgCol + (plus ? 0 : kUgRowBlock) + (d * kUgRows + i) * kUgCol;
-    for (int t = 0; t < kUgCol; ++t) {
-      const T w = ugw<T>(g, base + t);
-      if (w != T(0)) f(t - i, w);
-    }
-  } else {  // right row k = n-1-i, points n-1-t
-    const int k = n - 1 - i;
-    const int base = 4 * kUgCol + (plus ? 2 : 3) * kUgRowBlock + (d * kUgRows + k) * kUgCol;
-    for (int t = 0; t < kUgCol; ++t) {
-      const T w = ugw<T>(g, base + t);
-      if (w != T(0)) f(k - t, w);
-    }
-  }
-}
-
-// The six differenced quantities of load6 along axis d: D+ of the
-// velocities, D- of the d-face momentum fluxes.
-template <typename T, bool CURV>
-__device__ void diff6_ug(const T* __restrict__ F, const T* __restrict__ coef, long long np, long long p, int i,
-                         int n, long long st, int d, const UpG& g, bool shell, T r[6]) {
-#pragma unroll
-  for (int c = 0; c < 6; ++c) r[c] = T(0);
-  ug_row<T>(g, shell, true, i, n, d, [&](int off, T w) {
-    const long long q = p + off * st;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) r[c] += w * F[c * np + q];
-  });
-  ug_row<T>(g, shell, false, i, n, d, [&](int off, T w) {
-    T t[6];
-    load6<T, CURV>(F, coef, np, p + off * st, d, t);
-#pragma unroll
-    for (int c = 3; c < 6; ++c) r[c] += w * t[c];
-  });
-}
-
-// D+ of the three velocities only, along axis d.
+// Whether the pre-kernels have set DF of the point on a stage with A = 0: a
+// block face or a PML slab.
 template <typename T>
-__device__ void diff_v_ug(const T* __restrict__ F, long long np, long long p, int i, int n, long long st, int d,
-                          const UpG& g, bool shell, T r[3]) {
-  r[0] = r[1] = r[2] = T(0);
-  ug_row<T>(g, shell, true, i, n, d, [&](int off, T w) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) r[c] += w * F[c * np + p + off * st];
-  });
+__device__ __forceinline__ bool df_set(const VolumeArgs<T>& a, int i, int j, int k) {
+  const int w = a.npml;
+  return i == 0 || i == a.nq - 1 || j == 0 || j == a.nr - 1 || k == 0 || k == a.ns - 1 || (a.pml[0] && i < w) ||
+         (a.pml[1] && i >= a.nq - w) || (a.pml[2] && j < w) || (a.pml[3] && j >= a.nr - w) || (a.pml[4] && k < w) ||
+         (a.pml[5] && k >= a.ns - w);
 }
 
-// D- of the three fluxes J*metric_j(d)*sigma_{c,j} (the PML split).
+// Two blocks' arguments of a launch over one block or a scenario's two.
 template <typename T>
-__device__ void diff_pml_flux_ug(const T* __restrict__ F, const T* __restrict__ coef, long long np, long long p,
-                                 int i, int n, long long st, int d, int j, const UpG& g, bool shell, T r[3]) {
-  r[0] = r[1] = r[2] = T(0);
-  ug_row<T>(g, shell, false, i, n, d, [&](int off, T w) {
-    const long long q = p + off * st;
-    const T a = coef[(d * 3 + j) * np + q];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) r[c] += w * (a * F[sig(c, j) * np + q]);
-  });
-}
-
-// Operator dispatch on the compile-time fd of a kernel.
-template <typename T, bool CURV, int FD>
-__device__ __forceinline__ void diff6_op(const T* __restrict__ F, const T* __restrict__ coef, long long np,
-                                         long long p, int i, int n, long long st, int d, T r[6]) {
-  if (FD) diff6_up<T, CURV, FD ? FD : 1>(F, coef, np, p, i, n, st, d, r);
-  else diff6<T, CURV>(F, coef, np, p, i, n, st, d, r);
-}
-
-
+struct BlockPair {
+  VolumeArgs<T> a[2];
+  long long n0;  // threads, planes or CTAs of block 0 (by the kernel)
+};
 
 // ---------------------------------------------------------------------------
 // Main stencil kernel (2.5-D tiled).  Computes, for every point of the block,
 //   DF <- A*DF + L(F)      and      F_out <- F + B*dt*DF
 // (scale_rates + set_rates + update_fields, src/fields.f90:49-171,
 // src/JU_xJU_yJU_z6.f90:12-812 and 16141-16449, src/RHS_Interior.f90:133-274),
-// with the Kahan-compensated update in FP32C mode.  Boundary penalties, PML
-// terms and the plastic return map are applied afterwards by the correction
-// kernels below (they are linear in DF, so the order of the sums changes only
-// rounding).
+// with the Kahan-compensated update in FP32C mode.  Boundary penalties and the
+// PML damping are folded into DF beforehand by the pre-kernels below (they are
+// linear in DF, so the order of the sums changes only rounding).
 //
 // A CTA of TQ x TR threads owns a (q,r) tile and marches along s through a
 // chunk of planes.  Per plane the tile plus a 3-point halo in q and r is
@@ -575,10 +399,11 @@ __global__ void __launch_bounds__(TQ * TR, MINB) stencil_kernel_tiled(const __gr
     du[6] = mu * (g[0][1] + g[1][0]);
     du[7] = mu * (g[0][2] + g[2][0]);
     du[8] = mu * (g[1][2] + g[2][1]);
+    const bool keep = a.A != T(0), set = !keep && df_set(a, q, r, s);
 #pragma unroll
     for (int c = 0; c < 9; ++c) {
       const T f0 = F[c * np + p];
-      const T df = a.A * a.DF[c * np + p] + du[c];
+      const T df = (keep ? a.A * a.DF[c * np + p] : (set ? a.DF[c * np + p] : T(0))) + du[c];
       a.DF[c * np + p] = df;
       if (KAHAN) {
         const T y = a.Bdt * df - (T)comp_get(a.C, c * np + p);
@@ -593,32 +418,57 @@ __global__ void __launch_bounds__(TQ * TR, MINB) stencil_kernel_tiled(const __gr
 }
 
 // Per-point form of the same stencil kernel: every neighbour value is read
-// through L1/L2 (kept for cross-checks of the tiled kernel).
-// smode 1 restricts it to the 12 s-boundary planes (grid z = 12), the part
-// the TMA kernel leaves out.
+// through L1/L2.  It runs the upwind operators that the TMA kernel does not
+// take (the table operators, order 5, and FP64) and serves as a cross-check
+// of the other kernels.  One launch covers one block or a scenario's two:
+// planes [0, n0) of the grid are block 0's.
 template <typename T, bool CURV, bool KAHAN, int FD = 0>
-__global__ void __launch_bounds__(256) stencil_kernel_pointwise(const __grid_constant__ VolumeArgs<T> a, int smode) {
+__global__ void __launch_bounds__(256) stencil_kernel_pointwise(const __grid_constant__ BlockPair<T> P) {
+  __shared__ T tab[kRowWords<FD>];
+  load_rows<T, FD>(tab, P.a[0].ug);
+  const int blk = (long long)blockIdx.z >= P.n0 ? 1 : 0;
+  const VolumeArgs<T>& a = P.a[blk];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = smode ? (blockIdx.z < 6 ? (int)blockIdx.z : a.ns - 12 + (int)blockIdx.z) : (int)blockIdx.z;
+  const int k = (int)blockIdx.z - (blk ? (int)P.n0 : 0);
   if (i >= a.nq || j >= a.nr) return;
   const long long np = a.np;
   const long long p = i + (long long)a.pq * (j + (long long)a.nr * k);
+  const T* __restrict__ F = a.Fin + p;
+  const T* __restrict__ coef = a.coef + p;
   T g[3][3], dv[3];
-  const T Jinv = CURV ? a.coef[9 * np + p] : T(1);
-  const int idx[3] = {i, j, k}, nn[3] = {a.nq, a.nr, a.ns};
-  const long long st[3] = {1, a.pq, (long long)a.pq * a.nr};
+  const T Jinv = CURV ? coef[9 * np] : T(1);
+  const bool shell = FD == 3 && ug_shell(a, i, j, k);
 #pragma unroll
-  const bool shell = FD == 3 && ug_shell(a, idx, nn);
   for (int d = 0; d < 3; ++d) {
+    const long long st = d == 0 ? 1 : (d == 1 ? (long long)a.pq : (long long)a.pq * a.nr);
     T o[6];
-    if (FD == 3) diff6_ug<T, CURV>(a.Fin, a.coef, np, p, idx[d], nn[d], st[d], d, a.ug, shell, o);
-    else diff6_op<T, CURV, FD == 3 ? 0 : FD>(a.Fin, a.coef, np, p, idx[d], nn[d], st[d], d, o);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) o[c] = T(0);
+    visit_row<T, FD>(
+        tab, a.ug, shell, d == 0 ? i : (d == 1 ? j : k), d == 0 ? a.nq : (d == 1 ? a.nr : a.ns), d,
+        [&](int off, T w) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) o[c] += w * F[c * np + off * st];
+        },
+        [&](int off, T w) {
+          const long long q = off * st;
+          if (CURV) {
+            const T m0 = w * coef[(d * 3) * np + q], m1 = w * coef[(d * 3 + 1) * np + q],
+                    m2 = w * coef[(d * 3 + 2) * np + q];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              o[3 + c] += m0 * F[sig(c, 0) * np + q] + m1 * F[sig(c, 1) * np + q] + m2 * F[sig(c, 2) * np + q];
+          } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[3 + c] += w * F[sig(c, d) * np + q];
+          }
+        });
     const T rh = a.rh[d];
     if (CURV) {
       T m[3];
 #pragma unroll
-      for (int jj = 0; jj < 3; ++jj) m[jj] = a.coef[(d * 3 + jj) * np + p] * Jinv;
+      for (int jj = 0; jj < 3; ++jj) m[jj] = coef[(d * 3 + jj) * np] * Jinv;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         dv[c] = d == 0 ? rh * o[3 + c] : dv[c] + rh * o[3 + c];
@@ -634,10 +484,9 @@ __global__ void __launch_bounds__(256) stencil_kernel_pointwise(const __grid_con
       }
     }
   }
-  const T* coef = a.coef;
-  const T lam = CURV ? coef[10 * np + p] : coef[0 * np + p];
-  const T mu = CURV ? coef[11 * np + p] : coef[1 * np + p];
-  const T rinv = CURV ? coef[12 * np + p] : coef[2 * np + p];
+  const T lam = coef[(CURV ? 10 : 0) * np];
+  const T mu = coef[(CURV ? 11 : 1) * np];
+  const T rinv = coef[(CURV ? 12 : 2) * np];
   const T l2m = lam + T(2) * mu;
   T du[9];
   du[0] = rinv * dv[0];
@@ -649,10 +498,11 @@ __global__ void __launch_bounds__(256) stencil_kernel_pointwise(const __grid_con
   du[6] = mu * (g[0][1] + g[1][0]);
   du[7] = mu * (g[0][2] + g[2][0]);
   du[8] = mu * (g[1][2] + g[2][1]);
+  const bool keep = a.A != T(0), set = !keep && df_set(a, i, j, k);
 #pragma unroll
   for (int c = 0; c < 9; ++c) {
-    const T f0 = a.Fin[c * np + p];
-    const T df = a.A * a.DF[c * np + p] + du[c];
+    const T f0 = F[c * np];
+    const T df = (keep ? a.A * a.DF[c * np + p] : (set ? a.DF[c * np + p] : T(0))) + du[c];
     a.DF[c * np + p] = df;
     if (KAHAN) {
       const T y = a.Bdt * df - (T)comp_get(a.C, c * np + p);
@@ -665,47 +515,6 @@ __global__ void __launch_bounds__(256) stencil_kernel_pointwise(const __grid_con
   }
 }
 
-// ---------------------------------------------------------------------------
-// PML kernel (src/RHS_Interior.f90:1782-2201, src/fields.f90:70-105,131-166):
-// for every point inside one or more active slabs, the damping terms of the
-// rates, DQ <- A*DQ + sources - (d+cfs)*Q (plus the face penalty on the
-// slab's own boundary, src/RHS_Interior.f90:1560-1700) and Q <- Q + B*dt*DQ.
-// One thread per point of the block; points outside every slab exit.
-// The PML slab union of a block as up to six disjoint boxes: the q slabs
-// over the whole (r, s) extent, the r slabs between them, the s slabs inside
-// both; start[b] is the number of points in boxes before b.
-struct PmlBoxes {
-  int n;
-  int lo[6][3], dim[6][3];
-  long long start[7];
-};
-
-template <typename T>
-PmlBoxes pml_boxes(const VolumeArgs<T>& a) {
-  PmlBoxes B;
-  B.n = 0;
-  B.start[0] = 0;
-  const int nq = a.nq, nr = a.nr, ns = a.ns, w = a.npml;
-  const int qlo = a.pml[0] ? w : 0, qhi = a.pml[1] ? nq - w : nq;
-  const int rlo = a.pml[2] ? w : 0, rhi = a.pml[3] ? nr - w : nr;
-  const int slo = a.pml[4] ? w : 0, shi = a.pml[5] ? ns - w : ns;
-  auto add = [&](int q0, int q1, int r0, int r1, int s0, int s1) {
-    if (q1 <= q0 || r1 <= r0 || s1 <= s0) return;
-    const int b = B.n++;
-    B.lo[b][0] = q0; B.lo[b][1] = r0; B.lo[b][2] = s0;
-    B.dim[b][0] = q1 - q0; B.dim[b][1] = r1 - r0; B.dim[b][2] = s1 - s0;
-    B.start[b + 1] = B.start[b] + (long long)(q1 - q0) * (r1 - r0) * (s1 - s0);
-  };
-  add(0, qlo, 0, nr, 0, ns);
-  add(qhi, nq, 0, nr, 0, ns);
-  add(qlo, qhi, 0, rlo, 0, ns);
-  add(qlo, qhi, rhi, nr, 0, ns);
-  add(qlo, qhi, rlo, rhi, 0, slo);
-  add(qlo, qhi, rlo, rhi, shi, ns);
-  for (int b = B.n; b < 6; ++b) B.start[b + 1] = B.start[b];
-  return B;
-}
-
 // Offset of block point (i, j, k) within the slab of `side`.
 template <typename T>
 __device__ __forceinline__ long long slab_point(const VolumeArgs<T>& a, int side, int i, int j, int k) {
@@ -716,157 +525,16 @@ __device__ __forceinline__ long long slab_point(const VolumeArgs<T>& a, int side
   return i + (long long)a.nq * (j + (long long)a.nr * (hi ? k - (a.ns - npml) : k));
 }
 
-// FP32 fields: capped at 80 registers for three CTAs per SM (24 warps to
-// hide the latency of its dependent loads; measured 0.39 -> 0.31 ms per
-// correction launch on config 2 despite some spilling).
-template <typename T, bool CURV, bool KAHAN, int FD>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 1) pml_kernel(const __grid_constant__ VolumeArgs<T> a,
-                                                                           const __grid_constant__ PmlBoxes bx) {
-  // one thread per point of the slab union, enumerated box by box (q
-  // fastest within a box)
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  int b = 0;
-  while (b < bx.n && t >= bx.start[b + 1]) ++b;
-  if (b >= bx.n) return;
-  const long long l = t - bx.start[b];
-  const int i = bx.lo[b][0] + (int)(l % bx.dim[b][0]);
-  const int j = bx.lo[b][1] + (int)((l / bx.dim[b][0]) % bx.dim[b][1]);
-  const int k = bx.lo[b][2] + (int)(l / ((long long)bx.dim[b][0] * bx.dim[b][1]));
-  const int nq = a.nq, nr = a.nr, ns = a.ns, npml = a.npml;
-  const int idx[3] = {i, j, k}, nn[3] = {nq, nr, ns};
-  bool any = false;
-#pragma unroll
-  for (int side = 0; side < 6; ++side) {
-    const int ax = side >> 1;
-    if (a.pml[side] && ((side & 1) ? idx[ax] >= nn[ax] - npml : idx[ax] < npml)) any = true;
-  }
-  if (!any) return;
-  const long long np = a.np;
-  const long long p = i + (long long)a.pq * (j + (long long)nr * k);
-  const long long st[3] = {1, a.pq, (long long)a.pq * nr};
-  const T* __restrict__ F = a.Fin;
-  const T* __restrict__ coef = a.coef;
-  const bool shell = FD == 3 && ug_shell(a, idx, nn);
-  // velocity gradient at the point
-  T g[3][3];
-  const T Jinv = CURV ? coef[9 * np + p] : T(1);
-  // every loop over axes and sides is unrolled so that the per-axis index,
-  // extent and stride are compile-time selections (no local-memory arrays)
-  {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      T o[3];
-      if (FD == 3) diff_v_ug<T>(F, np, p, idx[d], nn[d], st[d], d, a.ug, shell, o);
-      else if (FD) diff_v_up<T, FD == 3 ? 1 : (FD ? FD : 1)>(F, np, p, idx[d], nn[d], st[d], d, o);
-      else diff_v<T>(F, np, p, idx[d], nn[d], st[d], o);
-      const T rh = a.rh[d];
-      for (int c = 0; c < 3; ++c) {
-        if (CURV) {
-          for (int jj = 0; jj < 3; ++jj) {
-            const T m = coef[(d * 3 + jj) * np + p] * Jinv;
-            g[c][jj] = d == 0 ? m * (rh * o[c]) : g[c][jj] + m * (rh * o[c]);
-          }
-        } else {
-          g[c][d] = a.cart_metric[d] * rh * o[c];
-        }
-      }
-    }
-  }
-  const T lam = CURV ? coef[10 * np + p] : coef[0 * np + p];
-  const T mu = CURV ? coef[11 * np + p] : coef[1 * np + p];
-  const T rinv = CURV ? coef[12 * np + p] : coef[2 * np + p];
-  const T rhoinv = CURV ? rinv / Jinv : rinv;
-  const T l2m = lam + T(2) * mu;
-  const double d0 = a.pml_d0;  // 6/(2*1) * ln(1/1e-3), src/RHS_Interior.f90:1815
-  const T cfs = T(1);
-  T corr[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) corr[c] = T(0);
-  // reference order of the layers: s-low, s-high, r-low, r-high, q-low, q-high
-#pragma unroll
-  for (int oi = 0; oi < 6; ++oi) {
-    const int side = oi < 2 ? 4 + oi : (oi < 4 ? oi : oi - 4);
-    if (!a.pml[side]) continue;
-    const int axis = side >> 1;
-    const bool hi = side & 1;
-    const int ii = idx[axis], n = nn[axis];
-    if (!(hi ? (ii >= n - npml) : (ii < npml))) continue;
-    // damping profile in grid-index units (src/RHS_Interior.f90:1855,1973,2092),
-    // in the field precision
-    const int off = hi ? ii + 1 - (n - npml) : (axis == 2 ? ii + 1 - npml : ii - npml);
-    const T damp = (T)d0 * (fabs((T)off / (T)npml));
-    const long long sp = slab_point(a, side, i, j, k);
-    const long long snp = a.slab_np[side];
-    T* __restrict__ Q = a.Q[side];
-    T* __restrict__ DQ = a.DQ[side];
-    T qv[9];
-    for (int c = 0; c < 9; ++c) qv[c] = Q[c * snp + sp];
-    // per-axis split of the stress divergence along physical axis `axis`
-    T sd[3];
-    if (CURV) {
-      T acc3[3] = {T(0), T(0), T(0)};
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        T r3[3];
-        if (FD == 3) diff_pml_flux_ug<T>(F, coef, np, p, idx[d], nn[d], st[d], d, axis, a.ug, shell, r3);
-        else if (FD) diff_pml_flux_up<T, FD == 3 ? 1 : (FD ? FD : 1)>(F, coef, np, p, idx[d], nn[d], st[d], d, axis, r3);
-        else diff_pml_flux<T>(F, coef, np, p, idx[d], nn[d], st[d], d, axis, r3);
-        for (int c = 0; c < 3; ++c) acc3[c] += a.rh[d] * r3[c];
-      }
-      for (int c = 0; c < 3; ++c) sd[c] = acc3[c] * Jinv;
-    } else {
-      T o[6];
-      if (FD == 3) diff6_ug<T, false>(F, coef, np, p, idx[axis], nn[axis], st[axis], axis, a.ug, shell, o);
-      else diff6_op<T, false, FD == 3 ? 0 : FD>(F, coef, np, p, idx[axis], nn[axis], st[axis], axis, o);
-      for (int c = 0; c < 3; ++c) sd[c] = a.cart_metric[axis] * a.rh[axis] * o[3 + c];
-    }
-    corr[0] -= damp * qv[0] * rhoinv;
-    corr[1] -= damp * qv[1] * rhoinv;
-    corr[2] -= damp * qv[2] * rhoinv;
-    corr[3] -= damp * (l2m * qv[3] + lam * qv[4] + lam * qv[5]);
-    corr[4] -= damp * (lam * qv[3] + l2m * qv[4] + lam * qv[5]);
-    corr[5] -= damp * (lam * qv[3] + lam * qv[4] + l2m * qv[5]);
-    corr[6] -= mu * damp * qv[6];
-    corr[7] -= mu * damp * qv[7];
-    corr[8] -= mu * damp * qv[8];
-    T src[9];
-    for (int c = 0; c < 9; ++c) src[c] = T(0);
-    src[0] = sd[0];
-    src[1] = sd[1];
-    src[2] = sd[2];
-    // velocity-gradient sources (src/RHS_Interior.f90:1890-1907, 2008-2025, 2125-2142)
-    if (axis == 0) { src[3] = g[0][0]; src[6] = g[1][0]; src[7] = g[2][0]; }
-    else if (axis == 1) { src[4] = g[1][1]; src[6] = g[0][1]; src[8] = g[2][1]; }
-    else { src[5] = g[2][2]; src[7] = g[0][2]; src[8] = g[1][2]; }
-    T dq[9];
-    for (int c = 0; c < 9; ++c) dq[c] = a.A * DQ[c * snp + sp] + src[c] - (damp + cfs) * qv[c];
-    const bool on_face = hi ? (ii == n - 1) : (ii == 0);
-    if (on_face && a.bc[side] >= 1 && a.bc[side] <= 3) {
-      T u[9], sat[9], ubc[9];
-      for (int c = 0; c < 9; ++c) u[c] = F[c * np + p];
-      const int na = axis == 0 ? nr : nq;
-      const long long f = axis == 0 ? (j + (long long)nr * k) : (axis == 1 ? (i + (long long)nq * k) : (i + (long long)nq * j));
-      const long long nf = (long long)na * (axis == 2 ? nr : ns);
-      boundary_sat(u, a.face[side], nf, f, a.bc[side], hi, a.bc_form, sat, ubc);
-      for (int c = 0; c < 9; ++c) dq[c] -= a.tau_h[axis] * (T)ubc[c];
-    }
-    for (int c = 0; c < 9; ++c) {
-      DQ[c * snp + sp] = dq[c];
-      Q[c * snp + sp] = qv[c] + a.Bdt * dq[c];
-    }
-  }
-  add_correction<T, KAHAN>(a, p, corr);
-}
-
 // ---------------------------------------------------------------------------
-// PML pre-kernel (FP32 fields whose stencil is the TMA kernel): the same slab
-// update as pml_kernel, run before the stencil of its stage.  Everything it
-// needs is stage input (F, Q, DQ), so the damping terms of the rates are
-// folded into DF (DF + corr/A, or corr on a stage with A = 0) and the
-// stencil's A*DF + du carries them: F_out and its compensation are not read
-// and written a second time, and no velocity gradient is handed over.  The
-// face pre-kernel, which runs first, has folded the boundary forcing of the
-// auxiliary fields into DQ at the slab's own face.
+// PML pre-kernel (src/RHS_Interior.f90:1782-2201, src/fields.f90:70-105,
+// 131-166): for every point inside one or more active slabs, the damping terms
+// of the rates, DQ <- A*DQ + sources - (d+cfs)*Q and Q <- Q + B*dt*DQ.  It
+// runs before the stencil of its stage.  Everything it needs is stage input
+// (F, Q, DQ), so the damping terms are folded into DF (DF + corr/A, or corr
+// on a stage with A = 0) and the stencil's A*DF + du carries them: F_out and
+// its compensation are not read and written a second time, and no velocity
+// gradient is handed over.  The face pre-kernel, which runs first, has folded
+// the boundary forcing of the auxiliary fields into DQ at the slab's own face.
 //
 // The slab union is cut into regions along the slab edges, up to 26, so that
 // the sides a point lies in are the same for a whole CTA: the axis of a side
@@ -940,28 +608,37 @@ struct PmlPair {
   int n0;
 };
 
-__device__ __forceinline__ float at(const float* base, unsigned byte) {
-  return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(base) + byte);
+// Element at a byte offset; O is unsigned, or size_t where a component is 4
+// GiB or more (and for FP64 fields, whose kernel waits on the FP64 unit, not
+// on address arithmetic).
+template <typename T, typename O>
+__device__ __forceinline__ T& at(T* base, O byte) {
+  return *reinterpret_cast<T*>(reinterpret_cast<char*>(base) + byte);
+}
+template <typename T, typename O>
+__device__ __forceinline__ T at(const T* base, O byte) {
+  return *reinterpret_cast<const T*>(reinterpret_cast<const char*>(base) + byte);
 }
 
-template <bool CURV, int FD>
-__device__ __forceinline__ void pml_pre_point(const VolumeArgs<float>& a, int i, int j, int k, unsigned sides,
-                                              const float* tab) {
+template <typename T, typename O, bool CURV, int FD>
+__device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int j, int k, unsigned sides,
+                                              const T* tab) {
   const int nq = a.nq, nr = a.nr, ns = a.ns, npml = a.npml;
   const long long np = a.np;
-  const unsigned o = 4u * (unsigned)(i + a.pq * (j + nr * k));  // byte offset of the point in a component
-  const float* __restrict__ F = a.Fin;
-  const float* __restrict__ coef = a.coef;
-  const float Jinv = CURV ? at(coef + 9 * np, o) : 1.0f;
-  const float lam = at(coef + (CURV ? 10 : 0) * np, o), mu = at(coef + (CURV ? 11 : 1) * np, o);
-  const float rinv = at(coef + (CURV ? 12 : 2) * np, o);
-  const float rhoinv = CURV ? rinv / Jinv : rinv;
-  const float l2m = lam + 2.0f * mu;
+  const O o = (O)sizeof(T) * ((O)i + (O)a.pq * ((O)j + (O)nr * (O)k));  // byte offset of the point in a component
+  const T* __restrict__ F = a.Fin;
+  const T* __restrict__ coef = a.coef;
+  const T Jinv = CURV ? at(coef + 9 * np, o) : T(1);
+  const T lam = at(coef + (CURV ? 10 : 0) * np, o), mu = at(coef + (CURV ? 11 : 1) * np, o);
+  const T rinv = at(coef + (CURV ? 12 : 2) * np, o);
+  const T rhoinv = CURV ? rinv / Jinv : rinv;
+  const T l2m = lam + T(2) * mu;
+  const bool shell = FD == 3 && ug_shell(a, i, j, k);
   // on a stage with A = 0, DF and DQ hold only what the face pre-kernel put there
-  const bool keep = a.A != 0.0f;
-  float corr[9];
+  const bool keep = a.A != T(0);
+  T corr[9];
 #pragma unroll
-  for (int c = 0; c < 9; ++c) corr[c] = 0.0f;
+  for (int c = 0; c < 9; ++c) corr[c] = T(0);
 #pragma unroll 1
   while (sides) {
     const int side = __ffs(sides) - 1;
@@ -970,68 +647,37 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<float>& a, int i,
     const bool hi = side & 1;
     const int ii = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 0 ? nq : (axis == 1 ? nr : ns);
     // flux components of physical axis `axis`: sigma_{c,axis}
-    const float* __restrict__ S0 = F + (axis == 0 ? 3 : (axis == 1 ? 6 : 7)) * np;
-    const float* __restrict__ S1 = F + (axis == 0 ? 6 : (axis == 1 ? 4 : 8)) * np;
-    const float* __restrict__ S2 = F + (axis == 0 ? 7 : (axis == 1 ? 8 : 5)) * np;
-    float sd[3] = {0.0f, 0.0f, 0.0f}, gv[3] = {0.0f, 0.0f, 0.0f};
+    const T* __restrict__ S0 = F + (axis == 0 ? 3 : (axis == 1 ? 6 : 7)) * np;
+    const T* __restrict__ S1 = F + (axis == 0 ? 6 : (axis == 1 ? 4 : 8)) * np;
+    const T* __restrict__ S2 = F + (axis == 0 ? 7 : (axis == 1 ? 8 : 5)) * np;
+    T sd[3] = {T(0), T(0), T(0)}, gv[3] = {T(0), T(0), T(0)};
     // derivative along computational axis d of the velocities (o6[0..2]) and
     // of the fluxes J*metric_axis(d)*sigma_{c,axis} (o6[3..5])
     auto direction = [&](int d) {
-      const int id = d == 0 ? i : (d == 1 ? j : k), nd = d == 0 ? nq : (d == 1 ? nr : ns);
-      const unsigned st = 4u * (unsigned)(d == 0 ? 1 : (d == 1 ? a.pq : a.pq * nr));
-      const float* __restrict__ M = CURV ? coef + (d * 3 + axis) * np : coef;
-      float o6[6];
+      const O st = (O)sizeof(T) * (d == 0 ? (O)1 : (d == 1 ? (O)a.pq : (O)a.pq * (O)nr));
+      const T* __restrict__ M = CURV ? coef + (d * 3 + axis) * np : coef;
+      T o6[6];
 #pragma unroll
-      for (int c = 0; c < 6; ++c) o6[c] = 0.0f;
-      auto vel = [&](unsigned q, float w) {
+      for (int c = 0; c < 6; ++c) o6[c] = T(0);
+      visit_row<T, FD>(
+          tab, a.ug, shell, d == 0 ? i : (d == 1 ? j : k), d == 0 ? nq : (d == 1 ? nr : ns), d,
+          [&](int off, T w) {
+            const O q = o + (O)off * st;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) o6[c] += w * at(F + c * np, q);
-      };
-      auto flux = [&](unsigned q, float w) {
-        const float m = CURV ? w * at(M, q) : w;
-        o6[3] += m * at(S0, q);
-        o6[4] += m * at(S1, q);
-        o6[5] += m * at(S2, q);
-      };
-      const int kind = sbp_kind(id, nd);
-      if (kind == 0 && FD) {
-        const float cf[7] = WQL_UP_CF;
-#pragma unroll
-        for (int of = -4; of <= 4; ++of) {
-          if (of >= -2) vel(o + (unsigned)of * st, cf[of + 2]);
-          if (of <= 2) flux(o + (unsigned)of * st, -cf[2 - of]);
-        }
-      } else if (kind == 0) {
-        const float cs[3] = {float(kC1), float(kC2), float(kC3)};
-#pragma unroll
-        for (int s = 1; s <= 3; ++s) {
-          vel(o + (unsigned)s * st, cs[s - 1]);
-          flux(o + (unsigned)s * st, cs[s - 1]);
-          vel(o - (unsigned)s * st, -cs[s - 1]);
-          flux(o - (unsigned)s * st, -cs[s - 1]);
-        }
-      } else {
-        // left row kind = -1-row reads points 0.., right row kind = 1+row
-        // the mirrored points with negated weights (the upwind pair swaps
-        // its two tables there)
-        const int row = kind < 0 ? -kind - 1 : kind - 1;
-        constexpr int NC = FD ? 10 : 9;
-        const float sgn = kind < 0 ? 1.0f : -1.0f;
-        const unsigned dir = kind < 0 ? st : 0u - st;
-        const float* wv = tab + (FD && kind > 0 ? 60 : 0) + row * NC;
-        const float* wf = FD ? tab + (kind > 0 ? 0 : 60) + row * NC : wv;
-        const unsigned q = o - (unsigned)row * dir;
-#pragma unroll
-        for (int t = 0; t < NC; ++t) {
-          vel(q + (unsigned)t * dir, sgn * wv[t]);
-          flux(q + (unsigned)t * dir, sgn * wf[t]);
-        }
-      }
-      const float rh = a.rh[d];
-      const float mt = CURV ? at(M, o) * Jinv : a.cart_metric[d];
+            for (int c = 0; c < 3; ++c) o6[c] += w * at(F + c * np, q);
+          },
+          [&](int off, T w) {
+            const O q = o + (O)off * st;
+            const T m = CURV ? w * at(M, q) : w;
+            o6[3] += m * at(S0, q);
+            o6[4] += m * at(S1, q);
+            o6[5] += m * at(S2, q);
+          });
+      const T rh = a.rh[d];
+      const T mt = rh * (CURV ? at(M, o) * Jinv : a.cart_metric[d]);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        gv[c] += mt * (rh * o6[c]);
+        gv[c] += mt * o6[c];
         sd[c] += rh * o6[3 + c];
       }
     };
@@ -1042,67 +688,64 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<float>& a, int i,
       direction(axis);
     }
     // Q and DQ are read after the derivatives (held across them, they spill)
-    float qv[9], dq[9];
+    T qv[9], dq[9];
     const bool forced = (hi ? ii == n - 1 : ii == 0) && a.bc[side] >= 1 && a.bc[side] <= 3;
     const long long sp = slab_point(a, side, i, j, k), snp = a.slab_np[side];
-    float* __restrict__ Q = a.Q[side] + sp;
-    float* __restrict__ DQ = a.DQ[side] + sp;
+    T* __restrict__ Q = a.Q[side] + sp;
+    T* __restrict__ DQ = a.DQ[side] + sp;
 #pragma unroll
     for (int c = 0; c < 9; ++c) {
       qv[c] = Q[c * snp];
-      dq[c] = keep || forced ? DQ[c * snp] : 0.0f;
+      dq[c] = keep || forced ? DQ[c * snp] : T(0);
     }
-    const float sc = CURV ? Jinv : a.cart_metric[axis];
+    const T sc = CURV ? Jinv : a.cart_metric[axis];
     // damping profile in grid-index units (src/RHS_Interior.f90:1855,1973,2092)
     const int off = hi ? ii + 1 - (n - npml) : (axis == 2 ? ii + 1 - npml : ii - npml);
-    const float damp = (float)a.pml_d0 * (fabsf((float)off / (float)npml));
-    const float cfs = 1.0f;
-    corr[0] -= damp * qv[0] * rhoinv;
-    corr[1] -= damp * qv[1] * rhoinv;
-    corr[2] -= damp * qv[2] * rhoinv;
-    corr[3] -= damp * (l2m * qv[3] + lam * qv[4] + lam * qv[5]);
-    corr[4] -= damp * (lam * qv[3] + l2m * qv[4] + lam * qv[5]);
-    corr[5] -= damp * (lam * qv[3] + lam * qv[4] + l2m * qv[5]);
-    corr[6] -= mu * damp * qv[6];
-    corr[7] -= mu * damp * qv[7];
-    corr[8] -= mu * damp * qv[8];
+    const T damp = (T)a.pml_d0 * (fabs((T)off / (T)npml));
+    const T cfs = T(1);
+    const T dr = damp * rhoinv, dm = mu * damp;
+    const T tr = damp * (lam * (qv[3] + qv[4] + qv[5])), d2 = dm + dm;
+    corr[0] -= dr * qv[0];
+    corr[1] -= dr * qv[1];
+    corr[2] -= dr * qv[2];
+    corr[3] -= tr + d2 * qv[3];
+    corr[4] -= tr + d2 * qv[4];
+    corr[5] -= tr + d2 * qv[5];
+    corr[6] -= dm * qv[6];
+    corr[7] -= dm * qv[7];
+    corr[8] -= dm * qv[8];
     // velocity-gradient sources (src/RHS_Interior.f90:1890-1907, 2008-2025, 2125-2142)
-    float src[9];
+    T src[9];
     src[0] = sd[0] * sc;
     src[1] = sd[1] * sc;
     src[2] = sd[2] * sc;
-    src[3] = axis == 0 ? gv[0] : 0.0f;
-    src[4] = axis == 1 ? gv[1] : 0.0f;
-    src[5] = axis == 2 ? gv[2] : 0.0f;
-    src[6] = axis == 0 ? gv[1] : (axis == 1 ? gv[0] : 0.0f);
-    src[7] = axis == 0 ? gv[2] : (axis == 2 ? gv[0] : 0.0f);
-    src[8] = axis == 1 ? gv[2] : (axis == 2 ? gv[1] : 0.0f);
+    src[3] = axis == 0 ? gv[0] : T(0);
+    src[4] = axis == 1 ? gv[1] : T(0);
+    src[5] = axis == 2 ? gv[2] : T(0);
+    src[6] = axis == 0 ? gv[1] : (axis == 1 ? gv[0] : T(0));
+    src[7] = axis == 0 ? gv[2] : (axis == 2 ? gv[0] : T(0));
+    src[8] = axis == 1 ? gv[2] : (axis == 2 ? gv[1] : T(0));
+    const T dc = damp + cfs;
 #pragma unroll
     for (int c = 0; c < 9; ++c) {
-      const float nw = (keep ? a.A * dq[c] : dq[c]) + src[c] - (damp + cfs) * qv[c];
+      const T nw = (keep ? a.A * dq[c] : dq[c]) + src[c] - dc * qv[c];
       DQ[c * snp] = nw;
       Q[c * snp] = qv[c] + a.Bdt * nw;
     }
   }
   const bool face = i == 0 || i == nq - 1 || j == 0 || j == nr - 1 || k == 0 || k == ns - 1;
-  const float inv = keep ? 1.0f / a.A : 1.0f;
-  float df[9];
+  const T inv = keep ? T(1) / a.A : T(1);
+  T df[9];
 #pragma unroll
-  for (int c = 0; c < 9; ++c) df[c] = keep || face ? at(a.DF + c * np, o) : 0.0f;
+  for (int c = 0; c < 9; ++c) df[c] = keep || face ? at(a.DF + c * np, o) : T(0);
 #pragma unroll
-  for (int c = 0; c < 9; ++c)
-    *reinterpret_cast<float*>(reinterpret_cast<char*>(a.DF + c * np) + o) = df[c] + corr[c] * inv;
+  for (int c = 0; c < 9; ++c) at(a.DF + c * np, o) = df[c] + corr[c] * inv;
 }
 
-template <bool CURV, int FD>
-__global__ void __launch_bounds__(256, 3) pml_pre_kernel(const __grid_constant__ PmlPair<float> P) {
-  __shared__ float tab[120];
-  if (FD) {
-    if (threadIdx.x < 120) tab[threadIdx.x] = (&c_up_f[0][0][0])[threadIdx.x];
-  } else if (threadIdx.x < 54) {
-    tab[threadIdx.x] = (&c_sbp_f[0][0])[threadIdx.x];
-  }
-  __syncthreads();
+template <typename T, typename O, bool CURV, int FD>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) pml_pre_kernel(const __grid_constant__ PmlPair<T> P) {
+  __shared__ T tab[kRowWords<FD>];
+  load_rows<T, FD>(tab, P.a[0].ug);
   const int blk = (int)blockIdx.x >= P.n0 ? 1 : 0;
   const int t = (int)blockIdx.x - (blk ? P.n0 : 0);
   const PmlTiles& B = P.t[blk];
@@ -1115,25 +758,40 @@ __global__ void __launch_bounds__(256, 3) pml_pre_kernel(const __grid_constant__
   const int j = (br << lr) + ((e >> lw) & ((1 << lr) - 1));
   const int k = (bs << (8 - lw - lr)) + (e >> (lw + lr));
   if (i >= B.dim[b][0] || j >= B.dim[b][1] || k >= B.dim[b][2]) return;
-  pml_pre_point<CURV, FD>(P.a[blk], B.lo[b][0] + i, B.lo[b][1] + j, B.lo[b][2] + k, (unsigned)B.sides[b], tab);
+  pml_pre_point<T, O, CURV, FD>(P.a[blk], B.lo[b][0] + i, B.lo[b][1] + j, B.lo[b][2] + k, (unsigned)B.sides[b], tab);
+}
+
+template <typename T, typename O, bool CURV>
+void launch_pml_pre_fd(const PmlPair<T>& P, unsigned g, cudaStream_t s) {
+  switch (P.a[0].fd) {
+    case 0: pml_pre_kernel<T, O, CURV, 0><<<g, 256, 0, s>>>(P); return;
+    case 1: pml_pre_kernel<T, O, CURV, 1><<<g, 256, 0, s>>>(P); return;
+    case 2: pml_pre_kernel<T, O, CURV, 2><<<g, 256, 0, s>>>(P); return;
+    default: pml_pre_kernel<T, O, CURV, 3><<<g, 256, 0, s>>>(P); return;
+  }
 }
 
 // Launches the PML pre-kernel over one block (a1 null) or two.
-int launch_pml_pre(const VolumeArgs<float>& a0, const VolumeArgs<float>* a1, bool curv, cudaStream_t s) {
-  PmlPair<float> P;
-  const VolumeArgs<float>* a[2] = {&a0, a1 ? a1 : &a0};
+template <typename T>
+int launch_pml_pre(const VolumeArgs<T>& a0, const VolumeArgs<T>* a1, bool curv, cudaStream_t s) {
+  if (a0.npml == 0 && !(a1 && a1->npml)) return 0;
+  PmlPair<T> P;
+  const VolumeArgs<T>* a[2] = {&a0, a1 ? a1 : &a0};
   int n[2];
+  bool wide = sizeof(T) == 8;
   for (int b = 0; b < 2; ++b) {
     P.a[b] = *a[b];
     P.t[b] = pml_tiles(*a[b]);
-    n[b] = a[b]->pml_pre ? P.t[b].start[P.t[b].n] : 0;
+    n[b] = a[b]->npml > 0 ? P.t[b].start[P.t[b].n] : 0;
+    wide = wide || a[b]->np >= (1LL << 30);
   }
   if (!a1) n[1] = 0;
   P.n0 = n[0];
   if (n[0] + n[1] == 0) return 0;
   const unsigned g = (unsigned)(n[0] + n[1]);
-  if (a0.fd) curv ? pml_pre_kernel<true, 1><<<g, 256, 0, s>>>(P) : pml_pre_kernel<false, 1><<<g, 256, 0, s>>>(P);
-  else curv ? pml_pre_kernel<true, 0><<<g, 256, 0, s>>>(P) : pml_pre_kernel<false, 0><<<g, 256, 0, s>>>(P);
+  if (wide) curv ? launch_pml_pre_fd<T, size_t, true>(P, g, s) : launch_pml_pre_fd<T, size_t, false>(P, g, s);
+  else if constexpr (sizeof(T) == 4)
+    curv ? launch_pml_pre_fd<T, unsigned, true>(P, g, s) : launch_pml_pre_fd<T, unsigned, false>(P, g, s);
   return 1;
 }
 
@@ -1150,11 +808,13 @@ int launch_pml_pre(const VolumeArgs<float>& a0, const VolumeArgs<float>* a1, boo
 //   Deta <- A*Deta + (relaxed strain-rate forcing - eta) / tau
 // and eta <- eta + B*dt*Deta.  Inside a PML slab the strain rates lose the
 // damped auxiliary fields (pml_damping_and_q, src/RHS_Interior.f90:
-// 2287-2387), so this kernel runs before the PML kernel advances Q.  The
+// 2287-2387) of the stage's input.  The
 // velocity gradient comes from the TMA stencil (FP32C) or is formed here
 // with the block's operator.
 template <typename T, bool CURV, bool KAHAN, int FD>
 __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __grid_constant__ VolumeArgs<T> a) {
+  __shared__ T tab[kRowWords<FD>];
+  if (a.G == nullptr) load_rows<T, FD>(tab, a.ug);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -1163,7 +823,6 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
   const long long np = a.np;
   const long long p = i + (long long)a.pq * (j + (long long)nr * k);
   const int idx[3] = {i, j, k}, nn[3] = {nq, nr, ns};
-  const long long st[3] = {1, a.pq, (long long)a.pq * nr};
   const T* __restrict__ F = a.Fin;
   const T* __restrict__ coef = a.coef;
   const T Jinv = CURV ? coef[9 * np + p] : T(1);
@@ -1177,12 +836,18 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
       for (int jj = 0; jj < 3; ++jj) g[c][jj] = a.G[(c * 3 + jj) * np + p];
   }
   if (a.G == nullptr) {
+    const bool shell = FD == 3 && ug_shell(a, i, j, k);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      T o[3];
-      if (FD == 3) diff_v_ug<T>(F, np, p, idx[d], nn[d], st[d], d, a.ug, ug_shell(a, idx, nn), o);
-      else if (FD) diff_v_up<T, FD == 3 ? 1 : (FD ? FD : 1)>(F, np, p, idx[d], nn[d], st[d], d, o);
-      else diff_v<T>(F, np, p, idx[d], nn[d], st[d], o);
+      const long long st = d == 0 ? 1 : (d == 1 ? (long long)a.pq : (long long)a.pq * nr);
+      T o[3] = {T(0), T(0), T(0)};
+      visit_row<T, FD>(
+          tab, a.ug, shell, idx[d], nn[d], d,
+          [&](int off, T w) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[c] += w * F[c * np + p + off * st];
+          },
+          [](int, T) {});
       const T rh = a.rh[d];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -1228,9 +893,9 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
       const long long snp = a.slab_np[side];
       const T* Q = a.Q[side];
       const T* DQ = a.DQ[side];
-      // the stage-input Q; after the PML pre-kernel has advanced it by
-      // B*dt*DQ that step is taken back (to the rounding of Q)
-      auto q_in = [&](int c) { return a.pml_pre ? Q[c * snp + sp] - a.Bdt * DQ[c * snp + sp] : Q[c * snp + sp]; };
+      // the stage-input Q: the PML pre-kernel has advanced it by B*dt*DQ,
+      // which is taken back (to the rounding of Q)
+      auto q_in = [&](int c) { return Q[c * snp + sp] - a.Bdt * DQ[c * snp + sp]; };
       // Q components of the normal strain and the two shear strains of this axis
       const int cn = 3 + axis;
       const int c1 = axis == 0 ? 6 : (axis == 1 ? 6 : 7);
@@ -1312,47 +977,10 @@ __global__ void __launch_bounds__(256) mms_kernel(const __grid_constant__ Volume
 }
 
 // ---------------------------------------------------------------------------
-// Face kernel: outer-boundary SAT (src/RHS_Interior.f90:1516-1703 with
+// Face pre-kernel: the outer-boundary SAT (src/RHS_Interior.f90:1516-1703 with
 // src/BoundaryConditions.f90:777-918 + structure(), or the weighted form of
 // src/BoundaryConditions3.f90:777-903) and the fault SAT computed by the
-// interface kernel (src/RHS_Interior.f90:1757-1772).  One thread per face
-// point; a point on several faces is handled once, by its lowest side.
-template <typename T, bool KAHAN>
-__global__ void __launch_bounds__(256) face_kernel(const __grid_constant__ VolumeArgs<T> a) {
-  const int nq = a.nq, nr = a.nr, ns = a.ns;
-  const long long nfs[6] = {(long long)nr * ns, (long long)nr * ns, (long long)nq * ns, (long long)nq * ns,
-                            (long long)nq * nr, (long long)nq * nr};
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  int side = 0;
-  while (side < 6 && t >= nfs[side]) {
-    t -= nfs[side];
-    ++side;
-  }
-  if (side >= 6) return;
-  const int axis = side >> 1;
-  int i, j, k;
-  if (axis == 0) { i = (side & 1) ? nq - 1 : 0; j = (int)(t % nr); k = (int)(t / nr); }
-  else if (axis == 1) { i = (int)(t % nq); j = (side & 1) ? nr - 1 : 0; k = (int)(t / nq); }
-  else { i = (int)(t % nq); j = (int)(t / nq); k = (side & 1) ? ns - 1 : 0; }
-  const int idx[3] = {i, j, k}, nn[3] = {nq, nr, ns};
-  // owner: the lowest side containing the point
-  for (int s2 = 0; s2 < side; ++s2) {
-    const int ax2 = s2 >> 1;
-    if (idx[ax2] == ((s2 & 1) ? nn[ax2] - 1 : 0)) return;
-  }
-  const long long np = a.np;
-  const long long p = i + (long long)a.pq * (j + (long long)nr * k);
-  T u[9], tot[9], corr[9];
-  for (int c = 0; c < 9; ++c) u[c] = a.Fin[c * np + p];
-  mms_deviation(a, p, u);
-  const bool any = face_penalty(a, i, j, k, u, tot, [](int, const T (&)[9]) {});
-  for (int c = 0; c < 9; ++c) corr[c] = -tot[c];
-  if (any) add_correction<T, KAHAN>(a, p, corr);
-}
-
-// ---------------------------------------------------------------------------
-// Face pre-kernel (for the stencil variant without a face pass): the
-// boundary and fault penalty tot of each face point (as in the face kernel)
+// interface kernel (src/RHS_Interior.f90:1757-1772) of each face point, tot,
 // folded into the rates before the stencil kernel runs, DF <- DF - tot/A, or
 // DF <- -tot on a stage with A = 0, so that the stencil's A*DF + du (or
 // DF + du on face points when A = 0) carries it.  On a PML side the same
@@ -1360,7 +988,7 @@ __global__ void __launch_bounds__(256) face_kernel(const __grid_constant__ Volum
 // (src/RHS_Interior.f90:1560-1700): it is folded into DQ in the same way,
 // for the PML pre-kernel to pick up.  One thread per face point, a point on
 // several faces taken by its lowest side.
-template <typename T>
+template <typename T, bool PML>
 __device__ __forceinline__ void face_pre_point(const VolumeArgs<T>& a, long long t) {
   const int nq = a.nq, nr = a.nr, ns = a.ns;
   const long long nfs[6] = {(long long)nr * ns, (long long)nr * ns, (long long)nq * ns, (long long)nq * ns,
@@ -1397,7 +1025,7 @@ __device__ __forceinline__ void face_pre_point(const VolumeArgs<T>& a, long long
   }
   mms_deviation(a, p, u);
   face_penalty(a, i, j, k, u, tot, [&](int s2, const T (&ubc)[9]) {
-    if (!a.pml_pre || !a.pml[s2]) return;
+    if (!PML || !a.pml[s2]) return;
     const long long sp = slab_point(a, s2, i, j, k), snp = a.slab_np[s2];
     const T th = a.tau_h[s2 >> 1];
     T* DQ = a.DQ[s2];
@@ -1409,25 +1037,15 @@ __device__ __forceinline__ void face_pre_point(const VolumeArgs<T>& a, long long
   for (int c = 0; c < 9; ++c) a.DF[c * np + p] = keep ? df[c] - tot[c] / a.A : -tot[c];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) face_pre_kernel(const __grid_constant__ VolumeArgs<T> a) {
-  face_pre_point(a, blockIdx.x * (long long)blockDim.x + threadIdx.x);
-}
-
-// Both blocks of a scenario in one launch: threads [0, n0) take block 0's
-// face points, the rest block 1's (one launch of about twice the threads
-// hides the latency of these sub-wave launches better than two).
-template <typename T>
-struct FacePair {
-  VolumeArgs<T> a[2];
-  long long n0;
-};
-
-template <typename T>
-__global__ void __launch_bounds__(256) face_pre_kernel2(const __grid_constant__ FacePair<T> P) {
+// One launch covers one block or both of a scenario: threads [0, n0) take
+// block 0's face points, the rest block 1's (one launch of about twice the
+// threads hides the latency of these sub-wave launches better than two).
+// PML: some side has a slab.
+template <typename T, bool PML>
+__global__ void __launch_bounds__(256) face_pre_kernel(const __grid_constant__ BlockPair<T> P) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t < P.n0) face_pre_point(P.a[0], t);
-  else face_pre_point(P.a[1], t - P.n0);
+  if (t < P.n0) face_pre_point<T, PML>(P.a[0], t);
+  else face_pre_point<T, PML>(P.a[1], t - P.n0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1552,9 +1170,9 @@ void launch_tiled(const VolumeArgs<T>& a, cudaStream_t s) {
 
 // Stencil-kernel variants (the tuning table): 1 per-point, 2 tiled 32x8 at
 // 1 CTA/SM, 3 tiled 32x8 at 3 CTAs/SM in FP32, 4 tiled 64x8 at 1 CTA/SM,
-// 5 TMA-pipelined (FP32), 6 accepted as 5; 0 picks the
-// fastest measured on a 2 x 201^3 curvilinear block pair (TMA in FP32,
-// tiled 32x8 in FP64).
+// 5 TMA-pipelined (FP32), 6 accepted as 5; 0 picks the TMA kernel in FP32
+// and in FP64 the kernel of wql_stencil_fp64.cu (7 here; blocks with an axis
+// under 12 points take the tiled kernel).
 //
 // A tiled axis of n points with tiles of T keeps every closure row inside
 // the tile that owns it plus a 3-point halo unless the shifted last tile
@@ -1568,7 +1186,7 @@ inline bool tiles_ok_up(int n, int T) { return n <= T + 4 || n >= T + 6; }
 template <typename T>
 int effective_variant(const VolumeArgs<T>& a) {
   constexpr bool f32 = sizeof(T) == 4;
-  int v = a.kernel != 0 ? a.kernel : (f32 ? 5 : 2);
+  int v = a.kernel != 0 ? a.kernel : (f32 ? 5 : (a.plan64 && a.plan64->ok && !a.fd ? 7 : 2));
   if ((v == 5 || v == 6) && !(f32 && a.C != nullptr)) v = 2;
   if (a.fd) {
     // the order-6 upwind pair: the TMA kernel (compensated FP32) or per
@@ -1582,9 +1200,7 @@ int effective_variant(const VolumeArgs<T>& a) {
   return v;
 }
 
-// Whether the block's stencil runs as the TMA kernel.  Its penalties are
-// folded into DF beforehand by the face pre-kernel (launch_pre); the other
-// variants get them afterwards from the face kernel (launch_corrections).
+// Whether the block's stencil runs as the TMA kernel.
 template <typename T>
 bool stencil_is_tma(const VolumeArgs<T>& a) {
   const int v = effective_variant(a);
@@ -1592,24 +1208,38 @@ bool stencil_is_tma(const VolumeArgs<T>& a) {
 }
 
 template <typename T, bool CURV, bool KAHAN>
+void launch_pointwise(const VolumeArgs<T>& a0, const VolumeArgs<T>* a1, cudaStream_t s) {
+  BlockPair<T> P;
+  P.a[0] = a0;
+  P.a[1] = a1 ? *a1 : a0;
+  P.n0 = a0.ns;
+  dim3 blk(32, 8, 1), grd((std::max(a0.nq, P.a[1].nq) + 31) / 32, (a0.nr + 7) / 8, a0.ns + (a1 ? a1->ns : 0));
+  switch (a0.fd) {
+    case 0: stencil_kernel_pointwise<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(P); return;
+    case 1: stencil_kernel_pointwise<T, CURV, KAHAN, 1><<<grd, blk, 0, s>>>(P); return;
+    case 2: stencil_kernel_pointwise<T, CURV, KAHAN, 2><<<grd, blk, 0, s>>>(P); return;
+    default: stencil_kernel_pointwise<T, CURV, KAHAN, 3><<<grd, blk, 0, s>>>(P); return;
+  }
+}
+
+template <typename T, bool CURV, bool KAHAN>
 void launch_stencil(const VolumeArgs<T>& a, cudaStream_t s) {
   constexpr bool f32 = sizeof(T) == 4;
   const int v = effective_variant(a);
   switch (v) {
-    case 1: {
-      dim3 blk(32, 8, 1), grd((a.nq + 31) / 32, (a.nr + 7) / 8, a.ns);
-      if (a.fd == 1) stencil_kernel_pointwise<T, CURV, KAHAN, 1><<<grd, blk, 0, s>>>(a, 0);
-      else if (a.fd == 2) stencil_kernel_pointwise<T, CURV, KAHAN, 2><<<grd, blk, 0, s>>>(a, 0);
-      else if (a.fd == 3) stencil_kernel_pointwise<T, CURV, KAHAN, 3><<<grd, blk, 0, s>>>(a, 0);
-      else stencil_kernel_pointwise<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(a, 0);
-      return;
-    }
+    case 1: launch_pointwise<T, CURV, KAHAN>(a, nullptr, s); return;
     case 3: launch_tiled<T, CURV, KAHAN, 32, 8, f32 ? 3 : 1>(a, s); return;
     case 4: launch_tiled<T, CURV, KAHAN, 64, 8, 1>(a, s); return;
     case 5:
     case 6:
       if constexpr (f32 && KAHAN) {
         launch_stencil_tma(a, CURV, s);
+        return;
+      }
+      [[fallthrough]];
+    case 7:
+      if constexpr (!f32) {
+        launch_stencil_fp64(a, nullptr, CURV, s);
         return;
       }
       [[fallthrough]];
@@ -1621,27 +1251,11 @@ template <typename T, bool CURV, bool KAHAN>
 int launch_corr(const VolumeArgs<T>& a, cudaStream_t s) {
   int n = 0;
   dim3 blk(32, 8, 1), grd((a.nq + 31) / 32, (a.nr + 7) / 8, a.ns);
-  if (a.anel) {  // before the PML kernel: it reads Q of the stage's input
+  if (a.anel) {
     if (a.fd == 1) anelastic_kernel<T, CURV, KAHAN, 1><<<grd, blk, 0, s>>>(a);
     else if (a.fd == 2) anelastic_kernel<T, CURV, KAHAN, 2><<<grd, blk, 0, s>>>(a);
     else if (a.fd == 3) anelastic_kernel<T, CURV, KAHAN, 3><<<grd, blk, 0, s>>>(a);
     else anelastic_kernel<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(a);
-    ++n;
-  }
-  if (a.npml > 0 && !a.pml_pre) {
-    const PmlBoxes bx = pml_boxes(a);
-    const unsigned nblk = (unsigned)((bx.start[bx.n] + 255) / 256);
-    if (bx.start[bx.n] > 0) {
-      if (a.fd == 1) pml_kernel<T, CURV, KAHAN, 1><<<nblk, 256, 0, s>>>(a, bx);
-      else if (a.fd == 2) pml_kernel<T, CURV, KAHAN, 2><<<nblk, 256, 0, s>>>(a, bx);
-      else if (a.fd == 3) pml_kernel<T, CURV, KAHAN, 3><<<nblk, 256, 0, s>>>(a, bx);
-      else pml_kernel<T, CURV, KAHAN, 0><<<nblk, 256, 0, s>>>(a, bx);
-    }
-    ++n;
-  }
-  if (!stencil_is_tma(a)) {
-    const long long nface = 2LL * ((long long)a.nr * a.ns + (long long)a.nq * a.ns + (long long)a.nq * a.nr);
-    face_kernel<T, KAHAN><<<(unsigned)((nface + 255) / 256), 256, 0, s>>>(a);
     ++n;
   }
   if (a.mp) {
@@ -1678,26 +1292,36 @@ void launch_volume(const VolumeArgs<T>& a, bool curv, void* stream) {
 }
 
 template <typename T>
-int launch_pre(const VolumeArgs<T>& a, bool curv, void* stream) {
-  if (!stencil_is_tma(a)) return 0;
-  const long long nface = 2LL * ((long long)a.nr * a.ns + (long long)a.nq * a.ns + (long long)a.nq * a.nr);
-  face_pre_kernel<T><<<(unsigned)((nface + 255) / 256), 256, 0, (cudaStream_t)stream>>>(a);
-  if constexpr (sizeof(T) == 4) return 1 + launch_pml_pre(a, nullptr, curv, (cudaStream_t)stream);
-  return 1;
-}
-
-template <typename T>
-int launch_pre2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, bool curv, void* stream) {
-  FacePair<T> P;
+int launch_pre(const VolumeArgs<T>& a0, const VolumeArgs<T>* a1, bool curv, void* stream) {
+  BlockPair<T> P;
   P.a[0] = a0;
-  P.a[1] = a1;
+  P.a[1] = a1 ? *a1 : a0;
   auto nface = [](const VolumeArgs<T>& a) {
     return 2LL * ((long long)a.nr * a.ns + (long long)a.nq * a.ns + (long long)a.nq * a.nr);
   };
   P.n0 = nface(a0);
-  const long long n = P.n0 + nface(a1);
-  face_pre_kernel2<T><<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(P);
-  return 1 + launch_pml_pre(a0, &a1, curv, (cudaStream_t)stream);
+  const long long n = P.n0 + (a1 ? nface(*a1) : 0);
+  const unsigned g = (unsigned)((n + 255) / 256);
+  if (a0.npml > 0 || (a1 && a1->npml > 0)) face_pre_kernel<T, true><<<g, 256, 0, (cudaStream_t)stream>>>(P);
+  else face_pre_kernel<T, false><<<g, 256, 0, (cudaStream_t)stream>>>(P);
+  return 1 + launch_pml_pre(a0, a1, curv, (cudaStream_t)stream);
+}
+
+template <typename T>
+int launch_volume2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, bool curv, void* stream) {
+  const int v = effective_variant(a0);
+  if (v != effective_variant(a1) || !(v == 1 || v == 5 || v == 6 || v == 7)) return 0;
+  cudaStream_t s = (cudaStream_t)stream;
+  const bool kahan = a0.C != nullptr;
+  if (v == 1) {
+    if (a0.nr != a1.nr) return 0;
+    if (curv) kahan ? launch_pointwise<T, true, true>(a0, &a1, s) : launch_pointwise<T, true, false>(a0, &a1, s);
+    else kahan ? launch_pointwise<T, false, true>(a0, &a1, s) : launch_pointwise<T, false, false>(a0, &a1, s);
+    return 1;
+  }
+  if constexpr (sizeof(T) == 4) launch_stencil_tma2(a0, a1, curv, stream);
+  else launch_stencil_fp64(a0, &a1, curv, stream);
+  return 1;
 }
 
 template <typename T>
@@ -1736,9 +1360,10 @@ template void launch_source<float>(const VolumeArgs<float>&, const int*, const i
 template void launch_volume<double>(const VolumeArgs<double>&, bool, void*);
 template void launch_volume<float>(const VolumeArgs<float>&, bool, void*);
 template int launch_corrections<double>(const VolumeArgs<double>&, bool, void*);
-template int launch_pre<double>(const VolumeArgs<double>&, bool, void*);
-template int launch_pre<float>(const VolumeArgs<float>&, bool, void*);
-template int launch_pre2<float>(const VolumeArgs<float>&, const VolumeArgs<float>&, bool, void*);
+template int launch_pre<double>(const VolumeArgs<double>&, const VolumeArgs<double>*, bool, void*);
+template int launch_pre<float>(const VolumeArgs<float>&, const VolumeArgs<float>*, bool, void*);
+template int launch_volume2<double>(const VolumeArgs<double>&, const VolumeArgs<double>&, bool, void*);
+template int launch_volume2<float>(const VolumeArgs<float>&, const VolumeArgs<float>&, bool, void*);
 template int launch_corrections<float>(const VolumeArgs<float>&, bool, void*);
 template bool stencil_is_tma<float>(const VolumeArgs<float>&);
 template bool stencil_is_tma<double>(const VolumeArgs<double>&);
