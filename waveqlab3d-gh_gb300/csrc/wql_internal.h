@@ -202,9 +202,10 @@ constexpr int kFrameOff[9] = {FR_UFACE, FR_VFACE, FR_S, FR_UHAT, FR_VHAT, FR_SVE
 // three stages, 32 x 10 and 64 x 6 on 2 x 201^3 blocks).
 constexpr int kTmaTQ = 32, kTmaTR = 12, kTmaStages = 2;
 // Cartesian blocks whose q extent fills 40-wide tiles better (76 points: 2
-// tiles of 40 use 95 % of their columns, 3 of 32 use 79 %) take this width;
-// 15 consumer warps, the same 128-register cap.
+// tiles of 40 use 95 % of their columns, 3 of 32 use 79 %) take 40 x 8 tiles:
+// five whole consumer warps a role.
 constexpr int kTmaTQWide = 40;
+constexpr int tma_rows(int tq) { return tq == kTmaTQWide ? 8 : kTmaTR; }
 struct StencilMaps {
   CUtensorMap fbox[2], flead[2];  // per field buffer
   CUtensorMap ca, cb, cc, cl;     // coefficients: q-halo rows, r-halo columns, tile, lead plane

@@ -25,21 +25,31 @@
 //                      the remaining 7 coefficients, the rates DF and the
 //                      compensation C on the tile;
 //   lead (plane s+3) : the 9 field components and J*metric_s on the tile.
-// Each consumer thread works on two neighbouring q points with packed FP32
-// instructions (a point per thread took about 900 issue slots a plane, a pair
-// takes about 1100 at twice the points: 0.774 -> 0.756 ms per launch on 2 x
-// 201^3, 0.140 -> 0.124 ms on the 2 x 76x101x151 upwind pair) and keeps the
-// velocities and the s-face momentum flux of planes s-3..s+3 in registers (the first six read directly at
-// the start of a chunk, then one pushed per step from the lead tile), so
-// the s derivative of a central row needs no shared memory (lead planes
-// outside 0..ns-1 load as zeros and are never used: the 12 s closure rows
-// take the planes of their stencil that the window holds from it and read
-// the at most three others from global memory); the q and r derivatives read the
-// main box, the curvilinear q and r fluxes formed once per box point into
-// the stage (one mbarrier phase among the consumer threads per step).  The r
-// tiles follow the ownership rule of tile_span (the last
-// tile is shifted to end on the last point), which keeps every r closure row
-// inside tile + halo.  DF, F_out and C are stored directly from registers.
+// Two roles of consumer threads cover the tile, each thread two neighbouring q
+// points with packed FP32 instructions: the stress threads difference the
+// velocities and update the six stresses, the velocity threads form and
+// difference the momentum fluxes and update the three velocities.  They share
+// only the stage's data.  What bounded the kernel was a warp's own instruction
+// chain, about 3000 cycles a plane whether four or six warps took the tile
+// (one point a thread: 900 issue slots; two: 1100), longer than a plane's
+// loads at the rate of HBM; with the roles each chain is half as long and an
+// SM has twelve of them (three a scheduler).  2 x 201^3 curvilinear, per
+// launch: 0.779 ms one point a thread, 0.756 two, 0.725 with the roles = 77 %
+// of the measured HBM rate; 2 x 101/93x107x113 150, 150, 142 us.  32 x 8 tiles
+// with three stages ran 0.757 ms there (more halo).
+// A role keeps its three quantities of planes s-3..s+3 (velocities, or s-face
+// fluxes) in registers (the first six read directly at the start of a chunk,
+// then one pushed per step from the lead tile), so the s derivative of a
+// central row needs no shared memory (lead planes outside 0..ns-1 load as
+// zeros and are never used: the 12 s closure rows take the planes of their
+// stencil that the window holds from it and read the at most three others
+// from global memory); the q and r derivatives read the main box, the
+// curvilinear q and r fluxes formed once per box point into the stage, over
+// the metrics they come from, after the stress threads have taken theirs (one
+// mbarrier phase from them, one among the velocity threads per step).  The r
+// tiles follow the ownership rule of tile_span (the last tile is shifted to
+// end on the last point), which keeps every r closure row inside tile + halo.
+// DF, F_out and C are stored directly from registers.
 //
 // Every mbarrier wait is bounded; a wait that runs out sets *err and the
 // thread leaves its loop (the producer first waits, again bounded, for the
@@ -59,8 +69,9 @@ namespace {
 
 template <bool CURV, int FD, int TQ_ = kTmaTQ>
 struct TmaTile {
-  static constexpr int TQ = TQ_, TR = kTmaTR, NC = TQ * TR;
-  static constexpr int NT = (NC / 2 + 31) / 32 * 32;  // consumer threads: one per two q points, whole warps
+  static constexpr int TQ = TQ_, TR = tma_rows(TQ_), NC = TQ * TR;
+  static constexpr int NS = CURV ? kTmaStages : 3;  // ring depth: what fits in shared memory
+  static constexpr int NT = (NC / 2 + 31) / 32 * 32;  // consumer threads of a role: one per two q points, whole warps
   // r halo: 3 rows for the central operator, 4 for the upwind pair
   static constexpr int HR = FD ? 4 : 3;
   static constexpr int BQ = TQ + 16, BR = TR + 2 * HR;  // field box: q from q0-8, r from r0-HR
@@ -182,83 +193,490 @@ __device__ __forceinline__ unsigned bf16_pair(float lo, float hi) {
   return r;
 }
 
-// s derivative of the six differenced quantities on a closure row (planes
-// 0..5 and ns-6..ns-1).  The s window already holds most of the planes a
-// closure row reads (planes s-3..s+3 for the central operator; velocities of
-// s-2..s+4 and fluxes of s-4..s+2 for the upwind pair); the at most three
-// planes of a row outside it are read from global memory.  Each row is a
-// separate instantiation (the weights, offsets and window positions are
+__device__ __forceinline__ f2 g2(const float* p) { return *reinterpret_cast<const f2*>(p); }
+
+// s derivative of the three velocities (VEL) or momentum fluxes on a closure
+// row (planes 0..5 and ns-6..ns-1).  The s window already holds most of the
+// planes a closure row reads (planes s-3..s+3 for the central operator;
+// velocities of s-2..s+4 and fluxes of s-4..s+2 for the upwind pair); the at
+// most three planes of a row outside it are read from global memory.  Each row
+// is a separate instantiation (the weights, offsets and window positions are
 // compile-time constants, so the window stays in registers); the columns are
 // summed in the order of the operator table, zero weights skipped.
-template <bool CURV, int FD, int ROW, bool RIGHT, int T>
-__device__ __forceinline__ void s_close_col(const VolumeArgs<float>& a, long long p, const f2 (&qv)[7][6],
-                                            f2 acc[6]) {
-  constexpr float wv = (float)s_close_w(FD, RIGHT, false, ROW, T);
-  constexpr float wf = (float)s_close_w(FD, RIGHT, true, ROW, T);
+template <bool CURV, int FD, bool VEL, int ROW, bool RIGHT, int T>
+__device__ __forceinline__ void s_close_col(const VolumeArgs<float>& a, long long p, const f2 (&qv)[7][3],
+                                            f2 (&acc)[3]) {
+  constexpr float w = (float)s_close_w(FD, RIGHT, !VEL, ROW, T);
   constexpr int off = s_close_off(RIGHT, ROW, T);  // plane offset from s
-  constexpr int iv = s_close_vpos(FD, RIGHT, ROW, T), iflux = s_close_fpos(FD, RIGHT, ROW, T);
-  const long long np = a.np, pp = p + off * ((long long)a.pq * a.nr);
-  const float* F = a.Fin;
-  auto g2 = [&](const float* base) { return *reinterpret_cast<const f2*>(base + pp); };
-  if constexpr (wv != 0.0f) {
+  constexpr int iw = VEL ? s_close_vpos(FD, RIGHT, ROW, T) : s_close_fpos(FD, RIGHT, ROW, T);
+  if constexpr (w != 0.0f) {
     f2 x[3];
-    if constexpr (iv >= 0 && iv <= 6) {
+    if constexpr (iw >= 0 && iw <= 6) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = qv[iv][c];
+      for (int c = 0; c < 3; ++c) x[c] = qv[iw][c];
     } else {
+      const long long np = a.np, pp = p + off * ((long long)a.pq * a.nr);
+      const float* F = a.Fin + pp;
+      if constexpr (VEL) {
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = g2(F + c * np);
+        for (int c = 0; c < 3; ++c) x[c] = g2(F + c * np);
+      } else if constexpr (CURV) {
+        const float* M = a.coef + pp;
+        const f2 a0 = g2(M + 6 * np), a1 = g2(M + 7 * np), a2 = g2(M + 8 * np);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          x[c] = dot3(a0, g2(F + sig(c, 0) * np), a1, g2(F + sig(c, 1) * np), a2, g2(F + sig(c, 2) * np));
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[c] = g2(F + sig(c, 2) * np);
+      }
     }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) acc[c] = fma2(pack(wv, wv), x[c], acc[c]);
-  }
-  if constexpr (wf != 0.0f) {
-    f2 x[3];
-    if constexpr (iflux >= 0 && iflux <= 6) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = qv[iflux][3 + c];
-    } else if constexpr (CURV) {
-      const f2 a0 = g2(a.coef + 6 * np), a1 = g2(a.coef + 7 * np), a2 = g2(a.coef + 8 * np);
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        x[c] = dot3(a0, g2(F + sig(c, 0) * np), a1, g2(F + sig(c, 1) * np), a2, g2(F + sig(c, 2) * np));
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) x[c] = g2(F + sig(c, 2) * np);
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) acc[3 + c] = fma2(pack(wf, wf), x[c], acc[3 + c]);
+    for (int c = 0; c < 3; ++c) acc[c] = fma2(pack(w, w), x[c], acc[c]);
   }
 }
 
-template <bool CURV, int FD, int ROW, bool RIGHT, int... T>
-__device__ __forceinline__ void s_close_row(const VolumeArgs<float>& a, long long p, const f2 (&qv)[7][6],
-                                            f2 o[6], std::integer_sequence<int, T...>) {
-  f2 acc[6] = {0, 0, 0, 0, 0, 0};
-  (s_close_col<CURV, FD, ROW, RIGHT, T>(a, p, qv, acc), ...);
+template <bool CURV, int FD, bool VEL, int ROW, bool RIGHT, int... T>
+__device__ __forceinline__ void s_close_row(const VolumeArgs<float>& a, long long p, const f2 (&qv)[7][3], f2 (&o)[3],
+                                            std::integer_sequence<int, T...>) {
 #pragma unroll
-  for (int c = 0; c < 6; ++c) o[c] = acc[c];
+  for (int c = 0; c < 3; ++c) o[c] = 0;
+  (s_close_col<CURV, FD, VEL, ROW, RIGHT, T>(a, p, qv, o), ...);
 }
 
 // ks = sbp_kind(s, ns), nonzero: -1..-6 left rows 0..5, 1..6 right rows 0..5.
-template <bool CURV, int FD>
-__device__ __forceinline__ void s_closure(const VolumeArgs<float>& a, long long p, int ks, const f2 (&qv)[7][6],
-                                          f2 o[6]) {
+template <bool CURV, int FD, bool VEL>
+__device__ __forceinline__ void s_closure(const VolumeArgs<float>& a, long long p, int ks, const f2 (&qv)[7][3],
+                                          f2 (&o)[3]) {
   using Cols = std::make_integer_sequence<int, FD ? 10 : 9>;
   switch (ks) {
-    case -1: s_close_row<CURV, FD, 0, false>(a, p, qv, o, Cols{}); break;
-    case -2: s_close_row<CURV, FD, 1, false>(a, p, qv, o, Cols{}); break;
-    case -3: s_close_row<CURV, FD, 2, false>(a, p, qv, o, Cols{}); break;
-    case -4: s_close_row<CURV, FD, 3, false>(a, p, qv, o, Cols{}); break;
-    case -5: s_close_row<CURV, FD, 4, false>(a, p, qv, o, Cols{}); break;
-    case -6: s_close_row<CURV, FD, 5, false>(a, p, qv, o, Cols{}); break;
-    case 1: s_close_row<CURV, FD, 0, true>(a, p, qv, o, Cols{}); break;
-    case 2: s_close_row<CURV, FD, 1, true>(a, p, qv, o, Cols{}); break;
-    case 3: s_close_row<CURV, FD, 2, true>(a, p, qv, o, Cols{}); break;
-    case 4: s_close_row<CURV, FD, 3, true>(a, p, qv, o, Cols{}); break;
-    case 5: s_close_row<CURV, FD, 4, true>(a, p, qv, o, Cols{}); break;
-    default: s_close_row<CURV, FD, 5, true>(a, p, qv, o, Cols{}); break;
+    case -1: s_close_row<CURV, FD, VEL, 0, false>(a, p, qv, o, Cols{}); break;
+    case -2: s_close_row<CURV, FD, VEL, 1, false>(a, p, qv, o, Cols{}); break;
+    case -3: s_close_row<CURV, FD, VEL, 2, false>(a, p, qv, o, Cols{}); break;
+    case -4: s_close_row<CURV, FD, VEL, 3, false>(a, p, qv, o, Cols{}); break;
+    case -5: s_close_row<CURV, FD, VEL, 4, false>(a, p, qv, o, Cols{}); break;
+    case -6: s_close_row<CURV, FD, VEL, 5, false>(a, p, qv, o, Cols{}); break;
+    case 1: s_close_row<CURV, FD, VEL, 0, true>(a, p, qv, o, Cols{}); break;
+    case 2: s_close_row<CURV, FD, VEL, 1, true>(a, p, qv, o, Cols{}); break;
+    case 3: s_close_row<CURV, FD, VEL, 2, true>(a, p, qv, o, Cols{}); break;
+    case 4: s_close_row<CURV, FD, VEL, 3, true>(a, p, qv, o, Cols{}); break;
+    case 5: s_close_row<CURV, FD, VEL, 4, true>(a, p, qv, o, Cols{}); break;
+    default: s_close_row<CURV, FD, VEL, 5, true>(a, p, qv, o, Cols{}); break;
   }
+}
+
+// q derivative (index spacing) of three quantities of a pair of points: row(c)
+// is the start of quantity c's row in the box, lq the box column of the even
+// point; box columns lq-4 .. lq+5, five aligned pairs, serve both points.
+// VEL: the velocities (the upwind pair's D+), else the fluxes (its D-).
+template <int FD, bool VEL, typename Row>
+__device__ __forceinline__ void deriv_q(Row&& row, int lq, int kq0, int kq1, int lleft, int lright, const float* tab,
+                                        f2 (&o)[3]) {
+  const float c1 = float(kC1), c2 = float(kC2), c3 = float(kC3);
+  const float cf[7] = WQL_UP_CF;
+  if (kq0 == 0 || kq1 == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float* x = row(c) + lq;
+      const f2 m4 = g2(x - 4), m2 = g2(x - 2), z = g2(x), p2 = g2(x + 2), p4 = g2(x + 4);
+      float x0, x1, a1, a2, a3, a4, b2, b3, b4, b5, u0, u1;  // a_k at -k, b_k at +k
+      unpack(z, x0, x1);
+      unpack(m2, a2, a1);
+      unpack(m4, a4, a3);
+      unpack(p2, b2, b3);
+      unpack(p4, b4, b5);
+      if (FD && VEL) {  // offsets -2..4
+        f2 u = mul2(pack(cf[0], cf[0]), m2);
+        u = fma2(pack(cf[2], cf[2]), z, u);
+        u = fma2(pack(cf[4], cf[4]), p2, u);
+        u = fma2(pack(cf[6], cf[6]), p4, u);
+        unpack(u, u0, u1);
+        u0 += cf[1] * a1 + cf[3] * x1 + cf[5] * b3;
+        u1 += cf[1] * x0 + cf[3] * b2 + cf[5] * b4;
+      } else if (FD) {  // offsets -4..2
+        f2 u = mul2(pack(-cf[0], -cf[0]), p2);
+        u = fma2(pack(-cf[2], -cf[2]), z, u);
+        u = fma2(pack(-cf[4], -cf[4]), m2, u);
+        u = fma2(pack(-cf[6], -cf[6]), m4, u);
+        unpack(u, u0, u1);
+        u0 -= cf[1] * x1 + cf[3] * a1 + cf[5] * a3;
+        u1 -= cf[1] * b2 + cf[3] * x0 + cf[5] * a2;
+      } else {
+        unpack(mul2(pack(c2, c2), sub2(p2, m2)), u0, u1);
+        u0 += c1 * (x1 - a1) + c3 * (b3 - a3);
+        u1 += c1 * (b2 - x0) + c3 * (b4 - a2);
+      }
+      o[c] = pack(u0, u1);
+    }
+  }
+  if (kq0 != 0 || kq1 != 0) {
+    // one or both points on a closure row: both rows of a pair read the same
+    // columns (points 0.. or n-1.., at box columns lleft.. or lright..) with
+    // their own weights; the upwind pair's right rows swap its two tables
+    const bool left = kq0 < 0;
+    constexpr int NCOL = FD ? 10 : 9;
+    const int r0 = kq0 ? (left ? -kq0 : kq0) - 1 : 0, r1 = kq1 ? (left ? -kq1 : kq1) - 1 : 0;
+    const float sg0 = kq0 ? (left ? 1.0f : -1.0f) : 0.0f, sg1 = kq1 ? (left ? 1.0f : -1.0f) : 0.0f;
+    const float* w = tab + (FD && (left != VEL) ? 60 : 0);
+    const int l0 = left ? lleft : lright, dl = left ? 1 : -1;
+    float u0[3], u1[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) u0[c] = u1[c] = 0.0f;
+#pragma unroll 3
+    for (int e = 0; e < NCOL; ++e) {
+      const float v0 = sg0 * w[r0 * NCOL + e], v1 = sg1 * w[r1 * NCOL + e];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float x = row(c)[l0 + e * dl];
+        u0[c] += v0 * x;
+        u1[c] += v1 * x;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      float i0 = 0.0f, i1 = 0.0f;
+      if (kq0 == 0 || kq1 == 0) unpack(o[c], i0, i1);
+      o[c] = pack(kq0 ? u0[c] : i0, kq1 ? u1[c] : i1);
+    }
+  }
+}
+
+// r derivative: val(l, c) is quantity c at box row l.
+template <int FD, bool VEL, typename Val>
+__device__ __forceinline__ void deriv_r(Val&& val, int lr, int kr, const float* tab, f2 (&o)[3]) {
+  const float c1 = float(kC1), c2 = float(kC2), c3 = float(kC3);
+  const float cf[7] = WQL_UP_CF;
+  if (kr == 0 && FD) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[c] = 0;
+#pragma unroll
+    for (int i = 0; i < 7; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        o[c] = VEL ? fma2(pack(cf[i], cf[i]), val(lr + i - 2, c), o[c])
+                   : fma2(pack(-cf[6 - i], -cf[6 - i]), val(lr + i - 4, c), o[c]);
+  } else if (kr == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      o[c] = fma2(pack(c1, c1), sub2(val(lr + 1, c), val(lr - 1, c)),
+                  fma2(pack(c2, c2), sub2(val(lr + 2, c), val(lr - 2, c)),
+                       mul2(pack(c3, c3), sub2(val(lr + 3, c), val(lr - 3, c)))));
+  } else {
+    const bool left = kr < 0;
+    constexpr int NCOL = FD ? 10 : 9;
+    const int rw = (left ? -kr : kr) - 1;
+    const float sgn = left ? 1.0f : -1.0f;
+    const float* w = tab + (FD && (left != VEL) ? 60 : 0) + rw * NCOL;
+    const int l0 = lr + (left ? -rw : rw), dl = left ? 1 : -1;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[c] = 0;
+#pragma unroll 3
+    for (int e = 0; e < NCOL; ++e) {
+      const float v = sgn * w[e];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) o[c] = fma2(pack(v, v), val(l0 + e * dl, c), o[c]);
+    }
+  }
+}
+
+// s derivative of the window's three quantities.
+template <bool CURV, int FD, bool VEL>
+__device__ __forceinline__ void deriv_s(const VolumeArgs<float>& a, long long p, int ks, const f2 (&qv)[7][3],
+                                        f2 (&o)[3]) {
+  const float c1 = float(kC1), c2 = float(kC2), c3 = float(kC3);
+  const float cf[7] = WQL_UP_CF;
+  if (ks == 0 && FD) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[c] = 0;
+#pragma unroll
+    for (int i = 0; i < 7; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        o[c] = VEL ? fma2(pack(cf[i], cf[i]), qv[i][c], o[c]) : fma2(pack(-cf[6 - i], -cf[6 - i]), qv[i][c], o[c]);
+  } else if (ks == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      o[c] = fma2(pack(c1, c1), sub2(qv[4][c], qv[2][c]),
+                  fma2(pack(c2, c2), sub2(qv[5][c], qv[1][c]), mul2(pack(c3, c3), sub2(qv[6][c], qv[0][c]))));
+  } else {
+    s_closure<CURV, FD, VEL>(a, p, ks, qv, o);
+  }
+}
+
+// The work of the consumer threads of one role on a tile's chunk.  VEL: the
+// threads that difference the velocities and update the six stresses; else
+// those that form and difference the momentum fluxes and update the three
+// velocities.  Both roles cover every pair of points of the tile; they share
+// nothing but the stage's data.
+template <bool CURV, int FD, int TQW, bool VEL>
+__device__ __forceinline__ bool tma_consume(const VolumeArgs<float>& a, float* sm, uint64_t* full, uint64_t* empty,
+                                            uint64_t* fluxbar, uint64_t* metbar, int q0, const TileSpan& spr,
+                                            int s_begin, int nstep, int tid, const float* tab, int tb) {
+  using TL = TmaTile<CURV, FD, TQW>;
+  constexpr int TQ = TL::TQ, TR = TL::TR, NC = TL::NC, NT = TL::NT, BQ = TL::BQ, BR = TL::BR, HR = TL::HR, NS = TL::NS;
+  const int nq = a.nq, nr = a.nr, ns = a.ns, r0 = spr.origin;
+  const int tx = 2 * (tid % (TQ / 2));
+  const bool live = tid < NC / 2;  // the last warp of a 40-wide tile is half empty
+  const int ty = live ? tid / (TQ / 2) : TR - 1;
+  const int q = q0 + tx, r = r0 + ty;
+  // q = nq - 1 of an odd nq shares its pair with the pad column, which is
+  // inside the row pitch: its values are computed from zeros and stored
+  const bool own = live && q < nq && r >= spr.own_lo && r < spr.own_hi;
+  const int kq0 = sbp_kind(q, nq), kq1 = q + 1 < nq ? sbp_kind(q + 1, nq) : 0, kr = sbp_kind(r, nr);
+  // points whose DF the pre-kernels have set on a stage with A = 0: the
+  // block's faces and the PML slabs (here the q and r sides, true for the
+  // whole column)
+  const int npml = a.npml;
+  const bool fold_r = r == 0 || r == nr - 1 || (a.pml[2] && r < npml) || (a.pml[3] && r >= nr - npml);
+  auto fold_q = [&](int i) {
+    return i == 0 || i == nq - 1 || (a.pml[0] && i < npml) || (a.pml[1] && i >= nq - npml);
+  };
+  const bool fold0 = fold_r || fold_q(q), fold1 = fold_r || fold_q(q + 1);
+  const long long np = a.np;
+  const long long sts = (long long)a.pq * nr;
+  const long long col = q + (long long)a.pq * r;
+  const int lq = tx + 8, lr = ty + HR, li = ty * TQ + tx;
+  const int lleft = 8 - q0, lright = nq - 1 - q0 + 8;  // box columns of points 0 and nq-1
+  constexpr int W0 = FD ? (VEL ? -2 : -4) : -3;        // plane of the window's first entry, from s
+
+  // s window: the three velocities, or the three s-face fluxes, of the seven
+  // planes the operator reads.  Its first six entries come straight from
+  // global memory, all loads in flight at once; planes outside the block stay
+  // zero (only central rows read the window).
+  f2 qv[7][3];
+#pragma unroll
+  for (int i = 0; i < 7; ++i) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) qv[i][c] = 0;
+    const int pl = s_begin + W0 + i;
+    if (i < 6 && pl >= 0 && pl < ns && q < nq && r < nr) {
+      const long long pp = col + sts * pl;
+      const float* F = a.Fin;
+      if (VEL) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) qv[i][c] = g2(F + c * np + pp);
+      } else if (CURV) {
+        const f2 a0 = g2(a.coef + 6 * np + pp), a1 = g2(a.coef + 7 * np + pp), a2 = g2(a.coef + 8 * np + pp);
+        f2 sg[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) sg[c] = g2(F + (3 + c) * np + pp);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) qv[i][c] = dot3(a0, sg[sig(c, 0) - 3], a1, sg[sig(c, 1) - 3], a2, sg[sig(c, 2) - 3]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) qv[i][c] = g2(F + sig(c, 2) * np + pp);
+      }
+    }
+  }
+
+  for (int t = 0; t < nstep; ++t) {
+    const int T = tb + t;
+    const int st = T % NS;
+    const int s = s_begin + t;  // output plane
+    const int ks = sbp_kind(s, ns);
+    const long long p = col + sts * s;
+    if (!mbar_wait(&full[st], (T / NS) & 1)) {
+      atomicExch(a.err, 2);
+      return false;
+    }
+    float* S = sm + st * TL::STAGE_W;
+    float* FB = S + TL::OFF_F;
+    float* CA = S + TL::OFF_CA;
+    float* CB = S + TL::OFF_CB;
+    const float* CC = S + TL::OFF_CC;
+    const float* LF = S + TL::OFF_LF;
+    auto fb2 = [&](int c, int rr, int qq) -> f2 { return g2(FB + (c * BR + rr) * BQ + qq); };
+    const bool fold_s = s == 0 || s == ns - 1 || (a.pml[4] && s < npml) || (a.pml[5] && s >= ns - npml);
+    const comp_t* CKs = reinterpret_cast<const comp_t*>(S + TL::OFF_CK);
+    // DF <- A*DF + du and the compensated update of component c.  The
+    // pre-kernels have folded the boundary and fault penalties and the PML
+    // damping into DF of their points: DF + term/A, or the term itself on the
+    // first stage (A = 0, where DF holds nothing else).
+    auto update = [&](int c, f2 du) {
+      const f2 f0 = fb2(c, lr, lq);
+      const f2 dfs = g2(S + TL::OFF_DF + c * NC + li);
+      f2 df;
+      if (a.A != 0.0f) {
+        df = fma2(pack(a.A, a.A), dfs, du);
+      } else {
+        float d0, d1;
+        unpack(dfs, d0, d1);
+        df = add2(pack(fold_s || fold0 ? d0 : 0.0f, fold_s || fold1 ? d1 : 0.0f), du);
+      }
+      *reinterpret_cast<f2*>(a.DF + c * np + p) = df;
+      // -C of the pair: two bfloat16 (low half the even point), widened
+      const unsigned ck = *reinterpret_cast<const unsigned*>(CKs + c * NC + li) ^ 0x80008000u;
+      const f2 y = fma2(pack(a.Bdt, a.Bdt), df, pack(__uint_as_float(ck << 16), __uint_as_float(ck & 0xffff0000u)));
+      const f2 tt = add2(f0, y);
+      float e0, e1;
+      unpack(sub2(sub2(tt, f0), y), e0, e1);
+      *reinterpret_cast<unsigned*>(a.C + c * np + p) = bf16_pair(e0, e1);
+      *reinterpret_cast<f2*>(a.Fout + c * np + p) = tt;
+    };
+
+    if constexpr (VEL) {
+      // own J*metric_q and J*metric_r, before the flux threads write over them
+      f2 mq[3], mr[3];
+      if (CURV) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          mq[j] = g2(CA + (j * TR + ty) * BQ + lq);
+          mr[j] = g2(CB + (j * BR + lr) * TQ + tx);
+        }
+        mbar_arrive(&metbar[st]);
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) qv[6][c] = g2(LF + c * NC + li);
+      if (own) {
+        f2 g[3][3];
+        const f2 Jinv = CURV ? g2(CC + 3 * NC + li) : 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          f2 o[3];
+          if (d == 0)
+            deriv_q<FD, true>([&](int c) -> const float* { return FB + (c * BR + lr) * BQ; }, lq, kq0, kq1, lleft,
+                              lright, tab, o);
+          else if (d == 1) deriv_r<FD, true>([&](int l, int c) { return fb2(c, l, lq); }, lr, kr, tab, o);
+          else deriv_s<CURV, FD, true>(a, p, ks, qv, o);
+          const float rh = a.rh[d];
+          if (CURV) {
+            const f2 Jr = mul2(Jinv, pack(rh, rh));
+#pragma unroll
+            for (int jj = 0; jj < 3; ++jj) {
+              const f2 mt = mul2(d == 0 ? mq[jj] : (d == 1 ? mr[jj] : g2(CC + jj * NC + li)), Jr);
+#pragma unroll
+              for (int c = 0; c < 3; ++c) g[c][jj] = d == 0 ? mul2(mt, o[c]) : fma2(mt, o[c], g[c][jj]);
+            }
+          } else {
+            const float sc = a.cart_metric[d] * rh;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) g[c][d] = mul2(pack(sc, sc), o[c]);
+          }
+        }
+        if (a.G != nullptr) {  // anelastic: every point hands its velocity gradient over
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int jj = 0; jj < 3; ++jj) *reinterpret_cast<f2*>(a.G + (c * 3 + jj) * np + p) = g[c][jj];
+        }
+        const f2 lam = g2(CC + (CURV ? 4 : 0) * NC + li);
+        const f2 mu = g2(CC + (CURV ? 5 : 1) * NC + li);
+        const f2 l2m = fma2(pack(2.0f, 2.0f), mu, lam);
+        update(3, fma2(l2m, g[0][0], mul2(lam, add2(g[1][1], g[2][2]))));
+        update(4, fma2(l2m, g[1][1], mul2(lam, add2(g[0][0], g[2][2]))));
+        update(5, fma2(l2m, g[2][2], mul2(lam, add2(g[0][0], g[1][1]))));
+        update(6, mul2(mu, add2(g[0][1], g[1][0])));
+        update(7, mul2(mu, add2(g[0][2], g[2][0])));
+        update(8, mul2(mu, add2(g[1][2], g[2][1])));
+      }
+    } else {
+      {
+        f2 f[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) f[c] = g2(LF + (3 + c) * NC + li);
+        if (CURV) {
+          const float* LC = S + TL::OFF_LC;
+          const f2 a0 = g2(LC + li), a1 = g2(LC + NC + li), a2 = g2(LC + 2 * NC + li);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) qv[6][c] = dot3(a0, f[sig(c, 0) - 3], a1, f[sig(c, 1) - 3], a2, f[sig(c, 2) - 3]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) qv[6][c] = f[sig(c, 2) - 3];
+        }
+      }
+      // curvilinear: the q- and r-face momentum fluxes J*metric*sigma of the
+      // main plane, formed once per box point and written over the
+      // coefficients they come from (CA becomes the q flux on the q-extended
+      // rows, CB the r flux on the r-extended columns), once the other role
+      // has taken its metrics; each position is handled by one thread
+      if (CURV) {
+        // x: the first coefficient of the position, xs: words from one to the next
+        auto flux = [&](float* x, int xs, const f2 (&sg)[6]) {
+          f2 m[3];
+#pragma unroll
+          for (int j = 0; j < 3; ++j) m[j] = g2(x + j * xs);
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            *reinterpret_cast<f2*>(x + c * xs) =
+                dot3(m[0], sg[sig(c, 0) - 3], m[1], sg[sig(c, 1) - 3], m[2], sg[sig(c, 2) - 3]);
+        };
+        f2 sg[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) sg[c] = fb2(3 + c, lr, lq);
+        if (!mbar_wait(&metbar[st], (T / NS) & 1)) {
+          atomicExch(a.err, 4);
+          return false;
+        }
+        flux(CA + ty * BQ + lq, TR * BQ, sg);
+        flux(CB + lr * TQ + tx, BR * TQ, sg);
+        // the halos: lanes 0..15 take the q halo of the warp's own two rows (4
+        // pairs each side), lanes 16..31 of all warps together the r halo (HR
+        // rows each side, TQ/2 pairs each)
+        const int lane = tid & 31, warp = tid >> 5;
+        constexpr int kRHalo = 2 * HR * (TQ / 2), kRPass = NT / 2;
+#pragma unroll
+        for (int e0 = 0; e0 < kRHalo; e0 += kRPass) {
+          const bool isq = lane < 16;
+          const int e = e0 + warp * 16 + (lane - 16);
+          if (isq ? e0 == 0 : e < kRHalo) {
+            const int h = lane & 7, rw = e / (TQ / 2);
+            const int row = isq ? 2 * warp + (lane >> 3) : (rw < HR ? rw : rw + TR);
+            const int qq = isq ? (h < 4 ? 2 * h : TQ + 2 * h) : 2 * (e % (TQ / 2)) + 8;
+            const int rr = isq ? row + HR : row;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) sg[c] = fb2(3 + c, rr, qq);
+            flux(isq ? CA + row * BQ + qq : CB + row * TQ + (qq - 8), isq ? TR * BQ : BR * TQ, sg);
+          }
+        }
+        // a warp forms every q flux of its own rows (the q derivative needs
+        // only those: warp sync); the r fluxes of other rows come from other
+        // warps: every thread of the role arrives here and waits (bounded)
+        // just before the r derivative
+        __syncwarp();
+        mbar_arrive(fluxbar);
+      }
+      if (own) {
+        f2 dv[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const int d = k == 0 ? 0 : (k == 1 ? 2 : 1);  // q, s, then r
+          if (CURV && k == 2 && !mbar_wait(fluxbar, T & 1)) {
+            atomicExch(a.err, 3);
+            return false;
+          }
+          f2 o[3];
+          if (d == 0)
+            deriv_q<FD, false>([&](int c) -> const float* {
+              return CURV ? CA + (c * TR + ty) * BQ : FB + (sig(c, 0) * BR + lr) * BQ;
+            }, lq, kq0, kq1, lleft, lright, tab, o);
+          else if (d == 1)
+            deriv_r<FD, false>([&](int l, int c) {
+              return CURV ? g2(CB + (c * BR + l) * TQ + tx) : fb2(sig(c, 1), l, lq);
+            }, lr, kr, tab, o);
+          else deriv_s<CURV, FD, false>(a, p, ks, qv, o);
+          const float sc = CURV ? a.rh[d] : a.cart_metric[d] * a.rh[d];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) dv[c] = k == 0 ? mul2(pack(sc, sc), o[c]) : fma2(pack(sc, sc), o[c], dv[c]);
+        }
+        const f2 rinv = g2(CC + (CURV ? 6 : 2) * NC + li);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) update(c, mul2(rinv, dv[c]));
+      } else if (CURV && !mbar_wait(fluxbar, T & 1)) {  // the same phase for threads without a point
+        atomicExch(a.err, 3);
+        return false;
+      }
+      // order this thread's shared-memory writes (the fluxes) before the
+      // producer's next bulk copy into the stage
+      if (CURV) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    if ((tid & 31) == 0) mbar_arrive(&empty[st]);
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) qv[i][c] = qv[i + 1][c];
+  }
+  return true;
 }
 
 struct MapArgs {
@@ -270,18 +688,22 @@ struct MapArgs {
 // the CTA has used before this tile (the same count in every thread), so a
 // persistent CTA keeps its mbarriers and the producer runs ahead into the
 // next tile.  Returns false after a wait ran out (the error word is set).
-template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int FD, int TQW = kTmaTQ>
 __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapArgs& m, int schunk, int bx, int by,
                                          int bz, const float* tab, int& tb) {
   using TL = TmaTile<CURV, FD, TQW>;
-  constexpr int TQ = TL::TQ, TR = TL::TR, NC = TL::NC, NT = TL::NT, BQ = TL::BQ, BR = TL::BR, HR = TL::HR;
+  constexpr int TQ = TL::TQ, TR = TL::TR, NC = TL::NC, NT = TL::NT, BQ = TL::BQ, BR = TL::BR, HR = TL::HR, NS = TL::NS;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   // 128-byte aligned start, derived from the shared array itself so the
   // compiler keeps every access in the shared address space
   float* sm = reinterpret_cast<float*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
   uint64_t* full = reinterpret_cast<uint64_t*>(sm + NS * TL::STAGE_W);
   uint64_t* empty = full + NS;
-  uint64_t* fluxbar = empty + NS;  // consumer-only: fluxes of the step written
+  uint64_t* fluxbar = empty + NS;   // flux threads: fluxes of the step written
+  // stress threads: metrics of the stage read.  One per stage: those threads
+  // can be a step ahead of the flux threads that wait here, and a stage is
+  // filled again only after both roles have left it
+  uint64_t* metbar = fluxbar + 1;
 
   const int tid = threadIdx.x;
   const int nq = a.nq, nr = a.nr, ns = a.ns;
@@ -292,8 +714,8 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
   const int s_end = min(ns, s_begin + schunk);
   const int nstep = s_end - s_begin;
 
-  if (tid >= NT) {  // producer warp: one thread issues every copy
-    if (tid == NT) {
+  if (tid >= 2 * NT) {  // producer warp: one thread issues every copy
+    if (tid == 2 * NT) {
       for (int t = 0; t < nstep; ++t) {
         const int T = tb + t;
         const int st = T % NS;
@@ -329,397 +751,19 @@ __device__ __forceinline__ bool tma_body(const VolumeArgs<float>& a, const MapAr
     return true;
   }
 
-  // ---- consumers: one thread per pair of neighbouring q points (q, q+1) of the tile
-  const int tx = 2 * (tid % (TQ / 2));
-  const bool live = tid < NC / 2;  // the last warp of a 40-wide tile is half empty
-  const int ty = live ? tid / (TQ / 2) : TR - 1;
-  const int q = q0 + tx, r = r0 + ty;
-  // q = nq - 1 of an odd nq shares its pair with the pad column, which is
-  // inside the row pitch: its values are computed from zeros and stored
-  const bool own = live && q < nq && r >= spr.own_lo && r < spr.own_hi;
-  const int kq0 = sbp_kind(q, nq), kq1 = q + 1 < nq ? sbp_kind(q + 1, nq) : 0, kr = sbp_kind(r, nr);
-  // points whose DF the pre-kernels have set on a stage with A = 0: the
-  // block's faces and the PML slabs (here the q and r sides, true for the
-  // whole column)
-  const int npml = a.npml;
-  const bool fold_r = r == 0 || r == nr - 1 || (a.pml[2] && r < npml) || (a.pml[3] && r >= nr - npml);
-  auto fold_q = [&](int i) {
-    return i == 0 || i == nq - 1 || (a.pml[0] && i < npml) || (a.pml[1] && i >= nq - npml);
-  };
-  const bool fold0 = fold_r || fold_q(q), fold1 = fold_r || fold_q(q + 1);
-  const long long np = a.np;
-  const long long sts = (long long)a.pq * nr;
-  const long long col = q + (long long)a.pq * r;
-  const int lq = tx + 8, lr = ty + HR, li = ty * TQ + tx;
-  const float c1 = float(kC1), c2 = float(kC2), c3 = float(kC3);
-  const float cf[7] = WQL_UP_CF;
-  auto g2 = [](const float* p) { return *reinterpret_cast<const f2*>(p); };
-
-  // s window: velocities of planes s-3..s+3 and the s-face flux of the same
-  // planes (central operator), or velocities of s-2..s+4 and fluxes of
-  // s-4..s+2 (upwind pair: the planes D+ and D- read)
-  f2 qv[7][6];
-  // the window's first six entries straight from global memory, all loads
-  // in flight at once; planes outside the block stay zero (only central
-  // rows read the window)
-#pragma unroll
-  for (int i = 0; i < 7; ++i) {
-#pragma unroll
-    for (int c = 0; c < 6; ++c) qv[i][c] = 0;
-    const int plv = s_begin + (FD ? -2 : -3) + i, pl = s_begin + (FD ? -4 : -3) + i;
-    const float* F = a.Fin;
-    if (i < 6 && plv >= 0 && plv < ns && q < nq && r < nr) {
-      const long long pp = col + sts * plv;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) qv[i][c] = g2(F + c * np + pp);
-    }
-    if (i < 6 && pl >= 0 && pl < ns && q < nq && r < nr) {
-      const long long pp = col + sts * pl;
-      if (CURV) {
-        const f2 a0 = g2(a.coef + 6 * np + pp), a1 = g2(a.coef + 7 * np + pp), a2 = g2(a.coef + 8 * np + pp);
-        f2 sg[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) sg[c] = g2(F + (3 + c) * np + pp);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) qv[i][3 + c] = dot3(a0, sg[sig(c, 0) - 3], a1, sg[sig(c, 1) - 3], a2, sg[sig(c, 2) - 3]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) qv[i][3 + c] = g2(F + sig(c, 2) * np + pp);
-      }
-    }
-  }
-
-  for (int t = 0; t < nstep; ++t) {
-    const int T = tb + t;
-    const int st = T % NS;
-    const int s = s_begin + t;  // output plane
-    const int ks = sbp_kind(s, ns);
-    const long long p = col + sts * s;
-    if (!mbar_wait(&full[st], (T / NS) & 1)) {
-      atomicExch(a.err, 2);
-      return false;
-    }
-    float* S = sm + st * TL::STAGE_W;
-    // push the lead plane(s) into the s window
-    {
-      const float* LF = S + TL::OFF_LF;
-      f2 f[9];
-#pragma unroll
-      for (int c = 0; c < 9; ++c) f[c] = g2(LF + c * NC + li);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) qv[6][c] = f[c];
-      if (CURV) {
-        const float* LC = S + TL::OFF_LC;
-        const f2 a0 = g2(LC + li), a1 = g2(LC + NC + li), a2 = g2(LC + 2 * NC + li);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) qv[6][3 + c] = dot3(a0, f[sig(c, 0)], a1, f[sig(c, 1)], a2, f[sig(c, 2)]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) qv[6][3 + c] = f[sig(c, 2)];
-      }
-    }
-
-    // curvilinear: the q- and r-face momentum fluxes J*metric*sigma of the
-    // main plane, formed once per box point and written over the
-    // coefficients they come from (CA becomes the q flux on the q-extended
-    // rows, CB the r flux on the r-extended columns); each position is
-    // handled by one thread, which reads its coefficients first
-    float* FB = S + TL::OFF_F;
-    float* CA = S + TL::OFF_CA;
-    float* CB = S + TL::OFF_CB;
-    const float* CC = S + TL::OFF_CC;
-    auto fb2 = [&](int c, int rr, int qq) -> f2 { return g2(FB + (c * BR + rr) * BQ + qq); };
-    f2 mq[3], mr[3];  // own J*metric_q, J*metric_r
-    if (CURV) {
-      // x: the first coefficient of the position, xs: words from one to the
-      // next; (rr, qq): the position in the field box
-      auto flux = [&](float* x, int xs, const f2 (&sg)[6], f2 (&m)[3]) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j) m[j] = g2(x + j * xs);
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          *reinterpret_cast<f2*>(x + c * xs) =
-              dot3(m[0], sg[sig(c, 0) - 3], m[1], sg[sig(c, 1) - 3], m[2], sg[sig(c, 2) - 3]);
-      };
-      f2 sg[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) sg[c] = fb2(3 + c, lr, lq);
-      flux(CA + ty * BQ + lq, TR * BQ, sg, mq);
-      flux(CB + lr * TQ + tx, BR * TQ, sg, mr);
-      // the halos: lanes 0..15 take the q halo of the warp's own two rows (4
-      // pairs each side), lanes 16..31 of all warps together the r halo (HR
-      // rows each side, TQ/2 pairs each)
-      const int lane = tid & 31, warp = tid >> 5;
-      constexpr int kRHalo = 2 * HR * (TQ / 2), kRPass = NT / 2;
-#pragma unroll
-      for (int e0 = 0; e0 < kRHalo; e0 += kRPass) {
-        const bool isq = lane < 16;
-        const int e = e0 + warp * 16 + (lane - 16);
-        if (isq ? e0 == 0 : e < kRHalo) {
-          const int h = lane & 7, rw = e / (TQ / 2);
-          const int row = isq ? 2 * warp + (lane >> 3) : (rw < HR ? rw : rw + TR);
-          const int qq = isq ? (h < 4 ? 2 * h : TQ + 2 * h) : 2 * (e % (TQ / 2)) + 8;
-          const int rr = isq ? row + HR : row;
-          f2 m[3];
-#pragma unroll
-          for (int c = 0; c < 6; ++c) sg[c] = fb2(3 + c, rr, qq);
-          flux(isq ? CA + row * BQ + qq : CB + row * TQ + (qq - 8), isq ? TR * BQ : BR * TQ, sg, m);
-        }
-      }
-      // a warp forms every q flux of its own rows (the q derivative needs
-      // only those: warp sync); the r fluxes of other rows come from other
-      // warps: every consumer thread arrives here and waits (bounded) just
-      // before the r derivative, so the q and s derivatives overlap the wait
-      __syncwarp();
-      mbar_arrive(fluxbar);
-    }
-
-    if (own) {
-      f2 g[3][3], dv[3];
-      const f2 Jinv = CURV ? g2(CC + 3 * NC + li) : 0;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int d = k == 0 ? 0 : (k == 1 ? 2 : 1);  // q, s, then r
-        if (CURV && k == 2 && !mbar_wait(fluxbar, T & 1)) {
-          atomicExch(a.err, 3);
-          return false;
-        }
-        f2 o[6];
-        if (d == 0) {
-          // the quantities along the row: box columns lq-4 .. lq+5 as five
-          // aligned pairs serve both points
-          auto row = [&](int c) -> const float* {
-            return c < 3 ? FB + (c * BR + lr) * BQ : (CURV ? CA + ((c - 3) * TR + ty) * BQ : FB + (sig(c - 3, 0) * BR + lr) * BQ);
-          };
-          if (kq0 == 0 || kq1 == 0) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-              const float* x = row(c) + lq;
-              const f2 m4 = g2(x - 4), m2 = g2(x - 2), z = g2(x), p2 = g2(x + 2), p4 = g2(x + 4);
-              float x0, x1, a1, a2, a3, a4, b2, b3, b4, b5;  // a_k at -k, b_k at +k
-              unpack(z, x0, x1);
-              unpack(m2, a2, a1);
-              unpack(m4, a4, a3);
-              unpack(p2, b2, b3);
-              unpack(p4, b4, b5);
-              if (FD) {
-                // offsets -2..4 of D+ (velocities), -4..2 of D- (fluxes)
-                f2 u;
-                if (c < 3) {
-                  u = mul2(pack(cf[0], cf[0]), m2);
-                  u = fma2(pack(cf[2], cf[2]), z, u);
-                  u = fma2(pack(cf[4], cf[4]), p2, u);
-                  u = fma2(pack(cf[6], cf[6]), p4, u);
-                  float u0, u1;
-                  unpack(u, u0, u1);
-                  u0 += cf[1] * a1 + cf[3] * x1 + cf[5] * b3;
-                  u1 += cf[1] * x0 + cf[3] * b2 + cf[5] * b4;
-                  o[c] = pack(u0, u1);
-                } else {
-                  u = mul2(pack(-cf[0], -cf[0]), p2);
-                  u = fma2(pack(-cf[2], -cf[2]), z, u);
-                  u = fma2(pack(-cf[4], -cf[4]), m2, u);
-                  u = fma2(pack(-cf[6], -cf[6]), m4, u);
-                  float u0, u1;
-                  unpack(u, u0, u1);
-                  u0 -= cf[1] * x1 + cf[3] * a1 + cf[5] * a3;
-                  u1 -= cf[1] * b2 + cf[3] * x0 + cf[5] * a2;
-                  o[c] = pack(u0, u1);
-                }
-              } else {
-                float u0, u1;
-                unpack(mul2(pack(c2, c2), sub2(p2, m2)), u0, u1);
-                u0 += c1 * (x1 - a1) + c3 * (b3 - a3);
-                u1 += c1 * (b2 - x0) + c3 * (b4 - a2);
-                o[c] = pack(u0, u1);
-              }
-            }
-          }
-          if (kq0 != 0 || kq1 != 0) {
-            // one or both points on a closure row: both rows of a pair read
-            // the same columns (points 0.. or n-1..) with their own weights
-            const bool left = kq0 < 0;
-            constexpr int NCOL = FD ? 10 : 9;
-            const int r0_ = kq0 ? (left ? -kq0 : kq0) - 1 : 0, r1_ = kq1 ? (left ? -kq1 : kq1) - 1 : 0;
-            const float sg0 = kq0 ? (left ? 1.0f : -1.0f) : 0.0f, sg1 = kq1 ? (left ? 1.0f : -1.0f) : 0.0f;
-            // the upwind pair's right rows swap its two tables
-            const float* wv = tab + (FD && !left ? 60 : 0);
-            const float* wf = FD ? tab + (left ? 60 : 0) : wv;
-            const int l0 = (left ? 0 : nq - 1) - q0 + 8, dl = left ? 1 : -1;
-            float u0[6], u1[6];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) u0[c] = u1[c] = 0.0f;
-#pragma unroll 1
-            for (int e = 0; e < NCOL; ++e) {
-              const float v0 = sg0 * wv[r0_ * NCOL + e], v1 = sg1 * wv[r1_ * NCOL + e];
-              const float f0 = FD ? sg0 * wf[r0_ * NCOL + e] : v0, f1 = FD ? sg1 * wf[r1_ * NCOL + e] : v1;
-              const int l = l0 + e * dl;
-#pragma unroll
-              for (int c = 0; c < 6; ++c) {
-                const float x = row(c)[l];
-                u0[c] += (c < 3 ? v0 : f0) * x;
-                u1[c] += (c < 3 ? v1 : f1) * x;
-              }
-            }
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-              float i0 = 0.0f, i1 = 0.0f;
-              if (kq0 == 0 || kq1 == 0) unpack(o[c], i0, i1);
-              o[c] = pack(kq0 ? u0[c] : i0, kq1 ? u1[c] : i1);
-            }
-          }
-        } else if (d == 2) {
-          if (ks == 0 && FD) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = 0;
-#pragma unroll
-            for (int i = 0; i < 7; ++i) {
-#pragma unroll
-              for (int c = 0; c < 3; ++c) o[c] = fma2(pack(cf[i], cf[i]), qv[i][c], o[c]);
-#pragma unroll
-              for (int c = 3; c < 6; ++c) o[c] = fma2(pack(-cf[6 - i], -cf[6 - i]), qv[i][c], o[c]);
-            }
-          } else if (ks == 0) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c)
-              o[c] = fma2(pack(c1, c1), sub2(qv[4][c], qv[2][c]),
-                          fma2(pack(c2, c2), sub2(qv[5][c], qv[1][c]), mul2(pack(c3, c3), sub2(qv[6][c], qv[0][c]))));
-          } else {
-            f2 os[6];
-            s_closure<CURV, FD>(a, p, ks, qv, os);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = os[c];
-          }
-        } else {
-          auto rvals = [&](int l, int c) -> f2 {
-            return c < 3 ? fb2(c, l, lq) : (CURV ? g2(CB + ((c - 3) * BR + l) * TQ + tx) : fb2(sig(c - 3, 1), l, lq));
-          };
-          if (kr == 0 && FD) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = 0;
-#pragma unroll
-            for (int of = -4; of <= 4; ++of) {
-              if (of >= -2)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) o[c] = fma2(pack(cf[of + 2], cf[of + 2]), rvals(lr + of, c), o[c]);
-              if (of <= 2)
-#pragma unroll
-                for (int c = 3; c < 6; ++c) o[c] = fma2(pack(-cf[2 - of], -cf[2 - of]), rvals(lr + of, c), o[c]);
-            }
-          } else if (kr == 0) {
-#pragma unroll
-            for (int c = 0; c < 6; ++c)
-              o[c] = fma2(pack(c1, c1), sub2(rvals(lr + 1, c), rvals(lr - 1, c)),
-                          fma2(pack(c2, c2), sub2(rvals(lr + 2, c), rvals(lr - 2, c)),
-                               mul2(pack(c3, c3), sub2(rvals(lr + 3, c), rvals(lr - 3, c)))));
-          } else {
-#pragma unroll
-            for (int c = 0; c < 6; ++c) o[c] = 0;
-            const bool left = kr < 0;
-            constexpr int NCOL = FD ? 10 : 9;
-            const int rw = (left ? -kr : kr) - 1;
-            const float sgn = left ? 1.0f : -1.0f;
-            const float* wv = tab + (FD && !left ? 60 : 0) + rw * NCOL;
-            const float* wf = FD ? tab + (left ? 60 : 0) + rw * NCOL : wv;
-            const int l0 = lr + (left ? -rw : rw), dl = left ? 1 : -1;
-#pragma unroll 1
-            for (int e = 0; e < NCOL; ++e) {
-              const float v = sgn * wv[e], f = FD ? sgn * wf[e] : v;
-#pragma unroll
-              for (int c = 0; c < 6; ++c) o[c] = fma2(c < 3 ? pack(v, v) : pack(f, f), rvals(l0 + e * dl, c), o[c]);
-            }
-          }
-        }
-        const float rh = a.rh[d];
-        if (CURV) {
-          const f2 Jr = mul2(Jinv, pack(rh, rh));
-          f2 mt[3];
-#pragma unroll
-          for (int jj = 0; jj < 3; ++jj) mt[jj] = mul2(d == 0 ? mq[jj] : (d == 1 ? mr[jj] : g2(CC + jj * NC + li)), Jr);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            dv[c] = k == 0 ? mul2(pack(rh, rh), o[3 + c]) : fma2(pack(rh, rh), o[3 + c], dv[c]);
-#pragma unroll
-            for (int jj = 0; jj < 3; ++jj) g[c][jj] = k == 0 ? mul2(mt[jj], o[c]) : fma2(mt[jj], o[c], g[c][jj]);
-          }
-        } else {
-          const float sc = a.cart_metric[d] * rh;
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            dv[c] = k == 0 ? mul2(pack(sc, sc), o[3 + c]) : fma2(pack(sc, sc), o[3 + c], dv[c]);
-            g[c][d] = mul2(pack(sc, sc), o[c]);
-          }
-        }
-      }
-      if (a.G != nullptr) {  // anelastic: every point hands its velocity gradient over
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int jj = 0; jj < 3; ++jj) *reinterpret_cast<f2*>(a.G + (c * 3 + jj) * np + p) = g[c][jj];
-      }
-      const f2 lam = g2(CC + (CURV ? 4 : 0) * NC + li);
-      const f2 mu = g2(CC + (CURV ? 5 : 1) * NC + li);
-      const f2 rinv = g2(CC + (CURV ? 6 : 2) * NC + li);
-      const f2 l2m = fma2(pack(2.0f, 2.0f), mu, lam);
-      f2 du[9];
-      du[0] = mul2(rinv, dv[0]);
-      du[1] = mul2(rinv, dv[1]);
-      du[2] = mul2(rinv, dv[2]);
-      du[3] = fma2(l2m, g[0][0], mul2(lam, add2(g[1][1], g[2][2])));
-      du[4] = fma2(l2m, g[1][1], mul2(lam, add2(g[0][0], g[2][2])));
-      du[5] = fma2(l2m, g[2][2], mul2(lam, add2(g[0][0], g[1][1])));
-      du[6] = mul2(mu, add2(g[0][1], g[1][0]));
-      du[7] = mul2(mu, add2(g[0][2], g[2][0]));
-      du[8] = mul2(mu, add2(g[1][2], g[2][1]));
-      // the pre-kernels have folded the boundary and fault penalties and the
-      // PML damping into DF of their points: DF + term/A, or the term itself
-      // on the first stage (A = 0, where DF holds nothing else)
-      const bool fold_s = s == 0 || s == ns - 1 || (a.pml[4] && s < npml) || (a.pml[5] && s >= ns - npml);
-      const comp_t* CKs = reinterpret_cast<const comp_t*>(S + TL::OFF_CK);
-      const f2 A2 = pack(a.A, a.A), B2 = pack(a.Bdt, a.Bdt);
-#pragma unroll
-      for (int c = 0; c < 9; ++c) {
-        const f2 f0 = fb2(c, lr, lq);
-        const f2 dfs = g2(S + TL::OFF_DF + c * NC + li);
-        f2 df;
-        if (a.A != 0.0f) {
-          df = fma2(A2, dfs, du[c]);
-        } else {
-          float d0, d1;
-          unpack(dfs, d0, d1);
-          df = add2(pack(fold_s || fold0 ? d0 : 0.0f, fold_s || fold1 ? d1 : 0.0f), du[c]);
-        }
-        *reinterpret_cast<f2*>(a.DF + c * np + p) = df;
-        // -C of the pair: two bfloat16 (low half the even point), widened
-        const unsigned ck = *reinterpret_cast<const unsigned*>(CKs + c * NC + li) ^ 0x80008000u;
-        const f2 y = fma2(B2, df, pack(__uint_as_float(ck << 16), __uint_as_float(ck & 0xffff0000u)));
-        const f2 tt = add2(f0, y);
-        float e0, e1;
-        unpack(sub2(sub2(tt, f0), y), e0, e1);
-        *reinterpret_cast<unsigned*>(a.C + c * np + p) = bf16_pair(e0, e1);
-        *reinterpret_cast<f2*>(a.Fout + c * np + p) = tt;
-      }
-    } else if (CURV && !mbar_wait(fluxbar, T & 1)) {  // the same phase for threads without a point
-      atomicExch(a.err, 3);
-      return false;
-    }
-    // order this thread's shared-memory writes (the fluxes) before the
-    // producer's next bulk copy into the stage
-    if (CURV) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if ((tid & 31) == 0) mbar_arrive(&empty[st]);
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-#pragma unroll
-      for (int c = 0; c < 6; ++c) qv[i][c] = qv[i + 1][c];
-  }
+  // ---- consumers: two warps' worth of threads for every pair of points, one per role
+  const bool ok = tid < NT ? tma_consume<CURV, FD, TQW, true>(a, sm, full, empty, fluxbar, metbar, q0, spr, s_begin,
+                                                                  nstep, tid, tab, tb)
+                           : tma_consume<CURV, FD, TQW, false>(a, sm, full, empty, fluxbar, metbar, q0, spr,
+                                                                   s_begin, nstep, tid - NT, tab, tb);
   tb += nstep;
-  return true;
+  return ok;
 }
 
 // Shared-memory ring of a persistent CTA: NS stages then the mbarriers.
-template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int FD, int TQW = kTmaTQ>
 struct Ring {
+  static constexpr int NS = TmaTile<CURV, FD, TQW>::NS;
   float* sm;
   uint64_t *full, *empty, *fluxbar;
   float* tab;  // closure weights
@@ -730,7 +774,7 @@ struct Ring {
     full = reinterpret_cast<uint64_t*>(sm + NS * TL::STAGE_W);
     empty = full + NS;
     fluxbar = empty + NS;
-    tab = reinterpret_cast<float*>(fluxbar + 1);
+    tab = reinterpret_cast<float*>(fluxbar + 1 + NS);
   }
   // one thread initialises the barriers once per CTA
   __device__ void init() {
@@ -745,9 +789,10 @@ struct Ring {
     if (threadIdx.x == 0) {
       for (int i = 0; i < NS; ++i) {
         mbar_init(&full[i], 1);
-        mbar_init(&empty[i], TL::NT / 32);
+        mbar_init(&empty[i], 2 * TL::NT / 32);
       }
       mbar_init(fluxbar, TL::NT);
+      for (int i = 0; i < NS; ++i) mbar_init(fluxbar + 1 + i, TL::NT);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -755,7 +800,7 @@ struct Ring {
   // the producer's copies of the last stages land before the CTA leaves
   // (tb = stages issued)
   __device__ void drain(int tb) {
-    if (threadIdx.x == TmaTile<CURV, FD, TQW>::NT)
+    if (threadIdx.x == 2 * TmaTile<CURV, FD, TQW>::NT)
       for (int T = max(0, tb - NS); T < tb; ++T) mbar_wait(&full[T % NS], (T / NS) & 1);
   }
 };
@@ -763,28 +808,28 @@ struct Ring {
 // Each CTA takes tiles w = blockIdx.x, blockIdx.x + gridDim.x, ... of the
 // tq x tr x nchunk tiles of the block (q fastest, so neighbouring CTAs share
 // halos in L2); with one CTA per tile that is one tile each.
-template <bool CURV, int NS, int FD, int TQW>
-__global__ void __launch_bounds__(TmaTile<CURV, FD, TQW>::NT + 32, 1)
+template <bool CURV, int FD, int TQW>
+__global__ void __launch_bounds__(2 * TmaTile<CURV, FD, TQW>::NT + 32, 1)
     stencil_kernel_tma(const __grid_constant__ VolumeArgs<float> a, const __grid_constant__ MapArgs m, int schunk,
                        int tq, int tr, int ntile) {
-  Ring<CURV, NS, FD, TQW> ring;
+  Ring<CURV, FD, TQW> ring;
   ring.init();
   int tb = 0;
   for (int w = blockIdx.x; w < ntile; w += gridDim.x)
-    if (!tma_body<CURV, NS, FD, TQW>(a, m, schunk, w % tq, (w / tq) % tr, w / (tq * tr), ring.tab, tb)) break;
+    if (!tma_body<CURV, FD, TQW>(a, m, schunk, w % tq, (w / tq) % tr, w / (tq * tr), ring.tab, tb)) break;
   ring.drain(tb);
 }
 
 // One launch over many blocks (of one or many scenarios): CTA i works on the
 // descriptor whose CTA range holds i, found by binary search in the packed
 // table (descriptors sorted by cta0).
-template <bool CURV, int NS>
-__global__ void __launch_bounds__(TmaTile<CURV, 0>::NT + 32, 1)
+template <bool CURV>
+__global__ void __launch_bounds__(2 * TmaTile<CURV, 0>::NT + 32, 1)
     stencil_kernel_tma_batch(const TmaBatchDesc* __restrict__ d, int nd, long long total) {
   // the entry's arguments are copied to shared memory: read from there they
   // cost no registers across the plane loop (held in registers they spill)
   __shared__ VolumeArgs<float> sa;
-  Ring<CURV, NS, 0> ring;
+  Ring<CURV, 0> ring;
   const long long cta = blockIdx.x;
   int lo = 0, hi = nd - 1;
   while (lo < hi) {
@@ -800,13 +845,13 @@ __global__ void __launch_bounds__(TmaTile<CURV, 0>::NT + 32, 1)
   }
   // the table was written by a host copy: order that write before the
   // tensor-map proxy reads the entry's maps (in the thread that issues copies)
-  if (threadIdx.x == TmaTile<CURV, 0>::NT)
+  if (threadIdx.x == 2 * TmaTile<CURV, 0>::NT)
     for (int i = 0; i < 9; ++i)
       asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(&D.m[i]) : "memory");
   ring.init();  // its barrier also publishes sa
   int tb = 0;
   const long long l = cta - D.cta0;
-  tma_body<CURV, NS, 0>(sa, *reinterpret_cast<const MapArgs*>(&D.m), D.schunk, (int)(l % D.tq),
+  tma_body<CURV, 0>(sa, *reinterpret_cast<const MapArgs*>(&D.m), D.schunk, (int)(l % D.tq),
                             (int)((l / D.tq) % D.tr), (int)(l / ((long long)D.tq * D.tr)), ring.tab, tb);
   ring.drain(tb);
 }
@@ -822,19 +867,19 @@ struct TwoBlocks {
   int ntile0;
 };
 
-template <bool CURV, int NS, int FD, int TQW>
-__global__ void __launch_bounds__(TmaTile<CURV, FD, TQW>::NT + 32, 1)
+template <bool CURV, int FD, int TQW>
+__global__ void __launch_bounds__(2 * TmaTile<CURV, FD, TQW>::NT + 32, 1)
     stencil_kernel_tma2(const __grid_constant__ TwoBlocks P) {
-  Ring<CURV, NS, FD, TQW> ring;
+  Ring<CURV, FD, TQW> ring;
   ring.init();
   int tb = 0;
   const int w = blockIdx.x;
   if (w < P.ntile0) {
-    tma_body<CURV, NS, FD, TQW>(P.a[0], P.m[0], P.schunk[0], w % P.tq[0], (w / P.tq[0]) % P.tr[0],
+    tma_body<CURV, FD, TQW>(P.a[0], P.m[0], P.schunk[0], w % P.tq[0], (w / P.tq[0]) % P.tr[0],
                               w / (P.tq[0] * P.tr[0]), ring.tab, tb);
   } else {
     const int l = w - P.ntile0;
-    tma_body<CURV, NS, FD, TQW>(P.a[1], P.m[1], P.schunk[1], l % P.tq[1], (l / P.tq[1]) % P.tr[1],
+    tma_body<CURV, FD, TQW>(P.a[1], P.m[1], P.schunk[1], l % P.tq[1], (l / P.tq[1]) % P.tr[1],
                               l / (P.tq[1] * P.tr[1]), ring.tab, tb);
   }
   ring.drain(tb);
@@ -890,21 +935,21 @@ MapArgs stage_maps(const StencilMaps& sm) {
 }
 
 template <bool CURV, int FD, int TQW = kTmaTQ>
-constexpr size_t tma_smem_bytes(int NS) {
-  return sizeof(float) * (size_t)NS * TmaTile<CURV, FD, TQW>::STAGE_W + (2 * NS + 1) * sizeof(uint64_t) + 120 * sizeof(float) + 128;
+constexpr size_t tma_smem_bytes() {
+  constexpr int NS = TmaTile<CURV, FD, TQW>::NS;
+  return sizeof(float) * (size_t)NS * TmaTile<CURV, FD, TQW>::STAGE_W + (3 * NS + 1) * sizeof(uint64_t) + 120 * sizeof(float) + 128;
 }
-static_assert(tma_smem_bytes<true, 0>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<false, 0>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<true, 1>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<false, 1>(kTmaStages) <= 227 * 1024,
+static_assert(tma_smem_bytes<true, 0>() <= 227 * 1024 &&
+                  tma_smem_bytes<false, 0>() <= 227 * 1024 &&
+                  tma_smem_bytes<true, 1>() <= 227 * 1024 &&
+                  tma_smem_bytes<false, 1>() <= 227 * 1024,
               "the stage ring must fit in the shared memory of one CTA");
-static_assert(tma_smem_bytes<false, 0, kTmaTQWide>(kTmaStages) <= 227 * 1024 &&
-                  tma_smem_bytes<false, 1, kTmaTQWide>(kTmaStages) <= 227 * 1024,
+static_assert(tma_smem_bytes<false, 0, kTmaTQWide>() <= 227 * 1024 &&
+                  tma_smem_bytes<false, 1, kTmaTQWide>() <= 227 * 1024,
               "the wide Cartesian stage ring must fit in the shared memory of one CTA");
 
 template <typename K>
-size_t prepare(K kern, int NS, int stage_words) {
-  const size_t smem = sizeof(float) * (size_t)NS * stage_words + (2 * NS + 1) * sizeof(uint64_t) + 120 * sizeof(float) + 128;
+size_t prepare(K kern, size_t smem) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   return smem;
 }
@@ -914,22 +959,22 @@ size_t prepare(K kern, int NS, int stage_words) {
 // tiles statically interleaved that measured slower on 2 x 201^3 blocks
 // (0.54 ms against 0.50 ms per launch): the chunks holding the s closure
 // rows take longer, and the hardware's dynamic CTA scheduling balances them.
-template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int FD, int TQW = kTmaTQ>
 void launch_tma(const VolumeArgs<float>& a, const StencilMaps& sm, cudaStream_t s) {
   using TL = TmaTile<CURV, FD, TQW>;
-  auto kern = stencil_kernel_tma<CURV, NS, FD, TQW>;
-  static const size_t smem = prepare(kern, NS, TL::STAGE_W);
+  auto kern = stencil_kernel_tma<CURV, FD, TQW>;
+  static const size_t smem = prepare(kern, tma_smem_bytes<CURV, FD, TQW>());
   const int tq = (a.nq + TL::TQ - 1) / TL::TQ, tr = (a.nr + TL::TR - 1) / TL::TR;
   const int schunk = chunk_planes(a);
   const int ntile = tq * tr * ((a.ns + schunk - 1) / schunk);
-  kern<<<ntile, TL::NT + 32, smem, s>>>(a, stage_maps(sm), schunk, tq, tr, ntile);
+  kern<<<ntile, 2 * TL::NT + 32, smem, s>>>(a, stage_maps(sm), schunk, tq, tr, ntile);
 }
 
-template <bool CURV, int NS, int FD, int TQW = kTmaTQ>
+template <bool CURV, int FD, int TQW = kTmaTQ>
 void launch_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, cudaStream_t s) {
   using TL = TmaTile<CURV, FD, TQW>;
-  auto kern = stencil_kernel_tma2<CURV, NS, FD, TQW>;
-  static const size_t smem = prepare(kern, NS, TL::STAGE_W);
+  auto kern = stencil_kernel_tma2<CURV, FD, TQW>;
+  static const size_t smem = prepare(kern, tma_smem_bytes<CURV, FD, TQW>());
   TwoBlocks P;
   const VolumeArgs<float>* a[2] = {&a0, &a1};
   int ntile[2];
@@ -947,16 +992,16 @@ void launch_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, cudaS
     ntile[b] = tiles[b] * ((a[b]->ns + P.schunk[b] - 1) / P.schunk[b]);
   }
   P.ntile0 = ntile[0];
-  kern<<<ntile[0] + ntile[1], TL::NT + 32, smem, s>>>(P);
+  kern<<<ntile[0] + ntile[1], 2 * TL::NT + 32, smem, s>>>(P);
 }
 
-template <bool CURV, int NS>
+template <bool CURV>
 void launch_tma_batch(const TmaBatchDesc* d, int nd, long long total, cudaStream_t s) {
   using TL = TmaTile<CURV, 0>;
-  auto kern = stencil_kernel_tma_batch<CURV, NS>;
-  static const size_t smem = prepare(kern, NS, TL::STAGE_W);
+  auto kern = stencil_kernel_tma_batch<CURV>;
+  static const size_t smem = prepare(kern, tma_smem_bytes<CURV, 0>());
   if (total <= 0) return;
-  kern<<<(unsigned)total, TL::NT + 32, smem, s>>>(d, nd, total);
+  kern<<<(unsigned)total, 2 * TL::NT + 32, smem, s>>>(d, nd, total);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -999,7 +1044,7 @@ int encode4(CUtensorMap* map, void* base, int nq, int nr, int ns, int ncomp, int
 
 int make_stencil_maps(StencilMaps& m, void* const F[2], void* coef, void* DF, void* C, int nq, int nr, int ns, int pq,
                       bool curv, int fd, int tq) {
-  const int TQ = (tq == kTmaTQWide && !curv) ? kTmaTQWide : kTmaTQ, TR = kTmaTR;
+  const int TQ = (tq == kTmaTQWide && !curv) ? kTmaTQWide : kTmaTQ, TR = tma_rows(TQ);
   const int hr = fd ? 4 : 3;  // r halo rows
   int rc = 0;
   m.ok = 0;
@@ -1060,21 +1105,21 @@ int tma_tile_width(int nq0, int nq1, bool curv) {
 
 void launch_stencil_tma_batch(const TmaBatchDesc* d, int nd, long long total, bool curv, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
-  if (curv) launch_tma_batch<true, kTmaStages>(d, nd, total, s);
-  else launch_tma_batch<false, kTmaStages>(d, nd, total, s);
+  if (curv) launch_tma_batch<true>(d, nd, total, s);
+  else launch_tma_batch<false>(d, nd, total, s);
 }
 
 void launch_stencil_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, bool curv, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   if (!curv && static_cast<const StencilMaps*>(a0.tma)->tq == kTmaTQWide) {
-    if (a0.fd) launch_tma2<false, kTmaStages, 1, kTmaTQWide>(a0, a1, s);
-    else launch_tma2<false, kTmaStages, 0, kTmaTQWide>(a0, a1, s);
+    if (a0.fd) launch_tma2<false, 1, kTmaTQWide>(a0, a1, s);
+    else launch_tma2<false, 0, kTmaTQWide>(a0, a1, s);
   } else if (a0.fd) {
-    if (curv) launch_tma2<true, kTmaStages, 1>(a0, a1, s);
-    else launch_tma2<false, kTmaStages, 1>(a0, a1, s);
+    if (curv) launch_tma2<true, 1>(a0, a1, s);
+    else launch_tma2<false, 1>(a0, a1, s);
   } else {
-    if (curv) launch_tma2<true, kTmaStages, 0>(a0, a1, s);
-    else launch_tma2<false, kTmaStages, 0>(a0, a1, s);
+    if (curv) launch_tma2<true, 0>(a0, a1, s);
+    else launch_tma2<false, 0>(a0, a1, s);
   }
 }
 
@@ -1082,14 +1127,14 @@ void launch_stencil_tma(const VolumeArgs<float>& a, bool curv, void* stream) {
   const StencilMaps& sm = *static_cast<const StencilMaps*>(a.tma);
   cudaStream_t s = (cudaStream_t)stream;
   if (!curv && sm.tq == kTmaTQWide) {
-    if (a.fd) launch_tma<false, kTmaStages, 1, kTmaTQWide>(a, sm, s);
-    else launch_tma<false, kTmaStages, 0, kTmaTQWide>(a, sm, s);
+    if (a.fd) launch_tma<false, 1, kTmaTQWide>(a, sm, s);
+    else launch_tma<false, 0, kTmaTQWide>(a, sm, s);
   } else if (a.fd) {
-    if (curv) launch_tma<true, kTmaStages, 1>(a, sm, s);
-    else launch_tma<false, kTmaStages, 1>(a, sm, s);
+    if (curv) launch_tma<true, 1>(a, sm, s);
+    else launch_tma<false, 1>(a, sm, s);
   } else {
-    if (curv) launch_tma<true, kTmaStages, 0>(a, sm, s);
-    else launch_tma<false, kTmaStages, 0>(a, sm, s);
+    if (curv) launch_tma<true, 0>(a, sm, s);
+    else launch_tma<false, 0>(a, sm, s);
   }
 }
 

@@ -1183,6 +1183,12 @@ void launch_tiled(const VolumeArgs<T>& a, cudaStream_t s) {
 inline bool tiles_ok(int n, int T) { return n <= T + 3 || n >= T + 6; }
 inline bool tiles_ok_up(int n, int T) { return n <= T + 4 || n >= T + 6; }
 
+// Rows of the TMA tiles that the block's tensor maps are shaped for.
+template <typename T>
+int tma_tile_rows(const VolumeArgs<T>& a) {
+  return tma_rows(a.tma ? static_cast<const StencilMaps*>(a.tma)->tq : kTmaTQ);
+}
+
 template <typename T>
 int effective_variant(const VolumeArgs<T>& a) {
   constexpr bool f32 = sizeof(T) == 4;
@@ -1191,10 +1197,10 @@ int effective_variant(const VolumeArgs<T>& a) {
   if (a.fd) {
     // the order-6 upwind pair: the TMA kernel (compensated FP32) or per
     // point; order 5 per point
-    if (a.fd != 1 || !(v == 5 || v == 6) || a.C == nullptr || !tiles_ok_up(a.nr, kTmaTR)) v = 1;
+    if (a.fd != 1 || !(v == 5 || v == 6) || a.C == nullptr || !tiles_ok_up(a.nr, tma_tile_rows(a))) v = 1;
     return v;
   }
-  if ((v == 5 || v == 6) && !tiles_ok(a.nr, kTmaTR)) v = 1;
+  if ((v == 5 || v == 6) && !tiles_ok(a.nr, tma_tile_rows(a))) v = 1;
   if ((v == 2 || v == 3) && !(tiles_ok(a.nq, 32) && tiles_ok(a.nr, 8))) v = 1;
   if (v == 4 && !(tiles_ok(a.nq, 64) && tiles_ok(a.nr, 8))) v = 1;
   return v;
