@@ -1384,6 +1384,19 @@ int batch_tables(wql_batch* B, int* phase) {
   std::vector<TmaBatchDesc> h;
   B->cur0.assign(n, 0);
   for (size_t i = 0; i < n; ++i) B->cur0[i] = B->members[i]->cur;
+  // s chunks of the packed launch of each mesh kind
+  int chunk[2];
+  for (int curv = 0; curv < 2; ++curv) {
+    std::vector<int> tiles, planes;
+    for (auto* S : B->members)
+      if (batch_tma(S) && (int)S->curv == curv)
+        for (int b = 0; b < 2; ++b) {
+          const auto& K = S->B[b];
+          tiles.push_back(((K.nq + kTmaTQ - 1) / kTmaTQ) * ((K.nr + kTmaTR - 1) / kTmaTR));
+          planes.push_back(K.ns);
+        }
+    chunk[curv] = choose_chunk(tiles.data(), planes.data(), (int)tiles.size());
+  }
   for (int ph = 0; ph < 2; ++ph)
     for (int stage = 1; stage <= 5; ++stage)
       for (int curv = 0; curv < 2; ++curv) {
@@ -1400,7 +1413,7 @@ int batch_tables(wql_batch* B, int* phase) {
             VolumeArgs<float> a = volume_args<float>(S, b, stage_A(S, stage), stage_Bdt(S, stage), stage == 5);
             if (!tma_eligible(a)) continue;
             TmaBatchDesc d;
-            const long long k = fill_tma_desc(a, d);
+            const long long k = fill_tma_desc(a, chunk[curv], d);
             d.cta0 = g.total;
             g.total += k;
             h.push_back(d);

@@ -214,6 +214,7 @@ struct StencilMaps {
   int cur;                        // which field buffer is the stage input
   int fd;                         // operator the boxes are shaped for (0 central, 1 upwind)
   int tq;                         // tile width along q the boxes are shaped for
+  int chunk2;                     // planes per s chunk of the launch over both blocks (0: not chosen yet)
   int ok;
 };
 // Fills m for a block (fd: 0 the central SBP-6 operator, 1 the upwind pair:
@@ -248,9 +249,13 @@ struct TmaBatchDesc {
   int schunk, tq, tr, nchunk;
   long long cta0;
 };
-// Fills d for one block (a.tma must point at the block's StencilMaps) and
-// returns the number of CTAs it needs.
-long long fill_tma_desc(const VolumeArgs<float>& a, TmaBatchDesc& d);
+// Fills d for one block (a.tma must point at the block's StencilMaps), with
+// s chunks of `chunk` planes where none is tuned, and returns the number of
+// CTAs it needs.
+long long fill_tma_desc(const VolumeArgs<float>& a, int chunk, TmaBatchDesc& d);
+// Planes per s chunk of a launch over nb blocks of tiles[b] (q, r) tiles and
+// ns[b] planes.
+int choose_chunk(const int* tiles, const int* ns, int nb);
 // Whether a block can go through the TMA stencil (FP32, r extent that keeps
 // the closure rows of the shifted last r tile inside the halo).
 bool tma_eligible(const VolumeArgs<float>& a);

@@ -59,7 +59,9 @@
 
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <utility>
+#include <vector>
 
 #include "wql_internal.h"
 #include "wql_stencil.cuh"
@@ -900,25 +902,55 @@ int sm_count() {
   return n[dev];
 }
 
-// Chunk length for a launch over both blocks with `tiles[b]` (q, r) tiles
-// each: 32 planes while that gives at least 8 waves of one CTA per SM, else
-// shorter chunks (down to 12 planes) for more CTAs.  Measured per launch
-// (planes per chunk: ms): 2 x 201^3 curvilinear, 1666 CTAs at 32 planes,
-// 16: 0.904, 24: 0.902, 32: 0.891; 2 x 401x201x201, 3094 CTAs at 32,
-// 16: 1.829, 24: 1.782, 32: 1.765; 2 x 76x101x151 Cartesian upwind, 270 CTAs
-// at 32, 12: 0.173, 16: 0.176, 24: 0.197, 32: 0.194.  Equal-length chunks
-// (29 planes on 201) measured slower than 32 with a short last chunk.
-int chunk_planes2(const VolumeArgs<float>* const a[2], const int tiles[2]) {
-  if (a[0]->schunk > 0) return a[0]->schunk;
-  const long long want = 8LL * sm_count();
-  int c = 32;
-  for (; c > 12; c -= 4) {
-    long long ncta = 0;
-    for (int b = 0; b < 2; ++b) ncta += (long long)tiles[b] * ((a[b]->ns + c - 1) / c);
-    if (ncta >= want) break;
+}  // namespace
+
+// Planes per s chunk of a launch over nb blocks of tiles[b] (q, r) tiles and
+// ns[b] planes.  With 8 or more waves of one CTA per SM at 32 planes, 32: the
+// scheduler evens out what is left (2 x 201^3, 11 waves: 4.40 ms a step at 32,
+// 4.45-4.52 at 12 to 29 and at 41 and more).  With fewer, the length that
+// ends soonest when the CTAs go to the SMs in launch order, as they become
+// free; a chunk costs its planes plus 2 for its start (the six window planes)
+// plus 0.5 for each plane with an s closure row.  Measured ms a step at the
+// chosen length and at the 12 planes that short launches took: 2 x 41^3 5: 0.217,
+// 0.265; 76/75 x 150^2 39: 1.09, 1.14; 101/93 x 107x113 26: 0.93, 0.95; upwind
+// 2 x 76x101x151 14: 1.38, 1.44 (correlation of the rule with the measured
+// times over 19 lengths: 0.91 to 1.00).
+int choose_chunk(const int* tiles, const int* ns, int nb) {
+  const int sms = sm_count();
+  auto ctas = [&](int c) {
+    long long n = 0;
+    for (int b = 0; b < nb; ++b) n += (long long)tiles[b] * ((ns[b] + c - 1) / c);
+    return n;
+  };
+  if (ctas(32) >= 8LL * sms) return 32;
+  int best = 32;
+  float best_t = 1e30f;
+  std::vector<float> heap;
+  for (int c = 4; c <= 48; ++c) {
+    if (ctas(c) > 8LL * sms) continue;
+    heap.assign(sms, 0.0f);  // a min-heap of the times at which the SMs are free
+    float end = 0.0f;
+    for (int b = 0; b < nb; ++b)
+      for (int z = 0; z < ns[b]; z += c) {
+        const int pl = std::min(c, ns[b] - z);
+        const int left = std::max(0, std::min(z + pl, 6) - z), right = std::max(0, z + pl - std::max(z, ns[b] - 6));
+        const float cost = 2.0f + pl + 0.5f * std::min(pl, left + right);
+        for (int t = 0; t < tiles[b]; ++t) {
+          std::pop_heap(heap.begin(), heap.end(), std::greater<float>());
+          heap.back() += cost;
+          end = std::max(end, heap.back());
+          std::push_heap(heap.begin(), heap.end(), std::greater<float>());
+        }
+      }
+    if (end < best_t) {
+      best_t = end;
+      best = c;
+    }
   }
-  return c;
+  return best;
 }
+
+namespace {
 
 MapArgs stage_maps(const StencilMaps& sm) {
   MapArgs m;
@@ -986,9 +1018,14 @@ void launch_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, cudaS
     P.tr[b] = (a[b]->nr + TL::TR - 1) / TL::TR;
     tiles[b] = P.tq[b] * P.tr[b];
   }
-  const int c = chunk_planes2(a, tiles);
+  // kept with block 0's maps: the blocks and their tiles do not change
+  StencilMaps& keep = *static_cast<StencilMaps*>(const_cast<void*>(a0.tma));
+  if (a0.schunk <= 0 && keep.chunk2 == 0) {
+    const int planes[2] = {a0.ns, a1.ns};
+    keep.chunk2 = choose_chunk(tiles, planes, 2);
+  }
   for (int b = 0; b < 2; ++b) {
-    P.schunk[b] = a[b]->schunk > 0 ? a[b]->schunk : c;
+    P.schunk[b] = a[b]->schunk > 0 ? a[b]->schunk : keep.chunk2;
     ntile[b] = tiles[b] * ((a[b]->ns + P.schunk[b] - 1) / P.schunk[b]);
   }
   P.ntile0 = ntile[0];
@@ -1051,6 +1088,7 @@ int make_stencil_maps(StencilMaps& m, void* const F[2], void* coef, void* DF, vo
   m.cur = 0;
   m.fd = fd;
   m.tq = TQ;
+  m.chunk2 = 0;
   for (int i = 0; i < 2 && !rc; ++i) {
     rc = encode4(&m.fbox[i], F[i], nq, nr, ns, 9, pq, TQ + 16, TR + 2 * hr, 9);
     // lead tiles: all 9 components of one plane, or (upwind) the 3
@@ -1075,13 +1113,13 @@ int make_stencil_maps(StencilMaps& m, void* const F[2], void* coef, void* DF, vo
   return rc;
 }
 
-long long fill_tma_desc(const VolumeArgs<float>& a, TmaBatchDesc& d) {
+long long fill_tma_desc(const VolumeArgs<float>& a, int chunk, TmaBatchDesc& d) {
   static_assert(sizeof(MapArgs) == sizeof(d.m), "map set layout");
   const StencilMaps& sm = *static_cast<const StencilMaps*>(a.tma);
   const MapArgs m = stage_maps(sm);
   std::memcpy(d.m, &m, sizeof(m));
   d.a = a;
-  d.schunk = chunk_planes(a);
+  d.schunk = a.schunk > 0 ? a.schunk : chunk;
   d.tq = (a.nq + kTmaTQ - 1) / kTmaTQ;
   d.tr = (a.nr + kTmaTR - 1) / kTmaTR;
   d.nchunk = (a.ns + d.schunk - 1) / d.schunk;
