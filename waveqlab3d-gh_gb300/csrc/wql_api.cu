@@ -1106,6 +1106,7 @@ VolumeArgs<T> volume_args(wql_scn* S, int b, double A, double Bdt, bool last) {
   a.npml = B.npml;
   a.A = (T)A;
   a.Bdt = (T)Bdt;
+  a.Ainv = A != 0.0 ? (T)(1.0 / A) : T(1);
   a.plastic = (S->plastic && last) ? 1 : 0;
   a.preset = S->fp.preset;
   if (S->fp.preset == PRE_SW_PARAM || S->fp.preset == PRE_RS_PARAM) a.preset = S->fp.s0_profile;
@@ -1131,6 +1132,7 @@ VolumeArgs<T> volume_args(wql_scn* S, int b, double A, double Bdt, bool last) {
     a.an_w[m] = S->an_w[m];
   }
   a.pml_d0 = 6.0 / (2.0 * 1.0) * std::log(1.0 / 1.0e-3);
+  a.pml_dn = B.npml ? (T)(a.pml_d0 / B.npml) : T(0);
   a.ms = (const T*)B.ms;
   a.mp = (const T*)B.mp;
   a.mms_T = (T)S->mms_T;

@@ -104,6 +104,8 @@ struct VolumeArgs {
   int schunk;         // planes per CTA along s for the tiled kernel (0: default)
   // RK
   T A, Bdt;
+  T Ainv;             // 1/A, or 1 on the stage with A = 0
+  T pml_dn;           // PML damping per layer, pml_d0 / npml
   // plasticity on the last stage
   int plastic;
   int preset;          // initial-stress preset for the plastic update (PRE_NONE: s0u)

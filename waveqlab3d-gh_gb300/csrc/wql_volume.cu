@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <utility>
 
 #include "wql_internal.h"
@@ -139,20 +140,13 @@ __device__ __forceinline__ void visit_row(const T* tab, const UpG& g, bool shell
       const T sgn = left ? T(1) : T(-1);
       const T* wv = tab + (FD && !left ? NR * NC : 0) + row * NC;
       const T* wf = FD ? tab + (left ? NR * NC : 0) + row * NC : wv;
-#pragma unroll
+#pragma unroll(FD == 1 ? 5 : (FD == 2 ? 7 : 3))
       for (int t = 0; t < NC; ++t) {
         const int off = left ? t - row : row - t;
-        if (FD == 0) {
-          const T w = wv[t];
-          if (w != T(0)) {
-            vel(off, sgn * w);
-            flux(off, sgn * w);
-          }
-        } else {
-          const T w = wv[t], x = wf[t];
-          if (w != T(0)) vel(off, sgn * w);
-          if (x != T(0)) flux(off, sgn * x);
-        }
+        // zero weights too: a test per column would put its latency before
+        // the column's loads
+        vel(off, sgn * wv[t]);
+        flux(off, sgn * wf[t]);
       }
     }
   }
@@ -639,12 +633,11 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int
   T corr[9];
 #pragma unroll
   for (int c = 0; c < 9; ++c) corr[c] = T(0);
-#pragma unroll 1
-  while (sides) {
-    const int side = __ffs(sides) - 1;
-    sides &= sides - 1;
-    const int axis = side >> 1;
-    const bool hi = side & 1;
+  // one side; the axis is a compile-time constant so that the bases of all
+  // loads are uniform
+  auto take_side = [&](auto ax, const bool hi) {
+    constexpr int axis = decltype(ax)::value;
+    const int side = 2 * axis + (hi ? 1 : 0);
     const int ii = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 0 ? nq : (axis == 1 ? nr : ns);
     // flux components of physical axis `axis`: sigma_{c,axis}
     const T* __restrict__ S0 = F + (axis == 0 ? 3 : (axis == 1 ? 6 : 7)) * np;
@@ -690,9 +683,9 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int
     // Q and DQ are read after the derivatives (held across them, they spill)
     T qv[9], dq[9];
     const bool forced = (hi ? ii == n - 1 : ii == 0) && a.bc[side] >= 1 && a.bc[side] <= 3;
-    const long long sp = slab_point(a, side, i, j, k), snp = a.slab_np[side];
-    T* __restrict__ Q = a.Q[side] + sp;
-    T* __restrict__ DQ = a.DQ[side] + sp;
+    const long long sp = slab_point(a, side, i, j, k), snp = hi ? a.slab_np[2 * axis + 1] : a.slab_np[2 * axis];
+    T* __restrict__ Q = (hi ? a.Q[2 * axis + 1] : a.Q[2 * axis]) + sp;
+    T* __restrict__ DQ = (hi ? a.DQ[2 * axis + 1] : a.DQ[2 * axis]) + sp;
 #pragma unroll
     for (int c = 0; c < 9; ++c) {
       qv[c] = Q[c * snp];
@@ -701,7 +694,7 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int
     const T sc = CURV ? Jinv : a.cart_metric[axis];
     // damping profile in grid-index units (src/RHS_Interior.f90:1855,1973,2092)
     const int off = hi ? ii + 1 - (n - npml) : (axis == 2 ? ii + 1 - npml : ii - npml);
-    const T damp = (T)a.pml_d0 * (fabs((T)off / (T)npml));
+    const T damp = a.pml_dn * (T)abs(off);
     const T cfs = T(1);
     const T dr = damp * rhoinv, dm = mu * damp;
     const T tr = damp * (lam * (qv[3] + qv[4] + qv[5])), d2 = dm + dm;
@@ -732,9 +725,15 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int
       DQ[c * snp] = nw;
       Q[c * snp] = qv[c] + a.Bdt * nw;
     }
-  }
+  };
+#pragma unroll 1
+  for (unsigned m = sides & 3; m; m &= m - 1) take_side(std::integral_constant<int, 0>{}, m & 1 ? false : true);
+#pragma unroll 1
+  for (unsigned m = sides >> 2 & 3; m; m &= m - 1) take_side(std::integral_constant<int, 1>{}, m & 1 ? false : true);
+#pragma unroll 1
+  for (unsigned m = sides >> 4 & 3; m; m &= m - 1) take_side(std::integral_constant<int, 2>{}, m & 1 ? false : true);
   const bool face = i == 0 || i == nq - 1 || j == 0 || j == nr - 1 || k == 0 || k == ns - 1;
-  const T inv = keep ? T(1) / a.A : T(1);
+  const T inv = a.Ainv;
   T df[9];
 #pragma unroll
   for (int c = 0; c < 9; ++c) df[c] = keep || face ? at(a.DF + c * np, o) : T(0);
