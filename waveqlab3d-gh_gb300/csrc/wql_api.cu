@@ -313,6 +313,10 @@ __global__ void dense_to_pitched(const double* __restrict__ in, int pq, int nq, 
 }
 
 
+// The field buffer that the next stage writes and nothing reads before: room
+// for one dense FP64 component (9 pitched components of at least 4 bytes).
+double* field_scratch(wql_scn* scn, int block) { return (double*)scn->B[block].F[scn->cur ^ 1]; }
+
 // Dense (nq-pitched) FP64 array to a pq-pitched array of T.
 template <typename T>
 __global__ void pad_rows(const double* in, T* out, int nq, int pq, long long npd) {
@@ -331,10 +335,11 @@ __global__ void station_kernel(const T* __restrict__ F, long long np, const long
   for (int c = 0; c < 3; ++c) out[i * 3 + c] = (double)F[c * np + p];
 }
 
+// Grid points only: the row pads hold no field values.
 template <typename T>
-__global__ void count_nonfinite(const T* a, long long n, unsigned int* cnt) {
+__global__ void count_nonfinite(const T* a, long long n, int nq, int pq, unsigned int* cnt) {
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p < n && !isfinite((double)a[p])) atomicAdd(cnt, 1u);
+  if (p < n && p % pq < nq && !isfinite((double)a[p])) atomicAdd(cnt, 1u);
 }
 
 // source_time (src/moment_tensor.f90:958-1011); false for an unknown type.
@@ -1646,9 +1651,9 @@ int wql_sync(wql_scn* scn, int check_nan) {
     for (int b = 0; b < 2; ++b) {
       const long long n = 9 * scn->B[b].np;
       if (scn->prec == WQL_FP64)
-        count_nonfinite<double><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const double*)scn->B[b].F[scn->cur], n, cnt);
+        count_nonfinite<double><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const double*)scn->B[b].F[scn->cur], n, scn->B[b].nq, scn->B[b].pq, cnt);
       else
-        count_nonfinite<float><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const float*)scn->B[b].F[scn->cur], n, cnt);
+        count_nonfinite<float><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const float*)scn->B[b].F[scn->cur], n, scn->B[b].nq, scn->B[b].pq, cnt);
     }
     unsigned int h = 0;
     CK(cudaStreamSynchronize(scn->stream));
@@ -1685,19 +1690,18 @@ int wql_get_field(wql_scn* scn, int block, int comp, double* host_out) {
     return fail(WQL_E_STATE, "components 9 and 10 (plastic strain rate and strain) need plastic_flow");
   const void* src = comp == 9 ? B.pl_lambda : (comp == 10 ? B.pl_gammap : B.F[scn->cur]);
   const long long off = comp > 8 ? 0 : comp * B.np;
-  CK(cudaStreamSynchronize(scn->stream));
   const long long rows = (long long)B.nr * B.ns;
-  double* tmp = nullptr;
-  CK(cudaMalloc(&tmp, B.npd * sizeof(double)));
+  // dense FP64 values go through the buffer that the next stage overwrites:
+  // an allocation and its release would wait for all work on the device
+  double* tmp = field_scratch(scn, block);
   const unsigned grid = (unsigned)std::min<long long>((B.npd + 255) / 256, 4096);
   if (scn->prec == WQL_FP64)
     pitched_to_dense<double><<<grid, 256, 0, scn->stream>>>((const double*)src + off, B.pq, B.nq, rows, tmp);
   else
     pitched_to_dense<float><<<grid, 256, 0, scn->stream>>>((const float*)src + off, B.pq, B.nq, rows, tmp);
-  cudaError_t e = cudaStreamSynchronize(scn->stream);
-  if (e == cudaSuccess) e = cudaMemcpy(host_out, tmp, B.npd * sizeof(double), cudaMemcpyDeviceToHost);
-  cudaFree(tmp);
-  if (e != cudaSuccess) return fail(WQL_E_CUDA, cudaGetErrorString(e));
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(host_out, tmp, B.npd * sizeof(double), cudaMemcpyDeviceToHost, scn->stream));
+  CK(cudaStreamSynchronize(scn->stream));
   return WQL_OK;
 }
 
@@ -1784,23 +1788,18 @@ int wql_set_field(wql_scn* scn, int block, int comp, const double* host_in) {
   if (!scn || !host_in || block < 0 || block > 1 || comp < 0 || comp > 8)
     return fail(WQL_E_INPUT, "bad argument");
   auto& B = scn->B[block];
-  CK(cudaStreamSynchronize(scn->stream));
   const long long rows = (long long)B.nr * B.ns;
-  double* tmp = nullptr;
-  CK(cudaMalloc(&tmp, B.npd * sizeof(double)));
-  cudaError_t e = cudaMemcpy(tmp, host_in, B.npd * sizeof(double), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) {
-    const unsigned grid = (unsigned)std::min<long long>((B.np + 255) / 256, 4096);
-    if (scn->prec == WQL_FP64)
-      dense_to_pitched<double><<<grid, 256, 0, scn->stream>>>(tmp, B.pq, B.nq, rows, (double*)B.F[scn->cur] + comp * B.np);
-    else
-      dense_to_pitched<float><<<grid, 256, 0, scn->stream>>>(tmp, B.pq, B.nq, rows, (float*)B.F[scn->cur] + comp * B.np);
-    // the new values carry no rounding error yet: clear their compensation
-    if (B.C) e = cudaMemsetAsync((comp_t*)B.C + comp * B.np, 0, B.np * sizeof(comp_t), scn->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(scn->stream);
-  }
-  cudaFree(tmp);
-  if (e != cudaSuccess) return fail(WQL_E_CUDA, cudaGetErrorString(e));
+  double* tmp = field_scratch(scn, block);
+  CK(cudaMemcpyAsync(tmp, host_in, B.npd * sizeof(double), cudaMemcpyHostToDevice, scn->stream));
+  const unsigned grid = (unsigned)std::min<long long>((B.np + 255) / 256, 4096);
+  if (scn->prec == WQL_FP64)
+    dense_to_pitched<double><<<grid, 256, 0, scn->stream>>>(tmp, B.pq, B.nq, rows, (double*)B.F[scn->cur] + comp * B.np);
+  else
+    dense_to_pitched<float><<<grid, 256, 0, scn->stream>>>(tmp, B.pq, B.nq, rows, (float*)B.F[scn->cur] + comp * B.np);
+  // the new values carry no rounding error yet: clear their compensation
+  if (B.C) CK(cudaMemsetAsync((comp_t*)B.C + comp * B.np, 0, B.np * sizeof(comp_t), scn->stream));
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(scn->stream));
   return WQL_OK;
 }
 
