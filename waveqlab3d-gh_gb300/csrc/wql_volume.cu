@@ -65,9 +65,19 @@ __device__ __forceinline__ void load6(const T* __restrict__ F, const T* __restri
 //   FD 0  SBP-6: [row 6][point 9]
 //   FD 1  upwind order 6: [D+, D-][row 6][point 10]
 //   FD 2  upwind order 5: [D+, D-][row 4][point 7]
-//   FD 3  a table operator: the whole table (UpG)
+//   FD 3..5  a table operator whose interior rows lie within -(FD-1)..FD (D+)
+//         and -FD..FD-1 (D-): the whole table (UpG), then the interior rows on
+//         that window, [interior, shell][D+, D-][2*FD]
 template <int FD>
-constexpr int kRowWords = FD == 0 ? 54 : (FD == 1 ? 120 : (FD == 2 ? 56 : kUgWords));
+constexpr int kRowWords = FD == 0 ? 54 : (FD == 1 ? 120 : (FD == 2 ? 56 : kUgWords + 8 * FD));
+
+// The narrowest window that holds a table operator's interior rows (orders 2
+// to 4 and DRP 3: 3; order 7, DRP 4, 5 and 66: 4; the others 5).
+inline int ug_window(const UpG& g) {
+  for (int w = 3; w < 5; ++w)
+    if (g.plo >= 1 - w && g.plo + g.pn - 1 <= w && g.mlo >= -w && g.mlo + g.mn - 1 <= w - 1) return w;
+  return 5;
+}
 
 template <typename T, int FD>
 __device__ __forceinline__ void load_rows(T* tab, const UpG& g) {
@@ -76,7 +86,12 @@ __device__ __forceinline__ void load_rows(T* tab, const UpG& g) {
     if constexpr (FD == 0) tab[e] = sbp_w<T>(e / 9, e % 9);
     else if constexpr (FD == 1) tab[e] = up_w<T>(e / 60, e / 10 % 6, e % 10);
     else if constexpr (FD == 2) tab[e] = upw<T, 2>(e / 28, e / 7 % 4, e % 7);
-    else tab[e] = ((const T*)g.w)[e];
+    else if (e < kUgWords) tab[e] = ((const T*)g.w)[e];
+    else {
+      const int x = e - kUgWords, k = x % (2 * FD), minus = x / (2 * FD) & 1, set = x / (4 * FD);
+      const int idx = k - (minus ? FD + g.mlo : FD - 1 + g.plo);
+      tab[e] = idx >= 0 && idx < (minus ? g.mn : g.pn) ? ((const T*)g.w)[(2 * set + minus) * kUgCol + idx] : T(0);
+    }
   }
   __syncthreads();
 }
@@ -85,19 +100,30 @@ __device__ __forceinline__ void load_rows(T* tab, const UpG& g) {
 // rows of the velocity and the flux operator at 0-based index i of n along
 // axis d (one operator for both in FD 0, D+ and D- else).  Interior rows and
 // closure columns are unrolled so that their loads are in flight together.
-// shell (FD 3): the point lies in the boundary shell, whose interior rows are
+// shell (FD 3..5): the point lies in the boundary shell, whose interior rows are
 // the near-boundary routine's.
 template <typename T, int FD, typename V, typename X>
 __device__ __forceinline__ void visit_row(const T* tab, const UpG& g, bool shell, int i, int n, int d, V&& vel,
                                           X&& flux) {
-  if constexpr (FD == 3) {
+  if constexpr (FD >= 3) {
     if (i >= g.R && i < n - g.R) {
-      // orders 2..9 and the DRP operators: D+ within -4..5, D- within -5..4
-      const T* wp = tab + (shell ? 2 * kUgCol : 0);
+      // a fixed window with zero weights outside the operator's own: with the
+      // operator's run-time bounds tested per offset, every offset waited for
+      // its own loads.  Only rows nearer to an end than the window (orders 2
+      // and 3, whose closures are shorter) clamp its points to the axis.
+      const T* wp = tab + kUgWords + (shell ? 4 * FD : 0);
+      if (i >= FD && i < n - FD) {
 #pragma unroll
-      for (int o = -5; o <= 5; ++o) {
-        if (o >= -4 && o >= g.plo && o < g.plo + g.pn) vel(o, wp[o - g.plo]);
-        if (o <= 4 && o >= g.mlo && o < g.mlo + g.mn) flux(o, wp[kUgCol + o - g.mlo]);
+        for (int k = 0; k < 2 * FD; ++k) {
+          vel(k + 1 - FD, wp[k]);
+          flux(k - FD, wp[2 * FD + k]);
+        }
+      } else {
+#pragma unroll 2
+        for (int k = 0; k < 2 * FD; ++k) {
+          vel(min(max(k + 1 - FD, -i), n - 1 - i), wp[k]);
+          flux(min(max(k - FD, -i), n - 1 - i), wp[2 * FD + k]);
+        }
       }
     } else {
       // left row i reads points 0.., right row k = n-1-i points n-1-t
@@ -106,10 +132,9 @@ __device__ __forceinline__ void visit_row(const T* tab, const UpG& g, bool shell
       const T* wp = tab + 4 * kUgCol + (left ? 0 : 2 * kUgRowBlock) + (d * kUgRows + row) * kUgCol;
 #pragma unroll 4
       for (int t = 0; t < kUgCol; ++t) {
-        const int off = left ? t - row : row - t;
-        const T wv = wp[t], wf = wp[kUgRowBlock + t];
-        if (wv != T(0)) vel(off, wv);
-        if (wf != T(0)) flux(off, wf);
+        const int off = min(max(left ? t - row : row - t, -i), n - 1 - i);
+        vel(off, wp[t]);
+        flux(off, wp[kUgRowBlock + t]);
       }
     }
   } else {
@@ -432,7 +457,7 @@ __global__ void __launch_bounds__(256) stencil_kernel_pointwise(const __grid_con
   const T* __restrict__ coef = a.coef + p;
   T g[3][3], dv[3];
   const T Jinv = CURV ? coef[9 * np] : T(1);
-  const bool shell = FD == 3 && ug_shell(a, i, j, k);
+  const bool shell = FD >= 3 && ug_shell(a, i, j, k);
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const long long st = d == 0 ? 1 : (d == 1 ? (long long)a.pq : (long long)a.pq * a.nr);
@@ -627,7 +652,7 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int
   const T rinv = at(coef + (CURV ? 12 : 2) * np, o);
   const T rhoinv = CURV ? rinv / Jinv : rinv;
   const T l2m = lam + T(2) * mu;
-  const bool shell = FD == 3 && ug_shell(a, i, j, k);
+  const bool shell = FD >= 3 && ug_shell(a, i, j, k);
   // on a stage with A = 0, DF and DQ hold only what the face pre-kernel put there
   const bool keep = a.A != T(0);
   T corr[9];
@@ -766,7 +791,7 @@ void launch_pml_pre_fd(const PmlPair<T>& P, unsigned g, cudaStream_t s) {
     case 0: pml_pre_kernel<T, O, CURV, 0><<<g, 256, 0, s>>>(P); return;
     case 1: pml_pre_kernel<T, O, CURV, 1><<<g, 256, 0, s>>>(P); return;
     case 2: pml_pre_kernel<T, O, CURV, 2><<<g, 256, 0, s>>>(P); return;
-    default: pml_pre_kernel<T, O, CURV, 3><<<g, 256, 0, s>>>(P); return;
+    default: pml_pre_kernel<T, O, CURV, 5><<<g, 256, 0, s>>>(P); return;
   }
 }
 
@@ -835,7 +860,7 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
       for (int jj = 0; jj < 3; ++jj) g[c][jj] = a.G[(c * 3 + jj) * np + p];
   }
   if (a.G == nullptr) {
-    const bool shell = FD == 3 && ug_shell(a, i, j, k);
+    const bool shell = FD >= 3 && ug_shell(a, i, j, k);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const long long st = d == 0 ? 1 : (d == 1 ? (long long)a.pq : (long long)a.pq * nr);
@@ -1223,7 +1248,12 @@ void launch_pointwise(const VolumeArgs<T>& a0, const VolumeArgs<T>* a1, cudaStre
     case 0: stencil_kernel_pointwise<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(P); return;
     case 1: stencil_kernel_pointwise<T, CURV, KAHAN, 1><<<grd, blk, 0, s>>>(P); return;
     case 2: stencil_kernel_pointwise<T, CURV, KAHAN, 2><<<grd, blk, 0, s>>>(P); return;
-    default: stencil_kernel_pointwise<T, CURV, KAHAN, 3><<<grd, blk, 0, s>>>(P); return;
+    default: break;
+  }
+  switch (ug_window(a0.ug)) {
+    case 3: stencil_kernel_pointwise<T, CURV, KAHAN, 3><<<grd, blk, 0, s>>>(P); return;
+    case 4: stencil_kernel_pointwise<T, CURV, KAHAN, 4><<<grd, blk, 0, s>>>(P); return;
+    default: stencil_kernel_pointwise<T, CURV, KAHAN, 5><<<grd, blk, 0, s>>>(P); return;
   }
 }
 
@@ -1259,7 +1289,7 @@ int launch_corr(const VolumeArgs<T>& a, cudaStream_t s) {
   if (a.anel) {
     if (a.fd == 1) anelastic_kernel<T, CURV, KAHAN, 1><<<grd, blk, 0, s>>>(a);
     else if (a.fd == 2) anelastic_kernel<T, CURV, KAHAN, 2><<<grd, blk, 0, s>>>(a);
-    else if (a.fd == 3) anelastic_kernel<T, CURV, KAHAN, 3><<<grd, blk, 0, s>>>(a);
+    else if (a.fd == 3) anelastic_kernel<T, CURV, KAHAN, 5><<<grd, blk, 0, s>>>(a);
     else anelastic_kernel<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(a);
     ++n;
   }
