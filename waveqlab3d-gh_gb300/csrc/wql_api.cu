@@ -1135,6 +1135,7 @@ VolumeArgs<T> volume_args(wql_scn* S, int b, double A, double Bdt, bool last) {
   for (int m = 0; m < 4; ++m) {
     a.an_tau[m] = S->an_tau[m];
     a.an_w[m] = S->an_w[m];
+    a.an_tinv[m] = S->anel ? (T)(1.0 / S->an_tau[m]) : T(0);
   }
   a.pml_d0 = 6.0 / (2.0 * 1.0) * std::log(1.0 / 1.0e-3);
   a.pml_dn = B.npml ? (T)(a.pml_d0 / B.npml) : T(0);

@@ -129,6 +129,7 @@ struct VolumeArgs {
   T* Deta;
   const T* qsinv;
   double an_tau[4], an_w[4];
+  T an_tinv[4];                  // 1/tau
   int* err;                      // device error word (pipeline wait timeouts)
   double pml_d0;                 // PML damping scale 3 ln(1000)
   const void* tma;               // host pointer to the block's StencilMaps (FP32 only)

@@ -833,12 +833,12 @@ int launch_pml_pre(const VolumeArgs<T>& a0, const VolumeArgs<T>* a1, bool curv, 
 // and eta <- eta + B*dt*Deta.  Inside a PML slab the strain rates lose the
 // damped auxiliary fields (pml_damping_and_q, src/RHS_Interior.f90:
 // 2287-2387) of the stage's input.  The
-// velocity gradient comes from the TMA stencil (FP32C) or is formed here
-// with the block's operator.
+// velocity gradient is formed here with the block's operator (blocks whose
+// stencil hands it over take anelastic_comp_kernel).
 template <typename T, bool CURV, bool KAHAN, int FD>
 __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __grid_constant__ VolumeArgs<T> a) {
   __shared__ T tab[kRowWords<FD>];
-  if (a.G == nullptr) load_rows<T, FD>(tab, a.ug);
+  load_rows<T, FD>(tab, a.ug);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -851,15 +851,7 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
   const T* __restrict__ coef = a.coef;
   const T Jinv = CURV ? coef[9 * np + p] : T(1);
   T g[3][3];
-  // the velocity gradient: from the TMA stencil of this stage (a.G), else
-  // formed here
-  if (a.G != nullptr) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int jj = 0; jj < 3; ++jj) g[c][jj] = a.G[(c * 3 + jj) * np + p];
-  }
-  if (a.G == nullptr) {
+  {
     const bool shell = FD >= 3 && ug_shell(a, i, j, k);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -968,6 +960,83 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
     }
   }
   add_correction<T, KAHAN>(a, p, corr);
+}
+
+// The same with the velocity gradient at hand (a.G): six threads a point, one
+// per stress component, 64 consecutive points of the pitched block a CTA, both
+// blocks in a launch.  One thread a point walked the six components with 80
+// registers and 24 warps an SM, each waiting on its 66 streams (0.204 ms a
+// block of 76x101x151, 46 % of HBM); a component's loads are now all in flight
+// in 48 warps.
+template <typename T, bool CURV, bool KAHAN>
+__global__ void __launch_bounds__(384, 4) anelastic_comp_kernel(const __grid_constant__ BlockPair<T> P) {
+  const int blk = (long long)blockIdx.x >= P.n0 ? 1 : 0;
+  const VolumeArgs<T>& a = P.a[blk];
+  const long long p = ((long long)blockIdx.x - (blk ? P.n0 : 0)) * 64 + (threadIdx.x & 63);
+  const int c = threadIdx.x >> 6;  // stress component 3 + c
+  const long long np = a.np;
+  if (p >= np) return;
+  const int i = (int)(p % a.pq), jk = (int)(p / a.pq), j = jk % a.nr, k = jk / a.nr;
+  if (i >= a.nq) return;
+  const T* __restrict__ coef = a.coef + p;
+  const T* __restrict__ G = a.G + p;
+  T* __restrict__ eta = a.eta + 4 * c * np + p;
+  T* __restrict__ deta = a.Deta + 4 * c * np + p;
+  T ev[4], dv[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    ev[m] = eta[m * np];
+    dv[m] = deta[m * np];
+  }
+  const T mu = coef[(CURV ? 11 : 1) * np], qs = a.qsinv[p];
+  // the component's strain rate e (twice the shear strain) and the trace
+  T e, tr = T(0), lam = T(0);
+  if (c < 3) {
+    const T g0 = G[0], g1 = G[4 * np], g2_ = G[8 * np];
+    e = c == 0 ? g0 : (c == 1 ? g1 : g2_);
+    tr = g0 + g1 + g2_;
+    lam = coef[(CURV ? 10 : 0) * np];
+  } else {
+    e = c == 3 ? G[np] + G[3 * np] : (c == 4 ? G[2 * np] + G[6 * np] : G[5 * np] + G[7 * np]);
+  }
+#pragma unroll
+  for (int side = 0; side < 6; ++side) {
+    if (!a.pml[side]) continue;
+    const int axis = side >> 1;
+    const bool hi = side & 1;
+    const int ii = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 0 ? a.nq : (axis == 1 ? a.nr : a.ns);
+    if (!(hi ? ii >= n - a.npml : ii < a.npml)) continue;
+    // the axes of a shear component: xy 0 1, xz 0 2, yz 1 2
+    if (c >= 3 && (c == 3 ? axis == 2 : (c == 4 ? axis == 1 : axis == 0))) continue;
+    const int off = hi ? ii + 1 - (n - a.npml) : (axis == 2 ? ii + 1 - a.npml : ii - a.npml);
+    const T damp = a.pml_dn * (T)abs(off);
+    const long long snp = a.slab_np[side], q = (c < 3 ? 3 + axis : 3 + c) * snp + slab_point(a, side, i, j, k);
+    // the stage-input Q (see anelastic_kernel)
+    const T dq = damp * (a.Q[side][q] - a.Bdt * a.DQ[side][q]);
+    if (c < 3) tr -= dq;
+    if (c >= 3 || c == axis) e -= dq;
+  }
+  // (w 2 mu qs) e + w ((lam + 2 mu) qp - 2 mu qs) tr, or (w mu qs) e
+  const T ms = mu * qs;
+  const T f = c < 3 ? T(2) * ms * e + ((lam + T(2) * mu) * (T(0.5) * qs) - T(2) * ms) * tr : ms * e;
+  const T corr = -(ev[0] + ev[1] + ev[2] + ev[3]);
+  const long long o = (3 + c) * np + p;
+  const T df = a.DF[o], f0 = a.Fout[o];
+  const T ck = KAHAN ? (T)comp_get(a.C, o) : T(0);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const T de = a.A * dv[m] + ((T)a.an_w[m] * f - ev[m]) * a.an_tinv[m];
+    deta[m * np] = de;
+    eta[m * np] = ev[m] + a.Bdt * de;
+  }
+  a.DF[o] = df + corr;
+  if (KAHAN) {
+    const T y = a.Bdt * corr - ck, t = f0 + y;
+    comp_put(a.C, o, (float)((t - f0) - y));
+    a.Fout[o] = t;
+  } else {
+    a.Fout[o] = f0 + a.Bdt * corr;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1286,11 +1355,17 @@ template <typename T, bool CURV, bool KAHAN>
 int launch_corr(const VolumeArgs<T>& a, cudaStream_t s) {
   int n = 0;
   dim3 blk(32, 8, 1), grd((a.nq + 31) / 32, (a.nr + 7) / 8, a.ns);
-  if (a.anel) {
+  if (a.anel && a.G == nullptr) {
     if (a.fd == 1) anelastic_kernel<T, CURV, KAHAN, 1><<<grd, blk, 0, s>>>(a);
     else if (a.fd == 2) anelastic_kernel<T, CURV, KAHAN, 2><<<grd, blk, 0, s>>>(a);
     else if (a.fd == 3) anelastic_kernel<T, CURV, KAHAN, 5><<<grd, blk, 0, s>>>(a);
     else anelastic_kernel<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(a);
+    ++n;
+  } else if (a.anel) {
+    BlockPair<T> P;
+    P.a[0] = P.a[1] = a;
+    P.n0 = (a.np + 63) / 64;
+    anelastic_comp_kernel<T, CURV, KAHAN><<<(unsigned)P.n0, 384, 0, s>>>(P);
     ++n;
   }
   if (a.mp) {
