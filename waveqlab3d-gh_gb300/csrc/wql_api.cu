@@ -134,7 +134,8 @@ struct wql_scn {
     void* DF = nullptr;
     void* C = nullptr;
     void* coef = nullptr;
-    double* face[6] = {};
+    double* face[6] = {};  // FP64 face data; in FP32C only the fault side's is kept after set-up
+    float* facef[6] = {};  // FP32C: the same in FP32
     int bc[6] = {};
     int pml[6] = {};
     int npml = 0;
@@ -537,10 +538,22 @@ int setup_block(wql_scn* S, int b) {
   for (int s = 0; s < 6; ++s) {
     const int axis = s / 2;
     const long long nf = axis == 0 ? (long long)B.nr * B.ns : (axis == 1 ? (long long)B.nq * B.ns : (long long)B.nq * B.nr);
-    if ((rc = S->alloc((void**)&B.face[s], kFaceWords * nf * sizeof(double), false))) return rc;
+    const bool scratch = S->prec == WQL_FP32C && s != (b == 0 ? 1 : 0);
+    if ((rc = S->alloc((void**)&B.face[s], kFaceWords * nf * sizeof(double), false, scratch))) return rc;
+    if (S->prec == WQL_FP32C && (rc = S->alloc((void**)&B.facef[s], kFaceWords * nf * sizeof(float), false))) return rc;
   }
   launch_faces(B.nq, B.nr, B.ns, metric, mat, mat + np, mat + 2 * np, B.face, S->stream);
   CK(cudaGetLastError());
+  for (int s = 0; s < 6 && S->prec == WQL_FP32C; ++s) {
+    const int axis = s / 2;
+    const long long nf = axis == 0 ? (long long)B.nr * B.ns : (axis == 1 ? (long long)B.nq * B.ns : (long long)B.nq * B.nr);
+    launch_face_f32(kFaceWords * nf, B.face[s], B.facef[s], S->stream);
+    CK(cudaGetLastError());
+    if (s != (b == 0 ? 1 : 0)) {
+      S->release(B.face[s]);
+      B.face[s] = nullptr;
+    }
+  }
   // coefficients
   const int ncoef = S->curv ? kCurvCoef : kCartCoef;
   if ((rc = S->alloc(&B.coef, ncoef * B.np * S->esz))) return rc;
@@ -1094,7 +1107,8 @@ VolumeArgs<T> volume_args(wql_scn* S, int b, double A, double Bdt, bool last) {
     a.tau_h[d] = (T)B.tau_h[d];
   }
   for (int s = 0; s < 6; ++s) {
-    a.face[s] = B.face[s];
+    if constexpr (sizeof(T) == 8) a.face[s] = B.face[s];
+    else a.face[s] = B.facef[s];
     a.bc[s] = B.bc[s];
     a.pml[s] = B.pml[s];
     a.Q[s] = (T*)B.Q[s];
@@ -1193,8 +1207,6 @@ void stage_head(wql_scn* S, StepCtx& c, int stage) {
   ia.fp64 = S->prec == WQL_FP64;
   ia.F0 = S->B[0].F[S->cur];
   ia.F1 = S->B[1].F[S->cur];
-  ia.face0 = S->B[0].face[1];
-  ia.face1 = S->B[1].face[0];
   ia.xij = S->xij;
   ia.S = S->S; ia.DS = S->DS; ia.W = S->W; ia.DW = S->DW; ia.trup = S->trup;
   ia.sat = S->sat;
@@ -1215,6 +1227,9 @@ void stage_head(wql_scn* S, StepCtx& c, int stage) {
   ia.C0 = S->B[0].C;
   ia.C1 = S->B[1].C;
   ia.fault_comp = S->fault_comp && S->B[0].C && S->B[1].C;
+  const bool f64 = ia.fp64 || ia.fault_comp;  // the algebra's type
+  ia.face0 = f64 ? (const void*)S->B[0].face[1] : S->B[0].facef[1];
+  ia.face1 = f64 ? (const void*)S->B[1].face[0] : S->B[1].facef[0];
   if (S->mms) {
     // T(t) and T'(t) of the manufactured solution at this stage's time, for
     // the interface here and the block phases of the same stage
@@ -2133,7 +2148,11 @@ int wql_estimate_device_bytes(const char* in_text, const char* base_dir, int pre
     res += 2 * al(9 * np * esz) + al(9 * np * esz) + al((curv ? kCurvCoef : kCartCoef) * np * esz);
     if (precision == WQL_FP32C) res += al(9 * np * (long long)sizeof(comp_t));
     const long long nfs[3] = {nr * ns, nq * ns, nq * nr};
-    for (int s2 = 0; s2 < 6; ++s2) res += al(kFaceWords * nfs[s2 / 2] * 8);
+    long long faces = 0;  // FP64 face data that is set-up scratch in FP32C
+    for (int s2 = 0; s2 < 6; ++s2) {
+      if (precision == WQL_FP32C) res += al(kFaceWords * nfs[s2 / 2] * 4);
+      (precision == WQL_FP64 || s2 == (b == 0 ? 1 : 0) ? res : faces) += al(kFaceWords * nfs[s2 / 2] * 8);
+    }
     const int dims[3] = {(int)nq, (int)nr, (int)ns};
     for (int s2 = 0; s2 < 6; ++s2) {
       const bool pml = (s2 % 2 == 0) ? bp.pml_lqrs[s2 / 2] : bp.pml_rqrs[s2 / 2];
@@ -2146,7 +2165,7 @@ int wql_estimate_device_bytes(const char* in_text, const char* base_dir, int pre
       if (precision == WQL_FP32C) res += al(9 * np * esz);
     }
     // set-up arrays of one block: x, metric, J, material (FP64)
-    transient = std::max(transient, al(3 * npd * 8) + al(9 * npd * 8) + al(npd * 8) + al(3 * npd * 8));
+    transient = std::max(transient, faces + al(3 * npd * 8) + al(9 * npd * 8) + al(npd * 8) + al(3 * npd * 8));
   }
   res += al(6 * nf * 8) + 2 * al(8 * nf * 8) + 3 * al(2 * nf * 8) + al(18 * nf * esz) + al(10 * nf * 8) + 2 * 512;
   if (P.w_fault) res += 2 * al((long long)frame_ring_cap(nf) * kFrameWords * nf * 4);

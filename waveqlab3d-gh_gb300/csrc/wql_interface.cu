@@ -178,21 +178,20 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
       v[c] -= c < 3 ? v_v : v_s;
     }
   }
-  const double* face = b == 0 ? a.face0 : a.face1;
+  const R* __restrict__ face0 = (const R*)a.face0;
+  const R* __restrict__ face1 = (const R*)a.face1;
+  const R* __restrict__ face = b == 0 ? face0 : face1;
   R n[3], m[3], l[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    n[c] = (R)face[(0 + c) * nf + f];
-    m[c] = (R)face[(3 + c) * nf + f];
-    l[c] = (R)face[(6 + c) * nf + f];
+    n[c] = face[(0 + c) * nf + f];
+    m[c] = face[(3 + c) * nf + f];
+    l[c] = face[(6 + c) * nf + f];
   }
-  const R gx = (R)face[9 * nf + f], gy = (R)face[10 * nf + f], gz = (R)face[11 * nf + f];
-  // material on each side (block 0 / block 1 face)
-  const R lam1 = (R)a.face0[12 * nf + f], mu1 = (R)a.face0[13 * nf + f], rho1 = (R)a.face0[14 * nf + f];
-  const R lam2 = (R)a.face1[12 * nf + f], mu2 = (R)a.face1[13 * nf + f], rho2 = (R)a.face1[14 * nf + f];
-  const R c1p = sqrt((R(2) * mu1 + lam1) / rho1), c1s = sqrt(mu1 / rho1);
-  const R c2p = sqrt((R(2) * mu2 + lam2) / rho2), c2s = sqrt(mu2 / rho2);
-  const R Z1p = rho1 * c1p, Z1s = rho1 * c1s, Z2p = rho2 * c2p, Z2s = rho2 * c2s;
+  const R gx = face[9 * nf + f], gy = face[10 * nf + f], gz = face[11 * nf + f];
+  // impedances of each side (block 0 / block 1 face) and their reciprocals
+  const R Z1p = face0[16 * nf + f], Z1s = face0[17 * nf + f], Z2p = face1[16 * nf + f], Z2s = face1[17 * nf + f];
+  const R i1p = face0[18 * nf + f], i1s = face0[19 * nf + f], i2p = face1[18 * nf + f], i2s = face1[19 * nf + f];
   double x[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) x[c] = a.xij[(b * 3 + c) * nf + f];
@@ -223,11 +222,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
   // characteristics (src/Interface_Condition.f90:809-828)
   const R p_n = Z1p * ur[0] - ur[3], p_m = Z1s * ur[1] - ur[4], p_l = Z1s * ur[2] - ur[5];
   const R q_n = Z2p * vr[0] + vr[3], q_m = Z2s * vr[1] + vr[4], q_l = Z2s * vr[2] + vr[5];
-  const R eta_s = R(1) / (R(1) / Z1s + R(1) / Z2s);
-  const R eta_p = R(1) / (R(1) / Z1p + R(1) / Z2p);
-  const R phi_n = eta_p * (q_n / Z2p - p_n / Z1p);
-  const R phi_m = eta_s * (q_m / Z2s - p_m / Z1s);
-  const R phi_l = eta_s * (q_l / Z2s - p_l / Z1s);
+  const R eta_s = R(1) / (i1s + i2s);
+  const R eta_p = R(1) / (i1p + i2p);
+  const R phi_n = eta_p * (q_n * i2p - p_n * i1p);
+  const R phi_m = eta_s * (q_m * i2s - p_m * i1s);
+  const R phi_l = eta_s * (q_l * i2s - p_l * i1s);
 
   double* S = a.S + (long long)b * 4 * nf;
   double* DS = a.DS + (long long)b * 4 * nf;
@@ -240,18 +239,18 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
   const int cpl = a.fp.coupling;
   if (cpl == CPL_LOCKED) {
     // Welded_Interface (src/Interface_Condition.f90:516-637)
-    P[0] = (q_n - phi_n) / Z2p; P[1] = (q_m - phi_m) / Z2s; P[2] = (q_l - phi_l) / Z2s;
-    Q[0] = (p_n + phi_n) / Z1p; Q[1] = (p_m + phi_m) / Z1s; Q[2] = (p_l + phi_l) / Z1s;
+    P[0] = (q_n - phi_n) * i2p; P[1] = (q_m - phi_m) * i2s; P[2] = (q_l - phi_l) * i2s;
+    Q[0] = (p_n + phi_n) * i1p; Q[1] = (p_m + phi_m) * i1s; Q[2] = (p_l + phi_l) * i1s;
     P[3] = Q[3] = phi_n; P[4] = Q[4] = phi_m; P[5] = Q[5] = phi_l;
   } else if (cpl == CPL_LINEAR) {
     // Linear_Friction with alpha = 1e14 (src/Interface_Condition.f90:639-742)
     const R al = R(1.0e14);
     const R tm = al / (al + eta_s) * phi_m, tl = al / (al + eta_s) * phi_l;
-    P[0] = (q_n - phi_n) / Z2p; Q[0] = (p_n + phi_n) / Z1p;
-    Q[1] = (p_m + tm) / Z1s + R(1) / (al + eta_s) * phi_m;
-    Q[2] = (p_l + tl) / Z1s + R(1) / (al + eta_s) * phi_l;
+    P[0] = (q_n - phi_n) * i2p; Q[0] = (p_n + phi_n) * i1p;
+    Q[1] = (p_m + tm) * i1s + R(1) / (al + eta_s) * phi_m;
+    Q[2] = (p_l + tl) * i1s + R(1) / (al + eta_s) * phi_l;
     P[1] = R(0);
-    P[2] = (q_l - tl) / Z2s - R(1) / (al + eta_s) * phi_l;
+    P[2] = (q_l - tl) * i2s - R(1) / (al + eta_s) * phi_l;
     P[3] = Q[3] = phi_n; P[4] = Q[4] = tm; P[5] = Q[5] = tl;
   } else {
     // prestress: static part + nucleation weight x the stage's uniform ramp
@@ -320,15 +319,15 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
       }
     }
     const R tmh = (R)tau_m_hat, tlh = (R)tau_l_hat, vm = (R)vv_m, vl = (R)vv_l;
-    P[0] = (q_n - phi_n) / Z2p;
-    Q[0] = (p_n + phi_n) / Z1p;
+    P[0] = (q_n - phi_n) * i2p;
+    Q[0] = (p_n + phi_n) * i1p;
     P[3] = Q[3] = phi_n;
     P[4] = Q[4] = tmh;
     P[5] = Q[5] = tlh;
-    Q[1] = (tmh + p_m) / Z1s + vm;
-    Q[2] = (tlh + p_l) / Z1s + vl;
-    P[1] = (q_m - tmh) / Z2s - vm;
-    P[2] = (q_l - tlh) / Z2s - vl;
+    Q[1] = (tmh + p_m) * i1s + vm;
+    Q[2] = (tlh + p_l) * i1s + vl;
+    P[1] = (q_m - tmh) * i2s - vm;
+    P[2] = (q_l - tlh) * i2s - vl;
   }
   const R srate = sqrt((Q[1] - P[1]) * (Q[1] - P[1]) + (Q[2] - P[2]) * (Q[2] - P[2]));
 
@@ -385,8 +384,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
   back(vr, vg);
 
   // SAT vector for this copy's block (src/CouplingForcing.f90:238-466)
-  const R norm = sqrt(gx * gx + gy * gy + gz * gz);
-  const R Zp = b == 0 ? Z1p : Z2p, Zs = b == 0 ? Z1s : Z2s;
+  const R norm = face[15 * nf + f];
+  const R Zp = b == 0 ? Z1p : Z2p, Zs = b == 0 ? Z1s : Z2s, iZp = b == 0 ? i1p : i2p, iZs = b == 0 ? i1s : i2s;
   R Mm[3][3], Pm[3][3];
   const R* e[3] = {n, m, l};
 #pragma unroll
@@ -395,7 +394,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
     for (int c = 0; c < 3; ++c) {
       // M = sum_k e_r[k] e_c[k] Z_k with Z = (Zp, Zs, Zs) by component index
       Mm[r][c] = e[r][0] * e[c][0] * Zp + e[r][1] * e[c][1] * Zs + e[r][2] * e[c][2] * Zs;
-      Pm[r][c] = e[r][0] * e[c][0] * R(1) / Zp + e[r][1] * e[c][1] * R(1) / Zs + e[r][2] * e[c][2] * R(1) / Zs;
+      Pm[r][c] = e[r][0] * e[c][0] * iZp + e[r][1] * e[c][1] * iZs + e[r][2] * e[c][2] * iZs;
     }
   R dch[3];
   if (b == 0) {
@@ -416,13 +415,13 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
   R rr[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) rr[r] = Pm[r][0] * dch[0] + Pm[r][1] * dch[1] + Pm[r][2] * dch[2];
-  const R lam = b == 0 ? lam1 : lam2, mu = b == 0 ? mu1 : mu2, rho = b == 0 ? rho1 : rho2;
+  const R lam = face[12 * nf + f], mu = face[13 * nf + f], irho = face[20 * nf + f];
   const R sgn = b == 0 ? R(1) : R(-1);
   const R l2m = R(2) * mu + lam;
   R sat[9];
-  sat[0] = norm / rho * dch[0];
-  sat[1] = norm / rho * dch[1];
-  sat[2] = norm / rho * dch[2];
+  sat[0] = norm * irho * dch[0];
+  sat[1] = norm * irho * dch[1];
+  sat[2] = norm * irho * dch[2];
   sat[3] = sgn * (l2m * gx * rr[0] + lam * gy * rr[1] + lam * gz * rr[2]);
   sat[4] = sgn * (l2m * gy * rr[1] + lam * gz * rr[2] + lam * gx * rr[0]);
   sat[5] = sgn * (l2m * gz * rr[2] + lam * gy * rr[1] + lam * gx * rr[0]);

@@ -11,8 +11,10 @@
 //           mode only; see comp_t)
 //   coef  : curvilinear: 13 x np = J*metric (3 directions x 3 components),
 //           1/J, lambda, mu, 1/(rho*J); Cartesian: 3 x np = lambda, mu, 1/rho
-//   face  : per side 15 x nface (FP64): n(3), m(3), l(3), grad(3) of the
-//           face-normal coordinate, lambda, mu, rho
+//   face  : per side 21 x nface, in the field type (the fault sides in FP64
+//           too): n(3), m(3), l(3), grad(3) of the face-normal coordinate,
+//           lambda, mu, rho, |grad|, the impedances Zp and Zs, 1/Zp, 1/Zs,
+//           1/rho (square roots and quotients taken once, at set-up)
 //   Q/DQ  : PML auxiliary fields on slabs of npml layers per active side
 //   G     : 9 x np velocity gradient hand-off (FP32C with attenuation)
 //   eta/Deta, qs : 24 x np memory variables and their rates, 1/Qs per point
@@ -40,7 +42,7 @@ namespace wql {
 // FP32 term (232 instead of 268).
 typedef unsigned short comp_t;
 
-constexpr int kFaceWords = 15;
+constexpr int kFaceWords = 21;
 constexpr int kCurvCoef = 13;
 constexpr int kCartCoef = 3;
 
@@ -81,7 +83,7 @@ struct VolumeArgs {
   const T* __restrict__ coef;
   T cart_metric[3];   // q_x, r_y, s_z for Cartesian blocks
   // outer faces (side 0..5 = -q,+q,-r,+r,-s,+s)
-  const double* face[6];
+  const T* face[6];
   int bc[6];          // 1 absorbing, 2 free surface, 3 clamped, else none
   int bc_form;
   T tau_h[3];         // tau0 / h per axis
@@ -152,8 +154,8 @@ struct InterfaceArgs {
   int fp64;                 // fields are double (1) or float (0)
   const void* F0;           // block 0 fields (9 x np0)
   const void* F1;           // block 1 fields (9 x np1)
-  const double* face0;      // block 0, side +q (15 x nf)
-  const double* face1;      // block 1, side -q (15 x nf)
+  const void* face0;        // block 0, side +q (kFaceWords x nf, in the algebra's type)
+  const void* face1;        // block 1, side -q
   const double* xij;        // 2 x 3 x nf fault-point coordinates per block copy
   double* S;                // 2 x 4 x nf
   double* DS;               // 2 x 4 x nf
@@ -296,6 +298,8 @@ void launch_anelastic_material(long long n, double c, const double den[4], const
                                double* mu, const double* rho, double* qsinv, void* stream);
 void launch_faces(int nq, int nr, int ns, const double* metric, const double* lam,
                   const double* mu, const double* rho, double* const face[6], void* stream);
+// FP64 face data rounded to FP32.
+void launch_face_f32(long long n, const double* in, float* out, void* stream);
 template <typename T>
 void launch_coef(int nq, int nr, int ns, int pq, bool curv, const double* metric, const double* J,
                  const double* lam, const double* mu, const double* rho, T* coef, void* stream);

@@ -123,7 +123,19 @@ __global__ void faces_kernel(int nq, int nr, int ns, const double* __restrict__ 
   o[11 * nf + f] = gz;
   o[12 * nf + f] = lam[p];
   o[13 * nf + f] = mu[p];
-  o[14 * nf + f] = rho[p];
+  const double r = rho[p], zp = r * sqrt((2.0 * mu[p] + lam[p]) / r), zs = r * sqrt(mu[p] / r);
+  o[14 * nf + f] = r;
+  o[15 * nf + f] = norm;
+  o[16 * nf + f] = zp;
+  o[17 * nf + f] = zs;
+  o[18 * nf + f] = 1.0 / zp;
+  o[19 * nf + f] = 1.0 / zs;
+  o[20 * nf + f] = 1.0 / r;
+}
+
+__global__ void face_f32_kernel(long long n, const double* __restrict__ in, float* __restrict__ out) {
+  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (p < n) out[p] = (float)in[p];
 }
 
 template <typename T>
@@ -166,6 +178,10 @@ void launch_faces(int nq, int nr, int ns, const double* metric, const double* la
   const int my = nr > ns ? nr : ns;
   dim3 blk(32, 4, 1), grd((mx + 31) / 32, (my + 3) / 4, 6);
   faces_kernel<<<grd, blk, 0, (cudaStream_t)stream>>>(nq, nr, ns, metric, lam, mu, rho, fp);
+}
+
+void launch_face_f32(long long n, const double* in, float* out, void* stream) {
+  face_f32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(n, in, out);
 }
 
 template <typename T>

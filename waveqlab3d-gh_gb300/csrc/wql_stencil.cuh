@@ -151,20 +151,18 @@ __device__ __forceinline__ TileSpan tile_span(int t, int n, int T_) {
 // alpha/theta form of src/BoundaryConditions3.f90:777-903 added directly.
 // Returns sat (added to DF with -tau/h) and ubc (added to DQ in a PML).
 template <typename R>
-__device__ void boundary_sat(const R u[9], const double* __restrict__ face, long long nf, long long f, int code,
+__device__ void boundary_sat(const R u[9], const R* __restrict__ face, long long nf, long long f, int code,
                              bool plus, int form, R sat[9], R ubc[9]) {
   R n[3], m[3], l[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    n[c] = (R)face[(0 + c) * nf + f];
-    m[c] = (R)face[(3 + c) * nf + f];
-    l[c] = (R)face[(6 + c) * nf + f];
+    n[c] = face[(0 + c) * nf + f];
+    m[c] = face[(3 + c) * nf + f];
+    l[c] = face[(6 + c) * nf + f];
   }
-  const R gx = (R)face[9 * nf + f], gy = (R)face[10 * nf + f], gz = (R)face[11 * nf + f];
-  const R lam = (R)face[12 * nf + f], mu = (R)face[13 * nf + f], rho = (R)face[14 * nf + f];
-  const R norm = sqrt(gx * gx + gy * gy + gz * gz);
-  const R cp = sqrt((R(2.0) * mu + lam) / rho), cs = sqrt(mu / rho);
-  const R Zp = rho * cp, Zs = rho * cs;
+  const R lam = face[12 * nf + f], mu = face[13 * nf + f];
+  const R norm = face[15 * nf + f], Zp = face[16 * nf + f], Zs = face[17 * nf + f];
+  const R iZp = face[18 * nf + f], iZs = face[19 * nf + f], irho = face[20 * nf + f];
   R r, alpha, theta;
   if (code == 1) { r = R(0.0); alpha = R(2.0); theta = R(0.0); }
   else if (code == 2) { r = R(1.0); alpha = R(1.0); theta = R(0.0); }
@@ -182,9 +180,9 @@ __device__ void boundary_sat(const R u[9], const double* __restrict__ face, long
   const R pl = R(0.5) * ((R(1.0) - r) * Zs * vl + sg * (R(1.0) + r) * Tl);
   const R pm = R(0.5) * ((R(1.0) - r) * Zs * vm + sg * (R(1.0) + r) * Tm);
   const R pn = R(0.5) * ((R(1.0) - r) * Zp * vn + sg * (R(1.0) + r) * Tn);
-  const R ql = R(0.5) * ((R(1.0) - r) * vl + sg * (R(1.0) + r) / Zs * Tl);
-  const R qm = R(0.5) * ((R(1.0) - r) * vm + sg * (R(1.0) + r) / Zs * Tm);
-  const R qn = R(0.5) * ((R(1.0) - r) * vn + sg * (R(1.0) + r) / Zp * Tn);
+  const R ql = R(0.5) * ((R(1.0) - r) * vl + sg * (R(1.0) + r) * iZs * Tl);
+  const R qm = R(0.5) * ((R(1.0) - r) * vm + sg * (R(1.0) + r) * iZs * Tm);
+  const R qn = R(0.5) * ((R(1.0) - r) * vn + sg * (R(1.0) + r) * iZp * Tn);
   const R Fx = l[0] * pl + m[0] * pm + n[0] * pn;
   const R Fy = l[1] * pl + m[1] * pm + n[1] * pn;
   const R Fz = l[2] * pl + m[2] * pm + n[2] * pn;
@@ -193,9 +191,9 @@ __device__ void boundary_sat(const R u[9], const double* __restrict__ face, long
   const R F_z = l[2] * ql + m[2] * qm + n[2] * qn;
   if (form == BC_WEIGHTED) {
     const R l2m = lam + R(2.0) * mu;
-    ubc[0] = alpha * norm / rho * Fx;
-    ubc[1] = alpha * norm / rho * Fy;
-    ubc[2] = alpha * norm / rho * Fz;
+    ubc[0] = alpha * norm * irho * Fx;
+    ubc[1] = alpha * norm * irho * Fy;
+    ubc[2] = alpha * norm * irho * Fz;
     ubc[3] = theta * norm * (l2m * n[0] * F_x + lam * (n[1] * F_y + n[2] * F_z));
     ubc[4] = theta * norm * (l2m * n[1] * F_y + lam * (n[0] * F_x + n[2] * F_z));
     ubc[5] = theta * norm * (l2m * n[2] * F_z + lam * (n[0] * F_x + n[1] * F_y));
@@ -215,9 +213,9 @@ __device__ void boundary_sat(const R u[9], const double* __restrict__ face, long
   ubc[6] = sg * (norm * (n[1] * F_x + n[0] * F_y));
   ubc[7] = sg * (norm * (n[2] * F_x + n[0] * F_z));
   ubc[8] = sg * (norm * (n[2] * F_y + n[1] * F_z));
-  sat[0] = R(1.0) / rho * ubc[0];
-  sat[1] = R(1.0) / rho * ubc[1];
-  sat[2] = R(1.0) / rho * ubc[2];
+  sat[0] = irho * ubc[0];
+  sat[1] = irho * ubc[1];
+  sat[2] = irho * ubc[2];
   sat[3] = (R(2.0) * mu + lam) * ubc[3] + lam * (ubc[4] + ubc[5]);
   sat[4] = (R(2.0) * mu + lam) * ubc[4] + lam * (ubc[3] + ubc[5]);
   sat[5] = (R(2.0) * mu + lam) * ubc[5] + lam * (ubc[3] + ubc[4]);

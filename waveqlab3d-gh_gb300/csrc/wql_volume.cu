@@ -1123,11 +1123,11 @@ __device__ __forceinline__ void face_pre_point(const VolumeArgs<T>& a, long long
     const T th = a.tau_h[s2 >> 1];
     T* DQ = a.DQ[s2];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) DQ[c * snp + sp] = keep ? DQ[c * snp + sp] - th * ubc[c] / a.A : -th * ubc[c];
+    for (int c = 0; c < 9; ++c) DQ[c * snp + sp] = keep ? DQ[c * snp + sp] - th * ubc[c] * a.Ainv : -th * ubc[c];
   });
   // a face point without a penalised side still defines DF when A = 0
 #pragma unroll
-  for (int c = 0; c < 9; ++c) a.DF[c * np + p] = keep ? df[c] - tot[c] / a.A : -tot[c];
+  for (int c = 0; c < 9; ++c) a.DF[c * np + p] = df[c] - tot[c] * a.Ainv;
 }
 
 // One launch covers one block or both of a scenario: threads [0, n0) take
