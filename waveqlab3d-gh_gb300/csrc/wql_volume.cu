@@ -610,6 +610,13 @@ PmlTiles pml_tiles(const VolumeArgs<T>& a) {
         P.lw[b] = narrow ? 3 : 5;
         P.lr[b] = narrow ? 3 : 2;
         const int ls = 8 - P.lw[b] - P.lr[b];
+        if (sizeof(T) == 8) {  // the FP64 unit is the bound: no idle lanes, 256 consecutive points
+          const long long pts = (long long)P.dim[b][0] * P.dim[b][1] * P.dim[b][2];
+          P.tq[b] = P.tr[b] = 1;
+          P.start[b + 1] = P.start[b] + (int)((pts + 255) / 256);
+          ++P.n;
+          continue;
+        }
         P.tq[b] = (P.dim[b][0] + (1 << P.lw[b]) - 1) >> P.lw[b];
         P.tr[b] = (P.dim[b][1] + (1 << P.lr[b]) - 1) >> P.lr[b];
         const int ts = (P.dim[b][2] + (1 << ls) - 1) >> ls;
@@ -743,10 +750,10 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int
     src[6] = axis == 0 ? gv[1] : (axis == 1 ? gv[0] : T(0));
     src[7] = axis == 0 ? gv[2] : (axis == 2 ? gv[0] : T(0));
     src[8] = axis == 1 ? gv[2] : (axis == 2 ? gv[1] : T(0));
-    const T dc = damp + cfs;
+    const T dc = damp + cfs, Ak = keep ? a.A : T(1);
 #pragma unroll
     for (int c = 0; c < 9; ++c) {
-      const T nw = (keep ? a.A * dq[c] : dq[c]) + src[c] - dc * qv[c];
+      const T nw = Ak * dq[c] + (src[c] - dc * qv[c]);
       DQ[c * snp] = nw;
       Q[c * snp] = qv[c] + a.Bdt * nw;
     }
@@ -778,9 +785,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) pml_pre_kernel(co
   const int l = t - B.start[b], lw = B.lw[b], lr = B.lr[b];
   const int bq = l % B.tq[b], br = (l / B.tq[b]) % B.tr[b], bs = l / (B.tq[b] * B.tr[b]);
   const int e = threadIdx.x;
-  const int i = (bq << lw) + (e & ((1 << lw) - 1));
-  const int j = (br << lr) + ((e >> lw) & ((1 << lr) - 1));
-  const int k = (bs << (8 - lw - lr)) + (e >> (lw + lr));
+  int i = (bq << lw) + (e & ((1 << lw) - 1));
+  int j = (br << lr) + ((e >> lw) & ((1 << lr) - 1));
+  int k = (bs << (8 - lw - lr)) + (e >> (lw + lr));
+  if (sizeof(T) == 8) {
+    const int x = l * 256 + e;
+    i = x % B.dim[b][0];
+    j = x / B.dim[b][0] % B.dim[b][1];
+    k = x / (B.dim[b][0] * B.dim[b][1]);
+  }
   if (i >= B.dim[b][0] || j >= B.dim[b][1] || k >= B.dim[b][2]) return;
   pml_pre_point<T, O, CURV, FD>(P.a[blk], B.lo[b][0] + i, B.lo[b][1] + j, B.lo[b][2] + k, (unsigned)B.sides[b], tab);
 }
