@@ -559,10 +559,9 @@ __device__ __forceinline__ long long slab_point(const VolumeArgs<T>& a, int side
 // the sides a point lies in are the same for a whole CTA: the axis of a side
 // and the arrays of its fluxes are uniform, and every load of a neighbour is
 // a uniform base plus one 32-bit offset that all of the neighbour's
-// quantities share.  A CTA takes a tile of 256 points of one region, 32 x 4 x
-// 2 (q, r, s) points, or 8 x 8 x 4 in the regions of the q slabs, whose rows
-// are only npml points long: neighbouring rows share their stencil reads in
-// L1.  Each direction's neighbours are visited once for both the flux and the
+// quantities share.  A CTA takes a tile of 256 points of one region, 4 to 32
+// points along q and 2 to 8 along r and s, whichever pads the region least:
+// neighbouring rows share their stencil reads in L1.  Each direction's neighbours are visited once for both the flux and the
 // velocity derivative; a closure row's columns are unrolled like the interior
 // row's, so their loads are in flight together (as a loop, their latencies
 // added up).
@@ -606,10 +605,6 @@ PmlTiles pml_tiles(const VolumeArgs<T>& a) {
           P.dim[b][d] = cut[d][c[d] + 1] - cut[d][c[d]];
         }
         P.sides[b] = sides;
-        const bool narrow = P.dim[b][0] <= 24;
-        P.lw[b] = narrow ? 3 : 5;
-        P.lr[b] = narrow ? 3 : 2;
-        const int ls = 8 - P.lw[b] - P.lr[b];
         if (sizeof(T) == 8) {  // the FP64 unit is the bound: no idle lanes, 256 consecutive points
           const long long pts = (long long)P.dim[b][0] * P.dim[b][1] * P.dim[b][2];
           P.tq[b] = P.tr[b] = 1;
@@ -617,6 +612,23 @@ PmlTiles pml_tiles(const VolumeArgs<T>& a) {
           ++P.n;
           continue;
         }
+        // the tile of 256 points that pads the region least; rows of 4 points
+        // half use their 32-byte sectors
+        float least = 1e30f;
+        int ls = 0;
+        for (int w2 = 5; w2 >= 2; --w2)
+          for (int r2 = 3; r2 >= 1; --r2) {
+            const int s2 = 8 - w2 - r2;
+            if (s2 < 1 || s2 > 3) continue;
+            auto up = [](int n, int l) { return (float)(((n + (1 << l) - 1) >> l) << l); };
+            const float v = up(P.dim[b][0], w2) * up(P.dim[b][1], r2) * up(P.dim[b][2], s2) * (w2 == 2 ? 1.1f : 1.0f);
+            if (v < 0.999f * least) {
+              least = v;
+              P.lw[b] = w2;
+              P.lr[b] = r2;
+              ls = s2;
+            }
+          }
         P.tq[b] = (P.dim[b][0] + (1 << P.lw[b]) - 1) >> P.lw[b];
         P.tr[b] = (P.dim[b][1] + (1 << P.lr[b]) - 1) >> P.lr[b];
         const int ts = (P.dim[b][2] + (1 << ls) - 1) >> ls;
