@@ -699,6 +699,7 @@ int setup_block(wql_scn* S, int b) {
   S->release(metric);
   S->release(J);
   S->release(mat);
+  CK(cudaStreamSynchronize(S->stream));  // the pool gives unused memory back at a synchronisation
   return WQL_OK;
 }
 

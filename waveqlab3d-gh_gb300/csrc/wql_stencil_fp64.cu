@@ -41,6 +41,7 @@ namespace {
 // 75x81x77 Cartesian, the same on curvilinear 67/59x71x73; three of 128 the
 // same as two).
 constexpr int kF64Threads = 192;
+constexpr size_t kF64Smem = 110 * 1024;  // most shared memory of a CTA
 
 struct F64Pair {
   VolumeArgs<double> a[2];
@@ -350,7 +351,7 @@ StencilPlan64 make_plan64(int nq, int nr, int ns, int sms) {
       }
     }
   }
-  if (best.ok && smem_of(best) > 110 * 1024) best.ok = 0;
+  if (best.ok && smem_of(best) > kF64Smem) best.ok = 0;
   return best;
 }
 
@@ -370,7 +371,8 @@ void launch_stencil_fp64(const VolumeArgs<double>& a0, const VolumeArgs<double>*
   P.n0 = n[0];
   if (!a1) n[1] = 0;
   auto kern = curv ? stencil_kernel_fp64<true> : stencil_kernel_fp64<false>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the same limit for every launch: threads stepping other scenarios set it too
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF64Smem);
   kern<<<n[0] + n[1], nt, smem, (cudaStream_t)stream>>>(P);
 }
 

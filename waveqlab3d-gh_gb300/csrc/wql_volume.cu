@@ -1458,7 +1458,7 @@ int launch_volume2(const VolumeArgs<T>& a0, const VolumeArgs<T>& a1, bool curv, 
   cudaStream_t s = (cudaStream_t)stream;
   const bool kahan = a0.C != nullptr;
   if (v == 1) {
-    if (a0.nr != a1.nr) return 0;
+    if (a0.nr != a1.nr || a0.ns + a1.ns > 65535) return 0;  // one grid over both blocks' planes
     if (curv) kahan ? launch_pointwise<T, true, true>(a0, &a1, s) : launch_pointwise<T, true, false>(a0, &a1, s);
     else kahan ? launch_pointwise<T, false, true>(a0, &a1, s) : launch_pointwise<T, false, false>(a0, &a1, s);
     return 1;
