@@ -1007,7 +1007,9 @@ __global__ void __launch_bounds__(384, 4) anelastic_comp_kernel(const __grid_con
   const int c = threadIdx.x >> 6;  // stress component 3 + c
   const long long np = a.np;
   if (p >= np) return;
-  const int i = (int)(p % a.pq), jk = (int)(p / a.pq), j = jk % a.nr, k = jk / a.nr;
+  // 32-bit divisions (a block has fewer than 2^32 points)
+  const unsigned pu = (unsigned)p, jk = pu / (unsigned)a.pq;
+  const int i = (int)(pu - jk * (unsigned)a.pq), k = (int)(jk / (unsigned)a.nr), j = (int)(jk - (unsigned)k * (unsigned)a.nr);
   if (i >= a.nq) return;
   const T* __restrict__ coef = a.coef + p;
   const T* __restrict__ G = a.G + p;
@@ -1125,7 +1127,7 @@ __device__ __forceinline__ void face_pre_point(const VolumeArgs<T>& a, long long
   if (side >= 6) return;
   const int axis = side >> 1;
   const int w = axis == 0 ? nr : nq;
-  const int c1 = (int)(t % w), c2 = (int)(t / w);
+  const int c2 = (int)((unsigned)t / (unsigned)w), c1 = (int)((unsigned)t - (unsigned)c2 * (unsigned)w);
   int i, j, k;
   if (axis == 0) { i = (side & 1) ? nq - 1 : 0; j = c1; k = c2; }
   else if (axis == 1) { i = c1; j = (side & 1) ? nr - 1 : 0; k = c2; }
