@@ -141,6 +141,14 @@ __device__ __forceinline__ void load_face(const void* F, const void* C, long lon
   for (int c = 0; c < 9; ++c) out[c] = k ? (R)f[c * np + p] - (R)comp_get(k, c * np + p) : (R)f[c * np + p];
 }
 
+// x / Z with iZ = 1/Z at hand: FP32 takes the quotient (see the impedances in
+// the kernel), FP64 multiplies (a quotient holds its unit some twenty times
+// longer).
+template <typename R>
+__device__ __forceinline__ R over(R x, R Z, R iZ) {
+  return sizeof(R) == 4 ? x / Z : x * iZ;
+}
+
 // T is the field type, R the arithmetic type of the characteristic algebra.
 // FP64 fields (R = T = double) keep every operation of the FP64 restatement.
 // FP32 fields either do the algebra in FP32 (R = float) or read the
@@ -156,7 +164,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
   const long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (f >= nf) return;
-  const int j = (int)(f % a.nr), k = (int)(f / a.nr);
+  const int k = (int)((unsigned)f / (unsigned)a.nr), j = (int)((unsigned)f - (unsigned)k * (unsigned)a.nr);
   // fields on both faces: block 0 at q = nq0-1, block 1 at q = 0
   R u[9], v[9];
   const long long pu = (a.nq0 - 1) + (long long)a.pq0 * (j + (long long)a.nr * k);
@@ -189,12 +197,51 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
     l[c] = face[(6 + c) * nf + f];
   }
   const R gx = face[9 * nf + f], gy = face[10 * nf + f], gz = face[11 * nf + f];
-  // impedances of each side (block 0 / block 1 face) and their reciprocals
-  const R Z1p = face0[16 * nf + f], Z1s = face0[17 * nf + f], Z2p = face1[16 * nf + f], Z2s = face1[17 * nf + f];
-  const R i1p = face0[18 * nf + f], i1s = face0[19 * nf + f], i2p = face1[18 * nf + f], i2s = face1[19 * nf + f];
+  // impedances of each side (block 0 / block 1 face) and their reciprocals.
+  // FP32 forms them from its own moduli and takes quotients below: the slip
+  // rate is a small difference of terms that agree only as far as x / Z, Z and
+  // eta come from the same numbers (with impedances and reciprocals rounded
+  // one by one from FP64 the slip of a rupture was off by 3.3e-7 instead of
+  // 4.8e-8 after 200 steps)
+  R Z1p, Z1s, Z2p, Z2s, i1p, i1s, i2p, i2s;
+  if (sizeof(R) == 4) {
+    const R lam1 = face0[12 * nf + f], mu1 = face0[13 * nf + f], rho1 = face0[14 * nf + f];
+    const R lam2 = face1[12 * nf + f], mu2 = face1[13 * nf + f], rho2 = face1[14 * nf + f];
+    Z1p = rho1 * sqrt((R(2) * mu1 + lam1) / rho1);
+    Z1s = rho1 * sqrt(mu1 / rho1);
+    Z2p = rho2 * sqrt((R(2) * mu2 + lam2) / rho2);
+    Z2s = rho2 * sqrt(mu2 / rho2);
+    i1p = R(1) / Z1p;
+    i1s = R(1) / Z1s;
+    i2p = R(1) / Z2p;
+    i2s = R(1) / Z2s;
+  } else {
+    Z1p = face0[16 * nf + f], Z1s = face0[17 * nf + f], Z2p = face1[16 * nf + f], Z2s = face1[17 * nf + f];
+    i1p = face0[18 * nf + f], i1s = face0[19 * nf + f], i2p = face1[18 * nf + f], i2s = face1[19 * nf + f];
+  }
   double x[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) x[c] = a.xij[(b * 3 + c) * nf + f];
+
+  double* S = a.S + (long long)b * 4 * nf;
+  double* DS = a.DS + (long long)b * 4 * nf;
+  double* W = a.W + (long long)b * nf;
+  double* DW = a.DW + (long long)b * nf;
+  double* trup = a.trup + (long long)b * nf;
+  const int cpl = a.fp.coupling;
+  // the slip, its rates and the prestress, read with the fields: one after
+  // another at their uses, their latencies were a fifth of a small fault's
+  // launch
+  double s0[4], ds0[4], pr[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    s0[c] = S[c * nf + f];
+    ds0[c] = DS[c * nf + f];
+  }
+  if (cpl == CPL_SW || cpl == CPL_RS) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) pr[c] = a.pre[((long long)b * 5 + c) * nf + f];
+  }
 
   // tractions on the face, then rotate velocities and tractions to (n,m,l)
   R ur[6], vr[6];
@@ -224,41 +271,33 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
   const R q_n = Z2p * vr[0] + vr[3], q_m = Z2s * vr[1] + vr[4], q_l = Z2s * vr[2] + vr[5];
   const R eta_s = R(1) / (i1s + i2s);
   const R eta_p = R(1) / (i1p + i2p);
-  const R phi_n = eta_p * (q_n * i2p - p_n * i1p);
-  const R phi_m = eta_s * (q_m * i2s - p_m * i1s);
-  const R phi_l = eta_s * (q_l * i2s - p_l * i1s);
-
-  double* S = a.S + (long long)b * 4 * nf;
-  double* DS = a.DS + (long long)b * 4 * nf;
-  double* W = a.W + (long long)b * nf;
-  double* DW = a.DW + (long long)b * nf;
-  double* trup = a.trup + (long long)b * nf;
+  const R phi_n = eta_p * (over(q_n, Z2p, i2p) - over(p_n, Z1p, i1p));
+  const R phi_m = eta_s * (over(q_m, Z2s, i2s) - over(p_m, Z1s, i1s));
+  const R phi_l = eta_s * (over(q_l, Z2s, i2s) - over(p_l, Z1s, i1s));
 
   R P[6], Q[6];
   double T0n = 0.0, T0m = 0.0, T0l = 0.0;
-  const int cpl = a.fp.coupling;
   if (cpl == CPL_LOCKED) {
     // Welded_Interface (src/Interface_Condition.f90:516-637)
-    P[0] = (q_n - phi_n) * i2p; P[1] = (q_m - phi_m) * i2s; P[2] = (q_l - phi_l) * i2s;
-    Q[0] = (p_n + phi_n) * i1p; Q[1] = (p_m + phi_m) * i1s; Q[2] = (p_l + phi_l) * i1s;
+    P[0] = over(q_n - phi_n, Z2p, i2p); P[1] = over(q_m - phi_m, Z2s, i2s); P[2] = over(q_l - phi_l, Z2s, i2s);
+    Q[0] = over(p_n + phi_n, Z1p, i1p); Q[1] = over(p_m + phi_m, Z1s, i1s); Q[2] = over(p_l + phi_l, Z1s, i1s);
     P[3] = Q[3] = phi_n; P[4] = Q[4] = phi_m; P[5] = Q[5] = phi_l;
   } else if (cpl == CPL_LINEAR) {
     // Linear_Friction with alpha = 1e14 (src/Interface_Condition.f90:639-742)
     const R al = R(1.0e14);
     const R tm = al / (al + eta_s) * phi_m, tl = al / (al + eta_s) * phi_l;
-    P[0] = (q_n - phi_n) * i2p; Q[0] = (p_n + phi_n) * i1p;
-    Q[1] = (p_m + tm) * i1s + R(1) / (al + eta_s) * phi_m;
-    Q[2] = (p_l + tl) * i1s + R(1) / (al + eta_s) * phi_l;
+    P[0] = over(q_n - phi_n, Z2p, i2p); Q[0] = over(p_n + phi_n, Z1p, i1p);
+    Q[1] = over(p_m + tm, Z1s, i1s) + R(1) / (al + eta_s) * phi_m;
+    Q[2] = over(p_l + tl, Z1s, i1s) + R(1) / (al + eta_s) * phi_l;
     P[1] = R(0);
-    P[2] = (q_l - tl) * i2s - R(1) / (al + eta_s) * phi_l;
+    P[2] = over(q_l - tl, Z2s, i2s) - R(1) / (al + eta_s) * phi_l;
     P[3] = Q[3] = phi_n; P[4] = Q[4] = tm; P[5] = Q[5] = tl;
   } else {
     // prestress: static part + nucleation weight x the stage's uniform ramp
-    const double* pre = a.pre + (long long)b * 5 * nf;
-    T0n = pre[f];
-    T0m = pre[nf + f];
-    T0l = pre[2 * nf + f];
-    const double wn = pre[3 * nf + f];
+    T0n = pr[0];
+    T0m = pr[1];
+    T0l = pr[2];
+    const double wn = pr[3];
     if (wn != 0.0) T0l = T0l + wn * a.ramp;
     // the friction law in FP64 for both field types
     const double phm = phi_m, phl = phi_l, phn = phi_n, es = eta_s;
@@ -268,7 +307,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
       // Slip_Weakening_Friction + solve (src/Interface_Condition.f90:745-916, 1147-1166)
       const double tau_lock = sqrt((T0l + phl) * (T0l + phl) + (T0m + phm) * (T0m + phm));
       const double sn = fmax(0.0, -(T0n + phn));
-      const double tau_str = tau_strength(a.fp, sn, S[3 * nf + f], x, a.t);
+      const double tau_str = tau_strength(a.fp, sn, s0[3], x, a.t);
       if (tau_lock > tau_str) {
         const double Phi = sqrt(phi_1 * phi_1 + phi_2 * phi_2);
         const double V = (Phi - tau_str) / es;
@@ -283,7 +322,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
       }
     } else {
       // rate_state_friction + solve + Regula_Falsi (src/Interface_Condition.f90:918-1146)
-      const double ra = pre[4 * nf + f];  // direct-effect parameter a(x)
+      const double ra = a.pre[((long long)b * 5 + 4) * nf + f];  // direct-effect parameter a(x)
       const RSParams rs = rs_params(a.fp, x, ra);
       const double psi = W[f];
       const double sn = fmax(0.0, -(T0n + phn));
@@ -319,15 +358,15 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
       }
     }
     const R tmh = (R)tau_m_hat, tlh = (R)tau_l_hat, vm = (R)vv_m, vl = (R)vv_l;
-    P[0] = (q_n - phi_n) * i2p;
-    Q[0] = (p_n + phi_n) * i1p;
+    P[0] = over(q_n - phi_n, Z2p, i2p);
+    Q[0] = over(p_n + phi_n, Z1p, i1p);
     P[3] = Q[3] = phi_n;
     P[4] = Q[4] = tmh;
     P[5] = Q[5] = tlh;
-    Q[1] = (tmh + p_m) * i1s + vm;
-    Q[2] = (tlh + p_l) * i1s + vl;
-    P[1] = (q_m - tmh) * i2s - vm;
-    P[2] = (q_l - tlh) * i2s - vl;
+    Q[1] = over(tmh + p_m, Z1s, i1s) + vm;
+    Q[2] = over(tlh + p_l, Z1s, i1s) + vl;
+    P[1] = over(q_m - tmh, Z2s, i2s) - vm;
+    P[2] = over(q_l - tlh, Z2s, i2s) - vl;
   }
   const R srate = sqrt((Q[1] - P[1]) * (Q[1] - P[1]) + (Q[2] - P[2]) * (Q[2] - P[2]));
 
@@ -343,7 +382,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
         fr[(FR_VFACE + c) * nf + f] = (float)((const T*)a.F1)[c * a.np1 + pv];
       }
 #pragma unroll
-      for (int c = 0; c < 4; ++c) fr[(FR_S + c) * nf + f] = (float)S[c * nf + f];
+      for (int c = 0; c < 4; ++c) fr[(FR_S + c) * nf + f] = (float)s0[c];
       const double T0[3] = {T0n, T0m, T0l};
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -361,10 +400,11 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? 5 : 3) interface_kernel(
 
   // slip and state: DS <- A*DS + rates, then the RK update of S and W
 #pragma unroll
-  for (int c = 0; c < 3; ++c) DS[c * nf + f] = a.A * DS[c * nf + f] + (double)(Q[c] - P[c]);
-  DS[3 * nf + f] = a.A * DS[3 * nf + f] + (double)srate;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) S[c * nf + f] += a.Bdt * DS[c * nf + f];
+  for (int c = 0; c < 4; ++c) {
+    const double ds = a.A * ds0[c] + (c < 3 ? (double)(Q[c] - P[c]) : (double)srate);
+    DS[c * nf + f] = ds;
+    S[c * nf + f] = s0[c] + a.Bdt * ds;
+  }
   if (cpl == CPL_RS) W[f] += a.Bdt * DW[f];
 
   // hat variables back to (x,y,z); grid values rotate back to themselves
