@@ -1,0 +1,59 @@
+"""Combinations of options that the other GPU tests do not reach, each against
+the oracle, FP64 or the same run without the option."""
+import numpy as np
+import pytest
+
+from gpu_helpers import rel_l2
+from test_gpu_kernel_edges import deck, start
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def wqlmod():
+    import wql
+    return wql
+
+
+@pytest.fixture(scope="module")
+def ctx(wqlmod):
+    c = wqlmod.Context(0)
+    yield c
+    c.close()
+
+
+def fill(sim, dims):
+    for b in range(2):
+        f = start((dims[3], dims[2], dims[b]), 10 + b)
+        for c in range(9):
+            sim.set_field(b, c, f[c])
+
+
+ANELASTIC = "&anelastic_list\n c = 2.0,\n weight_exp = 0.6,\n fref = 1.0 /\n"
+
+
+# (mesh, operator, (nq1, nq2, nr, ns), npml): row remainders, s slabs that overlap or meet, per-point and TMA gradients
+@pytest.mark.parametrize("mesh,op,dims,npml", [
+    ("cartesian", "traditional", (27, 22, 29, 18), 10),
+    ("curvilinear", "traditional", (33, 25, 20, 22), 12),
+    ("cartesian", "upwind 6", (41, 34, 25, 21), 14),
+    ("curvilinear", "upwind 6", (30, 31, 24, 28), 17),
+    ("cartesian", "upwind 4", (26, 23, 19, 20), 11),
+])
+def test_attenuation_in_slabs_that_overlap(wqlmod, oracle_lib, ctx, tmp_path, mesh, op, dims, npml):
+    """Where the two slabs of an axis overlap, the strain rates lose the + side's fields alone, in
+    the kernel that forms the gradient and in the one that is handed it.  FP32C is held to 1e-6 in
+    the velocities and in the stresses: ten times what FP32 coefficients and rates alone leave."""
+    text = deck(mesh, op, dims, npml, ",\n response = 'anelastic'") + ANELASTIC
+    path = tmp_path / "an.in"
+    path.write_text(text)
+    o = oracle_lib.Oracle(str(path))
+    runs = [wqlmod.Scenario(ctx, text=text, precision=p) for p in (wqlmod.FP64, wqlmod.FP32C)]
+    for r in [o] + runs:
+        fill(r, dims)
+        r.step(12)
+    for b in range(2):
+        ref, d, f = (r.fields(b) for r in [o] + runs)
+        assert rel_l2(d, ref) < 1e-11
+        assert rel_l2(f[:3], d[:3]) < 1e-6
+        assert rel_l2(f[3:], d[3:]) < 1e-6

@@ -1040,6 +1040,9 @@ __global__ void __launch_bounds__(384, 4) anelastic_comp_kernel(const __grid_con
     const bool hi = side & 1;
     const int ii = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 0 ? a.nq : (axis == 1 ? a.nr : a.ns);
     if (!(hi ? ii >= n - a.npml : ii < a.npml)) continue;
+    // where the two slabs of an axis overlap, the + side's Q alone counts
+    // (pml_damping_and_q takes the sides in turn, src/RHS_Interior.f90:2287-2387)
+    if (!hi && a.pml[side + 1] && ii >= n - a.npml) continue;
     // the axes of a shear component: xy 0 1, xz 0 2, yz 1 2
     if (c >= 3 && (c == 3 ? axis == 2 : (c == 4 ? axis == 1 : axis == 0))) continue;
     const int off = hi ? ii + 1 - (n - a.npml) : (axis == 2 ? ii + 1 - a.npml : ii - a.npml);
