@@ -17,8 +17,8 @@
  * last failure on the calling thread.  Host buffers are caller-owned;
  * device memory is owned by the scenario.  Arrays use the reference's
  * column-major point order (q fastest, then r, then s), without ghost layers.
- * Calls on one scenario must not overlap; different scenarios are
- * independent.
+ * Calls on one scenario must not overlap, but for wql_get_field among
+ * themselves or beside a step; different scenarios are independent.
  */
 #ifndef WQL_H
 #define WQL_H
@@ -119,15 +119,17 @@ int wql_get_info(wql_scn* scn, wql_info* info);
  * With the plastic_flow model (response = 'plastic', plastic_model other
  * than 'scec'), comp 9 and 10 read the plastic strain rate lambda and the
  * plastic strain gammap per point (P%P(:,:,:,1:2), src/plastic.f90:141,
- * src/plastic_material.f90:38-44); otherwise they return WQL_E_STATE. */
+ * src/plastic_material.f90:38-44); otherwise they return WQL_E_STATE.
+ * The values pass through an array of the scenario (at most 32 MiB) that
+ * nothing else uses, under a lock: a read changes no state of the run, and
+ * reads and writes from several threads take their turn.  Neither call
+ * allocates device memory.  A read that overlaps a step returns the values of
+ * some stage of it. */
 int wql_get_field(wql_scn* scn, int block, int comp, double* host_out);
 int wql_set_field(wql_scn* scn, int block, int comp, const double* host_in);
 
-/* wql_get_field without any device allocation, for callers that must not
- * allocate device memory (cudaMalloc/cudaFree synchronise the whole device,
- * so a monitoring thread reading a scenario would stall other threads'
- * streams; a memory-capped host may have no room left).  FP32 fields are
- * widened one s plane at a time through a fixed 8 MiB device array; a block
+/* wql_get_field through a fixed 8 MiB device array instead of the
+ * scenario's: FP32 fields are widened one s plane at a time; a block
  * whose pitched plane (pq*nr, pq = nq rounded up to a multiple of 8)
  * exceeds 1048576 points returns WQL_E_INPUT.  The first call on a device
  * resolves the array's address and must not happen during stream capture.

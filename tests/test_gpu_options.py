@@ -1,5 +1,7 @@
 """Combinations of options that the other GPU tests do not reach, each against
 the oracle, FP64 or the same run without the option."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -57,3 +59,60 @@ def test_attenuation_in_slabs_that_overlap(wqlmod, oracle_lib, ctx, tmp_path, me
         assert rel_l2(d, ref) < 1e-11
         assert rel_l2(f[:3], d[:3]) < 1e-6
         assert rel_l2(f[3:], d[3:]) < 1e-6
+
+
+# odd row lengths in both blocks; the upwind pair; an axis over 32 MiB of dense values (three chunks)
+@pytest.mark.parametrize("prec", ["fp64", "fp32c"])
+@pytest.mark.parametrize("mesh,op,dims,npml", [
+    ("curvilinear", "traditional", (33, 27, 21, 23), 6),
+    ("cartesian", "upwind 6", (41, 35, 22, 24), 0),
+    ("cartesian", "traditional", (355, 13, 150, 170), 0),
+])
+def test_reads_leave_a_run_as_it_is(wqlmod, ctx, mesh, op, dims, npml, prec):
+    """Reads between steps, between stages, and from other threads during steps: the run ends bit for
+    bit where it ends without them, and threads reading at once each get their own component."""
+    p = wqlmod.FP64 if prec == "fp64" else wqlmod.FP32C
+    plain, read = (wqlmod.Scenario(ctx, text=deck(mesh, op, dims, npml), precision=p) for _ in range(2))
+    for s in (plain, read):
+        fill(s, dims)
+    plain.step(9)
+    got = read.fields(0)
+    f = start((dims[3], dims[2], dims[0]), 10)
+    assert np.array_equal(got, f if prec == "fp64" else f.astype(np.float32).astype(float))
+    read.step(2)
+    read.fields(1)
+    for k in range(1, 6):
+        read.stage(k)
+        read.fields(k % 2)
+    done = threading.Event()
+
+    def monitor():
+        while not done.is_set():
+            read.field(0, 4)
+            read.field(1, 1)
+
+    t = [threading.Thread(target=monitor) for _ in range(2)]
+    for x in t:
+        x.start()
+    for _ in range(6):
+        read.step(1)
+        read.sync()
+    done.set()
+    for x in t:
+        x.join()
+    want = [plain.fields(b) for b in range(2)]
+    for b in range(2):
+        assert np.array_equal(read.fields(b), want[b])
+    wrong = []
+
+    def reader(c):
+        for _ in range(4):
+            if not np.array_equal(read.field(0, c), want[0][c]):
+                wrong.append(c)
+
+    t = [threading.Thread(target=reader, args=(c,)) for c in range(9)]
+    for x in t:
+        x.start()
+    for x in t:
+        x.join()
+    assert not wrong

@@ -235,6 +235,13 @@ struct wql_scn {
   size_t ev_used = 0;
   std::vector<std::pair<size_t, int>> ev_marks;  // (start event, kind 0 interface / 1 stencil / 2 corrections)
   int launches_last_step = 0;
+  // Field reads and writes pass through this array of dense FP64 values, rows
+  // of a block at a time.  It belongs to them alone, so that a read changes
+  // nothing that a step uses, and io_mu is held from the first chunk to the
+  // last, so that calls from several threads take it in turn.
+  double* io = nullptr;
+  long long io_words = 0;
+  std::mutex io_mu;
   cudaEvent_t next_event() {
     if (ev_used == ev_pool.size()) {
       cudaEvent_t e;
@@ -314,9 +321,11 @@ __global__ void dense_to_pitched(const double* __restrict__ in, int pq, int nq, 
 }
 
 
-// The field buffer that the next stage writes and nothing reads before: room
-// for one dense FP64 component (9 pitched components of at least 4 bytes).
-double* field_scratch(wql_scn* scn, int block) { return (double*)scn->B[block].F[scn->cur ^ 1]; }
+// Words of the array that field reads and writes pass through: a component of
+// the larger block, at most 32 MiB (whole rows of either block).
+long long io_words_of(long long npd0, long long npd1, int nq0, int nq1) {
+  return std::max<long long>(std::min(std::max(npd0, npd1), 4LL << 20), std::max(nq0, nq1));
+}
 
 // Dense (nq-pitched) FP64 array to a pq-pitched array of T.
 template <typename T>
@@ -336,11 +345,10 @@ __global__ void station_kernel(const T* __restrict__ F, long long np, const long
   for (int c = 0; c < 3; ++c) out[i * 3 + c] = (double)F[c * np + p];
 }
 
-// Grid points only: the row pads hold no field values.
 template <typename T>
-__global__ void count_nonfinite(const T* a, long long n, int nq, int pq, unsigned int* cnt) {
+__global__ void count_nonfinite(const T* a, long long n, unsigned int* cnt) {
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p < n && p % pq < nq && !isfinite((double)a[p])) atomicAdd(cnt, 1u);
+  if (p < n && !isfinite((double)a[p])) atomicAdd(cnt, 1u);
 }
 
 // source_time (src/moment_tensor.f90:958-1011); false for an unknown type.
@@ -940,6 +948,8 @@ int create(wql_ctx* ctx, Problem&& P, int precision, const wql_media* media, wql
   S->st_cap = station_ring_cap(Pr);
   for (int b = 0; b < 2; ++b)
     if ((rc = setup_block(S.get(), b))) return rc;
+  S->io_words = io_words_of(S->B[0].npd, S->B[1].npd, S->B[0].nq, S->B[1].nq);
+  if ((rc = S->alloc((void**)&S->io, S->io_words * sizeof(double), false))) return rc;
   // moment-tensor sources: the unified list goes to the preferred block when
   // the source lies in its box, else to the other block when it lies in
   // that one; per-block lists stay with their block; a source in no block is
@@ -1668,9 +1678,9 @@ int wql_sync(wql_scn* scn, int check_nan) {
     for (int b = 0; b < 2; ++b) {
       const long long n = 9 * scn->B[b].np;
       if (scn->prec == WQL_FP64)
-        count_nonfinite<double><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const double*)scn->B[b].F[scn->cur], n, scn->B[b].nq, scn->B[b].pq, cnt);
+        count_nonfinite<double><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const double*)scn->B[b].F[scn->cur], n, cnt);
       else
-        count_nonfinite<float><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const float*)scn->B[b].F[scn->cur], n, scn->B[b].nq, scn->B[b].pq, cnt);
+        count_nonfinite<float><<<(unsigned)((n + 255) / 256), 256, 0, scn->stream>>>((const float*)scn->B[b].F[scn->cur], n, cnt);
     }
     unsigned int h = 0;
     CK(cudaStreamSynchronize(scn->stream));
@@ -1707,17 +1717,18 @@ int wql_get_field(wql_scn* scn, int block, int comp, double* host_out) {
     return fail(WQL_E_STATE, "components 9 and 10 (plastic strain rate and strain) need plastic_flow");
   const void* src = comp == 9 ? B.pl_lambda : (comp == 10 ? B.pl_gammap : B.F[scn->cur]);
   const long long off = comp > 8 ? 0 : comp * B.np;
-  const long long rows = (long long)B.nr * B.ns;
-  // dense FP64 values go through the buffer that the next stage overwrites:
-  // an allocation and its release would wait for all work on the device
-  double* tmp = field_scratch(scn, block);
-  const unsigned grid = (unsigned)std::min<long long>((B.npd + 255) / 256, 4096);
-  if (scn->prec == WQL_FP64)
-    pitched_to_dense<double><<<grid, 256, 0, scn->stream>>>((const double*)src + off, B.pq, B.nq, rows, tmp);
-  else
-    pitched_to_dense<float><<<grid, 256, 0, scn->stream>>>((const float*)src + off, B.pq, B.nq, rows, tmp);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(host_out, tmp, B.npd * sizeof(double), cudaMemcpyDeviceToHost, scn->stream));
+  const long long rows = (long long)B.nr * B.ns, per = scn->io_words / B.nq;
+  std::lock_guard<std::mutex> lock(scn->io_mu);
+  for (long long r = 0; r < rows; r += per) {
+    const long long n = std::min(per, rows - r), at = off + r * B.pq;
+    const unsigned grid = (unsigned)std::min<long long>((n * B.nq + 255) / 256, 4096);
+    if (scn->prec == WQL_FP64)
+      pitched_to_dense<double><<<grid, 256, 0, scn->stream>>>((const double*)src + at, B.pq, B.nq, n, scn->io);
+    else
+      pitched_to_dense<float><<<grid, 256, 0, scn->stream>>>((const float*)src + at, B.pq, B.nq, n, scn->io);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(host_out + r * B.nq, scn->io, n * B.nq * sizeof(double), cudaMemcpyDeviceToHost, scn->stream));
+  }
   CK(cudaStreamSynchronize(scn->stream));
   return WQL_OK;
 }
@@ -1805,14 +1816,17 @@ int wql_set_field(wql_scn* scn, int block, int comp, const double* host_in) {
   if (!scn || !host_in || block < 0 || block > 1 || comp < 0 || comp > 8)
     return fail(WQL_E_INPUT, "bad argument");
   auto& B = scn->B[block];
-  const long long rows = (long long)B.nr * B.ns;
-  double* tmp = field_scratch(scn, block);
-  CK(cudaMemcpyAsync(tmp, host_in, B.npd * sizeof(double), cudaMemcpyHostToDevice, scn->stream));
-  const unsigned grid = (unsigned)std::min<long long>((B.np + 255) / 256, 4096);
-  if (scn->prec == WQL_FP64)
-    dense_to_pitched<double><<<grid, 256, 0, scn->stream>>>(tmp, B.pq, B.nq, rows, (double*)B.F[scn->cur] + comp * B.np);
-  else
-    dense_to_pitched<float><<<grid, 256, 0, scn->stream>>>(tmp, B.pq, B.nq, rows, (float*)B.F[scn->cur] + comp * B.np);
+  const long long rows = (long long)B.nr * B.ns, per = scn->io_words / B.nq;
+  std::lock_guard<std::mutex> lock(scn->io_mu);
+  for (long long r = 0; r < rows; r += per) {
+    const long long n = std::min(per, rows - r), at = comp * B.np + r * B.pq;
+    CK(cudaMemcpyAsync(scn->io, host_in + r * B.nq, n * B.nq * sizeof(double), cudaMemcpyHostToDevice, scn->stream));
+    const unsigned grid = (unsigned)std::min<long long>((n * B.pq + 255) / 256, 4096);
+    if (scn->prec == WQL_FP64)
+      dense_to_pitched<double><<<grid, 256, 0, scn->stream>>>(scn->io, B.pq, B.nq, n, (double*)B.F[scn->cur] + at);
+    else
+      dense_to_pitched<float><<<grid, 256, 0, scn->stream>>>(scn->io, B.pq, B.nq, n, (float*)B.F[scn->cur] + at);
+  }
   // the new values carry no rounding error yet: clear their compensation
   if (B.C) CK(cudaMemsetAsync((comp_t*)B.C + comp * B.np, 0, B.np * sizeof(comp_t), scn->stream));
   CK(cudaGetLastError());
@@ -2167,6 +2181,11 @@ int wql_estimate_device_bytes(const char* in_text, const char* base_dir, int pre
     }
     // set-up arrays of one block: x, metric, J, material (FP64)
     transient = std::max(transient, faces + al(3 * npd * 8) + al(9 * npd * 8) + al(npd * 8) + al(3 * npd * 8));
+  }
+  {
+    const int* n0 = P.btp[0].nqrs;
+    const int* n1 = P.btp[1].nqrs;
+    res += al(8 * io_words_of((long long)n0[0] * n0[1] * n0[2], (long long)n1[0] * n1[1] * n1[2], n0[0], n1[0]));
   }
   res += al(6 * nf * 8) + 2 * al(8 * nf * 8) + 3 * al(2 * nf * 8) + al(18 * nf * esz) + al(10 * nf * 8) + 2 * 512;
   if (P.w_fault) res += 2 * al((long long)frame_ring_cap(nf) * kFrameWords * nf * 4);
