@@ -542,10 +542,13 @@ __device__ __forceinline__ bool tma_consume(const VolumeArgs<float>& a, float* s
           else deriv_s<CURV, FD, true>(a, p, ks, qv, o);
           const float rh = a.rh[d];
           if (CURV) {
-            const f2 Jr = mul2(Jinv, pack(rh, rh));
+            // 1/h goes to the differences: taken into 1/J, its rounding is the
+            // same at every point of a regular grid and adds up
+#pragma unroll
+            for (int c = 0; c < 3; ++c) o[c] = mul2(pack(rh, rh), o[c]);
 #pragma unroll
             for (int jj = 0; jj < 3; ++jj) {
-              const f2 mt = mul2(d == 0 ? mq[jj] : (d == 1 ? mr[jj] : g2(CC + jj * NC + li)), Jr);
+              const f2 mt = mul2(d == 0 ? mq[jj] : (d == 1 ? mr[jj] : g2(CC + jj * NC + li)), Jinv);
 #pragma unroll
               for (int c = 0; c < 3; ++c) g[c][jj] = d == 0 ? mul2(mt, o[c]) : fma2(mt, o[c], g[c][jj]);
             }

@@ -479,11 +479,13 @@ __global__ void __launch_bounds__(256) stencil_kernel_pointwise(const __grid_con
         [&](int off, T w) {
           const unsigned q = pu + (unsigned)off * st;
           if (CURV) {
-            const T m0 = w * (Cu + (d * 3) * np)[q], m1 = w * (Cu + (d * 3 + 1) * np)[q],
-                    m2 = w * (Cu + (d * 3 + 2) * np)[q];
+            // the weight goes to the flux, not into its metrics (rounded there,
+            // it is off by the same at every point of a regular grid)
+            const T m0 = (Cu + (d * 3) * np)[q], m1 = (Cu + (d * 3 + 1) * np)[q], m2 = (Cu + (d * 3 + 2) * np)[q];
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-              o[3 + c] += m0 * (Fu + sig(c, 0) * np)[q] + m1 * (Fu + sig(c, 1) * np)[q] + m2 * (Fu + sig(c, 2) * np)[q];
+              o[3 + c] += w * (m0 * (Fu + sig(c, 0) * np)[q] + m1 * (Fu + sig(c, 1) * np)[q] +
+                               m2 * (Fu + sig(c, 2) * np)[q]);
           } else {
 #pragma unroll
             for (int c = 0; c < 3; ++c) o[3 + c] += w * (Fu + sig(c, d) * np)[q];
