@@ -120,7 +120,7 @@ int wql_get_info(wql_scn* scn, wql_info* info);
  * than 'scec'), comp 9 and 10 read the plastic strain rate lambda and the
  * plastic strain gammap per point (P%P(:,:,:,1:2), src/plastic.f90:141,
  * src/plastic_material.f90:38-44); otherwise they return WQL_E_STATE.
- * The values pass through an array of the scenario (at most 32 MiB) that
+ * The values pass through an array of the scenario (at most 64 MiB) that
  * nothing else uses, under a lock: a read changes no state of the run, and
  * reads and writes from several threads take their turn.  Neither call
  * allocates device memory.  A read that overlaps a step returns the values of

@@ -61,12 +61,12 @@ def test_attenuation_in_slabs_that_overlap(wqlmod, oracle_lib, ctx, tmp_path, me
         assert rel_l2(f[3:], d[3:]) < 1e-6
 
 
-# odd row lengths in both blocks; the upwind pair; an axis over 32 MiB of dense values (three chunks)
+# odd row lengths in both blocks; the upwind pair; a component of over 64 MiB (two chunks)
 @pytest.mark.parametrize("prec", ["fp64", "fp32c"])
 @pytest.mark.parametrize("mesh,op,dims,npml", [
     ("curvilinear", "traditional", (33, 27, 21, 23), 6),
     ("cartesian", "upwind 6", (41, 35, 22, 24), 0),
-    ("cartesian", "traditional", (355, 13, 150, 170), 0),
+    ("cartesian", "traditional", (355, 13, 170, 180), 0),
 ])
 def test_reads_leave_a_run_as_it_is(wqlmod, ctx, mesh, op, dims, npml, prec):
     """Reads between steps, between stages, and from other threads during steps: the run ends bit for

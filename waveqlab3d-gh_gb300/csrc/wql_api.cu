@@ -322,9 +322,9 @@ __global__ void dense_to_pitched(const double* __restrict__ in, int pq, int nq, 
 
 
 // Words of the array that field reads and writes pass through: a component of
-// the larger block, at most 32 MiB (whole rows of either block).
+// the larger block, at most 64 MiB (whole rows of either block).
 long long io_words_of(long long npd0, long long npd1, int nq0, int nq1) {
-  return std::max<long long>(std::min(std::max(npd0, npd1), 4LL << 20), std::max(nq0, nq1));
+  return std::max<long long>(std::min(std::max(npd0, npd1), 8LL << 20), std::max(nq0, nq1));
 }
 
 // Dense (nq-pitched) FP64 array to a pq-pitched array of T.
