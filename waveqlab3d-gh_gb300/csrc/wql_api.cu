@@ -456,6 +456,28 @@ void place_source(const BlockGrid& G, const MomentSource& m, int order, int alph
       }
 }
 
+// Tensor maps m of both blocks for TMA tiles tq wide, over the rates DF and the
+// compensation C, and the s chunk of the launch over both.
+int make_pair_maps(wql_scn* S, int tq, StencilMaps* const m[2], void* const DF[2], void* const C[2]) {
+  for (int b = 0; b < 2; ++b) {
+    const auto& B = S->B[b];
+    const int erc = make_stencil_maps(*m[b], B.F, B.coef, DF[b], C[b], B.nq, B.nr, B.ns, B.pq, S->curv, S->fd, tq);
+    if (erc) return fail(WQL_E_CUDA, "cuTensorMapEncodeTiled failed for the stencil maps (error " + std::to_string(erc) + ")");
+  }
+  const int nq[2] = {S->B[0].nq, S->B[1].nq}, ns[2] = {S->B[0].ns, S->B[1].ns};
+  m[0]->chunk2 = m[1]->chunk2 = pair_chunk(nq, S->B[0].nr, ns, m[0]->tq);
+  return WQL_OK;
+}
+
+// The scenario's own maps for tiles tq wide, unless they are that already.
+int use_tiles(wql_scn* S, int tq) {
+  if (S->B[0].maps.ok && S->B[0].maps.tq == tq) return WQL_OK;
+  StencilMaps* const m[2] = {&S->B[0].maps, &S->B[1].maps};
+  void* const DF[2] = {S->B[0].DF, S->B[1].DF};
+  void* const C[2] = {S->B[0].C, S->B[1].C};
+  return make_pair_maps(S, tq, m, DF, C);
+}
+
 int setup_block(wql_scn* S, int b) {
   const BlockParams& bp = S->P.btp[b];
   auto& B = S->B[b];
@@ -586,9 +608,6 @@ int setup_block(wql_scn* S, int b) {
   if ((rc = S->alloc(&B.DF, 9 * B.np * S->esz))) return rc;
   if (S->prec == WQL_FP32C) {
     if ((rc = S->alloc(&B.C, 9 * B.np * sizeof(comp_t)))) return rc;
-    const int erc = make_stencil_maps(B.maps, B.F, B.coef, B.DF, B.C, B.nq, B.nr, B.ns, B.pq, S->curv, S->fd,
-                                      tma_tile_width(S->P.btp[0].nqrs[0], S->P.btp[1].nqrs[0], S->curv));
-    if (erc) return fail(WQL_E_CUDA, "cuTensorMapEncodeTiled failed for the stencil maps (error " + std::to_string(erc) + ")");
   }
   if (S->prec == WQL_FP64 && !S->fd) {
     int sms = 0;
@@ -948,6 +967,7 @@ int create(wql_ctx* ctx, Problem&& P, int precision, const wql_media* media, wql
   S->st_cap = station_ring_cap(Pr);
   for (int b = 0; b < 2; ++b)
     if ((rc = setup_block(S.get(), b))) return rc;
+  if (S->prec == WQL_FP32C && (rc = use_tiles(S.get(), tma_tile_width(S->B[0].nq, S->B[1].nq, S->curv)))) return rc;
   S->io_words = io_words_of(S->B[0].npd, S->B[1].npd, S->B[0].nq, S->B[1].nq);
   if ((rc = S->alloc((void**)&S->io, S->io_words * sizeof(double), false))) return rc;
   // moment-tensor sources: the unified list goes to the preferred block when
@@ -2229,13 +2249,7 @@ int wql_batch_add(wql_batch* b, wql_scn* scn) {
   // the packed launch runs 32-wide tiles: a member set up with the wide
   // Cartesian tiles gets 32-wide tensor maps
   if (scn->prec == WQL_FP32C)
-    for (int k = 0; k < 2; ++k) {
-      auto& B = scn->B[k];
-      if (B.maps.tq == kTmaTQ) continue;
-      const int erc =
-          make_stencil_maps(B.maps, B.F, B.coef, B.DF, B.C, B.nq, B.nr, B.ns, B.pq, scn->curv, scn->fd, kTmaTQ);
-      if (erc) return fail(WQL_E_CUDA, "cuTensorMapEncodeTiled failed for the stencil maps (error " + std::to_string(erc) + ")");
-    }
+    if (const int rc = use_tiles(scn, kTmaTQ)) return rc;
   b->members.push_back(scn);
   return WQL_OK;
 }
@@ -2315,13 +2329,7 @@ int wql_set_tuning(wql_scn* scn, int kernel_variant, int schunk) {
   if (scn->prec == WQL_FP32C) {
     CK(cudaStreamSynchronize(scn->stream));  // no launch in flight reads the old maps
     const int want = kernel_variant == 6 ? kTmaTQ : tma_tile_width(scn->B[0].nq, scn->B[1].nq, scn->curv);
-    for (int k = 0; k < 2; ++k) {
-      auto& B = scn->B[k];
-      if (B.maps.tq == want) continue;
-      const int erc =
-          make_stencil_maps(B.maps, B.F, B.coef, B.DF, B.C, B.nq, B.nr, B.ns, B.pq, scn->curv, scn->fd, want);
-      if (erc) return fail(WQL_E_CUDA, "cuTensorMapEncodeTiled failed for the stencil maps (error " + std::to_string(erc) + ")");
-    }
+    if (const int rc = use_tiles(scn, want)) return rc;
   }
   scn->kernel_variant = kernel_variant;
   scn->schunk = schunk;

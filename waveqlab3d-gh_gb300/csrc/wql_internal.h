@@ -219,7 +219,7 @@ struct StencilMaps {
   int cur;                        // which field buffer is the stage input
   int fd;                         // operator the boxes are shaped for (0 central, 1 upwind)
   int tq;                         // tile width along q the boxes are shaped for
-  int chunk2;                     // planes per s chunk of the launch over both blocks (0: not chosen yet)
+  int chunk2;                     // planes per s chunk of the launch over both blocks (pair_chunk)
   int ok;
 };
 // Fills m for a block (fd: 0 the central SBP-6 operator, 1 the upwind pair:
@@ -261,6 +261,8 @@ long long fill_tma_desc(const VolumeArgs<float>& a, int chunk, TmaBatchDesc& d);
 // Planes per s chunk of a launch over nb blocks of tiles[b] (q, r) tiles and
 // ns[b] planes.
 int choose_chunk(const int* tiles, const int* ns, int nb);
+// The same for the launch over a scenario's two blocks on tiles tq wide.
+int pair_chunk(const int nq[2], int nr, const int ns[2], int tq);
 // Whether a block can go through the TMA stencil (FP32, r extent that keeps
 // the closure rows of the shifted last r tile inside the halo).
 bool tma_eligible(const VolumeArgs<float>& a);

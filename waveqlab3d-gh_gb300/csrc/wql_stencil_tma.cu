@@ -957,6 +957,12 @@ int choose_chunk(const int* tiles, const int* ns, int nb) {
   return best;
 }
 
+int pair_chunk(const int nq[2], int nr, const int ns[2], int tq) {
+  const int rows = (nr + tma_rows(tq) - 1) / tma_rows(tq);
+  const int tiles[2] = {(nq[0] + tq - 1) / tq * rows, (nq[1] + tq - 1) / tq * rows};
+  return choose_chunk(tiles, ns, 2);
+}
+
 namespace {
 
 MapArgs stage_maps(const StencilMaps& sm) {
@@ -1017,23 +1023,14 @@ void launch_tma2(const VolumeArgs<float>& a0, const VolumeArgs<float>& a1, cudaS
   TwoBlocks P;
   const VolumeArgs<float>* a[2] = {&a0, &a1};
   int ntile[2];
-  int tiles[2];
   for (int b = 0; b < 2; ++b) {
+    const StencilMaps& sm = *static_cast<const StencilMaps*>(a[b]->tma);
     P.a[b] = *a[b];
-    P.m[b] = stage_maps(*static_cast<const StencilMaps*>(a[b]->tma));
+    P.m[b] = stage_maps(sm);
     P.tq[b] = (a[b]->nq + TL::TQ - 1) / TL::TQ;
     P.tr[b] = (a[b]->nr + TL::TR - 1) / TL::TR;
-    tiles[b] = P.tq[b] * P.tr[b];
-  }
-  // kept with block 0's maps: the blocks and their tiles do not change
-  StencilMaps& keep = *static_cast<StencilMaps*>(const_cast<void*>(a0.tma));
-  if (a0.schunk <= 0 && keep.chunk2 == 0) {
-    const int planes[2] = {a0.ns, a1.ns};
-    keep.chunk2 = choose_chunk(tiles, planes, 2);
-  }
-  for (int b = 0; b < 2; ++b) {
-    P.schunk[b] = a[b]->schunk > 0 ? a[b]->schunk : keep.chunk2;
-    ntile[b] = tiles[b] * ((a[b]->ns + P.schunk[b] - 1) / P.schunk[b]);
+    P.schunk[b] = a[b]->schunk > 0 ? a[b]->schunk : sm.chunk2;
+    ntile[b] = P.tq[b] * P.tr[b] * ((a[b]->ns + P.schunk[b] - 1) / P.schunk[b]);
   }
   P.ntile0 = ntile[0];
   kern<<<ntile[0] + ntile[1], 2 * TL::NT + 32, smem, s>>>(P);
@@ -1095,7 +1092,7 @@ int make_stencil_maps(StencilMaps& m, void* const F[2], void* coef, void* DF, vo
   m.cur = 0;
   m.fd = fd;
   m.tq = TQ;
-  m.chunk2 = 0;
+  m.chunk2 = 32;
   for (int i = 0; i < 2 && !rc; ++i) {
     rc = encode4(&m.fbox[i], F[i], nq, nr, ns, 9, pq, TQ + 16, TR + 2 * hr, 9);
     // lead tiles: all 9 components of one plane, or (upwind) the 3
