@@ -192,11 +192,12 @@ int wql_station_index(wql_scn* scn, int block, int* ijk);
 int wql_get_seismograms(wql_scn* scn, int block, double* host_out);
 
 /* Autotuner: times the stencil-kernel candidates (WQL_FP32C: the TMA
- * kernel with s chunks of 12..48 planes or automatic, and on Cartesian
+ * kernel with s chunks of 4..48 planes or automatic, and on Cartesian
  * blocks that fill 40-wide tiles better both tile widths, variants 5 and 6;
- * WQL_FP64: default, tiled and per-point) on the scenario's own blocks, reps
- * launches each, into scratch arrays (the scenario's state is not
- * changed), applies the fastest with wql_set_tuning and returns it.
+ * WQL_FP64: default, tiled and per-point) on the scenario's own blocks,
+ * launched as a step launches them, reps launches each, into scratch arrays
+ * (the scenario's state is not changed), applies the fastest with
+ * wql_set_tuning and returns it; the default stays unless it is beaten by 2 %.
  * Results are cached per block shape, mesh type and precision. */
 int wql_autotune(wql_scn* scn, int reps, int* variant, int* schunk);
 

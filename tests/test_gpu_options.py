@@ -132,3 +132,30 @@ def test_curvilinear_rounding(wqlmod, ctx, op):
         err[mesh] = [np.hypot(*(rel_l2(f.fields(b)[c], d.fields(b)[c]) for b in range(2)))
                      for c in (slice(0, 3), slice(3, 9))]
     assert all(k < 1.1 * c for k, c in zip(err["curvilinear"], err["cartesian"])), err
+
+
+def stencil_ms(s, tuning=None, steps=40):
+    """Least device time of one step's stencil launches in five runs."""
+    if tuning:
+        s.set_tuning(*tuning)
+    s.step(3)
+    best = 1e9
+    for _ in range(5):
+        s.profile(True)
+        s.step(steps)
+        best = min(best, s.kernel_times()["stencil"][0] / steps)
+    s.profile(False)
+    return best
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32c"])
+@pytest.mark.parametrize("mesh,dims", [("cartesian", (41, 41, 41, 41)), ("curvilinear", (64, 64, 48, 57))])
+def test_autotune_is_no_slower_than_the_default(wqlmod, ctx, mesh, dims, prec):
+    """The trial launches what a step launches, so the choice cannot lose to the default by more than
+    the noise of launches of some 20 us."""
+    s = wqlmod.Scenario(ctx, text=deck(mesh, "traditional", dims, 0), precision=wqlmod.FP64 if prec == "fp64" else wqlmod.FP32C)
+    fill(s, dims)
+    default = stencil_ms(s)
+    choice = s.autotune(20)
+    tuned = stencil_ms(s)
+    assert tuned < 1.15 * default, (choice, tuned, default)
