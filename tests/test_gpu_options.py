@@ -159,3 +159,13 @@ def test_autotune_is_no_slower_than_the_default(wqlmod, ctx, mesh, dims, prec):
     choice = s.autotune(20)
     tuned = stencil_ms(s)
     assert tuned < 1.15 * default, (choice, tuned, default)
+
+
+@pytest.mark.parametrize("variant,launches", [(0, 5), (1, 5), (2, 10), (6, 5)])
+def test_profile_counts_launches(wqlmod, ctx, variant, launches):
+    """wql_kernel_times counts the stencil's launches: one a stage over both blocks, or one a block."""
+    s = wqlmod.Scenario(ctx, text=deck("curvilinear", "traditional", (33, 27, 21, 23), 0), precision=wqlmod.FP32C)
+    s.set_tuning(variant, 0)
+    s.profile(True)
+    s.step(3)
+    assert s.kernel_times()["stencil"][1] == 3 * launches

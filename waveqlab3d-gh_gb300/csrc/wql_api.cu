@@ -1311,9 +1311,15 @@ template <typename T>
 bool stage_pair_stencil(wql_scn* S, StepCtx& c, int stage) {
   const VolumeArgs<T> a0 = volume_args<T>(S, 0, stage_A(S, stage), stage_Bdt(S, stage), stage == 5);
   const VolumeArgs<T> a1 = volume_args<T>(S, 1, stage_A(S, stage), stage_Bdt(S, stage), stage == 5);
+  const size_t marks = S->ev_marks.size(), used = S->ev_used;
   mark_begin(S, 1);
   const int n = launch_volume2<T>(a0, a1, S->curv, S->stream);
-  mark_end(S);
+  if (n > 0) {
+    mark_end(S);
+  } else if (S->profiling) {  // nothing to time: each block's launch has its own mark
+    S->ev_marks.resize(marks);
+    S->ev_used = used;
+  }
   c.launches += n;
   return n > 0;
 }
