@@ -193,7 +193,7 @@ int wql_get_seismograms(wql_scn* scn, int block, double* host_out);
 
 /* Autotuner: times the stencil-kernel candidates (WQL_FP32C: the TMA
  * kernel with s chunks of 4..48 planes or automatic, and on Cartesian
- * blocks that fill 40-wide tiles better both tile widths, variants 5 and 6;
+ * blocks that take 40-wide tiles both tile widths, variants 5 and 6;
  * WQL_FP64: default, tiled and per-point) on the scenario's own blocks,
  * launched as a step launches them, reps launches each, into scratch arrays
  * (the scenario's state is not changed), applies the fastest with
@@ -278,7 +278,7 @@ int wql_kernel_times(wql_scn* scn, int kind, double* ms, int* launches);
  * (every neighbour read through the caches), 2 = tiled shared-memory kernel
  * with 32x8 tiles, 3 = the same at three blocks per SM (FP32), 4 = 64x8 tiles
  * (WQL_FP32C only), 5 = TMA-pipelined kernel (WQL_FP32C only; 32x12 tiles, or
- * 40x8 on Cartesian blocks whose q extent fills 40-wide tiles better), 6 = the
+ * 40x8 on Cartesian blocks that get done sooner on them), 6 = the
  * TMA kernel on 32x12 tiles always; schunk = planes per thread block along s
  * (0 = automatic). */
 int wql_set_tuning(wql_scn* scn, int kernel_variant, int schunk);

@@ -169,3 +169,29 @@ def test_profile_counts_launches(wqlmod, ctx, variant, launches):
     s.profile(True)
     s.step(3)
     assert s.kernel_times()["stencil"][1] == 3 * launches
+
+
+@pytest.mark.parametrize("op,nr", [("traditional", 12), ("traditional", 13), ("upwind 6", 13)])
+def test_tile_width_for_short_r_axes(wqlmod, ctx, op, nr):
+    """Rows whose closures 40 x 8 tiles would not hold take the 32 x 12 tiles, not the per-point kernel."""
+    dims, out = (76, 75, nr, 40), {}
+    for v in (0, 6, 1):
+        s = wqlmod.Scenario(ctx, text=deck("cartesian", op, dims, 0), precision=wqlmod.FP32C)
+        s.set_tuning(v, 0)
+        fill(s, dims)
+        s.step(4)
+        out[v] = np.stack([s.fields(b)[:, 3:-3, 3:-3, 3:70] for b in range(2)])
+    assert np.array_equal(out[0], out[6])
+    assert not np.array_equal(out[6], out[1])  # the two kernels round differently
+
+
+@pytest.mark.parametrize("dims", [(280, 280, 41, 41), (120, 120, 100, 100), (76, 75, 150, 150), (120, 160, 14, 60)])
+def test_tile_width_by_schedule(wqlmod, ctx, dims):
+    """The width that the schedules choose is no slower than 32-wide tiles (but for noise), and faster
+    where 40-wide ones save planes."""
+    s = wqlmod.Scenario(ctx, text=deck("cartesian", "traditional", dims, 0), precision=wqlmod.FP32C)
+    fill(s, dims)
+    default, narrow = stencil_ms(s, (0, 0), 20), stencil_ms(s, (6, 0), 20)
+    assert default < 1.08 * narrow
+    if dims[0] in (76, 120) and dims[2] in (150, 14):
+        assert default < 0.97 * narrow

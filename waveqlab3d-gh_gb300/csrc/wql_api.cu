@@ -186,6 +186,7 @@ struct wql_scn {
   bool anel = false;       // response = 'anelastic'
   double an_tau[4] = {}, an_w[4] = {};
   int schunk = 0;          // planes per CTA along s (0: default)
+  int tile_width = kTmaTQ; // TMA tiles' width along q (FP32C)
   bool plastic = false;
   bool pl_flow = false;  // plastic_flow (the reference's default model) instead of scec
   double pl_c = 1.36, pl_nu = 0.1934, pl_Tv = 0.03;
@@ -967,7 +968,11 @@ int create(wql_ctx* ctx, Problem&& P, int precision, const wql_media* media, wql
   S->st_cap = station_ring_cap(Pr);
   for (int b = 0; b < 2; ++b)
     if ((rc = setup_block(S.get(), b))) return rc;
-  if (S->prec == WQL_FP32C && (rc = use_tiles(S.get(), tma_tile_width(S->B[0].nq, S->B[1].nq, S->curv)))) return rc;
+  if (S->prec == WQL_FP32C) {
+    const int nq[2] = {S->B[0].nq, S->B[1].nq}, ns[2] = {S->B[0].ns, S->B[1].ns};
+    S->tile_width = tma_tile_width(nq, S->B[0].nr, ns, S->curv, S->fd);
+    if ((rc = use_tiles(S.get(), S->tile_width))) return rc;
+  }
   S->io_words = io_words_of(S->B[0].npd, S->B[1].npd, S->B[0].nq, S->B[1].nq);
   if ((rc = S->alloc((void**)&S->io, S->io_words * sizeof(double), false))) return rc;
   // moment-tensor sources: the unified list goes to the preferred block when
@@ -2065,11 +2070,11 @@ int wql_autotune(wql_scn* scn, int reps, int* variant, int* schunk) {
     if (it != cache.end()) return apply(it->second);
   }
   // candidates, the default first: the TMA kernel with several s chunk sizes
-  // (FP32C; on Cartesian blocks that fill 40-wide tiles better, with both
-  // tile widths), the tiled and per-point kernels (FP64)
+  // (FP32C; on Cartesian blocks that take 40-wide tiles, with both tile
+  // widths), the tiled and per-point kernels (FP64)
   std::vector<std::pair<int, int>> cand;
   if (scn->prec == WQL_FP32C) {
-    const bool wide = tma_tile_width(scn->B[0].nq, scn->B[1].nq, scn->curv) != kTmaTQ;
+    const bool wide = scn->tile_width != kTmaTQ;
     for (int c : {0, 4, 6, 8, 10, 12, 14, 16, 24, 32, 48})
       if (c <= scn->B[0].ns) {
         cand.push_back({5, c});
@@ -2106,8 +2111,7 @@ int wql_autotune(wql_scn* scn, int reps, int* variant, int* schunk) {
       StencilMaps* const m[2] = {&maps[0], &maps[1]};
       void* const DF[2] = {scratch[0][0], scratch[1][0]};
       void* const C[2] = {scratch[0][1], scratch[1][1]};
-      const int tq = c.first == 6 ? kTmaTQ : tma_tile_width(scn->B[0].nq, scn->B[1].nq, scn->curv);
-      if ((rc = make_pair_maps(scn, tq, m, DF, C))) break;
+      if ((rc = make_pair_maps(scn, c.first == 6 ? kTmaTQ : scn->tile_width, m, DF, C))) break;
     }
     // a stage's stencil as a step launches it: both blocks at once where the
     // variant has that
@@ -2325,8 +2329,7 @@ int wql_set_tuning(wql_scn* scn, int kernel_variant, int schunk) {
   // restore) the width chosen for the blocks at set-up
   if (scn->prec == WQL_FP32C) {
     CK(cudaStreamSynchronize(scn->stream));  // no launch in flight reads the old maps
-    const int want = kernel_variant == 6 ? kTmaTQ : tma_tile_width(scn->B[0].nq, scn->B[1].nq, scn->curv);
-    if (const int rc = use_tiles(scn, want)) return rc;
+    if (const int rc = use_tiles(scn, kernel_variant == 6 ? kTmaTQ : scn->tile_width)) return rc;
   }
   scn->kernel_variant = kernel_variant;
   scn->schunk = schunk;

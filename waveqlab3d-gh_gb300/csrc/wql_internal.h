@@ -206,11 +206,18 @@ constexpr int kFrameOff[9] = {FR_UFACE, FR_VFACE, FR_S, FR_UHAT, FR_VHAT, FR_SVE
 // stages fill one SM's shared memory (measured faster than 32 x 8 tiles with
 // three stages, 32 x 10 and 64 x 6 on 2 x 201^3 blocks).
 constexpr int kTmaTQ = 32, kTmaTR = 12, kTmaStages = 2;
-// Cartesian blocks whose q extent fills 40-wide tiles better (76 points: 2
-// tiles of 40 use 95 % of their columns, 3 of 32 use 79 %) take 40 x 8 tiles:
-// five whole consumer warps a role.
+// Cartesian blocks that need fewer of them (76/75 x 150^2: 76 a plane against
+// 78 of 32 x 12, so that the schedule ends sooner) take 40 x 8 tiles, five
+// whole consumer warps a role (tma_tile_width).
 constexpr int kTmaTQWide = 40;
 constexpr int tma_rows(int tq) { return tq == kTmaTQWide ? 8 : kTmaTR; }
+// A tiled axis of n points with tiles of T keeps every closure row inside
+// the tile that owns it plus a 3-point halo unless the shifted last tile
+// starts at 4 or 5 (then it would own left closure rows whose stencil
+// reaches point 0 from outside the halo).  With the upwind pair (halo 4,
+// closure rows reading points 0..9) only a last tile starting at 5 is excluded.
+constexpr bool tiles_ok(int n, int T) { return n <= T + 3 || n >= T + 6; }
+constexpr bool tiles_ok_up(int n, int T) { return n <= T + 4 || n >= T + 6; }
 struct StencilMaps {
   CUtensorMap fbox[2], flead[2];  // per field buffer
   CUtensorMap ca, cb, cc, cl;     // coefficients: q-halo rows, r-halo columns, tile, lead plane
@@ -227,9 +234,8 @@ struct StencilMaps {
 // returns 0 or a CUDA driver error code.
 int make_stencil_maps(StencilMaps& m, void* const F[2], void* coef, void* DF, void* C, int nq, int nr, int ns, int pq,
                       bool curv, int fd, int tq);
-// Tile width along q (kTmaTQ or kTmaTQWide) for a scenario whose blocks have
-// nq0 and nq1 points along q.
-int tma_tile_width(int nq0, int nq1, bool curv);
+// Tile width along q (kTmaTQ or kTmaTQWide) for a scenario's two blocks.
+int tma_tile_width(const int nq[2], int nr, const int ns[2], bool curv, int fd);
 // Launches the TMA stencil kernel (every plane of the block).
 void launch_stencil_tma(const VolumeArgs<float>& a, bool curv, void* stream);
 // The same for both blocks of a scenario in one launch.
@@ -260,9 +266,9 @@ struct TmaBatchDesc {
 long long fill_tma_desc(const VolumeArgs<float>& a, int chunk, TmaBatchDesc& d);
 // Planes per s chunk of a launch over nb blocks of tiles[b] (q, r) tiles and
 // ns[b] planes.
-int choose_chunk(const int* tiles, const int* ns, int nb);
+int choose_chunk(const int* tiles, const int* ns, int nb, float* end = nullptr);
 // The same for the launch over a scenario's two blocks on tiles tq wide.
-int pair_chunk(const int nq[2], int nr, const int ns[2], int tq);
+int pair_chunk(const int nq[2], int nr, const int ns[2], int tq, float* end = nullptr);
 // Whether a block can go through the TMA stencil (FP32, r extent that keeps
 // the closure rows of the shifted last r tile inside the halo).
 bool tma_eligible(const VolumeArgs<float>& a);

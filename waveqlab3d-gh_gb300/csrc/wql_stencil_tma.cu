@@ -922,19 +922,16 @@ int sm_count() {
 // 0.265; 76/75 x 150^2 39: 1.09, 1.14; 101/93 x 107x113 26: 0.93, 0.95; upwind
 // 2 x 76x101x151 14: 1.38, 1.44 (correlation of the rule with the measured
 // times over 19 lengths: 0.91 to 1.00).
-int choose_chunk(const int* tiles, const int* ns, int nb) {
+// The time at which it ends, in planes, goes to *end.
+int choose_chunk(const int* tiles, const int* ns, int nb, float* end_out) {
   const int sms = sm_count();
   auto ctas = [&](int c) {
     long long n = 0;
     for (int b = 0; b < nb; ++b) n += (long long)tiles[b] * ((ns[b] + c - 1) / c);
     return n;
   };
-  if (ctas(32) >= 8LL * sms) return 32;
-  int best = 32;
-  float best_t = 1e30f;
   std::vector<float> heap;
-  for (int c = 4; c <= 48; ++c) {
-    if (ctas(c) > 8LL * sms) continue;
+  auto schedule = [&](int c) {
     heap.assign(sms, 0.0f);  // a min-heap of the times at which the SMs are free
     float end = 0.0f;
     for (int b = 0; b < nb; ++b)
@@ -949,18 +946,30 @@ int choose_chunk(const int* tiles, const int* ns, int nb) {
           std::push_heap(heap.begin(), heap.end(), std::greater<float>());
         }
       }
-    if (end < best_t) {
-      best_t = end;
-      best = c;
+    return end;
+  };
+  int best = 32;
+  float best_t = 1e30f;
+  if (ctas(32) >= 8LL * sms) {
+    if (end_out) best_t = schedule(32);
+  } else {
+    for (int c = 4; c <= 48; ++c) {
+      if (ctas(c) > 8LL * sms) continue;
+      const float end = schedule(c);
+      if (end < best_t) {
+        best_t = end;
+        best = c;
+      }
     }
   }
+  if (end_out) *end_out = best_t;
   return best;
 }
 
-int pair_chunk(const int nq[2], int nr, const int ns[2], int tq) {
+int pair_chunk(const int nq[2], int nr, const int ns[2], int tq, float* end) {
   const int rows = (nr + tma_rows(tq) - 1) / tma_rows(tq);
   const int tiles[2] = {(nq[0] + tq - 1) / tq * rows, (nq[1] + tq - 1) / tq * rows};
-  return choose_chunk(tiles, ns, 2);
+  return choose_chunk(tiles, ns, 2, end);
 }
 
 namespace {
@@ -1133,16 +1142,27 @@ long long fill_tma_desc(const VolumeArgs<float>& a, int chunk, TmaBatchDesc& d) 
 
 bool tma_eligible(const VolumeArgs<float>& a) {
   // the packed launch runs the central operator on 32-wide tiles; tile_span
-  // keeps every r closure row inside tile + halo unless the shifted last
-  // tile starts at 4 or 5
+  // keeps every r closure row inside tile + halo for the sizes of tiles_ok
   return a.tma != nullptr && a.fd == 0 && static_cast<const StencilMaps*>(a.tma)->tq == kTmaTQ &&
-         (a.nr <= kTmaTR + 3 || a.nr >= kTmaTR + 6);
+         tiles_ok(a.nr, kTmaTR);
 }
 
-int tma_tile_width(int nq0, int nq1, bool curv) {
+// A plane of a 40 x 8 tile takes about as long as one of 32 x 12 (both are a
+// warp's chain of instructions), so what counts is the number of planes that
+// the fullest SM walks: 40 where its schedule ends 5 % sooner.  Over 168 pairs
+// (2 x 41 to 400 points in q, 14 to 150 in r) and both operators that is 0.1 %
+// slower than the better width on average and 5 % at worst; by the share of
+// the columns in use alone, 5.5 % and 28 % (2 x 280x41x41: 63.9 us a launch
+// with 40, 50.2 with 32; 76/75 x 150^2: 141.6 with 40, 156.6 with 32).
+int tma_tile_width(const int nq[2], int nr, const int ns[2], bool curv, int fd) {
   if (curv) return kTmaTQ;
-  auto used = [&](int T) { return (double)(nq0 + nq1) / (double)(((nq0 + T - 1) / T + (nq1 + T - 1) / T) * T); };
-  return used(kTmaTQWide) > used(kTmaTQ) + 0.02 ? kTmaTQWide : kTmaTQ;
+  auto ok = [&](int rows) { return fd ? tiles_ok_up(nr, rows) : tiles_ok(nr, rows); };
+  if (!ok(tma_rows(kTmaTQWide))) return kTmaTQ;
+  if (!ok(kTmaTR)) return kTmaTQWide;
+  float wide = 0.0f, narrow = 0.0f;
+  pair_chunk(nq, nr, ns, kTmaTQWide, &wide);
+  pair_chunk(nq, nr, ns, kTmaTQ, &narrow);
+  return 1.05f * wide < narrow ? kTmaTQWide : kTmaTQ;
 }
 
 void launch_stencil_tma_batch(const TmaBatchDesc* d, int nd, long long total, bool curv, void* stream) {

@@ -1348,14 +1348,8 @@ void launch_tiled(const VolumeArgs<T>& a, cudaStream_t s) {
 // and in FP64 the kernel of wql_stencil_fp64.cu (7 here; blocks with an axis
 // under 12 points take the tiled kernel).
 //
-// A tiled axis of n points with tiles of T keeps every closure row inside
-// the tile that owns it plus a 3-point halo unless the shifted last tile
-// starts at 4 or 5 (then it would own left closure rows whose stencil
-// reaches point 0 from outside the halo); such sizes run per point.
-// With the upwind pair (halo 4, closure rows reading points 0..9) only a
-// last tile starting at 5 is excluded.
-inline bool tiles_ok(int n, int T) { return n <= T + 3 || n >= T + 6; }
-inline bool tiles_ok_up(int n, int T) { return n <= T + 4 || n >= T + 6; }
+// Axes whose closure rows a tile would not hold (tiles_ok, tiles_ok_up) run per
+// point.
 
 // Rows of the TMA tiles that the block's tensor maps are shaped for.
 template <typename T>
