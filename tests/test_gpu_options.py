@@ -195,3 +195,29 @@ def test_tile_width_by_schedule(wqlmod, ctx, dims):
     assert default < 1.08 * narrow
     if dims[0] in (76, 120) and dims[2] in (150, 14):
         assert default < 0.97 * narrow
+
+
+def test_late_request_joins_the_running_one(wqlmod, ctx):
+    """A request whose set-up is done 7 ms before another's end joins it: the server does not queue the
+    rest of a run ahead of the device.  Four tries, since set-up times vary."""
+    import time
+    import wql_configs
+    medium, steps = wql_configs.config4_medium(48), 160
+    reqs = [wql_configs.config4_request(i, n_lo=24, n_hi=44, steps=steps, medium=medium) for i in range(2)]
+    srv = wqlmod.Server(ctx, hbm_budget_bytes=64 << 30, round_steps=4)
+
+    def serve(delay):
+        ids = [srv.submit(reqs[0][0], steps, media=reqs[0][1])]
+        while srv.stats()["active"] < 1 and srv.stats()["completed"] < 1:
+            time.sleep(0.0002)
+        time.sleep(delay)
+        ids.append(srv.submit(reqs[1][0], 8, media=reqs[1][1]))
+        for r in ids:
+            assert srv.wait(r, 300.0) == 1
+        return [srv.result(r, 0)[1] for r in ids]
+
+    t = [serve(0.3)[k] for _ in range(3) for k in range(2)]  # one after the other
+    run, setup = min(x[2] - x[1] for x in t[::2]), min(x[1] - x[0] for x in t[1::2])
+    tries = [serve(max(0.0, run - setup - 0.007)) for _ in range(4)]
+    srv.close()
+    assert any(b[1] < a[2] - 0.001 for a, b in tries), (run, setup, tries)

@@ -1,8 +1,8 @@
 // Request server: scenarios submitted from any thread are admitted by device
 // memory footprint, advanced together in a continuous batch (wql_batch_*),
 // retired when they reach their step count, and their seismograms and
-// timings kept until released.  One worker thread owns the GPU work; it is
-// written against the public C ABI only.
+// timings kept until released.  Written against the public C ABI and
+// wql::batch_throttle.
 //
 // Two threads own the GPU work.  The worker admits queued requests in
 // arrival order while the head's peak footprint (wql_estimate_device_bytes)
@@ -14,7 +14,10 @@
 // generation, uploads, set-up kernels on the scenario's own stream) while the
 // batch steps, so the device does not wait for a new request's set-up.
 // Requests that arrive while others run join the batch at the next round
-// after their set-up.
+// after their set-up.  The worker keeps at most two rounds queued: without
+// that it had queued all 120 steps of a small request half-way through its run,
+// went on to wait for its end, and requests whose set-up was done by then
+// joined an idle device.
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -29,6 +32,10 @@
 
 #include "../../../include/wql.h"
 #include "wql_input.h"
+
+namespace wql {
+int batch_throttle(::wql_batch* b);
+}
 
 namespace {
 
@@ -190,7 +197,8 @@ void wql_server::run() {
       k = std::min(k, r->nsteps - info.nstep);
     }
     if (k > 0) {
-      const int rc = wql_batch_step(batch, k);
+      int rc = wql_batch_step(batch, k);
+      if (!rc) rc = wql::batch_throttle(batch);
       if (rc) {
         const std::string e = last_error();
         for (auto* r : act) {

@@ -1411,8 +1411,12 @@ struct wql_batch {
   std::vector<int> key_tuning;  // variant, schunk per member
   std::vector<int> cur0;        // members' buffer index when the tables were built
   bool built = false;
+  cudaEvent_t round_end[2] = {};  // ends of the last two rounds (batch_throttle)
+  long long rounds = 0;
   ~wql_batch() {
     for (auto e : ev) cudaEventDestroy(e);
+    for (auto e : round_end)
+      if (e) cudaEventDestroy(e);
     if (joined) cudaEventDestroy(joined);
     if (d_dev) cudaFree(d_dev);
     if (stream) cudaStreamDestroy(stream);
@@ -1567,6 +1571,22 @@ int batch_step(wql_batch* B) {
   }
   return WQL_OK;
 }
+
+}  // namespace
+
+namespace wql {
+// Called after each wql_batch_step of a server: waits until the round before
+// that one is done, so that at most two rounds are queued.
+int batch_throttle(wql_batch* B) {
+  cudaEvent_t& e = B->round_end[B->rounds & 1];
+  if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  CK(cudaEventRecord(e, B->stream));
+  if (++B->rounds > 1) CK(cudaEventSynchronize(B->round_end[B->rounds & 1]));
+  return WQL_OK;
+}
+}  // namespace wql
+
+namespace {
 
 // One RK stage of the current step (stages 1..5 in order).
 void run_stage(wql_scn* S, StepCtx& c, int stage) {
