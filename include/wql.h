@@ -274,7 +274,7 @@ int wql_kernel_times(wql_scn* scn, int kind, double* ms, int* launches);
 
 /* Volume-stencil tuning: kernel_variant 0 = default (the TMA-pipelined kernel
  * in WQL_FP32C; in WQL_FP64 the kernel whose tiles follow the block's extents,
- * or tiled 32x8 where an axis has fewer than 12 points), 1 = per-point form
+ * or tiled 32x8 for a block that no split of it fits), 1 = per-point form
  * (every neighbour read through the caches), 2 = tiled shared-memory kernel
  * with 32x8 tiles, 3 = the same at three blocks per SM (FP32), 4 = 64x8 tiles
  * (WQL_FP32C only), 5 = TMA-pipelined kernel (WQL_FP32C only; 32x12 tiles, or

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from gpu_helpers import rel_l2
-from test_gpu_kernel_edges import deck, start
+from test_gpu_kernel_edges import CASES, deck, start
 
 pytestmark = pytest.mark.gpu
 
@@ -221,3 +221,32 @@ def test_late_request_joins_the_running_one(wqlmod, ctx):
     tries = [serve(max(0.0, run - setup - 0.007)) for _ in range(4)]
     srv.close()
     assert any(b[1] < a[2] - 0.001 for a, b in tries), (run, setup, tries)
+
+
+@pytest.mark.parametrize("mesh,op,dims,npml", CASES, ids=[f"{m}-{o}-{d}-{n}".replace(" ", "") for m, o, d, n in CASES])
+def test_fp32c_velocities_and_stresses(wqlmod, ctx, mesh, op, dims, npml):
+    """The edge sizes with velocities and stresses held apart, so that the larger ones do not hide the
+    others, to ten times the 1e-7 that FP32 coefficients leave."""
+    d, f = (wqlmod.Scenario(ctx, text=deck(mesh, op, dims, npml), precision=p) for p in (wqlmod.FP64, wqlmod.FP32C))
+    for s in (d, f):
+        fill(s, dims)
+        s.step(3)
+    for b in range(2):
+        x, y = f.fields(b), d.fields(b)
+        assert rel_l2(x[:3], y[:3]) < 1e-6
+        assert rel_l2(x[3:], y[3:]) < 1e-6
+
+
+@pytest.mark.parametrize("mesh,dims,npml", [("cartesian", (41, 34, 25, 21), 7), ("curvilinear", (33, 27, 29, 23), 8)])
+def test_return_map_beside_slabs(wqlmod, oracle_lib, ctx, tmp_path, mesh, dims, npml):
+    """Viscoplasticity on odd extents, where the box outside the slabs starts and ends in the middle of tiles."""
+    text = deck(mesh, "traditional", dims, npml, ",\n response = 'plastic',\n plastic_model = 'scec'")
+    text = text.replace("TPV5", "TPV26") + "&plastic_list\n cohesion = 0.5,\n friction = 0.02,\n Tv = 0.03 /\n"
+    path = tmp_path / "pl.in"
+    path.write_text(text)
+    o, d = oracle_lib.Oracle(str(path)), wqlmod.Scenario(ctx, text=text, precision=wqlmod.FP64)
+    for r in (o, d):
+        fill(r, dims)
+        r.step(6)
+    for b in range(2):
+        assert rel_l2(d.fields(b), o.fields(b)) < 1e-11

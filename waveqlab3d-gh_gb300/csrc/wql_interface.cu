@@ -150,7 +150,8 @@ __device__ __forceinline__ R over(R x, R Z, R iZ) {
 }
 
 // T is the field type, R the arithmetic type of the characteristic algebra.
-// FP64 fields (R = T = double) keep every operation of the FP64 restatement.
+// FP64 fields (R = T = double) follow the FP64 restatement, with products by the
+// reciprocals that set-up took in place of its quotients.
 // FP32 fields either do the algebra in FP32 (R = float) or read the
 // compensated face values and do it in FP64 (R = double); the slip, state,
 // their rates and the friction law are FP64 in every case.  FP32 algebra:

@@ -62,27 +62,6 @@ __device__ __forceinline__ void row_entry(int kind, int t, T& w, int& off) {
   }
 }
 
-// Closure entry t (0..9) of the upwind pair at a closure row (kind as
-// sbp_kind, nonzero): the D+ weight wv (velocities), the D- weight wf
-// (fluxes) and the offset from the point.  Left rows read points 0..9,
-// right rows the mirror images; the right rows of D+ are the negated left
-// rows of D- and the other way round.
-template <typename T>
-__device__ __forceinline__ void up_entry(int kind, int t, T& wv, T& wf, int& off) {
-  if (kind < 0) {
-    const int i = -kind - 1;
-    wv = up_w<T>(0, i, t);
-    wf = up_w<T>(1, i, t);
-    off = t - i;
-  } else {
-    const int k = kind - 1;
-    wv = -up_w<T>(1, k, t);
-    wf = -up_w<T>(0, k, t);
-    off = k - t;
-  }
-}
-
-
 // The upwind pair of a kernel's operator FD (1: order 6, 2: order 5):
 // closure rows R per end, closure columns NCOL, interior D+ offsets
 // -2..PHI (D- offsets -PHI..2).
@@ -114,22 +93,6 @@ __device__ __forceinline__ T up_cf(int o) {
   const T cf[7] = WQL_UP_CF;
   return cf[o + 2];
 }
-// Closure entry t (0..NCOL-1) of operator FD on axis ax, as up_entry.
-template <typename T, int FD>
-__device__ __forceinline__ void upx_entry(int kind, int t, int ax, T& wv, T& wf, int& off) {
-  if (kind < 0) {
-    const int i = -kind - 1;
-    wv = upw<T, FD>(0, i, t);
-    wf = upw<T, FD>(1, i, t);
-    off = t - i;
-  } else {
-    const int k = kind - 1;
-    wv = -upw<T, FD>(1, k, t);
-    wf = -upw<T, FD>(0, k, t);
-    off = k - t;
-  }
-}
-
 struct TileSpan {
   int origin, own_lo, own_hi;
 };
@@ -256,8 +219,8 @@ __device__ __forceinline__ void add_correction(const VolumeArgs<T>& a, long long
 // plus the fault SAT on the interface face (src/RHS_Interior.f90:1757-1772).
 // The caller subtracts tot from the rates.  on_side(side, ubc) is called for
 // each boundary side with the forcing of a PML slab's auxiliary fields (not
-// yet scaled by tau0/h).  Returns false if the point has no penalised face.  Inlined: as a call its array arguments went through
-// the stack.
+// yet scaled by tau0/h).  Returns false if the point has no penalised face.
+// Inlined: as a call its array arguments went through the stack.
 template <typename T, typename Fn>
 __device__ __forceinline__ bool face_penalty(const VolumeArgs<T>& a, int i, int j, int k, const T* u, T* tot,
                                              Fn&& on_side) {

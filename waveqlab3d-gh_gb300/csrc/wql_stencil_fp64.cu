@@ -327,10 +327,10 @@ size_t smem_of(const StencilPlan64& p) {
 // The split of a block: tiles of kq x kr over (q, r) and chunks of planes,
 // chosen for the fewest warp-steps on the fullest SM: the total over all CTAs
 // plus half a CTA's own (the tail), a chunk's six window planes counted as
-// 0.3 of a step.
+// 0.3 of a step.  Axes have at least 12 points, so closure rows from both ends
+// do not meet.
 StencilPlan64 make_plan64(int nq, int nr, int ns, int sms) {
   StencilPlan64 best{};
-  if (nq < 12 || nr < 12 || ns < 12) return best;  // closure rows from both ends would meet
   double best_cost = 1e300;
   for (int kq = 1; kq <= std::max(1, nq / 6); ++kq) {
     const int tw = (nq + kq - 1) / kq;

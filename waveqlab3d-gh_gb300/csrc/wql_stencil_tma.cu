@@ -422,12 +422,12 @@ __device__ __forceinline__ bool tma_consume(const VolumeArgs<float>& a, float* s
   constexpr int TQ = TL::TQ, TR = TL::TR, NC = TL::NC, NT = TL::NT, BQ = TL::BQ, BR = TL::BR, HR = TL::HR, NS = TL::NS;
   const int nq = a.nq, nr = a.nr, ns = a.ns, r0 = spr.origin;
   const int tx = 2 * (tid % (TQ / 2));
-  const bool live = tid < NC / 2;  // the last warp of a 40-wide tile is half empty
-  const int ty = live ? tid / (TQ / 2) : TR - 1;
+  static_assert(NT == NC / 2, "every thread of a role has a pair of points");
+  const int ty = tid / (TQ / 2);
   const int q = q0 + tx, r = r0 + ty;
   // q = nq - 1 of an odd nq shares its pair with the pad column, which is
   // inside the row pitch: its values are computed from zeros and stored
-  const bool own = live && q < nq && r >= spr.own_lo && r < spr.own_hi;
+  const bool own = q < nq && r >= spr.own_lo && r < spr.own_hi;
   const int kq0 = sbp_kind(q, nq), kq1 = q + 1 < nq ? sbp_kind(q + 1, nq) : 0, kr = sbp_kind(r, nr);
   // points whose DF the pre-kernels have set on a stage with A = 0: the
   // block's faces and the PML slabs (here the q and r sides, true for the

@@ -594,10 +594,13 @@ __device__ __forceinline__ long long slab_point(const VolumeArgs<T>& a, int side
 // a uniform base plus one 32-bit offset that all of the neighbour's
 // quantities share.  A CTA takes a tile of 256 points of one region, 4 to 32
 // points along q and 2 to 8 along r and s, whichever pads the region least:
-// neighbouring rows share their stencil reads in L1.  Each direction's neighbours are visited once for both the flux and the
-// velocity derivative; a closure row's columns are unrolled like the interior
-// row's, so their loads are in flight together (as a loop, their latencies
-// added up).
+// neighbouring rows share their stencil reads in L1.  Each direction's
+// neighbours are visited once for both the flux and the velocity derivative; a
+// closure row's columns are unrolled like the interior row's, so their loads
+// are in flight together (as a loop, their latencies added up).  At the 80
+// registers of three CTAs an SM every FP32 form spills 80 to 370 bytes a thread
+// (stores); with two CTAs and no spills the slabs take longer (2 x 401x201^2:
+// 13.8 ms a step against 12.95).
 struct PmlTiles {
   int n;
   int lo[26][3], dim[26][3];
@@ -641,6 +644,7 @@ PmlTiles pml_tiles(const VolumeArgs<T>& a) {
         if (sizeof(T) == 8) {  // the FP64 unit is the bound: no idle lanes, 256 consecutive points
           const long long pts = (long long)P.dim[b][0] * P.dim[b][1] * P.dim[b][2];
           P.tq[b] = P.tr[b] = 1;
+          P.lw[b] = P.lr[b] = 0;
           P.start[b + 1] = P.start[b] + (int)((pts + 255) / 256);
           ++P.n;
           continue;
@@ -703,7 +707,6 @@ __device__ __forceinline__ void pml_pre_point(const VolumeArgs<T>& a, int i, int
   const T lam = at(coef + (CURV ? 10 : 0) * np, o), mu = at(coef + (CURV ? 11 : 1) * np, o);
   const T rinv = at(coef + (CURV ? 12 : 2) * np, o);
   const T rhoinv = CURV ? rinv / Jinv : rinv;
-  const T l2m = lam + T(2) * mu;
   const bool shell = FD >= 3 && ug_shell(a, i, j, k);
   // on a stage with A = 0, DF and DQ hold only what the face pre-kernel put there
   const bool keep = a.A != T(0);
@@ -890,8 +893,8 @@ int launch_pml_pre(const VolumeArgs<T>& a0, const VolumeArgs<T>* a1, bool curv, 
 }
 
 // ---------------------------------------------------------------------------
-// three CTAs per SM: 80 registers, no spills (four would cap it at 64 and
-// spill)
+// three CTAs per SM: 80 registers, no spills in FP32 (four would cap it at 64
+// and spill; the FP64 forms spill 80 to 88 bytes at 80)
 #ifndef WQL_ANEL_MINB
 #define WQL_ANEL_MINB 3
 #endif
@@ -1038,17 +1041,15 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
 }
 
 // The same with the velocity gradient at hand (a.G): six threads a point, one
-// per stress component, 64 consecutive points of the pitched block a CTA, both
-// blocks in a launch.  One thread a point walked the six components with 80
+// per stress component, 64 consecutive points of the pitched block a CTA.  One
+// thread a point walked the six components with 80
 // registers and 24 warps an SM, each waiting on its 66 streams (0.204 ms a
 // block of 76x101x151, 46 % of HBM); a component's loads are now all in flight
 // in 48 warps, and the index takes 32-bit divisions (0.151 ms, 62 % of HBM in
 // its 552 B a point; 0.174 with 64-bit divisions).
 template <typename T, bool CURV, bool KAHAN>
-__global__ void __launch_bounds__(384, 4) anelastic_comp_kernel(const __grid_constant__ BlockPair<T> P) {
-  const int blk = (long long)blockIdx.x >= P.n0 ? 1 : 0;
-  const VolumeArgs<T>& a = P.a[blk];
-  const long long p = ((long long)blockIdx.x - (blk ? P.n0 : 0)) * 64 + (threadIdx.x & 63);
+__global__ void __launch_bounds__(384, 4) anelastic_comp_kernel(const __grid_constant__ VolumeArgs<T> a) {
+  const long long p = (long long)blockIdx.x * 64 + (threadIdx.x & 63);
   const int c = threadIdx.x >> 6;  // stress component 3 + c
   const long long np = a.np;
   if (p >= np) return;
@@ -1345,8 +1346,8 @@ void launch_tiled(const VolumeArgs<T>& a, cudaStream_t s) {
 // Stencil-kernel variants (the tuning table): 1 per-point, 2 tiled 32x8 at
 // 1 CTA/SM, 3 tiled 32x8 at 3 CTAs/SM in FP32, 4 tiled 64x8 at 1 CTA/SM,
 // 5 TMA-pipelined (FP32), 6 accepted as 5; 0 picks the TMA kernel in FP32
-// and in FP64 the kernel of wql_stencil_fp64.cu (7 here; blocks with an axis
-// under 12 points take the tiled kernel).
+// and in FP64 the kernel of wql_stencil_fp64.cu (7 here; a block that no split
+// fits, 22 x 17 points in q and r alone up to 420, takes the tiled kernel).
 //
 // Axes whose closure rows a tile would not hold (tiles_ok, tiles_ok_up) run per
 // point.
@@ -1440,10 +1441,7 @@ int launch_corr(const VolumeArgs<T>& a, cudaStream_t s) {
     else anelastic_kernel<T, CURV, KAHAN, 0><<<grd, blk, 0, s>>>(a);
     ++n;
   } else if (a.anel) {
-    BlockPair<T> P;
-    P.a[0] = P.a[1] = a;
-    P.n0 = (a.np + 63) / 64;
-    anelastic_comp_kernel<T, CURV, KAHAN><<<(unsigned)P.n0, 384, 0, s>>>(P);
+    anelastic_comp_kernel<T, CURV, KAHAN><<<(unsigned)((a.np + 63) / 64), 384, 0, s>>>(a);
     ++n;
   }
   if (a.mp) {
