@@ -1079,22 +1079,20 @@ __global__ void __launch_bounds__(384, 4) anelastic_comp_kernel(const __grid_con
     e = c == 3 ? G[np] + G[3 * np] : (c == 4 ? G[2 * np] + G[6 * np] : G[5 * np] + G[7 * np]);
   }
 #pragma unroll
-  for (int side = 0; side < 6; ++side) {
-    if (!a.pml[side]) continue;
-    const int axis = side >> 1;
-    const bool hi = side & 1;
+  for (int axis = 0; axis < 3; ++axis) {
     const int ii = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 0 ? a.nq : (axis == 1 ? a.nr : a.ns);
-    if (!(hi ? ii >= n - a.npml : ii < a.npml)) continue;
     // where the two slabs of an axis overlap, the + side's Q alone counts
     // (pml_damping_and_q takes the sides in turn, src/RHS_Interior.f90:2287-2387)
-    if (!hi && a.pml[side + 1] && ii >= n - a.npml) continue;
+    const bool hi = a.pml[2 * axis + 1] && ii >= n - a.npml;
+    if (!hi && !(a.pml[2 * axis] && ii < a.npml)) continue;
     // the axes of a shear component: xy 0 1, xz 0 2, yz 1 2
     if (c >= 3 && (c == 3 ? axis == 2 : (c == 4 ? axis == 1 : axis == 0))) continue;
     const int off = hi ? ii + 1 - (n - a.npml) : (axis == 2 ? ii + 1 - a.npml : ii - a.npml);
     const T damp = a.pml_dn * (T)abs(off);
-    const long long snp = a.slab_np[side], q = (c < 3 ? 3 + axis : 3 + c) * snp + slab_point(a, side, i, j, k);
+    const long long snp = hi ? a.slab_np[2 * axis + 1] : a.slab_np[2 * axis];
+    const long long q = (c < 3 ? 3 + axis : 3 + c) * snp + slab_point(a, 2 * axis + (hi ? 1 : 0), i, j, k);
     // the stage-input Q (see anelastic_kernel)
-    const T dq = damp * (a.Q[side][q] - a.Bdt * a.DQ[side][q]);
+    const T dq = damp * ((hi ? a.Q[2 * axis + 1] : a.Q[2 * axis])[q] - a.Bdt * (hi ? a.DQ[2 * axis + 1] : a.DQ[2 * axis])[q]);
     if (c < 3) tr -= dq;
     if (c >= 3 || c == axis) e -= dq;
   }
