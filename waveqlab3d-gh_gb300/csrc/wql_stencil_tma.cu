@@ -287,24 +287,18 @@ __device__ __forceinline__ void deriv_q(Row&& row, int lq, int kq0, int kq1, int
       unpack(m4, a4, a3);
       unpack(p2, b2, b3);
       unpack(p4, b4, b5);
-      // one chain a point, the packed half of it first, in an order that keeps
-      // the partial sums of the weights (and with them the rounding) small
-      if (FD && VEL) {  // offsets -2..4
-        f2 u = mul2(pack(cf[0], cf[0]), m2);
-        u = fma2(pack(cf[6], cf[6]), p4, u);
-        u = fma2(pack(cf[4], cf[4]), p2, u);
-        u = fma2(pack(cf[2], cf[2]), z, u);
-        unpack(u, u0, u1);
-        u0 = fmaf(cf[5], b3, fmaf(cf[1], a1, fmaf(cf[3], x1, u0)));
-        u1 = fmaf(cf[5], b4, fmaf(cf[1], x0, fmaf(cf[3], b2, u1)));
-      } else if (FD) {  // offsets -4..2
-        f2 u = mul2(pack(-cf[0], -cf[0]), p2);
-        u = fma2(pack(-cf[6], -cf[6]), m4, u);
-        u = fma2(pack(-cf[4], -cf[4]), m2, u);
-        u = fma2(pack(-cf[2], -cf[2]), z, u);
-        unpack(u, u0, u1);
-        u0 = fmaf(-cf[5], a3, fmaf(-cf[1], x1, fmaf(-cf[3], a1, u0)));
-        u1 = fmaf(-cf[5], a2, fmaf(-cf[1], b2, fmaf(-cf[3], x0, u1)));
+      if (FD) {
+        // offset by offset in ascending order, as the other axes: every order
+        // that packs the even offsets rounds worse (errors of 60 steps 0.4 to
+        // 2.5 % larger) and saves 1 % of the kernel at most
+        const float x[10] = {a4, a3, a2, a1, x0, x1, b2, b3, b4, b5};  // -4 .. 5
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+          const float w = VEL ? cf[i] : -cf[6 - i];
+          const int l = VEL ? i + 2 : i;
+          u0 = i ? fmaf(w, x[l], u0) : w * x[l];
+          u1 = i ? fmaf(w, x[l + 1], u1) : w * x[l + 1];
+        }
       } else {
         // the nearest pair first, as in the other axes: the errors of 60 steps
         // are 3 % smaller than with the farthest first
