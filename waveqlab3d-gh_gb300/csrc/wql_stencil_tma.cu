@@ -34,8 +34,8 @@
 // (one point a thread: 900 issue slots; two: 1100), longer than a plane's
 // loads at the rate of HBM; with the roles each chain is half as long and an
 // SM has twelve of them (three a scheduler).  2 x 201^3 curvilinear, per
-// launch: 0.779 ms one point a thread, 0.756 two, 0.725 with the roles = 77 %
-// of the measured HBM rate; 2 x 101/93x107x113 150, 150, 142 us.  32 x 8 tiles
+// launch: 0.779 ms one point a thread, 0.756 two, 0.727 with the roles = 76 %
+// of the measured HBM rate; 2 x 101/93x107x113 150, 150, 140 us.  32 x 8 tiles
 // with three stages ran 0.757 ms there (more halo).
 // A role keeps its three quantities of planes s-3..s+3 (velocities, or s-face
 // fluxes) in registers (the first six read directly at the start of a chunk,
@@ -907,15 +907,15 @@ int sm_count() {
 
 // Planes per s chunk of a launch over nb blocks of tiles[b] (q, r) tiles and
 // ns[b] planes.  With 8 or more waves of one CTA per SM at 32 planes, 32: the
-// scheduler evens out what is left (2 x 201^3, 11 waves: 4.40 ms a step at 32,
-// 4.45-4.52 at 12 to 29 and at 41 and more).  With fewer, the length that
+// scheduler evens out what is left (2 x 201^3, 11 waves: 4.43 ms a step at 32,
+// 1 to 3 % more at 12 to 29 and at 41 and more).  With fewer, the length that
 // ends soonest when the CTAs go to the SMs in launch order, as they become
 // free; a chunk costs its planes plus 2 for its start (the six window planes)
 // plus 0.5 for each plane with an s closure row.  Measured ms a step at the
-// chosen length and at the 12 planes that short launches took: 2 x 41^3 5: 0.217,
-// 0.265; 76/75 x 150^2 39: 1.09, 1.14; 101/93 x 107x113 26: 0.93, 0.95; upwind
-// 2 x 76x101x151 14: 1.38, 1.44 (correlation of the rule with the measured
-// times over 19 lengths: 0.91 to 1.00).
+// chosen length and at 12 planes: 2 x 41^3 5: 0.185, 0.236; 76/75 x 150^2 39:
+// 1.05, 1.11; 101/93 x 107x113 26: 0.90, 0.93; upwind 2 x 76x101x151 26: 1.30,
+// 1.35 (correlation of the rule with the measured times over 19 lengths: 0.91
+// to 1.00).
 // The time at which it ends, in planes, goes to *end.
 int choose_chunk(const int* tiles, const int* ns, int nb, float* end_out) {
   const int sms = sm_count();

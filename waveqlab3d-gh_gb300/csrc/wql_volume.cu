@@ -1045,8 +1045,9 @@ __global__ void __launch_bounds__(256, WQL_ANEL_MINB) anelastic_kernel(const __g
 // thread a point walked the six components with 80
 // registers and 24 warps an SM, each waiting on its 66 streams (0.204 ms a
 // block of 76x101x151, 46 % of HBM); a component's loads are now all in flight
-// in 48 warps, and the index takes 32-bit divisions (0.151 ms, 62 % of HBM in
-// its 552 B a point; 0.174 with 64-bit divisions).
+// in 48 warps, the index takes 32-bit divisions and an axis looks up one slab
+// side (0.131 ms, 72 % of HBM in its 552 B a point; 0.174 with 64-bit
+// divisions, 0.151 with a loop over the six sides, which spilled).
 template <typename T, bool CURV, bool KAHAN>
 __global__ void __launch_bounds__(384, 4) anelastic_comp_kernel(const __grid_constant__ VolumeArgs<T> a) {
   const long long p = (long long)blockIdx.x * 64 + (threadIdx.x & 63);
