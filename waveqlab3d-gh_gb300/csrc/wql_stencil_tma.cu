@@ -925,18 +925,31 @@ int choose_chunk(const int* tiles, const int* ns, int nb, float* end_out) {
     return n;
   };
   std::vector<float> heap;
-  auto schedule = [&](int c) {
+  // costs are multiples of a half plane: sums of them are exact
+  auto cost = [&](int b, int z, int c) {
+    const int pl = std::min(c, ns[b] - z);
+    const int left = std::max(0, std::min(z + pl, 6) - z), right = std::max(0, z + pl - std::max(z, ns[b] - 6));
+    return 2.0f + pl + 0.5f * std::min(pl, left + right);
+  };
+  // no schedule of chunks of c ends before this
+  auto bound = [&](int c) {
+    double total = 0.0;
+    for (int b = 0; b < nb; ++b)
+      for (int z = 0; z < ns[b]; z += c) total += (double)tiles[b] * cost(b, z, c);
+    return total / sms;
+  };
+  // its end, or any later time once it is later than `most`
+  auto schedule = [&](int c, float most) {
     heap.assign(sms, 0.0f);  // a min-heap of the times at which the SMs are free
     float end = 0.0f;
     for (int b = 0; b < nb; ++b)
       for (int z = 0; z < ns[b]; z += c) {
-        const int pl = std::min(c, ns[b] - z);
-        const int left = std::max(0, std::min(z + pl, 6) - z), right = std::max(0, z + pl - std::max(z, ns[b] - 6));
-        const float cost = 2.0f + pl + 0.5f * std::min(pl, left + right);
+        const float t1 = cost(b, z, c);
         for (int t = 0; t < tiles[b]; ++t) {
           std::pop_heap(heap.begin(), heap.end(), std::greater<float>());
-          heap.back() += cost;
+          heap.back() += t1;
           end = std::max(end, heap.back());
+          if (end > most) return end;
           std::push_heap(heap.begin(), heap.end(), std::greater<float>());
         }
       }
@@ -945,12 +958,17 @@ int choose_chunk(const int* tiles, const int* ns, int nb, float* end_out) {
   int best = 32;
   float best_t = 1e30f;
   if (ctas(32) >= 8LL * sms) {
-    if (end_out) best_t = schedule(32);
+    if (end_out) best_t = schedule(32, best_t);
   } else {
-    for (int c = 4; c <= 48; ++c) {
-      if (ctas(c) > 8LL * sms) continue;
-      const float end = schedule(c);
-      if (end < best_t) {
+    // the most promising length first; the shortest of equals
+    std::vector<std::pair<double, int>> order;
+    for (int c = 4; c <= 48; ++c)
+      if (ctas(c) <= 8LL * sms) order.push_back({bound(c), c});
+    std::sort(order.begin(), order.end());
+    for (const auto& [least, c] : order) {
+      if (least > best_t) break;
+      const float end = schedule(c, best_t);
+      if (end < best_t || (end == best_t && c < best)) {
         best_t = end;
         best = c;
       }
@@ -1149,7 +1167,7 @@ bool tma_eligible(const VolumeArgs<float>& a) {
 // the columns in use alone, 5.5 % and 28 % (2 x 280x41x41: 63.9 us a launch
 // with 40, 50.2 with 32; 76/75 x 150^2: 141.6 with 40, 156.6 with 32).
 int tma_tile_width(const int nq[2], int nr, const int ns[2], bool curv, int fd) {
-  if (curv) return kTmaTQ;
+  if (curv || fd > 1) return kTmaTQ;  // the other operators run per point
   auto ok = [&](int rows) { return fd ? tiles_ok_up(nr, rows) : tiles_ok(nr, rows); };
   if (!ok(tma_rows(kTmaTQWide))) return kTmaTQ;
   if (!ok(kTmaTR)) return kTmaTQWide;
